@@ -11,6 +11,7 @@
 #include "wv_kernels.cuh"
 #include "wv_plan.hpp"
 #include "wv_warpfft.cuh"
+#include "wv_fx_launch.hpp"
 #include "wv_adjoint.cuh"
 #include "wv_vinv_tc.cuh"
 #include "wv_vfwd_tc.cuh"
@@ -69,6 +70,7 @@ struct wv_handle {
     void* yadj = nullptr;   // [z][nt][y][kx]
     void* yout = nullptr;   // [z][4+2nt][y][kx]
     void* fadj = nullptr;   // [4+2nt][z][pos]
+    double* adjRows = nullptr;  // FP64: real rows of the x pass [z][3+3nt][y][Nx]
     double* st[4] = {};     // RK4 stage states (st[1..3]) for the step adjoint
     double* kb = nullptr;
     double* sb = nullptr;
@@ -98,6 +100,7 @@ struct wv_handle {
     // F-grid scalar advection (built on first use): full-spectrum descriptor copy,
     // z-derivative matrix, per-position flags and scratch
     bool scalarReady = false;
+    wvgpu::FxRows fx{};  // FP64: lines of the x pass (length Nx, two rows per line)
     dev::DescDev sd{};
     const void* scalarD = nullptr;
     const unsigned char* scalarFlags = nullptr;
@@ -384,18 +387,9 @@ size_t smem_xr2c(const Plan& p) { return (x_len(p) + p.Nx + 8 * x_len(p)) * size
 template <typename T>
 size_t smem_vfwd(const Plan& p, int nch) { return nch * p.zHalf * dev::kVfwdModes * sizeof(dev::cx2t<T>); }
 
-// The dynamic shared-memory cap is a process-wide attribute of each kernel,
-// not of a handle: only ever raise it, so a handle created for a smaller grid
-// cannot shrink the cap below what a live handle for a larger grid launches with.
-std::mutex g_smem_mutex;
 template <typename K>
 cudaError_t raise_smem_limit(K* kernel, int bytes) {
-    std::lock_guard<std::mutex> lock(g_smem_mutex);
-    cudaFuncAttributes a{};
-    cudaError_t e = cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(kernel));
-    if (e != cudaSuccess) return e;
-    if (a.maxDynamicSharedSizeBytes >= bytes) return cudaSuccess;
-    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return wvgpu::raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
 }
 
 template <typename T>
@@ -413,6 +407,10 @@ cudaError_t set_smem_limits(const Plan& p) {
     WV_SET((dev::k_xr2c_fields<T>), smem_xr2c<T>(p));
     WV_SET((dev::k_vfwd<T, true>), smem_vfwd<T>(p, 4));
     WV_SET((dev::k_vfwd<T, false>), smem_vfwd<T>(p, 4));
+    if constexpr (std::is_same<T, double>::value) {
+        e = wvgpu::fx_set_limits(p);
+        if (e != cudaSuccess) return e;
+    }
     if (p.fz.N > 0) {
         WV_SET((dev::k_vinv_fft<T, true>), dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, true>::modes));
         WV_SET((dev::k_vinv_fft<T, false>), dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, false>::modes));
@@ -529,6 +527,9 @@ void launch_yinv(wv_handle* h, const dev::YInvMap& map, const dev::cx<T>* z, dev
                  const dev::DescDev* over = nullptr) {
     const Plan& p = h->plan;
     const dev::DescDev& dd = over ? *over : h->dd;
+    if constexpr (std::is_same<T, double>::value) {
+        if (wvgpu::fx_yinv(p, dd, map, z, y, s)) return;
+    }
     const int ry = warp_ry<T>(p);
     if (ry) {
         const dim3 grid(cdiv(p.kxColumns, dev::kWG), dd.zTotal, map.nOut);
@@ -541,6 +542,9 @@ void launch_yinv(wv_handle* h, const dev::YInvMap& map, const dev::cx<T>* z, dev
 template <typename T>
 void launch_yfwd(wv_handle* h, const dev::cx<T>* ps, int nch, dev::cx<T>* f, cudaStream_t s) {
     const Plan& p = h->plan;
+    if constexpr (std::is_same<T, double>::value) {
+        if (wvgpu::fx_yfwd(p, h->dd, ps, nch, f, s)) return;
+    }
     const int ry = warp_ry<T>(p);
     if (ry) {
         const dim3 grid(cdiv(p.kxColumns, dev::kWG), h->dd.zTotal, nch);
@@ -554,6 +558,9 @@ template <typename T>
 void launch_xflux(wv_handle* h, const dev::cx<T>* y, dev::cx<T>* ps, unsigned long long* speed, cudaStream_t s,
                   void* physOut = nullptr, double* advOut = nullptr, const double* advIn = nullptr) {
     const Plan& p = h->plan;
+    if constexpr (std::is_same<T, double>::value) {
+        if (wvgpu::fx_xflux(p, h->dd, h->fx, y, ps, speed, static_cast<double*>(physOut), advOut, advIn, s)) return;
+    }
     const int rx = warp_rx<T>(p);
     if (rx) {
         const dim3 grid(cdiv(p.Ny, dev::kWG), h->dd.zTotal);
@@ -571,6 +578,9 @@ void launch_xc2r(wv_handle* h, const dev::cx<T>* y, double* fields, cudaStream_t
                  const dev::DescDev* over = nullptr) {
     const Plan& p = h->plan;
     const dev::DescDev& dd = over ? *over : h->dd;
+    if constexpr (std::is_same<T, double>::value) {
+        if (wvgpu::fx_xc2r(p, dd, h->fx, y, nch, fields, s)) return;
+    }
     const int rx = warp_rx<T>(p);
     if (rx) {
         const dim3 grid(cdiv(p.Ny, dev::kWG), dd.zTotal);
@@ -583,6 +593,9 @@ void launch_xc2r(wv_handle* h, const dev::cx<T>* y, double* fields, cudaStream_t
 template <typename T>
 void launch_xr2c(wv_handle* h, const double* fields, int nch, dev::cx<T>* ps, cudaStream_t s) {
     const Plan& p = h->plan;
+    if constexpr (std::is_same<T, double>::value) {
+        if (wvgpu::fx_xr2c(p, h->dd, h->fx, fields, nch, ps, s)) return;
+    }
     const int rx = warp_rx<T>(p);
     if (rx) {
         const dim3 grid(cdiv(p.Ny, dev::kWG), h->dd.zTotal);
@@ -590,6 +603,24 @@ void launch_xr2c(wv_handle* h, const double* fields, int nch, dev::cx<T>* ps, cu
         return;
     }
     dev::k_xr2c_fields<T><<<dim3(p.Ny, h->dd.zTotal), 256, smem_xr2c<T>(p), s>>>(h->dd, fields, nch, ps);
+}
+
+// The vertical transforms of FP64 handles on lane-held lines; false where the
+// length has none.
+template <typename T>
+bool launch_vinv_fx(wv_handle* h, bool flux, double elapsed, const double* Ap, const double* Am, const double* A0,
+                    dev::cx<T>* z, unsigned long long* speed, cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value)
+        return wvgpu::fx_vinv(h->plan, h->dd, flux, elapsed, Ap, Am, A0, z, speed, s);
+    return false;
+}
+template <typename T>
+bool launch_vfwd_fx(wv_handle* h, bool flux, const dev::cx<T>* f, int nch, double elapsed, const double* Ap, const double* Am,
+                    const double* A0, const unsigned long long* speed, int damping, double* Fp, double* Fm, double* F0,
+                    cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value)
+        return wvgpu::fx_vfwd(h->plan, h->dd, flux, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0, s);
+    return false;
 }
 
 // The flux's vertical inverse transform with the handle's kernel choice: the
@@ -621,6 +652,7 @@ void launch_vinv_flux(wv_handle* h, double elapsed, const double* Ap, const doub
             const size_t sm = dev::smem_vinv_wfft<T>(static_cast<int>(p.Nj), p.fz.N);
             WV_RSWITCH_Y(warp_rz<T>(p), (dev::k_vinv_wfft<T, RR><<<grid, 256, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed)));
         }
+    } else if (h->vinvKind == WV_VERTICAL_FFT && launch_vinv_fx<T>(h, true, elapsed, Ap, Am, A0, z, speed, s)) {
     } else if (h->vinvKind == WV_VERTICAL_FFT) {
         constexpr int modes = dev::VzShape<T, true>::modes;
         dev::k_vinv_fft<T, true><<<dim3(cdiv(p.Nkl, modes), d.members), 256,
@@ -698,6 +730,8 @@ cudaError_t launch_flux(wv_handle* h, double t, double t0, const double* Ap, con
         }
         fwdTC = true;
     }
+    if (!fwdTC && h->vfwdKind == WV_VERTICAL_FFT)
+        fwdTC = launch_vfwd_fx<T>(h, true, f, nt, elapsed, Ap, Am, A0, speed, damping ? 1 : 0, Fp, Fm, F0, s);
     if (!fwdTC && h->vfwdKind == WV_VERTICAL_FFT) {
         dev::k_vfwd_fft<T, true><<<dim3(cdiv(p.Nkl, dev::vf_modes<T>()), d.members), 256, dev::smem_vfwd_fft<T>(p.fz.N), s>>>(
             d, f, nt, elapsed, Ap, Am, A0, speed, damping ? 1 : 0, Fp, Fm, F0);
@@ -841,28 +875,45 @@ cudaError_t launch_scalar_advection(wv_handle* h, const double* scalar, const do
     const size_t smR2C = (L + p.Nx + 8 * L) * cb + 4 * p.Nx * sizeof(T);
     const size_t smC2R3 = (L + p.Nx + 3 * KX + 8 * L) * cb, smC2R1 = (L + p.Nx + 1 * KX + 8 * L) * cb;
     const unsigned gridE = static_cast<unsigned>(std::min<size_t>((R + 255) / 256, wvgpu::grid_cap(16)));
+    constexpr bool fp64 = std::is_same<T, double>::value;  // fixed-point lines
+    auto r2c = [&](const double* in, dev::cx<T>* out) {
+        if constexpr (fp64) if (wvgpu::fx_xr2c(p, sd, h->fx, in, 1, out, s)) return;
+        dev::k_xr2c_fields<T><<<dim3(Ny, Nz), 256, smR2C, s>>>(sd, in, 1, out);
+    };
+    auto yfwd = [&](dev::cx<T>* out) {
+        if constexpr (fp64) if (wvgpu::fx_yfwd(p, sd, sp, 1, out, s)) return;
+        dev::k_yfwd<T><<<dim3(cdiv(KX, dev::kYG), Nz, 1), 256, smem_y<T>(p), s>>>(sd, sp, 1, out);
+    };
+    auto yinv = [&](const dev::YInvMap& m) {
+        if constexpr (fp64) if (wvgpu::fx_yinv(p, sd, m, sf, sp, s)) return;
+        dev::k_yinv<T><<<dim3(cdiv(KX, dev::kYG), Nz), 256, smem_y<T>(p), s>>>(sd, m, sf, 0, sp);
+    };
+    auto c2r = [&](int nch, double* out, size_t sm) {
+        if constexpr (fp64) if (wvgpu::fx_xc2r(p, sd, h->fx, sp, nch, out, s)) return;
+        dev::k_xc2r_fields<T><<<dim3(Ny, Nz), 256, sm, s>>>(sd, sp, nch, out);
+    };
     // x r2c, y forward FFT of the scalar (channel 3 of sf), column derivatives (channels 0..2)
-    dev::k_xr2c_fields<T><<<dim3(Ny, Nz), 256, smR2C, s>>>(sd, scalar, 1, sp);
+    r2c(scalar, sp);
     dev::cx<T>* sf3 = sf + (size_t)3 * Nz * P;
-    dev::k_yfwd<T><<<dim3(cdiv(KX, dev::kYG), Nz, 1), 256, smem_y<T>(p), s>>>(sd, sp, 1, sf3);
+    yfwd(sf3);
     dev::k_scalar_derivs<T><<<cdiv(P, dev::kScalarCols), 256, Nz * dev::kScalarCols * cb, s>>>(sd, sf3, D, h->scalarFlags, hs, sf);
     dev::YInvMap map{};
     map.nOut = 3;
     for (int c = 0; c < 3; ++c) { map.src[c] = c; map.mulL[c] = 0; }
-    dev::k_yinv<T><<<dim3(cdiv(KX, dev::kYG), Nz), 256, smem_y<T>(p), s>>>(sd, map, sf, 0, sp);
-    dev::k_xc2r_fields<T><<<dim3(Ny, Nz), 256, smC2R3, s>>>(sd, sp, 3, h->scalarGrad);
+    yinv(map);
+    c2r(3, h->scalarGrad, smC2R3);
     dev::k_scalar_rhs<<<gridE, 256, 0, s>>>(h->scalarGrad, adv, R, rhs);
     h->metrics.kernel_launches += 6;
     if (antialias) {
-        dev::k_xr2c_fields<T><<<dim3(Ny, Nz), 256, smR2C, s>>>(sd, rhs, 1, sp);
-        dev::k_yfwd<T><<<dim3(cdiv(KX, dev::kYG), Nz, 1), 256, smem_y<T>(p), s>>>(sd, sp, 1, sf);
+        r2c(rhs, sp);
+        yfwd(sf);
         dev::k_scalar_mask<T><<<static_cast<unsigned>(std::min<size_t>((size_t(Nz) * P + 255) / 256, wvgpu::grid_cap(16))), 256, 0, s>>>(
             sd, sf, h->scalarFlags, hs);
         dev::YInvMap m1{};
         m1.nOut = 1;
         m1.src[0] = 0; m1.mulL[0] = 0;
-        dev::k_yinv<T><<<dim3(cdiv(KX, dev::kYG), Nz), 256, smem_y<T>(p), s>>>(sd, m1, sf, 0, sp);
-        dev::k_xc2r_fields<T><<<dim3(Ny, Nz), 256, smC2R1, s>>>(sd, sp, 1, rhs);
+        yinv(m1);
+        c2r(1, rhs, smC2R1);
         h->metrics.kernel_launches += 5;
     }
     return cudaGetLastError();
@@ -930,7 +981,8 @@ cudaError_t launch_inverse(wv_handle* h, double t, double t0, const double* Ap, 
     const auto& d = h->dd;
     auto* z = static_cast<dev::cx<T>*>(h->zspec);
     auto* y = static_cast<dev::cx<T>*>(h->yspec);
-    dev::k_vinv<T, false><<<dim3(cdiv(p.Nkl, dev::kVinvModes), d.members), 256, smem_vinv<T>(p), s>>>(d, Ap, Am, A0, t - t0, z, nullptr);
+    if (!launch_vinv_fx<T>(h, false, t - t0, Ap, Am, A0, z, nullptr, s))
+        dev::k_vinv<T, false><<<dim3(cdiv(p.Nkl, dev::kVinvModes), d.members), 256, smem_vinv<T>(p), s>>>(d, Ap, Am, A0, t - t0, z, nullptr);
     dev::YInvMap map{};
     map.nOut = nch;
     for (int c = 0; c < nch; ++c) { map.src[c] = c; map.mulL[c] = 0; }
@@ -950,8 +1002,9 @@ cudaError_t launch_forward(wv_handle* h, const double* fields, double t, double 
     auto* f = static_cast<dev::cx<T>*>(h->fspec);
     launch_xr2c<T>(h, fields, nch, ps, s);
     launch_yfwd<T>(h, ps, nch, f, s);
-    dev::k_vfwd<T, false><<<dim3(cdiv(p.Nkl, dev::kVfwdModes), d.members), 256, smem_vfwd<T>(p, nch), s>>>(
-        d, f, nch, t - t0, nullptr, nullptr, nullptr, nullptr, 0, Ap, Am, A0);
+    if (!launch_vfwd_fx<T>(h, false, f, nch, t - t0, nullptr, nullptr, nullptr, nullptr, 0, Ap, Am, A0, s))
+        dev::k_vfwd<T, false><<<dim3(cdiv(p.Nkl, dev::kVfwdModes), d.members), 256, smem_vfwd<T>(p, nch), s>>>(
+            d, f, nch, t - t0, nullptr, nullptr, nullptr, nullptr, 0, Ap, Am, A0);
     h->metrics.kernel_launches += 3;
     return cudaGetLastError();
 }
@@ -1039,6 +1092,10 @@ int ensure_adjoint(wv_handle* h) {
     if (e == cudaSuccess) e = alloc(h, nIn * p.Nz * p.positions * cb, &h->fadj);
     const size_t stateBytes = 6 * p.M * sizeof(double);
     void* tmp = nullptr;
+    if (e == cudaSuccess && h->precision == WV_PRECISION_FP64 && wvgpu::fx_has_rows(p)) {
+        e = alloc(h, (3 + 3 * nt) * p.Nx * p.Ny * p.Nz * sizeof(double), &tmp);
+        h->adjRows = static_cast<double*>(tmp);
+    }
     for (int i = 1; i < 4 && e == cudaSuccess; ++i) { e = alloc(h, stateBytes, &tmp); h->st[i] = static_cast<double*>(tmp); }
     if (e == cudaSuccess) { e = alloc(h, stateBytes, &tmp); h->kb = static_cast<double*>(tmp); }
     if (e == cudaSuccess) { e = alloc(h, stateBytes, &tmp); h->sb = static_cast<double*>(tmp); }
@@ -1088,6 +1145,14 @@ cudaError_t launch_flux_vjp(wv_handle* h, double t, double t0, const double* Ap,
     // forward fields of this state
     const dev::cx<T>* y = static_cast<const dev::cx<T>*>(h->yspec);
     if (!physIn) launch_flux_fields<T>(h, elapsed, Ap, Am, A0, static_cast<dev::cx<T>*>(h->yspec), s);
+    if constexpr (std::is_same<T, double>::value) {
+        // the fixed-point x pass gives the rows (the same bits whether kept or made here)
+        if (!physIn && h->adjRows &&
+            wvgpu::fx_xflux(p, d, h->fx, y, static_cast<double2*>(h->pspec), nullptr, h->adjRows, nullptr, nullptr, s)) {
+            physIn = h->adjRows;
+            h->metrics.kernel_launches += 1;
+        }
+    }
     // adjoint of projection and forward vertical transform, then inverse y FFTs
     bool done = false;  // the vertical forward map launched on warp lines
     if constexpr (!std::is_same<T, double>::value) {
@@ -1488,6 +1553,34 @@ static int create_handle(const wv_config* config, int precision, int members, wv
     for (int i = 0; i < dev::kMaxStages; ++i) { dd.fx.radix[i] = p.fx.radix[i]; dd.fy.radix[i] = p.fy.radix[i]; }
     dd.fz.N = p.fz.N; dd.fz.nstages = p.fz.nstages;
     for (int i = 0; i < dev::kMaxStages; ++i) dd.fz.radix[i] = p.fz.radix[i];
+    if (precision == WV_PRECISION_FP64) {  // fixed-point lines: their own factors and twiddles
+        auto fixed_point_fft = [](size_t N) {
+            const wvgpu::FFTFactors q = wvgpu::factor_fixed_point(static_cast<int>(N));
+            dev::FFTDev f{};
+            f.N = q.N; f.nstages = q.nstages;
+            for (int i = 0; i < dev::kMaxStages; ++i) f.radix[i] = q.radix[i];
+            return f;
+        };
+        for (dev::FFTDev* f : {&dd.fx, &dd.fy, &dd.fz})
+            if (f->N) *f = fixed_point_fft(f->N);
+        h->fx.x = fixed_point_fft(p.Nx);
+        auto table = [&](const std::vector<int32_t>& v, const dev::fxw** dst) {
+            if (e != cudaSuccess || v.empty()) return;
+            const int32_t* q = nullptr;
+            e = upload(h, v, &q);
+            *dst = reinterpret_cast<const dev::fxw*>(q);
+        };
+        table(wvgpu::fixed_point_twiddles(static_cast<int>(p.Nx)), &h->fx.twX);
+        table(wvgpu::fx_lane_table(p.Nx), &h->fx.twXLane);
+        table(wvgpu::fx_lane_table(p.Ny), &dd.fxTwY);
+        table(wvgpu::fx_lane_table(p.fz.N), &dd.fxTwZ);
+        // exp(+2 pi i k / 256): the forward table read backwards
+        const std::vector<int32_t> forward = wvgpu::fixed_point_twiddles(256);
+        std::vector<int32_t> phases(forward.size());
+        for (int k = 0; k < 256; ++k)
+            std::copy_n(forward.begin() + 4 * ((256 - k) % 256), 4, phases.begin() + 4 * k);
+        table(phases, &dd.fxPhase);
+    }
     std::vector<int32_t> ymap(p.ymap);
     std::vector<int32_t> posKy(p.posKy), colStart(p.colStart), modeWV(p.modeWV), modePos(p.modePos), modeComp(p.modeCompPos);
     std::vector<double> inertial(d.inertialScale), apmw(d.apmWProjectionPrefactor);
@@ -1541,8 +1634,16 @@ static int create_handle(const wv_config* config, int precision, int members, wv
         }
     };
     upT(p.Ccos, &dd.Ccos); upT(p.Csin, &dd.Csin); upT(p.CcosM, &dd.CcosM); upT(p.CsinM, &dd.CsinM);
-    upT(p.Fcos, &dd.Fcos); upT(p.Fsin, &dd.Fsin); upT(p.twx, &dd.twx); upT(p.twxN, &dd.twxN); upT(p.twy, &dd.twy);
-    if (p.fz.N > 0) { upT(p.twz, &dd.twz); upT(std::vector<double>(d.m.begin(), d.m.begin() + p.Nj), &dd.tMz); }
+    upT(p.Fcos, &dd.Fcos); upT(p.Fsin, &dd.Fsin); upT(p.twxN, &dd.twxN);
+    auto upTw = [&](const std::vector<double>& v, int N, const void** dst) {
+        if (precision != WV_PRECISION_FP64) { upT(v, dst); return; }
+        if (e != cudaSuccess) return;
+        const int32_t* q = nullptr;
+        e = upload(h, wvgpu::fixed_point_twiddles(N), &q);
+        *dst = q;
+    };
+    upTw(p.twx, p.fx.N, &dd.twx); upTw(p.twy, p.fy.N, &dd.twy);
+    if (p.fz.N > 0) { upTw(p.twz, p.fz.N, &dd.twz); upT(std::vector<double>(d.m.begin(), d.m.begin() + p.Nj), &dd.tMz); }
     upT(p.rowK, &dd.tRowK); upT(p.rowL, &dd.tRowL);
     {
         auto transpose = [](const std::vector<double>& a, size_t rows, size_t cols) {

@@ -1,0 +1,273 @@
+// Host side of the FP64 kernels on fixed-point lines.  See wv_fx_launch.hpp.
+#include "wv_fx_launch.hpp"
+#include "wv_fxflux.cuh"
+#include "wv_fxyz.cuh"
+#include "wv_fxany.cuh"
+#include "wv_internal.hpp"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <mutex>
+
+namespace wvgpu {
+namespace {
+
+unsigned cdiv(size_t a, size_t b) { return static_cast<unsigned>((a + b - 1) / b); }
+
+// Line lengths held by the lanes of a warp (wv_fxwarp.cuh).
+#define WV_FXW_SWITCH(N, ...)                             \
+    switch (N) {                                          \
+        case 16: { constexpr int NN = 16; __VA_ARGS__; } break;   \
+        case 32: { constexpr int NN = 32; __VA_ARGS__; } break;   \
+        case 64: { constexpr int NN = 64; __VA_ARGS__; } break;   \
+        case 128: { constexpr int NN = 128; __VA_ARGS__; } break; \
+        case 256: { constexpr int NN = 256; __VA_ARGS__; } break; \
+        default: break;                                   \
+    }
+inline bool fx_lane_length(size_t N) { return N == 16 || N == 32 || N == 64 || N == 128 || N == 256; }
+template <int N>
+std::vector<int32_t> lane_table() {
+    using W = dev::FxW<N>;
+    if (W::R3 > 1) return fixed_point_stage_twiddles(N, {8, W::R2, W::R3});
+    return fixed_point_stage_twiddles(N, {8, W::R2});
+}
+
+// The x pass: lane-held rows where the length allows (kx < Nx / 2 always holds on
+// the transform's own rows); else rows of up to 512 samples and 256 kx columns on
+// run-time stages; longer rows keep the block kernel.
+inline bool fx_x_lane(const Plan& p) { return fx_lane_length(p.Nx) && 2 * p.kxColumns <= p.Nx; }
+inline bool fx_x_any(const Plan& p) { return p.Nx <= 512 && p.kxColumns <= 256; }
+template <int N>
+size_t smem_xflux_fx() { return dev::FxW<N>::twiddles * sizeof(dev::fxw) + dev::kFxXWarps * dev::fx_xflux_warp_bytes(N); }
+// Warps of a y or z block: 8, fewer where the columns of a plane (the retained
+// columns) do not fill them; powers of two in y, as the tile's swizzle needs.
+inline int fx_y_warps(size_t Ny, size_t kxColumns) {
+    const size_t lines = 256 / Ny;
+    int warps = 1;
+    while (warps < dev::kFxYWarps && warps * lines < kxColumns) warps *= 2;
+    return warps;
+}
+inline int fx_z_warps(const Plan& p) {
+    // enough blocks for every SM before the blocks grow
+    const size_t lines = 256 / p.fz.N, units = (p.Nkl + lines - 1) / lines, sms = grid_cap(1);
+    return static_cast<int>(std::min<size_t>(dev::kFxZWarps, std::max<size_t>(1, (units + sms - 1) / sms)));
+}
+// Lines of any length along z: warps of a block, as shared memory allows.
+inline int fx_z_any_warps(const Plan& p, int lines) {
+    const size_t each = 2 * static_cast<size_t>(lines) * p.fz.N * 16, sms = grid_cap(1);
+    const size_t room = std::max<size_t>(1, (100 * 1024) / each);
+    return static_cast<int>(std::min<size_t>({room, dev::kFxAnyWarps, std::max<size_t>(1, (p.Nkl + sms - 1) / sms)}));
+}
+// The field kernels along x: one warp per row.
+struct FxFieldLaunch { int warps, grid; size_t smem; };
+inline FxFieldLaunch fx_field_launch(size_t Nx, size_t rows, int nch) {
+    FxFieldLaunch l{};
+    const int lines = (nch + 1) / 2;
+    const size_t each = 2 * static_cast<size_t>(lines) * Nx * 16;
+    l.warps = static_cast<int>(std::min<size_t>(dev::kFxAnyWarps, std::max<size_t>(1, (104 * 1024 - Nx * 16) / each)));
+    l.smem = dev::smem_fx_any_x(static_cast<int>(Nx), lines, l.warps);
+    l.grid = static_cast<int>(std::min<size_t>((rows + l.warps - 1) / l.warps, grid_cap(2)));
+    return l;
+}
+struct FxXLaunch { int warps, grid, pairs; size_t smem; };
+inline FxXLaunch fx_x_launch(const Plan& p, int members) {
+    FxXLaunch l{};
+    const int nt = p.targets.count, Nx = static_cast<int>(p.Nx);
+    l.pairs = dev::fx_xany_pairs(Nx, nt);
+    const size_t warp = dev::fx_xany_warp_bytes(Nx, nt, l.pairs), table = p.Nx * sizeof(dev::fxw);
+    const size_t most = 226 * 1024;
+    // 16 warps per SM (128 registers a thread) as two blocks where they fit
+    // beside each other, else one block of as many warps as shared memory holds
+    if (2 * (8 * warp + table) <= most) l.warps = 8;
+    else l.warps = static_cast<int>(std::min<size_t>(16, (most - table) / warp));
+    const size_t rows = p.Ny * p.Nz * members;
+    l.smem = table + l.warps * warp;
+    l.grid = static_cast<int>(std::min<size_t>((rows + l.warps - 1) / l.warps, grid_cap(l.warps == 8 ? 2 : 1)));
+    return l;
+}
+#define WV_FXX_SWITCH(KX, ...)                           \
+    if ((KX) <= 64) { constexpr int EK = 2; __VA_ARGS__; }      \
+    else if ((KX) <= 128) { constexpr int EK = 4; __VA_ARGS__; } \
+    else { constexpr int EK = 8; __VA_ARGS__; }
+
+}  // namespace
+
+std::vector<int32_t> fx_lane_table(size_t N) {
+    WV_FXW_SWITCH(N, return lane_table<NN>());
+    return {};
+}
+
+cudaError_t fx_set_limits(const Plan& p) {
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto* kernel, size_t bytes) {
+        if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(kernel), static_cast<int>(bytes));
+    };
+    WV_FXW_SWITCH(p.Ny, {
+        set(dev::k_yinv_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * (256 / NN)));
+        set(dev::k_yfwd_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * (256 / NN)));
+    });
+    if (!fx_lane_length(p.Ny)) {
+        // (the scalar pipeline has the most columns)
+        const size_t sm = dev::smem_fx_any_y(static_cast<int>(p.Ny), dev::fx_any_cols(static_cast<int>(p.Ny), 1 << 20));
+        set(dev::k_yinv_fxany<0>, sm);
+        set(dev::k_yfwd_fxany<0>, sm);
+    }
+    if (fx_x_any(p)) {
+        for (int nch = 1; nch <= 4; nch += 2) {
+            const FxFieldLaunch l = fx_field_launch(p.Nx, 1, nch);
+            set(dev::k_xc2r_fxany<2>, l.smem); set(dev::k_xc2r_fxany<4>, l.smem); set(dev::k_xc2r_fxany<8>, l.smem);
+            set(dev::k_xr2c_fxany<0>, l.smem);
+        }
+    }
+    if (p.fz.N > 0 && !fx_lane_length(p.fz.N)) {
+        const size_t inv = dev::smem_fx_any_z(p.fz.N, 4, fx_z_any_warps(p, 4)), two = dev::smem_fx_any_z(p.fz.N, 2, fx_z_any_warps(p, 2));
+        set(dev::k_vinv_fxany<true>, inv); set(dev::k_vinv_fxany<false>, two);
+        set(dev::k_vfwd_fxany<true>, two); set(dev::k_vfwd_fxany<false>, two);
+    }
+    WV_FXW_SWITCH(p.fz.N, {
+        set(dev::k_vinv_fx<NN, true>, dev::smem_fx_vinv<NN>(fx_z_warps(p)));
+        set(dev::k_vinv_fx<NN, false>, dev::smem_fx_vinv<NN>(fx_z_warps(p)));
+        set(dev::k_vfwd_fx<NN, true>, dev::smem_fx_vfwd<NN>(fx_z_warps(p)));
+        set(dev::k_vfwd_fx<NN, false>, dev::smem_fx_vfwd<NN>(fx_z_warps(p)));
+    });
+    if (fx_x_lane(p)) { WV_FXW_SWITCH(p.Nx, set(dev::k_xflux_fx<NN, 3>, smem_xflux_fx<NN>()); set(dev::k_xflux_fx<NN, 4>, smem_xflux_fx<NN>())); }
+    else if (fx_x_any(p)) { WV_FXX_SWITCH(p.kxColumns, set(dev::k_xflux_fxany<EK>, fx_x_launch(p, 1).smem)); }
+    return e;
+}
+
+bool fx_has_rows(const Plan& p) { return fx_x_lane(p) || fx_x_any(p); }
+
+bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* y, double2* ps,
+              unsigned long long* speed, double* physOut, double* advOut, const double* advIn, cudaStream_t s) {
+    if (fx_x_lane(p)) {
+        // one block per SM; fewer warps a block where there are too few rows to fill it
+        const size_t rows = p.Ny * p.Nz * d.members, perWarp = 256 / p.Nx;
+        const size_t units = (rows + perWarp - 1) / perWarp, sms = grid_cap(1);
+        const int warps = static_cast<int>(std::min<size_t>(dev::kFxXWarps, std::max<size_t>(1, (units + sms - 1) / sms)));
+        const int grid = static_cast<int>(std::min<size_t>((units + warps - 1) / warps, sms));
+        WV_FXW_SWITCH(p.Nx, {
+            auto* kernel = 8 * p.kxColumns <= 3 * p.Nx ? dev::k_xflux_fx<NN, 3> : dev::k_xflux_fx<NN, 4>;
+            kernel<<<grid, 32 * warps, smem_xflux_fx<NN>(), s>>>(d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
+        });
+        return true;
+    }
+    if (!fx_x_any(p)) return false;
+    const FxXLaunch l = fx_x_launch(p, d.members);
+    WV_FXX_SWITCH(p.kxColumns, (dev::k_xflux_fxany<EK><<<l.grid, 32 * l.warps, l.smem, s>>>(
+                                   d, r.x, r.twX, y, ps, speed, physOut, advOut, advIn, l.pairs)));
+    return true;
+}
+
+bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, const double2* z, double2* y, cudaStream_t s) {
+    const int Ny = static_cast<int>(p.Ny);
+    if (!fx_lane_length(p.Ny)) {
+        const int cols = dev::fx_any_cols(Ny, d.kxColumns);
+        dev::k_yinv_fxany<0><<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps,
+                               dev::smem_fx_any_y(Ny, cols), s>>>(d, map, z, y, cols);
+        return true;
+    }
+    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * (256 / Ny);
+    const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, map.nOut);
+    double ltop = 0.0;
+    for (double l : p.rowL) ltop = std::max(ltop, std::fabs(l));
+    uint64_t bits;
+    std::memcpy(&bits, &ltop, 8);
+    WV_FXW_SWITCH(p.Ny, (dev::k_yinv_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(
+                            d, map, z, y, static_cast<unsigned>(bits >> 32))));
+    return true;
+}
+
+bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, double2* f, cudaStream_t s) {
+    const int Ny = static_cast<int>(p.Ny);
+    if (!fx_lane_length(p.Ny)) {
+        const int cols = dev::fx_any_cols(Ny, d.kxColumns);
+        dev::k_yfwd_fxany<0><<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps,
+                               dev::smem_fx_any_y(Ny, cols), s>>>(d, ps, nch, f, cols);
+        return true;
+    }
+    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * (256 / Ny);
+    const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, nch);
+    WV_FXW_SWITCH(p.Ny, (dev::k_yfwd_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(d, ps, nch, f)));
+    return true;
+}
+
+bool fx_xc2r(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* y, int nch, double* fields, cudaStream_t s) {
+    if (p.Nx > 512 || d.kxColumns > 256) return false;
+    const FxFieldLaunch l = fx_field_launch(p.Nx, p.Ny * d.zTotal, nch);
+    WV_FXX_SWITCH(d.kxColumns, (dev::k_xc2r_fxany<EK><<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, y, nch, fields)));
+    return true;
+}
+
+bool fx_xr2c(const Plan& p, const dev::DescDev& d, const FxRows& r, const double* fields, int nch, double2* ps, cudaStream_t s) {
+    if (p.Nx > 512 || d.kxColumns > 256) return false;
+    const FxFieldLaunch l = fx_field_launch(p.Nx, p.Ny * d.zTotal, nch);
+    dev::k_xr2c_fxany<0><<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, fields, nch, ps);
+    return true;
+}
+
+bool fx_vinv(const Plan& p, const dev::DescDev& d, bool flux, double elapsed, const double* Ap, const double* Am,
+             const double* A0, double2* z, unsigned long long* speed, cudaStream_t s) {
+    if (p.fz.N == 0) return false;
+    if (!fx_lane_length(p.fz.N)) {
+        const int lines = flux ? 4 : 2, warps = fx_z_any_warps(p, lines);
+        const dim3 grid(cdiv(p.Nkl, warps), d.members);
+        const size_t sm = dev::smem_fx_any_z(p.fz.N, lines, warps);
+        if (flux) dev::k_vinv_fxany<true><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
+        else dev::k_vinv_fxany<false><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
+        return true;
+    }
+    const int warps = fx_z_warps(p);
+    const dim3 grid(cdiv(p.Nkl, warps * (256 / p.fz.N)), d.members);
+    WV_FXW_SWITCH(p.fz.N, {
+        const size_t sm = dev::smem_fx_vinv<NN>(warps);
+        if (flux) dev::k_vinv_fx<NN, true><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
+        else dev::k_vinv_fx<NN, false><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
+    });
+    return true;
+}
+
+bool fx_vfwd(const Plan& p, const dev::DescDev& d, bool flux, const double2* f, int nch, double elapsed, const double* Ap,
+             const double* Am, const double* A0, const unsigned long long* speed, int damping, double* Fp, double* Fm,
+             double* F0, cudaStream_t s) {
+    if (p.fz.N == 0) return false;
+    if (!fx_lane_length(p.fz.N)) {
+        const int warps = fx_z_any_warps(p, 2);
+        const dim3 grid(cdiv(p.Nkl, warps), d.members);
+        const size_t sm = dev::smem_fx_any_z(p.fz.N, 2, warps);
+        if (flux)
+            dev::k_vfwd_fxany<true><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
+        else
+            dev::k_vfwd_fxany<false><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
+        return true;
+    }
+    const int warps = fx_z_warps(p);
+    const dim3 grid(cdiv(p.Nkl, warps * (256 / p.fz.N)), d.members);
+    WV_FXW_SWITCH(p.fz.N, {
+        const size_t sm = dev::smem_fx_vfwd<NN>(warps);
+        if (flux)
+            dev::k_vfwd_fx<NN, true><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
+        else
+            dev::k_vfwd_fx<NN, false><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
+    });
+    return true;
+}
+
+}  // namespace wvgpu
+
+namespace wvgpu {
+
+// The dynamic shared-memory cap is a process-wide attribute of each kernel, not of
+// a handle: only ever raise it, so a handle created for a smaller grid cannot shrink
+// the cap below what a live handle for a larger grid launches with.
+cudaError_t raise_smem_limit(const void* kernel, int bytes) {
+    static std::mutex mutex;
+    std::lock_guard<std::mutex> lock(mutex);
+    cudaFuncAttributes a{};
+    cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess) return e;
+    if (a.maxDynamicSharedSizeBytes >= bytes) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+}  // namespace wvgpu

@@ -1,0 +1,425 @@
+// FFTs of FP64 data in 64-bit block fixed point on the integer pipes.
+//
+// The FP64 pipe of this GPU retires about 1.7 operations per SM and clock
+// (measured; 1/64 of the FP32 rate), which bounded every FP64 transform.  The
+// integer pipes add 62 64-bit values per SM and clock and run 16-18 32 x 32 ->
+// 64-bit multiply-adds, so a butterfly costs 10 to 30 times less there.  A line
+// of doubles is scaled by one power of two to 64-bit integers, transformed
+// exactly in its sums and to one unit in its products, and scaled back.
+//
+// Range: with B = sum |x_k| over the line (every partial sum of a DFT is at most
+// B in magnitude, twiddles having modulus 1), the scale puts B into
+// (2^59, 2^61): no sum overflows 63 bits and no product its accumulator.
+// Precision: the unit is 2^-60 B at worst; quantisation contributes 0.29 units
+// per entry and each twiddle product at most about one, so a 256-point line ends
+// near 7 units rms against the FP64 FFT's 2 x 2^-53 of the line's rms -- smaller
+// for every spectrum between flat (B = 18 rms) and steep (B = 4 rms).
+#pragma once
+
+#include <cstdint>
+#ifdef __CUDACC__
+#include <cuda_runtime.h>
+#endif
+
+#ifdef __CUDACC__
+#define WV_HD __host__ __device__ __forceinline__
+#else
+#define WV_HD inline
+#endif
+
+namespace wvgpu {
+namespace dev {
+
+struct alignas(16) fxc { long long x, y; };
+// Twiddle in Q62, each part as a signed high word and a signed low word
+// (value = h 2^32 + l): re_h, re_l, im_h, im_l.
+struct alignas(16) fxw { int ch, cl, sh, sl; };
+
+WV_HD fxc fx_add(fxc a, fxc b) { return {a.x + b.x, a.y + b.y}; }
+WV_HD fxc fx_sub(fxc a, fxc b) { return {a.x - b.x, a.y - b.y}; }
+template <bool INV> WV_HD fxc fx_mul_mi(fxc a) { return INV ? fxc{-a.y, a.x} : fxc{a.y, -a.x}; }
+
+// signed high and low words of x: x = h 2^32 + l, |l| <= 2^31
+WV_HD int fx_lo(long long x) { return static_cast<int>(static_cast<unsigned>(x)); }
+WV_HD int fx_hi(long long x) {
+    return static_cast<int>(x >> 32) + static_cast<int>(static_cast<unsigned>(x) >> 31);
+}
+constexpr long long kFxHalf = 1ll << 29;
+
+// x w (INV: x conj w), |x| < 2^61 (1 - 2^-9).  Twelve 32 x 32 -> 64 products: the
+// low x low terms (at most one unit) are dropped, the middle ones are rounded to
+// the unit and enter the high sum, whose operand carries the factor 4 of Q62.
+template <bool INV>
+WV_HD fxc fx_cmul(fxc a, fxw w) {
+    const int xh = fx_hi(a.x), xl = fx_lo(a.x), yh = fx_hi(a.y), yl = fx_lo(a.y);
+    const int sh = INV ? -w.sh : w.sh, sl = INV ? -w.sl : w.sl;
+    long long mr = kFxHalf, mi = kFxHalf;
+    mr += static_cast<long long>(xh) * w.cl; mr += static_cast<long long>(xl) * w.ch;
+    mr += static_cast<long long>(-yh) * sl;  mr += static_cast<long long>(yl) * -sh;
+    mi += static_cast<long long>(xh) * sl;   mi += static_cast<long long>(xl) * sh;
+    mi += static_cast<long long>(yh) * w.cl; mi += static_cast<long long>(yl) * w.ch;
+    const int xh4 = xh * 4, yh4 = yh * 4;
+    fxc r;
+    r.x = (mr >> 30) + static_cast<long long>(xh4) * w.ch + static_cast<long long>(yh4) * -sh;
+    r.y = (mi >> 30) + static_cast<long long>(xh4) * sh + static_cast<long long>(yh4) * w.ch;
+    return r;
+}
+// x c for a real Q62 constant (h, l)
+WV_HD long long fx_rmul(long long x, int ch, int cl) {
+    const int xh = fx_hi(x), xl = fx_lo(x);
+    long long m = kFxHalf;
+    m += static_cast<long long>(xh) * cl;
+    m += static_cast<long long>(xl) * ch;
+    return (m >> 30) + static_cast<long long>(xh * 4) * ch;
+}
+// high and low words of a Q62 constant
+WV_HD constexpr int fx_qh(long long q) { return static_cast<int>((q + 0x80000000ll) >> 32); }
+WV_HD constexpr int fx_ql(long long q) { return static_cast<int>(static_cast<unsigned>(q)); }
+
+// R-point DFTs of registers (forward: exp(-2 pi i k n / R); INV: conjugate).
+template <bool INV>
+WV_HD void fx_dft2(fxc& a, fxc& b) { const fxc t = fx_sub(a, b); a = fx_add(a, b); b = t; }
+template <bool INV>
+WV_HD void fx_dft4(fxc& v0, fxc& v1, fxc& v2, fxc& v3) {
+    const fxc a = fx_add(v0, v2), b = fx_sub(v0, v2), c = fx_add(v1, v3), d = fx_mul_mi<INV>(fx_sub(v1, v3));
+    v0 = fx_add(a, c); v1 = fx_add(b, d); v2 = fx_sub(a, c); v3 = fx_sub(b, d);
+}
+template <bool INV>
+WV_HD void fx_dft3(fxc& v0, fxc& v1, fxc& v2) {
+    constexpr long long q = 3993837246235628775ll;
+    const fxc t = fx_add(v1, v2), e = fx_sub(v1, v2);
+    const fxc m = {v0.x - (t.x >> 1), v0.y - (t.y >> 1)};
+    const fxc s = {fx_rmul(e.x, fx_qh(q), fx_ql(q)), fx_rmul(e.y, fx_qh(q), fx_ql(q))};
+    const fxc i = INV ? fxc{-s.y, s.x} : fxc{s.y, -s.x};  // -/+ i sin(60) (v1 - v2)
+    v0 = fx_add(v0, t); v1 = fx_add(m, i); v2 = fx_sub(m, i);
+}
+template <bool INV>
+WV_HD void fx_dft5(fxc& v0, fxc& v1, fxc& v2, fxc& v3, fxc& v4) {
+    // cos(72) = (sqrt5 - 1)/4, cos(144) = -(sqrt5 + 1)/4: sums of -1/4 and sqrt5/4
+    constexpr long long qd = 2578010857022246787ll;  // sqrt(5)/4
+    constexpr long long q1 = 4385974038932618941ll;  // sin 72
+    constexpr long long q2 = 2710681029835013083ll;  // sin 144
+    const fxc a = fx_add(v1, v4), b = fx_add(v2, v3), c = fx_sub(v1, v4), d = fx_sub(v2, v3);
+    const fxc t = fx_add(a, b), u = fx_sub(a, b);
+    const fxc du = {fx_rmul(u.x, fx_qh(qd), fx_ql(qd)), fx_rmul(u.y, fx_qh(qd), fx_ql(qd))};
+    const fxc m = {v0.x - (t.x >> 2), v0.y - (t.y >> 2)};
+    const fxc m1 = fx_add(m, du), m2 = fx_sub(m, du);
+    const fxc s1 = {fx_rmul(c.x, fx_qh(q1), fx_ql(q1)) + fx_rmul(d.x, fx_qh(q2), fx_ql(q2)),
+                    fx_rmul(c.y, fx_qh(q1), fx_ql(q1)) + fx_rmul(d.y, fx_qh(q2), fx_ql(q2))};
+    const fxc s2 = {fx_rmul(c.x, fx_qh(q2), fx_ql(q2)) - fx_rmul(d.x, fx_qh(q1), fx_ql(q1)),
+                    fx_rmul(c.y, fx_qh(q2), fx_ql(q2)) - fx_rmul(d.y, fx_qh(q1), fx_ql(q1))};
+    const fxc i1 = fx_mul_mi<INV>(s1), i2 = fx_mul_mi<INV>(s2);
+    v0 = fx_add(v0, t);
+    v1 = fx_add(m1, i1); v4 = fx_sub(m1, i1);
+    v2 = fx_add(m2, i2); v3 = fx_sub(m2, i2);
+}
+template <bool INV>
+WV_HD fxc fx_rot8(fxc a) {  // a exp(-/+ i pi/4)
+    constexpr long long q = 3260954456333195553ll;
+    const long long p = fx_rmul(a.x, fx_qh(q), fx_ql(q)), s = fx_rmul(a.y, fx_qh(q), fx_ql(q));
+    return INV ? fxc{p - s, p + s} : fxc{p + s, s - p};
+}
+template <bool INV>
+WV_HD void fx_dft8(fxc (&v)[8]) {
+    fx_dft4<INV>(v[0], v[2], v[4], v[6]);
+    fx_dft4<INV>(v[1], v[3], v[5], v[7]);
+    const fxc o0 = v[1], o1 = fx_rot8<INV>(v[3]), o2 = fx_mul_mi<INV>(v[5]), o3 = fx_mul_mi<INV>(fx_rot8<INV>(v[7]));
+    const fxc e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+    v[0] = fx_add(e0, o0); v[4] = fx_sub(e0, o0);
+    v[1] = fx_add(e1, o1); v[5] = fx_sub(e1, o1);
+    v[2] = fx_add(e2, o2); v[6] = fx_sub(e2, o2);
+    v[3] = fx_add(e3, o3); v[7] = fx_sub(e3, o3);
+}
+template <int R, bool INV>
+WV_HD void fx_dft(fxc (&v)[R]) {
+    if constexpr (R == 2) fx_dft2<INV>(v[0], v[1]);
+    else if constexpr (R == 3) fx_dft3<INV>(v[0], v[1], v[2]);
+    else if constexpr (R == 4) fx_dft4<INV>(v[0], v[1], v[2], v[3]);
+    else if constexpr (R == 5) fx_dft5<INV>(v[0], v[1], v[2], v[3], v[4]);
+    else fx_dft8<INV>(v);
+}
+
+// ---- doubles to and from the line's fixed point -----------------------------------
+
+// Words of a double's bits.
+WV_HD void fx_words(double v, unsigned& hi, unsigned& lo) {
+#ifdef __CUDA_ARCH__
+    hi = static_cast<unsigned>(__double2hiint(v));
+    lo = static_cast<unsigned>(__double2loint(v));
+#else
+    uint64_t u;
+    __builtin_memcpy(&u, &v, 8);
+    hi = static_cast<unsigned>(u >> 32);
+    lo = static_cast<unsigned>(u);
+#endif
+}
+WV_HD double fx_double(unsigned long long bits) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double(static_cast<long long>(bits));
+#else
+    double v;
+    __builtin_memcpy(&v, &bits, 8);
+    return v;
+#endif
+}
+WV_HD float fx_float(unsigned bits) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(bits);
+#else
+    float v;
+    __builtin_memcpy(&v, &bits, 4);
+    return v;
+#endif
+}
+WV_HD unsigned fx_float_bits(float v) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(v);
+#else
+    unsigned b;
+    __builtin_memcpy(&b, &v, 4);
+    return b;
+#endif
+}
+// |v| / 2^(e0) as a float from the high word of v (e0: the biased exponent of the
+// line's largest high word `top`, so the largest value lies in [1, 2))
+WV_HD float fx_rel(unsigned hi, unsigned top) {
+    const int r = static_cast<int>(hi & 0x7fffffffu) - static_cast<int>(top & 0x7ff00000u) + (127 << 20);
+    return fx_float(static_cast<unsigned>(r > 0 ? r : 0) << 3);
+}
+// bound of |re + i im|: max + (sqrt2 - 1) min >= the modulus
+WV_HD float fx_modulus(float a, float b) { return (a > b ? a : b) + 0.41422f * (a > b ? b : a); }
+
+// |v| as a float from the high word of v: 0 below 2^-126, inf from 2^128 on
+WV_HD float fx_mag(unsigned hi) {
+    int r = static_cast<int>(hi & 0x7fffffffu) - (896 << 20);
+    r = r < 0 ? 0 : r > (255 << 20) ? (255 << 20) : r;
+    return fx_float(static_cast<unsigned>(r) << 3);
+}
+// Whether a sum of fx_mag moduli gives a line's scale by itself; lines outside (all
+// zero, tiny, huge or non-finite) take their scale from their largest entry.
+WV_HD bool fx_plain_sum(float l1) { return l1 > 1e-30f && l1 < 1e30f; }
+
+// Scale of a line: the bit position of 2^e0.  l1: the sum of fx_modulus over the
+// line (its words were cut after 20 bits, hence the factor).
+struct fxscale {
+    int e0;   // biased exponent at bit `bit`
+    int bit;
+};
+WV_HD fxscale fx_scale(unsigned top, float l1) {
+    const float s = l1 * 1.0025f;
+    int el = static_cast<int>(fx_float_bits(s) >> 23) - 126;  // s < 2^el
+    if (el < -40) el = -40;                                   // (weighted rows of one dominant, weightless entry)
+    return {static_cast<int>(top >> 20), 61 - el};
+}
+// the same from a sum of fx_mag moduli
+WV_HD fxscale fx_scale(float l1) {
+    const int el = static_cast<int>(fx_float_bits(l1 * 1.0025f) >> 23) - 126;
+    return {1023, 61 - el};
+}
+WV_HD long long fx_from_double(double v, fxscale sc) {
+    unsigned hi, lo;
+    fx_words(v, hi, lo);
+    const int e = static_cast<int>((hi >> 20) & 0x7ffu);
+    unsigned long long m = (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;  // 2^e at bit 62
+    int rs = 61 - sc.bit + sc.e0 - e;  // one less than the full shift: the last bit rounds
+    if (rs > 63) rs = 63;              // (rs = 63 leaves 0)
+    if (e == 0) rs = 63;
+    m = ((m >> rs) + 1) >> 1;
+    const long long x = static_cast<long long>(m);
+    return static_cast<int>(hi) < 0 ? -x : x;
+}
+// Exponent of the unit (biased): real value = integer * 2^(unit - 1023).
+// kFxBad marks a line that held a non-finite value.
+constexpr int kFxBad = 1 << 28;
+WV_HD int fx_unit(fxscale sc) { return sc.e0 >= 0x7ff ? kFxBad : sc.e0 - sc.bit; }
+WV_HD int fx_clz(unsigned long long v) {
+#ifdef __CUDA_ARCH__
+    return __clzll(static_cast<long long>(v));
+#else
+    return v ? __builtin_clzll(v) : 64;
+#endif
+}
+// integer * 2^(unit - 1023) rounded to the nearest double (0 below the normal range, inf above)
+WV_HD double fx_to_double(long long x, int unit) {
+    const unsigned long long sign = static_cast<unsigned long long>(x) & 0x8000000000000000ull;
+    unsigned long long m = static_cast<unsigned long long>(x < 0 ? -x : x);
+    const int lz = fx_clz(m);
+    const int e = unit + 62 - lz;  // exponent field of the leading bit, less one (the hidden bit adds it)
+    m <<= (lz & 63);
+    const unsigned long long r = (m >> 11) + ((m >> 10) & 1ull);
+    unsigned long long bits = r + (static_cast<unsigned long long>(static_cast<unsigned>(e)) << 52);
+    if (x == 0 || e < 0) bits = 0;
+    if (e >= 0x7fe) bits = unit >= kFxBad / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull;
+    return fx_double(bits | sign);
+}
+
+#ifdef __CUDACC__
+// One stage over `lines` lines (as fft_stage): radix R from src to dst.
+template <int R, bool INV>
+__device__ __forceinline__ void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int Ns, int lines,
+                                         int ld, const fxw* __restrict__ tw, int tid, int nt) {
+    const int nb = N / R;
+    const int tstride = N / (Ns * R);
+    const bool p2 = (N & (N - 1)) == 0;
+    const int nbShift = __ffs(nb) - 1, nsShift = __ffs(Ns) - 1;
+    for (int it = tid; it < lines * nb; it += nt) {
+        int line, j, k, jq;
+        if (p2) {
+            line = it >> nbShift; j = it & (nb - 1); k = j & (Ns - 1); jq = j >> nsShift;
+        } else {
+            line = it / nb; j = it - line * nb; jq = j / Ns; k = j - jq * Ns;
+        }
+        const fxc* in = src + line * ld + j;
+        fxc v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = in[r * nb];
+        if (Ns > 1) {
+            const int ts = k * tstride;
+#pragma unroll
+            for (int r = 1; r < R; ++r) v[r] = fx_cmul<INV>(v[r], tw[r * ts]);
+        }
+        fx_dft<R, INV>(v);
+        fxc* out = dst + line * ld + jq * Ns * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) out[r * Ns] = v[r];
+    }
+}
+// Any other radix: one output per work item, an O(R) sum.
+template <bool INV>
+__device__ __forceinline__ void fx_stage_any(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int R, int Ns,
+                                             int lines, int ld, const fxw* __restrict__ tw, int tid, int nt) {
+    const int nb = N / R;
+    const int tstride = N / (Ns * R);
+    for (int it = tid; it < lines * N; it += nt) {
+        const int line = it / N, rem = it - line * N;
+        const int j = rem % nb, r = rem / nb;
+        const fxc* in = src + line * ld;
+        const int k = j % Ns;
+        const int step = (k * tstride + r * nb) % N;
+        fxc acc = in[j];
+        int e = step;
+        for (int m = 1; m < R; ++m) {
+            acc = fx_add(acc, fx_cmul<INV>(in[j + m * nb], tw[e]));
+            e += step;
+            if (e >= N) e -= N;
+        }
+        dst[line * ld + (j / Ns) * Ns * R + k + r * Ns] = acc;
+    }
+}
+
+struct FxFactors { int N, nstages; const int* radix; };
+
+// Lines of doubles (re, im) in place to fixed point: one group of warps per line
+// sums the moduli, then every entry is scaled.  unit[line] receives fx_unit.
+// Called by all threads of the block.
+__device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, int* unit) {
+    __shared__ unsigned redTop[32];
+    __shared__ float redSum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int per = lines < warps ? warps / lines : 1;  // warps of one line
+    const int groups = warps / per;
+    fxc* out = reinterpret_cast<fxc*>(lines_);
+    for (int l0 = 0; l0 < lines; l0 += groups) {
+        const int g = warp / per, line = l0 + g;
+        const bool has = g < groups && line < lines;
+        const int t = (warp - g * per) * 32 + lane, step = per * 32;
+        const double2* row = lines_ + line * ld;
+        auto total = [&](float sum) {  // over the warps of the line
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (per > 1) {
+                if (lane == 0) redSum[warp] = sum;
+                __syncthreads();
+                if (has) {
+                    sum = 0.f;
+                    for (int w = 0; w < per; ++w) sum += redSum[g * per + w];
+                }
+            }
+            return sum;
+        };
+        float sum = 0.f;
+        if (has)
+            for (int i = t; i < N; i += step) {
+                const double2 v = row[i];
+                sum += fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))),
+                                  fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
+            }
+        sum = total(sum);
+        fxscale sc = fx_scale(sum);
+        const bool odd = has && !fx_plain_sum(sum);
+        if (per > 1 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) {
+            unsigned top = 0;
+            if (has)
+                for (int i = t; i < N; i += step) {
+                    const double2 v = row[i];
+                    top = max(top, max(static_cast<unsigned>(__double2hiint(v.x)) & 0x7fffffffu,
+                                       static_cast<unsigned>(__double2hiint(v.y)) & 0x7fffffffu));
+                }
+            top = __reduce_max_sync(0xffffffffu, top);
+            if (per > 1) {
+                if (lane == 0) redTop[warp] = top;
+                __syncthreads();
+                if (has)
+                    for (int w = 0; w < per; ++w) top = max(top, redTop[g * per + w]);
+            }
+            float rel = 0.f;
+            if (has)
+                for (int i = t; i < N; i += step) {
+                    const double2 v = row[i];
+                    rel += fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
+                                      fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
+                }
+            rel = total(rel);
+            if (odd) sc = fx_scale(top, rel);
+        }
+        if (has) {
+            if (t == 0) unit[line] = fx_unit(sc);
+            for (int i = t; i < N; i += step) {
+                const double2 v = row[i];
+                out[line * ld + i] = fxc{fx_from_double(v.x, sc), fx_from_double(v.y, sc)};
+            }
+        }
+        if (per > 1 && l0 + groups < lines) __syncthreads();  // the partial results are reused
+    }
+    __syncthreads();
+}
+
+// All stages over fixed-point lines; returns the buffer holding the result.
+// WARP: the lines belong to one warp (no block barrier), else to the block.
+template <bool INV, bool WARP>
+__device__ inline fxc* fx_lines(fxc* a, fxc* b, const FxFactors f, int lines, int ld, const fxw* tw) {
+    const int tid = WARP ? (threadIdx.x & 31) : threadIdx.x, nt = WARP ? 32 : blockDim.x;
+    int Ns = 1;
+    for (int s = 0; s < f.nstages; ++s) {
+        const int R = f.radix[s];
+        if (R == 8) fx_stage<8, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
+        else if (R == 4) fx_stage<4, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
+        else if (R == 2) fx_stage<2, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
+        else if (R == 3) fx_stage<3, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
+        else if (R == 5) fx_stage<5, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
+        else fx_stage_any<INV>(a, b, f.N, R, Ns, lines, ld, tw, tid, nt);
+        if (WARP) __syncwarp(); else __syncthreads();
+        Ns *= R;
+        fxc* t = a; a = b; b = t;
+    }
+    return a;
+}
+
+// fft_lines of FP64 lines: scaled, transformed and scaled back in place.
+template <bool INV>
+__device__ inline double2* fx_fft_lines(double2* a, double2* b, const FxFactors f, int lines, int ld, const fxw* tw) {
+    __shared__ int unit[16];
+    fx_quantise(a, f.N, lines, ld, unit);
+    fxc* r = fx_lines<INV, false>(reinterpret_cast<fxc*>(a), reinterpret_cast<fxc*>(b), f, lines, ld, tw);
+    double2* out = reinterpret_cast<double2*>(r);
+    for (int i = threadIdx.x; i < lines * f.N; i += blockDim.x) {
+        const int line = i / f.N, k = i - line * f.N, u = unit[line];
+        const fxc v = r[line * ld + k];
+        out[line * ld + k] = make_double2(fx_to_double(v.x, u), fx_to_double(v.y, u));
+    }
+    __syncthreads();
+    return out;
+}
+#endif
+
+}  // namespace dev
+}  // namespace wvgpu

@@ -1,0 +1,442 @@
+// Fixed-point FFT lines (wv_fx.cuh) of 16 to 256 points held by lanes: a line of N
+// points belongs to N / 8 lanes of one warp, lane t holding points t + (N/8) e, e <
+// 8, before and after the transform; 32 / (N/8) lines ride in a warp.  The stages
+// are 8 x 2, 8 x 4, 8 x 8, 8 x 4 x 4 or 8 x 8 x 4 points of registers with one
+// exchange through shared memory between two stages (warp barriers only).
+//
+// What bounds these lines is the number of instructions issued: against the
+// run-time Stockham stages of wv_fx.cuh every index is a constant here, the first
+// and last stage work on registers, stage twiddles are stored in the order the
+// lanes read them, and the line buffers are padded by one entry in eight (no bank
+// conflicts on 16-byte accesses).
+#pragma once
+
+#include "wv_kernels.cuh"
+
+namespace wvgpu {
+namespace dev {
+
+template <int N> struct FxW {
+    static constexpr int G = N / 8;         // lanes of a line
+    static constexpr int lines = 32 / G;    // lines of a warp
+    static constexpr int buffer = N + N / 8;  // padded line buffer
+    static constexpr int R2 = N == 16 ? 2 : (N == 32 || N == 128) ? 4 : 8;
+    static constexpr int R3 = N >= 128 ? 4 : 1;
+    static constexpr int twiddles = (R2 - 1) * 8 + (R3 - 1) * 8 * R2;
+};
+__device__ __forceinline__ int fx_pad(int i) { return i + (i >> 3); }
+
+// Stage of radix R behind Ns points already combined; tw[(r - 1) Ns + k].
+template <int N, int R, int Ns, bool INV>
+__device__ __forceinline__ void fx_wstage(fxc (&v)[8], const fxw* __restrict__ tw, int t) {
+    constexpr int G = N / 8, B = 8 / R;
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        const int k = (t + G * b) & (Ns - 1);
+        fxc u[R];
+        u[0] = v[b];
+#pragma unroll
+        for (int r = 1; r < R; ++r) u[r] = fx_cmul<INV>(v[b + B * r], tw[(r - 1) * Ns + k]);
+        fx_dft<R, INV>(u);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[b + B * r] = u[r];
+    }
+}
+// v[b + B r], the outputs of a stage of radix R, to their places and back to lane order
+template <int N, int R, int Ns>
+__device__ __forceinline__ void fx_wexchange(fxc (&v)[8], fxc* __restrict__ x, int t) {
+    constexpr int G = N / 8, B = 8 / R;
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        const int j = t + G * b, k = j & (Ns - 1), jq = j / Ns;
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[fx_pad(jq * Ns * R + k + r * Ns)] = v[b + B * r];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+    __syncwarp();
+}
+// The whole line; x: this line's buffer, tw: the stage twiddles in shared memory.
+template <int N, bool INV>
+__device__ __forceinline__ void fx_fft_warp(fxc (&v)[8], fxc* __restrict__ x, const fxw* __restrict__ tw, int t) {
+    using W = FxW<N>;
+    fx_dft8<INV>(v);
+    fx_wexchange<N, 8, 1>(v, x, t);
+    fx_wstage<N, W::R2, 8, INV>(v, tw, t);
+    if constexpr (W::R3 > 1) {
+        fx_wexchange<N, W::R2, 8>(v, x, t);
+        fx_wstage<N, W::R3, 8 * W::R2, INV>(v, tw + (W::R2 - 1) * 8, t);
+    }
+}
+
+// maxima and sums over the lanes of a line
+template <int G>
+__device__ __forceinline__ unsigned fx_group_max(unsigned v) {
+    if constexpr (G == 32) return __reduce_max_sync(0xffffffffu, v);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+template <int G>
+__device__ __forceinline__ unsigned fx_group_add(unsigned v) {
+    if constexpr (G == 32) return __reduce_add_sync(0xffffffffu, v);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <int G>
+__device__ __forceinline__ float fx_group_sum(float v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// mantissa (2^e at bit 62; 0 below the normal range) and exponent of a double
+__device__ __forceinline__ unsigned long long fx_mantissa(double v, int& e) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
+    e = static_cast<int>((hi >> 20) & 0x7ffu);
+    const unsigned long long m = (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
+    return e == 0 ? 0ull : m;
+}
+__device__ __forceinline__ long long fx_align(unsigned long long m, int rs, bool negative) {
+    m = ((m >> min(rs, 63)) + 1) >> 1;
+    return negative ? -static_cast<long long>(m) : static_cast<long long>(m);
+}
+
+// What a line's entries are multiplied by: nothing, real weights w, or i w.
+enum FxWeight { kFxPlain, kFxReal, kFxImag };
+
+// C doubles of a lane, weighted, in the fixed point of their line.  count(c): how
+// often entry c enters the line's sum of moduli; spare: bits kept free (1 when two
+// rows share the line); wtop: high word of the largest |w|.
+template <int C, int G, FxWeight MODE, typename Count>
+__device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const double (&w)[C], unsigned wtop, int spare,
+                                                 Count count, fxc (&out)[C], int& unit) {
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        float m = fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v[c].x))),
+                             fx_mag(static_cast<unsigned>(__double2hiint(v[c].y))));
+        if (MODE != kFxPlain) m *= fx_mag(static_cast<unsigned>(__double2hiint(w[c])));
+        sum += count(c) * m;
+    }
+    sum = fx_group_sum<G>(sum);
+    fxscale sc = fx_scale(sum);
+    int wexp = 0;
+    const bool odd = !fx_plain_sum(sum);
+    if (__any_sync(0xffffffffu, odd)) {
+        unsigned top = 0;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            top = max(top, max(static_cast<unsigned>(__double2hiint(v[c].x)) & 0x7fffffffu,
+                               static_cast<unsigned>(__double2hiint(v[c].y)) & 0x7fffffffu));
+        top = fx_group_max<G>(top);
+        float rel = 0.f;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            float m = fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v[c].x)), top),
+                                 fx_rel(static_cast<unsigned>(__double2hiint(v[c].y)), top));
+            if (MODE != kFxPlain) m *= fx_rel(static_cast<unsigned>(__double2hiint(w[c])), wtop) * 1.00001f;
+            rel += count(c) * m;
+        }
+        rel = fx_group_sum<G>(rel);
+        if (odd) {
+            sc = fx_scale(top, rel);
+            if (MODE != kFxPlain) wexp = static_cast<int>((wtop >> 20) & 0x7ffu) - 1023;
+        }
+    }
+    sc.bit -= spare;
+    unit = sc.e0 >= 0x7ff ? kFxBad : sc.e0 + wexp - sc.bit;
+    const int base = 61 - sc.bit + sc.e0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        int ex, ey;
+        unsigned long long mx = fx_mantissa(v[c].x, ex), my = fx_mantissa(v[c].y, ey);
+        const bool nx = __double2hiint(v[c].x) < 0, ny = __double2hiint(v[c].y) < 0;
+        if constexpr (MODE != kFxPlain) {
+            int ew;
+            const unsigned long long mw = fx_mantissa(w[c], ew) << 1;
+            const bool nw = __double2hiint(w[c]) < 0;
+            mx = __umul64hi(mx, mw);  // 2^(e + ew - 1022) at bit 62
+            my = __umul64hi(my, mw);
+            const int b2 = base + wexp + 1022 - ew;
+            const long long wx = fx_align(mx, b2 - ex, nx != nw), wy = fx_align(my, b2 - ey, ny != nw);
+            out[c] = MODE == kFxImag ? fxc{-wy, wx} : fxc{wx, wy};
+        } else {
+            out[c].x = fx_align(mx, base - ex, nx);
+            out[c].y = fx_align(my, base - ey, ny);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// x pass of the FP64 flux: c2r of the velocities and of every derivative, the
+// quadratic products and their r2c, one (y, z) row per line of the warp and no
+// block barrier.  Two real rows share one complex line (Z = A + i B for the c2r,
+// S_a + i S_b for the r2c); each row keeps its own scale, so its rounding stays
+// relative to its own magnitude whatever its partner holds.  Products are formed as
+// (a b) >> 62 on velocities normalised to 62 bits and added at the largest unit of
+// a target's three.
+
+inline size_t fx_xflux_warp_bytes(int N) { return static_cast<size_t>(256 / N) * ((N + N / 8) * 16 + 40 * N); }
+constexpr int kFxXWarps = 15;  // 14.8 KB of shared memory and 32 x 128 registers each fill an SM
+
+// (a b) >> 62 rounded, |a| < 2^62, |b| < 2^61
+__device__ __forceinline__ long long fx_prod(long long a, long long b) {
+    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
+    long long m = kFxHalf;
+    m += static_cast<long long>(ah) * bl;
+    m += static_cast<long long>(al) * bh;
+    return (m >> 30) + static_cast<long long>(ah) * (bh * 4);
+}
+// A velocity normalised to 62 bits (leading bit of the row's largest: 61), cut to
+// the 53 a double holds: the fields that nonlinearFluxWithAdvectionFields returns
+// are then exactly those the flux used, and a flux given them forms the same
+// products bit for bit.  (Rounding up past the leading bit would change the
+// normalisation: the last step is dropped there.)
+__device__ __forceinline__ long long fx_round53(long long v) {
+    const long long most = (1ll << 62) - 512;
+    const long long r = (v + 256) & ~511ll;
+    return r > most ? most : r < -most ? -most : r;
+}
+__device__ __forceinline__ unsigned fx_abs_hi(long long v) {
+    return static_cast<unsigned>(static_cast<unsigned long long>(v < 0 ? -v : v) >> 32);
+}
+__device__ __forceinline__ int fx_pick(const int (&a)[3], int i) { return i == 0 ? a[0] : i == 1 ? a[1] : a[2]; }
+
+// physOut / advOut / advIn / maxSpeedBits as k_xflux.
+// EK: spectrum entries of a lane (kx < EK N / 8; 3 under the 2/3 rule).
+template <int N, int EK>
+__global__ void __launch_bounds__(32 * kFxXWarps, 1)
+    k_xflux_fx(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, double2* __restrict__ pspec,
+               unsigned long long* __restrict__ maxSpeedBits, double* __restrict__ physOut, double* __restrict__ advOut,
+               const double* __restrict__ advIn) {
+    using W = FxW<N>;
+    constexpr int G = W::G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
+    const int nIn = 4 + 2 * nt, nReal = 3 + 3 * nt;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int t = lane % G, line = lane / G;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
+    __syncthreads();
+    unsigned char* mine = smem_raw + W::twiddles * 16 + static_cast<size_t>(warp * W::lines + line) * (W::buffer * 16 + 40 * N);
+    fxc* x = reinterpret_cast<fxc*>(mine);                         // line buffer
+    long long* phys = reinterpret_cast<long long*>(x + W::buffer);  // u, v, w [3][N]
+    long long* S = phys + 3 * N;                                    // products of two targets [2][N]
+    const double* rowK = row_k<double>(d);
+    const size_t cstride = static_cast<size_t>(Ny) * KX;
+    const size_t R3 = static_cast<size_t>(N) * Ny * d.Nz;
+    const int rows = Ny * d.zTotal;
+    const unsigned wtop = static_cast<unsigned>(__double2hiint(rowK[KX - 1]));
+    for (int first = (blockIdx.x * warps + warp) * W::lines; first < rows; first += gridDim.x * warps * W::lines) {
+        const bool live = first + line < rows;
+        const int row = min(first + line, rows - 1);
+        const int z = row / Ny, y = row - z * Ny;
+        const double2* yrow = yspec + (static_cast<size_t>(z) * nIn * Ny + y) * KX;
+        int physUnit[3] = {0, 0, 0}, sUnit[2] = {0, 0}, unitNow = 0;
+        long long acc[8];  // products of the current target
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = 0;
+        for (int p = 0; 2 * p < nReal; ++p) {
+            fxc v[8];
+            int unit[2] = {0, 0};
+            {
+                // rows 2p and 2p + 1: spectrum entries k = t + G i, both rows' loads in flight
+                double2 raw[2][EK];
+                int weighted = 0;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int r = 2 * p + q;
+                    int ch = r;
+                    if (r >= 3) {
+                        const int tt = (r - 3) / 3, kind = (r - 3) - 3 * tt;
+                        if (kind == 0) weighted |= 1 << q;
+                        ch = kind == 0 ? d.tq[tt & 3] : kind == 1 ? 4 + tt : 4 + nt + tt;
+                    }
+                    const double2* h = yrow + ch * cstride;
+#pragma unroll
+                    for (int i = 0; i < EK; ++i) {
+                        const int k = t + G * i;
+                        raw[q][i] = k < KX && r < nReal ? h[k] : make_double2(0.0, 0.0);
+                    }
+                    if (t == 0) raw[q][0].y = 0.0;  // c2r semantics
+                }
+                fxc A[EK], B[EK];
+                auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
+#pragma unroll 1
+                for (int q = 0; q < 2; ++q) {  // one copy of the code: it must stay in the instruction cache
+                    double2 a[EK];
+                    double w[EK];
+#pragma unroll
+                    for (int i = 0; i < EK; ++i) {
+                        a[i] = q ? raw[1][i] : raw[0][i];
+                        A[i] = B[i];
+                    }
+                    int u;
+                    if ((weighted >> q) & 1) {
+#pragma unroll
+                        for (int i = 0; i < EK; ++i) w[i] = t + G * i < KX ? rowK[t + G * i] : 0.0;
+                        fx_quantise_lane<EK, G, kFxImag>(a, w, wtop, 1, count, B, u);
+                    } else {
+                        fx_quantise_lane<EK, G, kFxPlain>(a, w, 0u, 1, count, B, u);
+                    }
+                    unit[0] = unit[1];
+                    unit[1] = u;
+                }
+                // Z = A + i B at k and its mirror at N - k; nothing between
+#pragma unroll
+                for (int i = 0; i < EK; ++i) {
+                    const fxc a = A[i], b = B[i];
+                    v[i] = fxc{a.x - b.y, a.y + b.x};
+                    const int k = t + G * i;
+                    const fxc m = {a.x + b.y, b.x - a.y};
+                    x[fx_pad(k == 0 ? N - G * EK : N - k)] = k == 0 ? fxc{0, 0} : m;
+                }
+#pragma unroll
+                for (int e = EK; e < 8 - EK; ++e) v[e] = fxc{0, 0};
+                __syncwarp();
+#pragma unroll
+                for (int e = 8 - EK; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+                __syncwarp();
+            }
+            fx_fft_warp<N, true>(v, x, tw, t);
+            // samples x = t + G e: real part row 2p, imaginary part row 2p + 1
+#pragma unroll 1
+            for (int q = 0; q < 2; ++q) {
+                const int r = 2 * p + q;
+                if (r >= nReal) break;
+                const int uq = q ? unit[1] : unit[0];
+                long long smp[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) smp[e] = q ? v[e].y : v[e].x;
+                if (physOut && live && r >= 3) {
+                    double* keep = physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
+                }
+                if (r < 3) {
+                    // advecting velocity, normalised to 62 bits
+                    const size_t g = static_cast<size_t>(r) * R3 + (static_cast<size_t>(z) * Ny + y) * N;
+                    int un;
+                    if (advIn) {
+                        double a[8];
+                        unsigned top = 0;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            a[e] = advIn[g + t + G * e];
+                            top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
+                        }
+                        top = fx_group_max<G>(top);
+                        const fxscale sc{static_cast<int>(top >> 20), 61};
+                        un = fx_unit(sc);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            phys[r * N + t + G * e] = fx_from_double(a[e], sc);
+                            if (physOut && live)
+                                physOut[((static_cast<size_t>(z) * nReal + r) * Ny + y) * N + t + G * e] = a[e];
+                        }
+                    } else {
+                        unsigned top = 0;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) top = max(top, fx_abs_hi(smp[e]));
+                        top = fx_group_max<G>(top);
+                        const int sh = max(0, __clz(static_cast<int>(top)) - 2);
+                        un = uq - sh;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const long long s = fx_round53(smp[e] << sh);
+                            phys[r * N + t + G * e] = s;
+                            if (advOut && live) advOut[g + t + G * e] = fx_to_double(s, un);
+                            if (physOut && live)
+                                physOut[((static_cast<size_t>(z) * nReal + r) * Ny + y) * N + t + G * e] = fx_to_double(s, un);
+                        }
+                    }
+                    if (r == 0) physUnit[0] = un;
+                    else if (r == 1) physUnit[1] = un;
+                    else physUnit[2] = un;
+                    continue;  // phys is read back by the lane that wrote it
+                }
+                const int tt = (r - 3) / 3, kind = (r - 3) - 3 * tt;
+                const int un = fx_pick(physUnit, kind) + uq - 1023 + 62;
+                const long long* vel = phys + kind * N;
+                if (kind == 0) {
+                    unitNow = un;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] = -fx_prod(vel[t + G * e], smp[e]);
+                } else {
+                    const int now = max(unitNow, un);
+                    const int shS = min(63, now - unitNow), shP = min(63, now - un);
+                    unitNow = now;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        acc[e] = (acc[e] >> shS) - (fx_prod(vel[t + G * e], smp[e]) >> shP);
+                }
+                if (kind == 2) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) S[(tt & 1) * N + t + G * e] = acc[e];
+                    sUnit[0] = (tt & 1) ? sUnit[0] : unitNow;
+                    sUnit[1] = (tt & 1) ? unitNow : sUnit[1];
+                }
+            }
+            // targets finished so far: a full pair, or the last one, goes forward
+            const int done = min(nt, (2 * p + 2 - 3) / 3);
+            const int before = p == 0 ? 0 : min(nt, max(0, (2 * p - 3) / 3));
+            if (done > before && ((done & 1) == 0 || done == nt)) {
+                const bool both = (done & 1) == 0;
+                const int t0 = both ? done - 2 : done - 1;
+                int sh[2], u[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    unsigned sum = 0;
+                    if (q == 0 || both)
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) sum += (fx_abs_hi(S[q * N + t + G * e]) >> 9) + 1u;
+                    sum = fx_group_add<G>(sum);
+                    sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 60;  // sum |S| < 2^60 after the shift
+                    u[q] = sUnit[q] + sh[q] - 1;                            // the halves of the split below
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const long long a = S[t + G * e], b = both ? S[N + t + G * e] : 0;
+                    v[e].x = sh[0] >= 0 ? a >> sh[0] : a << -sh[0];
+                    v[e].y = sh[1] >= 0 ? b >> sh[1] : b << -sh[1];
+                }
+                fx_fft_warp<N, false>(v, x, tw, t);
+                __syncwarp();
+#pragma unroll
+                for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+                __syncwarp();
+                double2* out = pspec + ((static_cast<size_t>(z) * nt + t0) * Ny + y) * KX;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int k = t + G * i;
+                    const fxc a = v[i], b = k == 0 ? v[0] : x[fx_pad(N - k)];
+                    if (k < KX && live) {
+                        out[k] = make_double2(fx_to_double(a.x + b.x, u[0]), fx_to_double(a.y - b.y, u[0]));
+                        if (both) out[cstride + k] = make_double2(fx_to_double(a.y + b.y, u[1]), fx_to_double(b.x - a.x, u[1]));
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        // max |u_h| (only when adaptive damping consumes it)
+        if (maxSpeedBits) {
+            double m = 0.0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const double U = fx_to_double(phys[t + G * e], physUnit[0]);
+                const double V = fx_to_double(phys[N + t + G * e], physUnit[1]);
+                m = fmax(m, U * U + V * V);
+            }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if (t == 0) atomicMax(maxSpeedBits + z / d.Nz, (unsigned long long)__double_as_longlong(sqrt(m)));
+        }
+    }
+}
+
+}  // namespace dev
+}  // namespace wvgpu

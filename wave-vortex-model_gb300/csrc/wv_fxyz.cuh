@@ -1,0 +1,462 @@
+// The y and z passes of FP64 handles on lane-held fixed-point lines (wv_fxwarp.cuh).
+#pragma once
+
+#include "wv_fxwarp.cuh"
+
+namespace wvgpu {
+namespace dev {
+
+// ---- y ------------------------------------------------------------------------------
+
+constexpr int kFxYWarps = 8;
+// Shared memory: stage twiddles and, for each of `cols` columns, a line buffer; the
+// tile [y][cols] that makes the global accesses contiguous lies in the same bytes.
+template <int N>
+inline size_t smem_fxy(int cols) {
+    return static_cast<size_t>(FxW<N>::twiddles + cols * FxW<N>::buffer) * 16;
+}
+// Entry (y, c) of the tile: columns are exclusive-ored with y, so that eight lanes
+// of a line (consecutive y, one column) meet eight different banks.
+__device__ __forceinline__ int fx_tile(int y, int c, int cols) { return y * cols + (c ^ (y & min(7, cols - 1))); }
+
+// Inverse FFTs along y of output channel blockIdx.z, columns blockIdx.x cols ...,
+// plane blockIdx.y: yspec[z][ch][y][kx] from zspec[src][z][pos] (times i l).
+template <int N>
+__global__ void __launch_bounds__(32 * kFxYWarps, 2)
+    k_yinv_fx(DescDev d, YInvMap map, const double2* __restrict__ zspec, double2* __restrict__ yspec, unsigned ltop) {
+    using W = FxW<N>;
+    constexpr int G = W::G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int P = d.positions, KX = d.kxColumns;
+    const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
+    const int cols = (blockDim.x >> 5) * W::lines;
+    const int kx0 = blockIdx.x * cols, z = blockIdx.y, oc = blockIdx.z;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + own * W::buffer;
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwY[i];
+    const double2* in = zspec + (static_cast<size_t>(map.src[oc]) * d.zTotal + z) * P;
+    const int kx = kx0 + own;
+    double2 a[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int pos = kx < KX ? d.ymap[static_cast<size_t>(kx) * N + t + G * e] : -1;
+        a[e] = pos >= 0 ? in[pos] : make_double2(0.0, 0.0);
+    }
+    fxc v[8];
+    int unit;
+    double w[8];
+    auto count = [](int) { return 1.0f; };
+    if (map.mulL[oc]) {
+        const double* rowL = row_l<double>(d);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = rowL[t + G * e];
+        fx_quantise_lane<8, G, kFxImag>(a, w, ltop, 0, count, v, unit);
+    } else {
+        fx_quantise_lane<8, G, kFxPlain>(a, w, 0u, 0, count, v, unit);
+    }
+    __syncthreads();  // twiddles
+    fx_fft_warp<N, true>(v, x, tw, t);
+    __syncthreads();  // every line buffer read: the tile takes their place
+    double2* tile = reinterpret_cast<double2*>(tw + W::twiddles);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        tile[fx_tile(t + G * e, own, cols)] = make_double2(fx_to_double(v[e].x, unit), fx_to_double(v[e].y, unit));
+    __syncthreads();
+    double2* out = yspec + (static_cast<size_t>(z) * map.nOut + oc) * N * KX + kx0;
+    const int g = min(cols, KX - kx0);
+    for (int i = threadIdx.x; i < N * cols; i += blockDim.x) {
+        const int y = i / cols, c = i - y * cols;
+        if (c < g) out[static_cast<size_t>(y) * KX + c] = tile[fx_tile(y, c, cols)];
+    }
+}
+
+// Forward FFTs along y of channel blockIdx.z, gathered to the active rows:
+// fspec[c][z][pos] from pspec[z][c][y][kx].
+template <int N>
+__global__ void __launch_bounds__(32 * kFxYWarps, 2)
+    k_yfwd_fx(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec) {
+    using W = FxW<N>;
+    constexpr int G = W::G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int P = d.positions, KX = d.kxColumns;
+    const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
+    const int cols = (blockDim.x >> 5) * W::lines;
+    const int kx0 = blockIdx.x * cols, z = blockIdx.y, ch = blockIdx.z;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + own * W::buffer;
+    double2* tile = reinterpret_cast<double2*>(tw + W::twiddles);
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwY[i];
+    const double2* in = pspec + (static_cast<size_t>(z) * nch + ch) * N * KX + kx0;
+    const int g = min(cols, KX - kx0);
+    for (int i = threadIdx.x; i < N * cols; i += blockDim.x) {
+        const int y = i / cols, c = i - y * cols;
+        tile[fx_tile(y, c, cols)] = c < g ? in[static_cast<size_t>(y) * KX + c] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    double2 a[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
+    __syncthreads();  // the line buffers take the tile's place
+    fxc v[8];
+    int unit;
+    double w[8];
+    fx_quantise_lane<8, G, kFxPlain>(a, w, 0u, 0, [](int) { return 1.0f; }, v, unit);
+    fx_fft_warp<N, false>(v, x, tw, t);
+    const int kx = kx0 + own;
+    if (kx >= KX) return;
+    double2* out = fspec + (static_cast<size_t>(ch) * d.zTotal + z) * P;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int pos = d.ymap[static_cast<size_t>(kx) * N + t + G * e];
+        if (pos >= 0) out[pos] = make_double2(fx_to_double(v[e].x, unit), fx_to_double(v[e].y, unit));
+    }
+}
+
+// ---- phases ----------------------------------------------------------------------------
+
+// exp(i angle) rounded from fixed point: the angle in turns is the exact product of
+// its 53 bits with 1 / (2 pi) to 128 bits, the nearest of 256 table entries is
+// turned by the remainder |r| <= pi / 256 with Taylor sums (sine to r^7, cosine to
+// r^6; the next terms are below 2^-62).  About 170 integer instructions; the FP64
+// sincos it replaces takes some 50 operations of a pipe that retires 1.7 per clock
+// and SM (30 clocks against 1.3 a value).
+__device__ __forceinline__ void fx_phase(double angle, const fxw* __restrict__ table, double& cs, double& sn) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(angle));
+    const int e = static_cast<int>((hi >> 20) & 0x7ffu);
+    if (e >= 1023 + 31) {  // beyond 2^31 rad (and inf, NaN): the library's reduction
+        sincos(angle, &sn, &cs);
+        return;
+    }
+    const unsigned long long m = static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 |
+                                 static_cast<unsigned>(__double2loint(angle));
+    constexpr unsigned long long c1 = 0x28be60db9391054aull, c0 = 0x7f09d5f47d4d3770ull;  // 2^128 / (2 pi)
+    const unsigned long long lo = m * c1, add = __umul64hi(m, c0);
+    unsigned long long q1 = __umul64hi(m, c1), q0 = lo + add;
+    q1 += q0 < lo ? 1ull : 0ull;
+    const int s = 1075 - e;  // turns = (q1:q0) 2^-(64 + s); s > 21
+    unsigned long long f;
+    if (s < 64) f = (q0 >> s) | (q1 << (64 - s));
+    else f = s < 128 ? q1 >> (s - 64) : 0ull;
+    if (static_cast<int>(hi) < 0) f = 0ull - f;
+    const unsigned idx = static_cast<unsigned>((f + (1ull << 55)) >> 56) & 255u;
+    const long long r = static_cast<long long>(f - (static_cast<unsigned long long>(idx) << 56));  // turns, Q64
+    constexpr long long qpi = 3622009729038561421ll;  // pi / 4
+    const long long th = fx_rmul(r, fx_qh(qpi), fx_ql(qpi)) * 2;                // 2 pi r in Q62
+    const long long s2 = fx_prod(th, th);
+    constexpr long long k6 = 768614336404564651ll, k120 = 38430716820228233ll, k5040 = 915017067148291ll;
+    constexpr long long k24 = 192153584101141163ll, k720 = 6405119470038039ll, k2 = 2305843009213693952ll;
+    const long long ps = k6 - fx_prod(k120 - fx_rmul(s2, fx_qh(k5040), fx_ql(k5040)), s2);
+    const long long pc = k2 - fx_prod(k24 - fx_rmul(s2, fx_qh(k720), fx_ql(k720)), s2);
+    const fxc small = {-fx_prod(pc, s2), th - fx_prod(fx_prod(ps, s2), th)};  // cos r - 1, sin r
+    const fxw w = table[idx];
+    const fxc turned = fx_cmul<false>(small, w);
+    const long long tc = static_cast<long long>(w.ch) * 4294967296ll + w.cl, ts = static_cast<long long>(w.sh) * 4294967296ll + w.sl;
+    cs = fx_to_double(tc + turned.x, 1023 - 62);
+    sn = fx_to_double(ts + turned.y, 1023 - 62);
+}
+
+// ---- z ------------------------------------------------------------------------------
+
+// Field spectra u, v, w, eta of one (mode, j) (vinv_field_spectra's formulas with
+// the structure of the factors used: W's and the geostrophic u, v factors are
+// imaginary, and UAp Ap + conj(UAp) Am = Re(UAp) (Ap + Am) + i Im(UAp) (Ap - Am)).
+__device__ __forceinline__ void fx_field_spectra(const DescDev& d, const double* __restrict__ Ap, const double* __restrict__ Am,
+                                                 const double* __restrict__ A0, double elapsed, int w, unsigned char flags, int j,
+                                                 double2 (&f)[4]) {
+    const int idx = j + d.Nj * w;
+    double c, s;
+    fx_phase(d.omega[idx] * elapsed, d.fxPhase, c, s);
+    const zd p0 = zload(Ap + 2 * idx), m0 = zload(Am + 2 * idx), a = zload(A0 + 2 * idx);
+    const zd p = {p0.re * c - p0.im * s, p0.re * s + p0.im * c};
+    const zd m = {m0.re * c + m0.im * s, m0.im * c - m0.re * s};
+    const zd sum = {p.re + m.re, p.im + m.im}, dif = {p.re - m.re, p.im - m.im};
+    const zd uap = zload(d.UAp + 2 * idx), vap = zload(d.VAp + 2 * idx);
+    const double wi = d.WAp[2 * idx + 1], u0 = d.UA0[2 * idx + 1], v0 = d.VA0[2 * idx + 1];
+    const double nap = d.NAp[idx], na0 = d.NA0[idx];
+    f[0] = make_double2(uap.re * sum.re - uap.im * dif.im - u0 * a.im, uap.re * sum.im + uap.im * dif.re + u0 * a.re);
+    f[1] = make_double2(vap.re * sum.re - vap.im * dif.im - v0 * a.im, vap.re * sum.im + vap.im * dif.re + v0 * a.re);
+    f[2] = make_double2(-wi * sum.im, wi * sum.re);
+    f[3] = make_double2(nap * dif.re + na0 * a.re, nap * dif.im + na0 * a.im);
+    if (flags & 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) f[q].y = -f[q].y;
+    }
+    if (flags & 2) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) f[q].y = 0.0;
+    }
+}
+
+// Projection of one (mode, j) of the forward transforms: U, V, W, E are the unscaled
+// channel values, sc their normalisation.  One linear map for the flux and the
+// forward transform (projectFluxTargetMode, projectNonhydrostaticMode,
+// projectHydrostaticMode, kernel.cpp:299-431): with the real factors Cu, Cv, Cw
+//   wave = Cu U + Cv V + i Cw W,  a0 = i (k V - l U) vort + E buoy,
+//   b = (E - NA0 a0) ApmN,  cp = wave + b,  cm = wave - b.
+template <bool FLUX>
+__device__ __forceinline__ void fx_project(const DescDev& d, int w, int j, double2 U, double2 V, double2 W, double2 E, double sc,
+                                           double elapsed, double maxSpeed, int applyDamping, const double* __restrict__ Ap,
+                                           const double* __restrict__ Am, const double* __restrict__ A0,
+                                           double* __restrict__ Fp, double* __restrict__ Fm, double* __restrict__ F0) {
+    const int idx = j + d.Nj * w;
+    const double k = d.k[w], l = d.l[w];
+    const double vort = d.A0FromVorticity[idx], buoy = d.A0FromBuoyancy[idx], na0 = d.NA0[idx], apmn = d.ApmN[idx];
+    const double a0r = (l * U.y - k * V.y) * vort + E.x * buoy, a0i = (k * V.x - l * U.x) * vort + E.y * buoy;
+    double cpr, cpi, cmr, cmi;
+    if (w == 0) {
+        const double is = d.inertialScale[j];
+        cpr = is * (U.x + V.y); cpi = is * (U.y - V.x);
+        cmr = cpr; cmi = -cpi;
+    } else {
+        double wr, wi;
+        if (d.hydrostatic) {
+            const double g = -d.ApmD[2 * idx + 1];
+            wr = g * (k * U.x + l * V.x); wi = g * (k * U.y + l * V.y);
+        } else {
+            const double g = d.ApmDScaled[idx], h = (d.Kh[w] / 2.0) * d.apmWPrefactor[j];
+            wr = (d.cosAlpha[w] * U.x + d.sinAlpha[w] * V.x) * g - h * W.y;
+            wi = (d.cosAlpha[w] * U.y + d.sinAlpha[w] * V.y) * g + h * W.x;
+        }
+        const double br = (E.x - na0 * a0r) * apmn, bi = (E.y - na0 * a0i) * apmn;
+        cpr = wr + br; cpi = wi + bi; cmr = wr - br; cmi = wi - bi;
+    }
+    double c, s;
+    fx_phase(d.omega[idx] * elapsed, d.fxPhase, c, s);
+    c *= sc; s *= sc;
+    zd fp{cpr * c + cpi * s, cpi * c - cpr * s};  // cp conj(p)
+    zd fm{cmr * c - cmi * s, cmr * s + cmi * c};  // cm p
+    zd f0{a0r * sc, a0i * sc};
+    if (FLUX && applyDamping) {
+        const double sd = __dmul_rn(maxSpeed, d.damping[idx]);
+        fp = zadd(fp, zscale(zload(Ap + 2 * idx), sd));
+        fm = zadd(fm, zscale(zload(Am + 2 * idx), sd));
+        f0 = zadd(f0, zscale(zload(A0 + 2 * idx), sd));
+    }
+    zstore(Fp + 2 * idx, fp);
+    zstore(Fm + 2 * idx, fm);
+    zstore(F0 + 2 * idx, f0);
+}
+
+constexpr int kFxZWarps = 8;
+// Per line: its buffer and the field spectra [4][N/2] of its mode.
+template <int N>
+inline size_t smem_fx_vinv(int warps) {
+    return static_cast<size_t>(FxW<N>::twiddles) * 16 +
+           static_cast<size_t>(warps) * FxW<N>::lines * (FxW<N>::buffer * 16 + 2 * N * 16);
+}
+template <int N>
+inline size_t smem_fx_vfwd(int warps) {
+    return static_cast<size_t>(FxW<N>::twiddles) * 16 + static_cast<size_t>(warps) * FxW<N>::lines * FxW<N>::buffer * 16;
+}
+
+// k_vinv_fft (wv_vfft.cuh) in fixed point, one retained column per line: the pairs
+// (u | w), (v | eta) and, for the flux, (m w | -m u), (m eta | -m v).  The two channels of a
+// pair keep their own scales (the even and the odd part separate them again), so
+// neither rounds at the other's magnitude.
+template <int N, bool FLUX>
+__global__ void __launch_bounds__(32 * kFxZWarps, 2)
+    k_vinv_fx(DescDev d, const double* __restrict__ Ap, const double* __restrict__ Am, const double* __restrict__ A0,
+              double elapsed, double2* __restrict__ zspec, unsigned long long* __restrict__ maxSpeedBits) {
+    using W = FxW<N>;
+    constexpr int G = W::G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int Nj = d.Nj, P = d.positions;
+    const int lane = threadIdx.x & 31, t = lane % G;
+    const int own = (threadIdx.x >> 5) * W::lines + lane / G, perBlock = (blockDim.x >> 5) * W::lines;
+    const int member = blockIdx.y;
+    if (member > 0) {
+        const long long o = member * d.memberStride;
+        Ap += o; Am += o; A0 += o;
+        zspec += static_cast<size_t>(member) * d.Nz * P;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && maxSpeedBits) maxSpeedBits[member] = 0ull;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(own) * (W::buffer + 2 * N);
+    double2* fld = reinterpret_cast<double2*>(x + W::buffer);  // [4][N/2]
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwZ[i];
+    __syncthreads();
+    const int want = blockIdx.x * perBlock + own;
+    const bool live = want < d.Nkl;
+    const int mode = min(want, d.Nkl - 1);
+    const int w = d.modeWV[mode];
+    const unsigned char flags = d.modeFlags[mode];
+    const double* mz = static_cast<const double*>(d.tMz);
+    const unsigned mtop = static_cast<unsigned>(__double2hiint(mz[Nj - 1]));
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const int j = t + G * i;
+        double2 f[4];
+        if (j < Nj) fx_field_spectra(d, Ap, Am, A0, elapsed, w, flags, j, f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) fld[q * (N / 2) + j] = j < Nj ? f[q] : make_double2(0.0, 0.0);
+    }
+    int derivChan[4] = {-1, -1, -1, -1};
+    if constexpr (FLUX)
+        for (int q = 0; q < d.nt; ++q) derivChan[d.tq[q]] = 4 + q;
+    const int pos = d.modePos[mode], cpos = d.modeCompPos[mode];
+    auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
+    constexpr int kLines = FLUX ? 4 : 2;
+#pragma unroll 1
+    for (int l = 0; l < kLines; ++l) {
+        // fld slots of the cosine and sine channels: (0|2) (1|3) (2|0) (3|1)
+        const int qc = l < 2 ? l : l, qs = l < 2 ? l + 2 : l - 2;
+        const int chC = l < 2 ? l : derivChan[l], chS = l < 2 ? l + 2 : derivChan[l - 2];
+        double2 a[4];
+        double wgt[4];
+        fxc C[4], D[4];
+        int uC, uD;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = fld[qc * (N / 2) + t + G * i];
+        if (l < 2) {
+            fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, C, uC);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) wgt[i] = t + G * i < Nj ? mz[t + G * i] : 0.0;
+            fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, C, uC);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = fld[qs * (N / 2) + t + G * i];
+        if (l < 2) {
+            fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, D, uD);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) wgt[i] = -wgt[i];
+            fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, D, uD);
+        }
+        // 2 y[j] = C_j + i D_j, 2 y[N-j] = C_j - i D_j, 2 y[0] = C_0
+        fxc v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = t + G * i;
+            if (j == 0) D[i] = fxc{0, 0};
+            v[i] = fxc{C[i].x - D[i].y, C[i].y + D[i].x};
+            x[fx_pad(j == 0 ? N / 2 : N - j)] = j == 0 ? fxc{0, 0} : fxc{C[i].x + D[i].y, C[i].y - D[i].x};
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+        __syncwarp();
+        fx_fft_warp<N, false>(v, x, tw, t);
+#pragma unroll
+        for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+        __syncwarp();
+        // even part -> cosine channel, odd part -> sine channel, n = 0 .. N / 2
+        auto put = [&](int n, fxc a1, fxc b1) {
+            const double2 ev = make_double2(fx_to_double(a1.x + b1.x, uC - 2), fx_to_double(a1.y + b1.y, uC - 2));
+            const double2 od = make_double2(fx_to_double(a1.x - b1.x, uD - 2), fx_to_double(a1.y - b1.y, uD - 2));
+            if (!live) return;
+            if (chC >= 0) {
+                double2* base = zspec + (static_cast<size_t>(chC) * d.zTotal + n) * P;
+                base[pos] = ev;
+                if (cpos >= 0) base[cpos] = make_double2(ev.x, -ev.y);
+            }
+            if (chS >= 0) {
+                double2* base = zspec + (static_cast<size_t>(chS) * d.zTotal + n) * P;
+                base[pos] = od;
+                if (cpos >= 0) base[cpos] = make_double2(od.x, -od.y);
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int n = t + G * i;
+            put(n, v[i], n == 0 ? v[0] : x[fx_pad(N - n)]);
+        }
+        if (t == 0) put(N / 2, v[4], v[4]);
+        __syncwarp();
+    }
+}
+
+// k_vfwd_fft in fixed point, one retained column per line: (u | w), then (v | eta);
+// lane t projects the coefficients j = t + G i it holds.
+template <int N, bool FLUX>
+__global__ void __launch_bounds__(32 * kFxZWarps, 2)
+    k_vfwd_fx(DescDev d, const double2* __restrict__ fspec, int nch, double elapsed, const double* __restrict__ Ap,
+              const double* __restrict__ Am, const double* __restrict__ A0, const unsigned long long* __restrict__ maxSpeedBits,
+              int applyDamping, double* __restrict__ Fp, double* __restrict__ Fm, double* __restrict__ F0) {
+    using W = FxW<N>;
+    constexpr int G = W::G, L = N / 2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int Nj = d.Nj, P = d.positions;
+    const int lane = threadIdx.x & 31, t = lane % G;
+    const int own = (threadIdx.x >> 5) * W::lines + lane / G, perBlock = (blockDim.x >> 5) * W::lines;
+    const int member = blockIdx.y;
+    if (member > 0) {
+        const long long o = member * d.memberStride;
+        if (Ap) { Ap += o; Am += o; A0 += o; }
+        Fp += o; Fm += o; F0 += o;
+        fspec += static_cast<size_t>(member) * d.Nz * P;
+        if (maxSpeedBits) maxSpeedBits += member;
+    }
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(own) * W::buffer;
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwZ[i];
+    __syncthreads();
+    const int want = blockIdx.x * perBlock + own;
+    const bool live = want < d.Nkl;
+    const int mode = min(want, d.Nkl - 1);
+    const int w = d.modeWV[mode];
+    const bool conj = d.modeFlags[mode] & 1;
+    const int pos = d.modePos[mode];
+    int chanOfQ[4] = {-1, -1, -1, -1};
+    for (int c = 0; c < nch; ++c) chanOfQ[FLUX ? d.tq[c] : ((d.hydrostatic && c == 2) ? 3 : c)] = c;
+    // X[q][i]: slots 0 u, 1 v (cosine), 2 w, 3 eta (sine) of j = t + G i
+    double2 X[4][4];
+    const double sc = 1.0 / (static_cast<double>(L) * static_cast<double>(d.Nx) * static_cast<double>(d.Ny));
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const int cc = chanOfQ[l], cs = chanOfQ[2 + l];
+        const double2* hc = fspec + static_cast<size_t>(cc) * d.zTotal * P + pos;
+        const double2* hs = fspec + static_cast<size_t>(cs) * d.zTotal * P + pos;
+        double2 a[5], b[4];
+        double none5[5], none4[4];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const int zz = t + G * i;
+            a[i] = cc >= 0 && (i < 4 || t == 0) ? hc[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
+            if (i < 4) b[i] = cs >= 0 && zz != 0 ? hs[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
+        }
+        fxc C[5], S[4];
+        int uC, uS;
+        fx_quantise_lane<5, G, kFxPlain>(a, none5, 0u, 1, [&](int i) { return (i == 0 && t == 0) || i == 4 ? 1.0f : 2.0f; }, C, uC);
+        fx_quantise_lane<4, G, kFxPlain>(b, none4, 0u, 1, [&](int) { return 2.0f; }, S, uS);
+        // y[0] = c_0, y[L] = c_L, y[z] = c_z + s_z, y[N-z] = c_z - s_z
+        fxc v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int zz = t + G * i;
+            v[i] = fx_add(C[i], S[i]);
+            x[fx_pad(zz == 0 ? L : N - zz)] = zz == 0 ? C[4] : fx_sub(C[i], S[i]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+        __syncwarp();
+        fx_fft_warp<N, false>(v, x, tw, t);
+#pragma unroll
+        for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = t + G * i;
+            const fxc p = v[i], q = j == 0 ? v[0] : x[fx_pad(N - j)];
+            X[l][i] = make_double2(fx_to_double(p.x + q.x, uC - 1), fx_to_double(p.y + q.y, uC - 1));
+            // i times the odd part
+            X[2 + l][i] = make_double2(-fx_to_double(p.y - q.y, uS - 1), fx_to_double(p.x - q.x, uS - 1));
+        }
+        __syncwarp();
+    }
+    if (!live) return;
+    double maxSpeed = 0.0;
+    if (FLUX && applyDamping) maxSpeed = __longlong_as_double((long long)*maxSpeedBits);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int j = t + G * i;
+        if (j >= Nj) continue;
+        double2 U = X[0][i], V = X[1][i], Wv = X[2][i], E = X[3][i];
+        if (conj) { U.y = -U.y; V.y = -V.y; Wv.y = -Wv.y; E.y = -E.y; }
+        fx_project<FLUX>(d, w, j, U, V, Wv, E, sc, elapsed, maxSpeed, applyDamping, Ap, Am, A0, Fp, Fm, F0);
+    }
+}
+
+}  // namespace dev
+}  // namespace wvgpu

@@ -12,6 +12,9 @@ namespace wvgpu {
 // Cap of the grid-stride element-wise launches: perSm blocks per SM of the
 // current device (its multiprocessor count, queried once per device).
 size_t grid_cap(size_t perSm);
+// Raises a kernel's dynamic shared-memory cap to `bytes` (never lowers it: the cap
+// belongs to the process, not to a handle).
+cudaError_t raise_smem_limit(const void* kernel, int bytes);
 
 const Descriptor& handle_descriptor(const wv_handle* h);
 int handle_device(const wv_handle* h);

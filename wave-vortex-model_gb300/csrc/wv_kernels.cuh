@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "wv_ff.cuh"
+#include "wv_fx.cuh"
 
 namespace wvgpu {
 namespace dev {
@@ -196,6 +197,8 @@ __device__ void fft_stage(const cx<T>* __restrict__ src, cx<T>* __restrict__ dst
 // Runs all stages; returns the buffer holding the result (a or b).
 template <typename T, bool INV>
 __device__ cx<T>* fft_lines(cx<T>* a, cx<T>* b, const FFTDev& f, int lines, int ld, const cx<T>* tw) {
+    if constexpr (std::is_same<T, double>::value)  // FP64 lines run in fixed point; tw holds fxw entries
+        return fx_fft_lines<INV>(a, b, FxFactors{f.N, f.nstages, f.radix}, lines, ld, reinterpret_cast<const fxw*>(tw));
     int Ns = 1;
     for (int s = 0; s < f.nstages; ++s) {
         fft_stage<T, INV>(a, b, f.N, f.radix[s], Ns, lines, ld, tw);
@@ -317,6 +320,11 @@ struct DescDev {
     FFTDev fz;              // 2 (Nz - 1): vertical transforms as FFTs (N = 0: not available)
     const void* twz;        // cx<T>[2 (Nz - 1)]
     const void* tMz;        // T[Nj]: m_j in the working type
+    // FP64 handles: stage twiddles of the lane-held y and z lines (null: none) and
+    // exp(2 pi i k / 256) of the phases, in Q62
+    const fxw* fxTwY;
+    const fxw* fxTwZ;
+    const fxw* fxPhase;
 };
 
 // Row wavenumbers in the working type T of the xy stage.
@@ -1240,7 +1248,7 @@ __global__ void __launch_bounds__(256, VertOcc<T>::value) k_vfwd(DescDev d, cons
 // (PortableRuntime/src/WVRungeKutta.cpp:140-176).
 
 // acc = acc + scale * inc ; stage = base + cs * inc   (both from the same k)
-__global__ void k_accumulate_and_stage(double* __restrict__ acc, const double* __restrict__ inc, double scale,
+static __global__ void k_accumulate_and_stage(double* __restrict__ acc, const double* __restrict__ inc, double scale,
                                        const double* __restrict__ base, double cs, double* __restrict__ stage, int first, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double k = inc[i];
@@ -1252,7 +1260,7 @@ __global__ void k_accumulate_and_stage(double* __restrict__ acc, const double* _
 // The step's end: out = base + scale * (acc + k), with the arithmetic of
 // k_accumulate_and_stage at weight 1 followed by base + scale * acc, in one
 // pass (the final weighted sum is consumed here and not stored).
-__global__ void k_rk4_finish(const double* __restrict__ acc, const double* __restrict__ inc, const double* base, double scale,
+static __global__ void k_rk4_finish(const double* __restrict__ acc, const double* __restrict__ inc, const double* base, double scale,
                              double* out, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double a = __dadd_rn(acc[i], __dmul_rn(1.0, inc[i]));
@@ -1266,7 +1274,7 @@ __global__ void k_rk4_finish(const double* __restrict__ acc, const double* __res
 namespace wvgpu {
 namespace dev {
 // out = a*x + b*y (y may be null); n doubles
-__global__ void k_lincomb(double* __restrict__ out, double a, const double* __restrict__ x, double b,
+static __global__ void k_lincomb(double* __restrict__ out, double a, const double* __restrict__ x, double b,
                           const double* __restrict__ y, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = y ? __fma_rn(a, x[i], __dmul_rn(b, y[i])) : __dmul_rn(a, x[i]);
@@ -1274,7 +1282,7 @@ __global__ void k_lincomb(double* __restrict__ out, double a, const double* __re
 // One stage of the RK4 backward sweep after a flux VJP s: the step's
 // cotangent acc = x + s (first stage) or acc += s, and the next stage's flux
 // cotangent kb = a x + b s, with k_lincomb's rounding.
-__global__ void k_adj_stage(double* __restrict__ acc, bool first, double* __restrict__ kb, double a,
+static __global__ void k_adj_stage(double* __restrict__ acc, bool first, double* __restrict__ kb, double a,
                             const double* __restrict__ x, double b, const double* __restrict__ s, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double xi = x[i], si = s[i];
@@ -1283,13 +1291,13 @@ __global__ void k_adj_stage(double* __restrict__ acc, bool first, double* __rest
     }
 }
 // out += x
-__global__ void k_accumulate(double* __restrict__ out, const double* __restrict__ x, size_t n) {
+static __global__ void k_accumulate(double* __restrict__ out, const double* __restrict__ x, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] += x[i];
 }
 // RK4 dense output: out = iw y0 + ew y1 + isw k1 + esw k4, summed left to right
 // without contraction (WVFixedStepRK4::evaluateDenseOutput); grid.y = component.
-__global__ void k_rk4_dense(const double* __restrict__ y0, const double* __restrict__ y1, const double* __restrict__ k1,
+static __global__ void k_rk4_dense(const double* __restrict__ y0, const double* __restrict__ y1, const double* __restrict__ k1,
                             const double* __restrict__ k4, double iw, double ew, double isw, double esw, double* Ap,
                             double* Am, double* A0, size_t M2) {
     const int c = blockIdx.y;

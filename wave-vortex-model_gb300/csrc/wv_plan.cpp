@@ -49,6 +49,69 @@ FFTFactors factor_fft(int N) {
     return f;
 }
 
+FFTFactors factor_fixed_point(int N) {
+    FFTFactors f;
+    f.N = N;
+    int n = N, twos = 0;
+    auto push = [&](int r) { if (f.nstages < kMaxStages) f.radix[f.nstages++] = r; };
+    while (n % 2 == 0) { ++twos; n /= 2; }
+    while (twos >= 3 && twos != 4) { push(8); twos -= 3; }  // 4 twos: 4 x 4 rather than 8 x 2
+    while (twos >= 2) { push(4); twos -= 2; }
+    if (twos) push(2);
+    for (int p = 3; n > 1; p += 2) {
+        while (n % p == 0) { push(p); n /= p; }
+        if (p * p > n && n > 1) { push(n); n = 1; }
+    }
+    return f;
+}
+
+std::vector<int32_t> fixed_point_twiddles(int N) {
+    // the angle is reduced to the first octant in integers; long double carries
+    // at least 64 bits on both host architectures
+    const long double pi = 3.141592653589793238462643383279502884L;
+    auto q62 = [](long double v) { return std::llroundl(v * 4611686018427387904.0L); };
+    auto cosQ = [&](long long k) {  // cos(2 pi k / N)
+        k %= N;
+        if (2 * k > N) k = N - k;
+        const bool neg = 4 * k > N;
+        const long long a = neg ? N - 2 * k : 2 * k;  // angle pi a / N in [0, pi/2]
+        const long double v = 4 * a <= N ? std::cos(pi * a / N) : std::sin(pi * (N - 2 * a) / (2.0L * N));
+        return neg ? -q62(v) : q62(v);
+    };
+    auto sinQ = [&](long long k) {  // sin(2 pi k / N)
+        k %= N;
+        const bool neg = 2 * k > N;
+        if (neg) k = N - k;
+        long long a = 2 * k;  // angle pi a / N in [0, pi]
+        if (2 * a > N) a = N - a;
+        const long double v = 4 * a <= N ? std::sin(pi * a / N) : std::cos(pi * (N - 2 * a) / (2.0L * N));
+        return neg ? -q62(v) : q62(v);
+    };
+    std::vector<int32_t> out;
+    auto put = [&](long long q) {
+        out.push_back(static_cast<int32_t>((q + 0x80000000ll) >> 32));
+        out.push_back(static_cast<int32_t>(static_cast<uint32_t>(q)));
+    };
+    for (int k = 0; k < N; ++k) { put(cosQ(k)); put(-sinQ(k)); }
+    return out;
+}
+
+std::vector<int32_t> fixed_point_stage_twiddles(int N, std::initializer_list<int> radices) {
+    const std::vector<int32_t> all = fixed_point_twiddles(N);
+    std::vector<int32_t> out;
+    int Ns = 1;
+    for (const int R : radices) {
+        if (Ns > 1)
+            for (int r = 1; r < R; ++r)
+                for (int k = 0; k < Ns; ++k) {
+                    const int i = r * k * (N / (Ns * R));
+                    out.insert(out.end(), all.begin() + 4 * i, all.begin() + 4 * i + 4);
+                }
+        Ns *= R;
+    }
+    return out;
+}
+
 Status build_plan(const Descriptor& d, Plan& p) {
     const auto& c = d.c;
     p = Plan{};
