@@ -44,6 +44,18 @@ WV_HD int fx_lo(long long x) { return static_cast<int>(static_cast<unsigned>(x))
 WV_HD int fx_hi(long long x) {
     return static_cast<int>(x >> 32) + static_cast<int>(static_cast<unsigned>(x) >> 31);
 }
+// a b + c in one instruction (written out: the compiler otherwise splits most of the
+// sums below into products and 64-bit additions, 55 instructions for a complex
+// product instead of 26)
+WV_HD long long fx_mad(int a, int b, long long c) {
+#ifdef __CUDA_ARCH__
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+#else
+    return c + static_cast<long long>(a) * b;
+#endif
+}
 constexpr long long kFxHalf = 1ll << 29;
 
 // x w (INV: x conj w), |x| < 2^61 (1 - 2^-9).  Twelve 32 x 32 -> 64 products: the
@@ -52,25 +64,46 @@ constexpr long long kFxHalf = 1ll << 29;
 template <bool INV>
 WV_HD fxc fx_cmul(fxc a, fxw w) {
     const int xh = fx_hi(a.x), xl = fx_lo(a.x), yh = fx_hi(a.y), yl = fx_lo(a.y);
-    const int sh = INV ? -w.sh : w.sh, sl = INV ? -w.sl : w.sl;
-    long long mr = kFxHalf, mi = kFxHalf;
-    mr += static_cast<long long>(xh) * w.cl; mr += static_cast<long long>(xl) * w.ch;
-    mr += static_cast<long long>(-yh) * sl;  mr += static_cast<long long>(yl) * -sh;
-    mi += static_cast<long long>(xh) * sl;   mi += static_cast<long long>(xl) * sh;
-    mi += static_cast<long long>(yh) * w.cl; mi += static_cast<long long>(yl) * w.ch;
+    const int nh = -w.sh, nl = -w.sl;
+    const int sh = INV ? nh : w.sh, sl = INV ? nl : w.sl, mh = INV ? w.sh : nh, ml = INV ? w.sl : nl;
+    long long r = fx_mad(xh, w.cl, kFxHalf), i = fx_mad(xh, sl, kFxHalf);
+    r = fx_mad(xl, w.ch, r); i = fx_mad(xl, sh, i);
+    r = fx_mad(yh, ml, r);   i = fx_mad(yh, w.cl, i);
+    r = fx_mad(yl, mh, r);   i = fx_mad(yl, w.ch, i);
+    r >>= 30; i >>= 30;
     const int xh4 = xh * 4, yh4 = yh * 4;
-    fxc r;
-    r.x = (mr >> 30) + static_cast<long long>(xh4) * w.ch + static_cast<long long>(yh4) * -sh;
-    r.y = (mi >> 30) + static_cast<long long>(xh4) * sh + static_cast<long long>(yh4) * w.ch;
+    r = fx_mad(xh4, w.ch, r); i = fx_mad(xh4, sh, i);
+    r = fx_mad(yh4, mh, r);   i = fx_mad(yh4, w.ch, i);
+    return fxc{r, i};
+}
+#ifdef __CUDACC__
+// x w for |x| < 2^60 (1 - 2^-9): the middle terms as four high halves (32-bit sums;
+// each cuts its last bit, `two` gives the mean back), 25 instructions against 37.
+// two: the value 2 in a register the compiler cannot rebuild (fx_two); 0 on all-zero
+// lines, which stay exactly zero.
+template <bool INV>
+__device__ __forceinline__ fxc fx_cmul60(fxc a, fxw w, int two) {
+    const long long x4 = a.x << 2, y4 = a.y << 2;
+    const int xl = fx_lo(x4), yl = fx_lo(y4), xh = fx_hi(x4), yh = fx_hi(y4);
+    const int nh = -w.sh, nl = -w.sl;
+    const int sh = INV ? nh : w.sh, sl = INV ? nl : w.sl, mh = INV ? w.sh : nh, ml = INV ? w.sl : nl;
+    auto mad = [](int p, int q, int c) { int r; asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(p), "r"(q), "r"(c)); return r; };
+    auto mul = [](int p, int q) { long long r; asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(p), "r"(q)); return r; };
+    const int m = mad(xh, w.cl, mad(xl, w.ch, mad(yh, ml, mad(yl, mh, two))));
+    const int n = mad(xh, sl, mad(xl, sh, mad(yh, w.cl, mad(yl, w.ch, two))));
+    return fxc{mul(xh, w.ch) + mul(yh, mh) + static_cast<long long>(m), mul(xh, sh) + mul(yh, w.ch) + static_cast<long long>(n)};
+}
+__device__ __forceinline__ int fx_two() {
+    int r;
+    asm volatile("mov.u32 %0, 2;" : "=r"(r));
     return r;
 }
+#endif
 // x c for a real Q62 constant (h, l)
 WV_HD long long fx_rmul(long long x, int ch, int cl) {
-    const int xh = fx_hi(x), xl = fx_lo(x);
-    long long m = kFxHalf;
-    m += static_cast<long long>(xh) * cl;
-    m += static_cast<long long>(xl) * ch;
-    return (m >> 30) + static_cast<long long>(xh * 4) * ch;
+    const int xh = fx_hi(x);
+    const long long m = fx_mad(fx_lo(x), ch, fx_mad(xh, cl, kFxHalf)) >> 30;
+    return fx_mad(xh * 4, ch, m);
 }
 // high and low words of a Q62 constant
 WV_HD constexpr int fx_qh(long long q) { return static_cast<int>((q + 0x80000000ll) >> 32); }
@@ -191,9 +224,10 @@ WV_HD float fx_modulus(float a, float b) { return (a > b ? a : b) + 0.41422f * (
 
 // |v| as a float from the high word of v: 0 below 2^-126, inf from 2^128 on
 WV_HD float fx_mag(unsigned hi) {
-    int r = static_cast<int>(hi & 0x7fffffffu) - (896 << 20);
-    r = r < 0 ? 0 : r > (255 << 20) ? (255 << 20) : r;
-    return fx_float(static_cast<unsigned>(r) << 3);
+    unsigned a = hi & 0x7fffffffu;
+    a = a < (896u << 20) ? (896u << 20) : a;
+    a = a > (1151u << 20) ? (1151u << 20) : a;
+    return fx_float(a * 8u - (896u << 23));
 }
 // Whether a sum of fx_mag moduli gives a line's scale by itself; lines outside (all
 // zero, tiny, huge or non-finite) take their scale from their largest entry.
@@ -209,28 +243,34 @@ WV_HD fxscale fx_scale(unsigned top, float l1) {
     const float s = l1 * 1.0025f;
     int el = static_cast<int>(fx_float_bits(s) >> 23) - 126;  // s < 2^el
     if (el < -40) el = -40;                                   // (weighted rows of one dominant, weightless entry)
-    return {static_cast<int>(top >> 20), 61 - el};
+    const int e0 = static_cast<int>(top >> 20);
+    return {e0 < 200 ? 200 : e0, 61 - el};
 }
 // the same from a sum of fx_mag moduli
 WV_HD fxscale fx_scale(float l1) {
     const int el = static_cast<int>(fx_float_bits(l1 * 1.0025f) >> 23) - 126;
     return {1023, 61 - el};
 }
+// m (2^e at bit 62) shifted right by rs + 1 with the last bit rounded (up), negated
+// if asked
+WV_HD long long fx_shift_in(unsigned long long m, int rs, int sign) {
+    const long long s = sign >> 31;  // 0 or -1
+    return ((static_cast<long long>(m >> (rs > 63 ? 63 : rs)) ^ s) + (1 - s)) >> 1;
+}
+// (zeros and denormals leave through the shift: fx_scale keeps e0 far above them)
 WV_HD long long fx_from_double(double v, fxscale sc) {
     unsigned hi, lo;
     fx_words(v, hi, lo);
     const int e = static_cast<int>((hi >> 20) & 0x7ffu);
-    unsigned long long m = (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;  // 2^e at bit 62
-    int rs = 61 - sc.bit + sc.e0 - e;  // one less than the full shift: the last bit rounds
-    if (rs > 63) rs = 63;              // (rs = 63 leaves 0)
-    if (e == 0) rs = 63;
-    m = ((m >> rs) + 1) >> 1;
-    const long long x = static_cast<long long>(m);
-    return static_cast<int>(hi) < 0 ? -x : x;
+    const unsigned long long m = (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;  // 2^e at bit 62
+    return fx_shift_in(m, 61 - sc.bit + sc.e0 - e, static_cast<int>(hi));
 }
 // Exponent of the unit (biased): real value = integer * 2^(unit - 1023).
 // kFxBad marks a line that held a non-finite value.
 constexpr int kFxBad = 1 << 28;
+// unit of an all-zero line (fx_silent); units derived from it stay below half of it
+constexpr int kFxZero = -(1 << 24);
+WV_HD bool fx_silent(int unit) { return unit < kFxZero / 2; }
 WV_HD int fx_unit(fxscale sc) { return sc.e0 >= 0x7ff ? kFxBad : sc.e0 - sc.bit; }
 WV_HD int fx_clz(unsigned long long v) {
 #ifdef __CUDA_ARCH__
@@ -241,19 +281,56 @@ WV_HD int fx_clz(unsigned long long v) {
 }
 // integer * 2^(unit - 1023) rounded to the nearest double (0 below the normal range, inf above)
 WV_HD double fx_to_double(long long x, int unit) {
-    const unsigned long long sign = static_cast<unsigned long long>(x) & 0x8000000000000000ull;
-    unsigned long long m = static_cast<unsigned long long>(x < 0 ? -x : x);
-    const int lz = fx_clz(m);
-    const int e = unit + 62 - lz;  // exponent field of the leading bit, less one (the hidden bit adds it)
-    m <<= (lz & 63);
-    const unsigned long long r = (m >> 11) + ((m >> 10) & 1ull);
-    unsigned long long bits = r + (static_cast<unsigned long long>(static_cast<unsigned>(e)) << 52);
-    if (x == 0 || e < 0) bits = 0;
-    if (e >= 0x7fe) bits = unit >= kFxBad / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull;
-    return fx_double(bits | sign);
+    const long long s = x >> 63;
+    const unsigned long long a = static_cast<unsigned long long>((x ^ s) - s);
+    unsigned h = static_cast<unsigned>(a >> 32), l = static_cast<unsigned>(a);
+    const bool low = h == 0;  // the leading bit is in the low word
+    if (low) { h = l; l = 0; }
+#ifdef __CUDA_ARCH__
+    const int lz = __clz(static_cast<int>(h));
+#else
+    const int lz = h ? __builtin_clz(h) : 32;
+#endif
+    // leading bit to bit 62, half a unit of the 53 bits added, cut; the hidden bit
+    // and a carry past it add to the exponent field
+    unsigned long long m = (static_cast<unsigned long long>(h) << 32 | l) >> 1;
+    m <<= (lz & 31);
+    m = (m + 512) >> 10;
+    const int e = unit + (low ? 30 : 62) - lz;
+    unsigned long long bits = m + (static_cast<unsigned long long>(static_cast<unsigned>(e)) << 52);
+    if (e < 0 || h == 0) bits = 0;
+    if (e >= 0x7fe && h != 0) bits = unit >= kFxBad / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull;
+    if (unit >= kFxBad / 2) bits = 0x7ff8000000000000ull;
+    return fx_double(bits | (static_cast<unsigned long long>(x) & 0x8000000000000000ull));
 }
 
 #ifdef __CUDACC__
+// fx_to_double for a line's unit taken apart once: values of lines in the middle of
+// the exponent range need no checks of their own.  Magnitudes are one's complements
+// (one unit low below zero), rounded to 53 bits.
+struct FxUnit {
+    int unit;
+    unsigned keep, set;  // masks of the high word: 0 flushes the line, set makes it NaN
+};
+__device__ __forceinline__ FxUnit fx_out(int unit) {
+    const bool huge = unit > 1900, tiny = unit < 70;
+    return FxUnit{huge || tiny ? 1000 : unit, tiny ? 0u : 0xffffffffu, huge ? 0x7ff80000u : 0u};
+}
+__device__ __forceinline__ double fx_to_double(long long x, FxUnit o) {
+    unsigned lo = static_cast<unsigned>(x), hi = static_cast<unsigned>(static_cast<unsigned long long>(x) >> 32);
+    const unsigned s = static_cast<unsigned>(static_cast<int>(hi) >> 31);
+    lo ^= s;
+    hi ^= s;
+    int base = o.unit + 62;
+    if (hi == 0) { hi = lo; lo = 0; base -= 32; }
+    const int lz = __clz(static_cast<int>(hi));
+    const unsigned th = __funnelshift_l(lo, hi, lz), tl = lo << (lz & 31);
+    const unsigned long long m = (((static_cast<unsigned long long>(th) << 32 | tl) >> 1) + 512) >> 10;
+    unsigned h = static_cast<unsigned>(m >> 32) + (static_cast<unsigned>(base - lz) << 20);
+    if (hi == 0) h = 0;
+    h = ((h & o.keep) | (s & 0x80000000u)) | o.set;
+    return __hiloint2double(static_cast<int>(h), static_cast<int>(m));
+}
 // One stage over `lines` lines (as fft_stage): radix R from src to dst.
 template <int R, bool INV>
 __device__ __forceinline__ void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int Ns, int lines,

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
             double2* o = reinterpret_cast<double2*>(r + l * ld);
             for (int i = lane; i < Ny; i += 32) {
                 const fxc v = r[l * ld + i];
-                o[i] = make_double2(fx_to_double(v.x, u), fx_to_double(v.y, u));
+                o[i] = make_double2(fx_to_double(v.x, fx_out(u)), fx_to_double(v.y, fx_out(u)));
             }
         }
     }
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         for (int i = lane; i < Ny; i += 32) {
             const int pos = ym[i];
             const fxc v = r[l * ld + i];
-            if (pos >= 0) out[pos] = make_double2(fx_to_double(v.x, u), fx_to_double(v.y, u));
+            if (pos >= 0) out[pos] = make_double2(fx_to_double(v.x, fx_out(u)), fx_to_double(v.y, fx_out(u)));
         }
     }
 }
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
             const int u = __shfl_sync(0xffffffffu, units, c);
             double* o = fields + static_cast<size_t>(c) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
             const fxc* s = r + (c >> 1) * Nx;
-            for (int x = lane; x < Nx; x += 32) o[x] = fx_to_double((c & 1) ? s[x].y : s[x].x, u);
+            for (int x = lane; x < Nx; x += 32) o[x] = fx_to_double((c & 1) ? s[x].y : s[x].x, fx_out(u));
         }
         __syncwarp();
     }
@@ -258,9 +258,9 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
             double2* o = pspec + ((static_cast<size_t>(z) * nch + 2 * l) * Ny + y) * KX;
             for (int k = lane; k < KX; k += 32) {
                 const fxc a = r[l * Nx + k], b = r[l * Nx + (k == 0 ? 0 : Nx - k)];
-                o[k] = make_double2(fx_to_double(a.x + b.x, ua), fx_to_double(a.y - b.y, ua));
+                o[k] = make_double2(fx_to_double(a.x + b.x, fx_out(ua)), fx_to_double(a.y - b.y, fx_out(ua)));
                 if (2 * l + 1 < nch)
-                    o[static_cast<size_t>(Ny) * KX + k] = make_double2(fx_to_double(a.y + b.y, ub), fx_to_double(b.x - a.x, ub));
+                    o[static_cast<size_t>(Ny) * KX + k] = make_double2(fx_to_double(a.y + b.y, fx_out(ub)), fx_to_double(b.x - a.x, fx_out(ub)));
             }
         }
         __syncwarp();
@@ -341,13 +341,13 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         for (int n = lane; n <= L; n += 32) {
             const fxc a = row[n], b = row[n == 0 ? 0 : N - n];
             if (chC >= 0) {
-                const double2 ev = make_double2(fx_to_double(a.x + b.x, uC[l] - 2), fx_to_double(a.y + b.y, uC[l] - 2));
+                const double2 ev = make_double2(fx_to_double(a.x + b.x, fx_out(uC[l] - 2)), fx_to_double(a.y + b.y, fx_out(uC[l] - 2)));
                 double2* base = zspec + (static_cast<size_t>(chC) * d.zTotal + n) * P;
                 base[pos] = ev;
                 if (cpos >= 0) base[cpos] = make_double2(ev.x, -ev.y);
             }
             if (chS >= 0) {
-                const double2 od = make_double2(fx_to_double(a.x - b.x, uD[l] - 2), fx_to_double(a.y - b.y, uD[l] - 2));
+                const double2 od = make_double2(fx_to_double(a.x - b.x, fx_out(uD[l] - 2)), fx_to_double(a.y - b.y, fx_out(uD[l] - 2)));
                 double2* base = zspec + (static_cast<size_t>(chS) * d.zTotal + n) * P;
                 base[pos] = od;
                 if (cpos >= 0) base[cpos] = make_double2(od.x, -od.y);
@@ -421,8 +421,8 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
             const fxc p = F[l * N + j], q = F[l * N + (j == 0 ? 0 : N - j)];
-            X[l] = make_double2(fx_to_double(p.x + q.x, uC[l] - 1), fx_to_double(p.y + q.y, uC[l] - 1));
-            X[2 + l] = make_double2(-fx_to_double(p.y - q.y, uS[l] - 1), fx_to_double(p.x - q.x, uS[l] - 1));
+            X[l] = make_double2(fx_to_double(p.x + q.x, fx_out(uC[l] - 1)), fx_to_double(p.y + q.y, fx_out(uC[l] - 1)));
+            X[2 + l] = make_double2(-fx_to_double(p.y - q.y, fx_out(uS[l] - 1)), fx_to_double(p.x - q.x, fx_out(uS[l] - 1)));
         }
         if (conj) {
 #pragma unroll

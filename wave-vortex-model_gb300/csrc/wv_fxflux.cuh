@@ -36,12 +36,12 @@ __device__ __forceinline__ void fx_load_row(const double2* __restrict__ h, int K
     }
     auto count = [&](int i) { const int k = lane + 32 * i; return k == 0 || 2 * k == Nx ? 1.0f : 2.0f; };
     if (useK) {
-        fx_quantise_lane<EK, 32, kFxImag>(v, w, static_cast<unsigned>(__double2hiint(rowK[KX - 1])), 1, count, row, unit);
+        fx_quantise_lane<EK, 32, kFxImag, 0>(v, w, static_cast<unsigned>(__double2hiint(rowK[KX - 1])), 1, count, row, unit);
 #pragma unroll
         for (int i = 0; i < EK; ++i)
             if (2 * (lane + 32 * i) == Nx) row[i].y = 0;
     } else {
-        fx_quantise_lane<EK, 32, kFxPlain>(v, w, 0u, 1, count, row, unit);
+        fx_quantise_lane<EK, 32, kFxPlain, 0>(v, w, 0u, 1, count, row, unit);
     }
 }
 
@@ -229,11 +229,12 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                 const int t = t0 + 2 * i;
                 const int ua = __shfl_sync(0xffffffffu, units, 2 * i), ub = __shfl_sync(0xffffffffu, units, 2 * i + 1);
                 double2* out = pspec + ((static_cast<size_t>(z) * nt + t) * Ny + y) * KX;
+                const FxUnit oa = fx_out(ua), ob = fx_out(ub);
                 for (int k = lane; k < KX; k += 32) {
                     const fxc a = res[i * Nx + k], b = res[i * Nx + (k == 0 ? 0 : Nx - k)];
-                    out[k] = make_double2(fx_to_double(a.x + b.x, ua), fx_to_double(a.y - b.y, ua));
+                    out[k] = make_double2(fx_to_double(a.x + b.x, oa), fx_to_double(a.y - b.y, oa));
                     if (t + 1 < nt)
-                        out[cstride + k] = make_double2(fx_to_double(a.y + b.y, ub), fx_to_double(b.x - a.x, ub));
+                        out[cstride + k] = make_double2(fx_to_double(a.y + b.y, ob), fx_to_double(b.x - a.x, ob));
                 }
             }
             __syncwarp();

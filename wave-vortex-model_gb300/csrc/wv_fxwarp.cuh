@@ -28,7 +28,7 @@ __device__ __forceinline__ int fx_pad(int i) { return i + (i >> 3); }
 
 // Stage of radix R behind Ns points already combined; tw[(r - 1) Ns + k].
 template <int N, int R, int Ns, bool INV>
-__device__ __forceinline__ void fx_wstage(fxc (&v)[8], const fxw* __restrict__ tw, int t) {
+__device__ __forceinline__ void fx_wstage(fxc (&v)[8], const fxw* __restrict__ tw, int t, int two) {
     constexpr int G = N / 8, B = 8 / R;
 #pragma unroll
     for (int b = 0; b < B; ++b) {
@@ -36,7 +36,7 @@ __device__ __forceinline__ void fx_wstage(fxc (&v)[8], const fxw* __restrict__ t
         fxc u[R];
         u[0] = v[b];
 #pragma unroll
-        for (int r = 1; r < R; ++r) u[r] = fx_cmul<INV>(v[b + B * r], tw[(r - 1) * Ns + k]);
+        for (int r = 1; r < R; ++r) u[r] = fx_cmul60<INV>(v[b + B * r], tw[(r - 1) * Ns + k], two);
         fx_dft<R, INV>(u);
 #pragma unroll
         for (int r = 0; r < R; ++r) v[b + B * r] = u[r];
@@ -57,16 +57,16 @@ __device__ __forceinline__ void fx_wexchange(fxc (&v)[8], fxc* __restrict__ x, i
     for (int e = 0; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
     __syncwarp();
 }
-// The whole line; x: this line's buffer, tw: the stage twiddles in shared memory.
+// The whole line (sum of moduli below 2^60); x: this line's buffer, tw: the stage twiddles in shared memory.
 template <int N, bool INV>
-__device__ __forceinline__ void fx_fft_warp(fxc (&v)[8], fxc* __restrict__ x, const fxw* __restrict__ tw, int t) {
+__device__ __forceinline__ void fx_fft_warp(fxc (&v)[8], fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two) {
     using W = FxW<N>;
     fx_dft8<INV>(v);
     fx_wexchange<N, 8, 1>(v, x, t);
-    fx_wstage<N, W::R2, 8, INV>(v, tw, t);
+    fx_wstage<N, W::R2, 8, INV>(v, tw, t, two);
     if constexpr (W::R3 > 1) {
         fx_wexchange<N, W::R2, 8>(v, x, t);
-        fx_wstage<N, W::R3, 8 * W::R2, INV>(v, tw + (W::R2 - 1) * 8, t);
+        fx_wstage<N, W::R3, 8 * W::R2, INV>(v, tw + (W::R2 - 1) * 8, t, two);
     }
 }
 
@@ -92,16 +92,11 @@ __device__ __forceinline__ float fx_group_sum(float v) {
     return v;
 }
 
-// mantissa (2^e at bit 62; 0 below the normal range) and exponent of a double
+// mantissa (2^e at bit 62) and exponent of a double
 __device__ __forceinline__ unsigned long long fx_mantissa(double v, int& e) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
     e = static_cast<int>((hi >> 20) & 0x7ffu);
-    const unsigned long long m = (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
-    return e == 0 ? 0ull : m;
-}
-__device__ __forceinline__ long long fx_align(unsigned long long m, int rs, bool negative) {
-    m = ((m >> min(rs, 63)) + 1) >> 1;
-    return negative ? -static_cast<long long>(m) : static_cast<long long>(m);
+    return (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
 }
 
 // What a line's entries are multiplied by: nothing, real weights w, or i w.
@@ -110,7 +105,7 @@ enum FxWeight { kFxPlain, kFxReal, kFxImag };
 // C doubles of a lane, weighted, in the fixed point of their line.  count(c): how
 // often entry c enters the line's sum of moduli; spare: bits kept free (1 when two
 // rows share the line); wtop: high word of the largest |w|.
-template <int C, int G, FxWeight MODE, typename Count>
+template <int C, int G, FxWeight MODE, int FRAME = 1, typename Count>
 __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const double (&w)[C], unsigned wtop, int spare,
                                                  Count count, fxc (&out)[C], int& unit) {
     float sum = 0.f;
@@ -124,6 +119,7 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
     sum = fx_group_sum<G>(sum);
     fxscale sc = fx_scale(sum);
     int wexp = 0;
+    bool zero = false;
     const bool odd = !fx_plain_sum(sum);
     if (__any_sync(0xffffffffu, odd)) {
         unsigned top = 0;
@@ -142,30 +138,31 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
         }
         rel = fx_group_sum<G>(rel);
         if (odd) {
+            zero = top == 0;
             sc = fx_scale(top, rel);
             if (MODE != kFxPlain) wexp = static_cast<int>((wtop >> 20) & 0x7ffu) - 1023;
         }
     }
-    sc.bit -= spare;
-    unit = sc.e0 >= 0x7ff ? kFxBad : sc.e0 + wexp - sc.bit;
+    sc.bit -= spare + FRAME;
+    unit = zero ? kFxZero : sc.e0 >= 0x7ff ? kFxBad : sc.e0 + wexp - sc.bit;
     const int base = 61 - sc.bit + sc.e0;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         int ex, ey;
         unsigned long long mx = fx_mantissa(v[c].x, ex), my = fx_mantissa(v[c].y, ey);
-        const bool nx = __double2hiint(v[c].x) < 0, ny = __double2hiint(v[c].y) < 0;
+        const int sx = __double2hiint(v[c].x), sy = __double2hiint(v[c].y);
         if constexpr (MODE != kFxPlain) {
             int ew;
             const unsigned long long mw = fx_mantissa(w[c], ew) << 1;
-            const bool nw = __double2hiint(w[c]) < 0;
+            const int sw = __double2hiint(w[c]);
             mx = __umul64hi(mx, mw);  // 2^(e + ew - 1022) at bit 62
             my = __umul64hi(my, mw);
             const int b2 = base + wexp + 1022 - ew;
-            const long long wx = fx_align(mx, b2 - ex, nx != nw), wy = fx_align(my, b2 - ey, ny != nw);
+            const long long wx = fx_shift_in(mx, b2 - ex, sx ^ sw), wy = fx_shift_in(my, b2 - ey, sy ^ sw);
             out[c] = MODE == kFxImag ? fxc{-wy, wx} : fxc{wx, wy};
         } else {
-            out[c].x = fx_align(mx, base - ex, nx);
-            out[c].y = fx_align(my, base - ey, ny);
+            out[c].x = fx_shift_in(mx, base - ex, sx);
+            out[c].y = fx_shift_in(my, base - ey, sy);
         }
     }
 }
@@ -184,11 +181,9 @@ constexpr int kFxXWarps = 15;  // 14.8 KB of shared memory and 32 x 128 register
 
 // (a b) >> 62 rounded, |a| < 2^62, |b| < 2^61
 __device__ __forceinline__ long long fx_prod(long long a, long long b) {
-    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
-    long long m = kFxHalf;
-    m += static_cast<long long>(ah) * bl;
-    m += static_cast<long long>(al) * bh;
-    return (m >> 30) + static_cast<long long>(ah) * (bh * 4);
+    const int ah = fx_hi(a), bh = fx_hi(b);
+    const long long m = fx_mad(fx_lo(a), bh, fx_mad(ah, fx_lo(b), kFxHalf)) >> 30;
+    return fx_mad(ah, bh * 4, m);
 }
 // A velocity normalised to 62 bits (leading bit of the row's largest: 61), cut to
 // the 53 a double holds: the fields that nonlinearFluxWithAdvectionFields returns
@@ -226,6 +221,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
     fxc* x = reinterpret_cast<fxc*>(mine);                         // line buffer
     long long* phys = reinterpret_cast<long long*>(x + W::buffer);  // u, v, w [3][N]
     long long* S = phys + 3 * N;                                    // products of two targets [2][N]
+    const int two = fx_two();
     const double* rowK = row_k<double>(d);
     const size_t cstride = static_cast<size_t>(Ny) * KX;
     const size_t R3 = static_cast<size_t>(N) * Ny * d.Nz;
@@ -236,13 +232,13 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
         const int row = min(first + line, rows - 1);
         const int z = row / Ny, y = row - z * Ny;
         const double2* yrow = yspec + (static_cast<size_t>(z) * nIn * Ny + y) * KX;
-        int physUnit[3] = {0, 0, 0}, sUnit[2] = {0, 0}, unitNow = 0;
+        int physUnit[3] = {0, 0, 0}, sUnit[2] = {0, 0}, unitNow = 0;  // (as fx_unit)
         long long acc[8];  // products of the current target
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[e] = 0;
         for (int p = 0; 2 * p < nReal; ++p) {
             fxc v[8];
-            int unit[2] = {0, 0};
+            int unit[2] = {kFxZero, kFxZero};
             {
                 // rows 2p and 2p + 1: spectrum entries k = t + G i, both rows' loads in flight
                 double2 raw[2][EK];
@@ -302,7 +298,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
                 for (int e = 8 - EK; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
                 __syncwarp();
             }
-            fx_fft_warp<N, true>(v, x, tw, t);
+            fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
             // samples x = t + G e: real part row 2p, imaginary part row 2p + 1
 #pragma unroll 1
             for (int q = 0; q < 2; ++q) {
@@ -395,7 +391,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
 #pragma unroll
                         for (int e = 0; e < 8; ++e) sum += (fx_abs_hi(S[q * N + t + G * e]) >> 9) + 1u;
                     sum = fx_group_add<G>(sum);
-                    sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 60;  // sum |S| < 2^60 after the shift
+                    sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 59;  // sum |S| < 2^59 after the shift
                     u[q] = sUnit[q] + sh[q] - 1;                            // the halves of the split below
                 }
 #pragma unroll
@@ -404,19 +400,20 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
                     v[e].x = sh[0] >= 0 ? a >> sh[0] : a << -sh[0];
                     v[e].y = sh[1] >= 0 ? b >> sh[1] : b << -sh[1];
                 }
-                fx_fft_warp<N, false>(v, x, tw, t);
+                fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(sUnit[0], both ? sUnit[1] : sUnit[0])) ? 0 : two);
                 __syncwarp();
 #pragma unroll
                 for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
                 __syncwarp();
                 double2* out = pspec + ((static_cast<size_t>(z) * nt + t0) * Ny + y) * KX;
+                const FxUnit o0 = fx_out(u[0]), o1 = fx_out(u[1]);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int k = t + G * i;
                     const fxc a = v[i], b = k == 0 ? v[0] : x[fx_pad(N - k)];
                     if (k < KX && live) {
-                        out[k] = make_double2(fx_to_double(a.x + b.x, u[0]), fx_to_double(a.y - b.y, u[0]));
-                        if (both) out[cstride + k] = make_double2(fx_to_double(a.y + b.y, u[1]), fx_to_double(b.x - a.x, u[1]));
+                        out[k] = make_double2(fx_to_double(a.x + b.x, o0), fx_to_double(a.y - b.y, o0));
+                        if (both) out[cstride + k] = make_double2(fx_to_double(a.y + b.y, o1), fx_to_double(b.x - a.x, o1));
                     }
                 }
                 __syncwarp();

@@ -55,12 +55,13 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
         fx_quantise_lane<8, G, kFxPlain>(a, w, 0u, 0, count, v, unit);
     }
     __syncthreads();  // twiddles
-    fx_fft_warp<N, true>(v, x, tw, t);
+    fx_fft_warp<N, true>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
     __syncthreads();  // every line buffer read: the tile takes their place
     double2* tile = reinterpret_cast<double2*>(tw + W::twiddles);
+    const FxUnit o = fx_out(unit);
 #pragma unroll
     for (int e = 0; e < 8; ++e)
-        tile[fx_tile(t + G * e, own, cols)] = make_double2(fx_to_double(v[e].x, unit), fx_to_double(v[e].y, unit));
+        tile[fx_tile(t + G * e, own, cols)] = make_double2(fx_to_double(v[e].x, o), fx_to_double(v[e].y, o));
     __syncthreads();
     double2* out = yspec + (static_cast<size_t>(z) * map.nOut + oc) * N * KX + kx0;
     const int g = min(cols, KX - kx0);
@@ -101,14 +102,15 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
     int unit;
     double w[8];
     fx_quantise_lane<8, G, kFxPlain>(a, w, 0u, 0, [](int) { return 1.0f; }, v, unit);
-    fx_fft_warp<N, false>(v, x, tw, t);
+    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
     const int kx = kx0 + own;
     if (kx >= KX) return;
     double2* out = fspec + (static_cast<size_t>(ch) * d.zTotal + z) * P;
+    const FxUnit o = fx_out(unit);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const int pos = d.ymap[static_cast<size_t>(kx) * N + t + G * e];
-        if (pos >= 0) out[pos] = make_double2(fx_to_double(v[e].x, unit), fx_to_double(v[e].y, unit));
+        if (pos >= 0) out[pos] = make_double2(fx_to_double(v[e].x, o), fx_to_double(v[e].y, o));
     }
 }
 
@@ -336,14 +338,15 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
 #pragma unroll
         for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
-        fx_fft_warp<N, false>(v, x, tw, t);
+        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uD)) ? 0 : fx_two());
 #pragma unroll
         for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();
         // even part -> cosine channel, odd part -> sine channel, n = 0 .. N / 2
+        const FxUnit oC = fx_out(uC - 2), oD = fx_out(uD - 2);
         auto put = [&](int n, fxc a1, fxc b1) {
-            const double2 ev = make_double2(fx_to_double(a1.x + b1.x, uC - 2), fx_to_double(a1.y + b1.y, uC - 2));
-            const double2 od = make_double2(fx_to_double(a1.x - b1.x, uD - 2), fx_to_double(a1.y - b1.y, uD - 2));
+            const double2 ev = make_double2(fx_to_double(a1.x + b1.x, oC), fx_to_double(a1.y + b1.y, oC));
+            const double2 od = make_double2(fx_to_double(a1.x - b1.x, oD), fx_to_double(a1.y - b1.y, oD));
             if (!live) return;
             if (chC >= 0) {
                 double2* base = zspec + (static_cast<size_t>(chC) * d.zTotal + n) * P;
@@ -431,7 +434,8 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
 #pragma unroll
         for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
-        fx_fft_warp<N, false>(v, x, tw, t);
+        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two());
+        const FxUnit oC = fx_out(uC - 1), oS = fx_out(uS - 1);
 #pragma unroll
         for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();
@@ -439,9 +443,9 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
         for (int i = 0; i < 4; ++i) {
             const int j = t + G * i;
             const fxc p = v[i], q = j == 0 ? v[0] : x[fx_pad(N - j)];
-            X[l][i] = make_double2(fx_to_double(p.x + q.x, uC - 1), fx_to_double(p.y + q.y, uC - 1));
+            X[l][i] = make_double2(fx_to_double(p.x + q.x, oC), fx_to_double(p.y + q.y, oC));
             // i times the odd part
-            X[2 + l][i] = make_double2(-fx_to_double(p.y - q.y, uS - 1), fx_to_double(p.x - q.x, uS - 1));
+            X[2 + l][i] = make_double2(-fx_to_double(p.y - q.y, oS), fx_to_double(p.x - q.x, oS));
         }
         __syncwarp();
     }
