@@ -1044,6 +1044,10 @@ cudaError_t set_smem_limits_adj(const Plan& p) {
 #define WV_SET(kernel, bytes)                                                                                   \
     e = raise_smem_limit(kernel, static_cast<int>(bytes)); \
     if (e != cudaSuccess) return e;
+    if constexpr (std::is_same<T, double>::value) {
+        e = wvgpu::fx_set_limits_adj(p);
+        if (e != cudaSuccess) return e;
+    }
     WV_SET((dev::k_vfwd_adj<T>), smem_vfwd_adj<T>(p));
     WV_SET((dev::k_xadj<T>), smem_xadj<T>(p));
     WV_SET((dev::k_yfwd_pair<T>), smem_ypair<T>(p));
@@ -1163,6 +1167,8 @@ cudaError_t launch_flux_vjp(wv_handle* h, double t, double t0, const double* Ap,
             done = true;
         }
     }
+    if constexpr (std::is_same<T, double>::value)
+        done = h->vfwdKind == WV_VERTICAL_FFT && wvgpu::fx_vfwd_adj(p, d, Fpb, Fmb, F0b, elapsed, za, s);
     if (done) {
     } else if (h->vfwdKind == WV_VERTICAL_FFT)
         dev::k_vfwd_adj_fft<T><<<dim3(cdiv(p.Nkl, dev::vf_modes<T>()), d.members), 256, dev::smem_vadj_fft<T>(p.fz.N), s>>>(
@@ -1173,8 +1179,12 @@ cudaError_t launch_flux_vjp(wv_handle* h, double t, double t0, const double* Ap,
     amap.nOut = nt;
     for (int c = 0; c < nt; ++c) { amap.src[c] = c; amap.mulL[c] = 0; }
     launch_yinv<T>(h, amap, za, ya, s);
+    bool xdone = false;
+    if constexpr (std::is_same<T, double>::value)
+        xdone = wvgpu::fx_xadj(p, d, h->fx, ya, yo, static_cast<const double*>(physIn), s);
     const int rx = warp_rx<T>(p);
-    if (rx) {
+    if (xdone) {
+    } else if (rx) {
         const dim3 grid(cdiv(p.Ny, dev::kWG), p.Nz);
         WV_RSWITCH_X(T, rx, (dev::k_xadj_w<T, RR><<<grid, 256, smem_xadj_w<T>(p), s>>>(
                                  d, y, ya, yo, static_cast<const dev::cx<T>*>(physIn))));
@@ -1190,7 +1200,9 @@ cudaError_t launch_flux_vjp(wv_handle* h, double t, double t0, const double* Ap,
         pm.srcA[4 + t2] = 4 + nt + t2;
         pm.srcB[4 + t2] = -1;
     }
-    {
+    bool ydone = false;
+    if constexpr (std::is_same<T, double>::value) ydone = wvgpu::fx_yfwd_pair(p, d, pm, yo, nIn, fa, s);
+    if (!ydone) {
         const int ry = warp_ry<T>(p);
         if (ry) {
             const dim3 grid(cdiv(p.kxColumns, dev::kWG), d.zTotal, pm.nOut);
@@ -1209,6 +1221,8 @@ cudaError_t launch_flux_vjp(wv_handle* h, double t, double t0, const double* Ap,
             vdone = true;
         }
     }
+    if constexpr (std::is_same<T, double>::value)
+        vdone = h->vinvKind == WV_VERTICAL_FFT && wvgpu::fx_vinv_adj(p, d, fa, elapsed, Apb, Amb, A0b, s);
     if (vdone) {
     } else if (h->vinvKind == WV_VERTICAL_FFT)
         dev::k_vinv_adj_fft<T><<<dim3(cdiv(p.Nkl, dev::VzLines<T>::value / 4), d.members), 256, dev::smem_vadj_fft<T>(p.fz.N), s>>>(

@@ -3,6 +3,7 @@
 #include "wv_fxflux.cuh"
 #include "wv_fxyz.cuh"
 #include "wv_fxany.cuh"
+#include "wv_fxadj.cuh"
 #include "wv_internal.hpp"
 
 #include <algorithm>
@@ -38,6 +39,7 @@ std::vector<int32_t> lane_table() {
 // run-time stages; longer rows keep the block kernel.
 inline bool fx_x_lane(const Plan& p) { return fx_lane_length(p.Nx) && 2 * p.kxColumns <= p.Nx; }
 inline bool fx_x_any(const Plan& p) { return p.Nx <= 512 && p.kxColumns <= 256; }
+constexpr size_t kFxCoUnits = 6;
 template <int N>
 size_t smem_xflux_fx() { return dev::FxW<N>::twiddles * sizeof(dev::fxw) + dev::kFxXWarps * dev::fx_xflux_warp_bytes(N); }
 // Warps of a y or z block: 8, fewer where the columns of a plane (the retained
@@ -48,10 +50,11 @@ inline int fx_y_warps(size_t Ny, size_t kxColumns) {
     while (warps < dev::kFxYWarps && warps * lines < kxColumns) warps *= 2;
     return warps;
 }
-inline int fx_z_warps(const Plan& p) {
-    // enough blocks for every SM before the blocks grow
-    const size_t lines = 256 / p.fz.N, units = (p.Nkl + lines - 1) / lines, sms = grid_cap(1);
-    return static_cast<int>(std::min<size_t>(dev::kFxZWarps, std::max<size_t>(1, (units + sms - 1) / sms)));
+// Column sets of a z block (its warps: sets x lines of a column): enough blocks for
+// every SM before the blocks grow to 8 warps.
+inline int fx_z_sets(const Plan& p, int lines) {
+    const size_t columns = 256 / p.fz.N, units = (p.Nkl + columns - 1) / columns, sms = grid_cap(1);
+    return static_cast<int>(std::min<size_t>(dev::kFxZWarps / lines, std::max<size_t>(1, units / sms)));
 }
 // Lines of any length along z: warps of a block, as shared memory allows.
 inline int fx_z_any_warps(const Plan& p, int lines) {
@@ -126,14 +129,64 @@ cudaError_t fx_set_limits(const Plan& p) {
         set(dev::k_vfwd_fxany<true>, two); set(dev::k_vfwd_fxany<false>, two);
     }
     WV_FXW_SWITCH(p.fz.N, {
-        set(dev::k_vinv_fx<NN, true>, dev::smem_fx_vinv<NN>(fx_z_warps(p)));
-        set(dev::k_vinv_fx<NN, false>, dev::smem_fx_vinv<NN>(fx_z_warps(p)));
-        set(dev::k_vfwd_fx<NN, true>, dev::smem_fx_vfwd<NN>(fx_z_warps(p)));
-        set(dev::k_vfwd_fx<NN, false>, dev::smem_fx_vfwd<NN>(fx_z_warps(p)));
+        set(dev::k_vinv_fx<NN, true>, dev::smem_fx_z<NN>(4, 2));
+        set(dev::k_vinv_fx<NN, false>, dev::smem_fx_z<NN>(2, 4));
+        set(dev::k_vfwd_fx<NN, true>, dev::smem_fx_z<NN>(2, 4));
+        set(dev::k_vfwd_fx<NN, false>, dev::smem_fx_z<NN>(2, 4));
     });
-    if (fx_x_lane(p)) { WV_FXW_SWITCH(p.Nx, set(dev::k_xflux_fx<NN, 3>, smem_xflux_fx<NN>()); set(dev::k_xflux_fx<NN, 4>, smem_xflux_fx<NN>())); }
+    if (fx_x_lane(p)) { WV_FXW_SWITCH(p.Nx, set(dev::k_xflux_fx<NN, 3>, smem_xflux_fx<NN>()); set(dev::k_xflux_fx<NN, 4>, smem_xflux_fx<NN>()); set(dev::k_xflux_fxco<NN, 3>, dev::smem_xflux_co<NN>()); set(dev::k_xflux_fxco<NN, 4>, dev::smem_xflux_co<NN>())); }
     else if (fx_x_any(p)) { WV_FXX_SWITCH(p.kxColumns, set(dev::k_xflux_fxany<EK>, fx_x_launch(p, 1).smem)); }
     return e;
+}
+
+cudaError_t fx_set_limits_adj(const Plan& p) {
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto* kernel, size_t bytes) {
+        if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(kernel), static_cast<int>(bytes));
+    };
+    WV_FXW_SWITCH(p.fz.N, {
+        set(dev::k_vfwd_adj_fx<NN>, dev::smem_fx_z<NN>(2, 4));
+        set(dev::k_vinv_adj_fx<NN>, dev::smem_fx_vinv_adj<NN>(2));
+    });
+    WV_FXW_SWITCH(p.Ny, set(dev::k_yfwd_pair_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * (256 / NN))));
+    if (fx_x_lane(p)) { WV_FXW_SWITCH(p.Nx, set(dev::k_xadj_fx<NN>, dev::smem_xadj_fx<NN>())); }
+    return e;
+}
+
+bool fx_vfwd_adj(const Plan& p, const dev::DescDev& d, const double* Fpb, const double* Fmb, const double* F0b, double elapsed,
+                 double2* zadj, cudaStream_t s) {
+    if (!fx_lane_length(p.fz.N)) return false;
+    const int sets = fx_z_sets(p, 2);
+    WV_FXW_SWITCH(p.fz.N, (dev::k_vfwd_adj_fx<NN><<<cdiv(p.Nkl, sets * (256 / NN)), 64 * sets, dev::smem_fx_z<NN>(2, sets), s>>>(
+                              d, Fpb, Fmb, F0b, elapsed, zadj)));
+    return true;
+}
+
+bool fx_vinv_adj(const Plan& p, const dev::DescDev& d, const double2* fadj, double elapsed, double* Apb, double* Amb,
+                 double* A0b, cudaStream_t s) {
+    if (!fx_lane_length(p.fz.N)) return false;
+    const int sets = fx_z_sets(p, 4);
+    WV_FXW_SWITCH(p.fz.N, (dev::k_vinv_adj_fx<NN><<<cdiv(p.Nkl, sets * (256 / NN)), 128 * sets, dev::smem_fx_vinv_adj<NN>(sets), s>>>(
+                              d, fadj, elapsed, Apb, Amb, A0b)));
+    return true;
+}
+
+bool fx_yfwd_pair(const Plan& p, const dev::DescDev& d, const dev::YFwdPairMap& map, const double2* y, int nIn, double2* f,
+                  cudaStream_t s) {
+    if (!fx_lane_length(p.Ny)) return false;
+    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(256 / p.Ny);
+    const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, map.nOut);
+    WV_FXW_SWITCH(p.Ny, (dev::k_yfwd_pair_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(d, map, y, nIn, f)));
+    return true;
+}
+
+bool fx_xadj(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* yadj, double2* yout, const double* rowsIn,
+             cudaStream_t s) {
+    if (!fx_x_lane(p) || !rowsIn) return false;
+    const size_t rows = p.Ny * static_cast<size_t>(d.zTotal), lines = 256 / p.Nx;
+    WV_FXW_SWITCH(p.Nx, (dev::k_xadj_fx<NN><<<cdiv(rows, lines), 32 * dev::kFxCoWarps, dev::smem_xadj_fx<NN>(), s>>>(
+                            d, r.twXLane, yadj, yout, rowsIn)));
+    return true;
 }
 
 bool fx_has_rows(const Plan& p) { return fx_x_lane(p) || fx_x_any(p); }
@@ -144,6 +197,14 @@ bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& r, const doubl
         // one block per SM; fewer warps a block where there are too few rows to fill it
         const size_t rows = p.Ny * p.Nz * d.members, perWarp = 256 / p.Nx;
         const size_t units = (rows + perWarp - 1) / perWarp, sms = grid_cap(1);
+        if (p.Nx == 256 || units <= kFxCoUnits * sms) {
+            WV_FXW_SWITCH(p.Nx, {
+                auto* kernel = 8 * p.kxColumns <= 3 * p.Nx ? dev::k_xflux_fxco<NN, 3> : dev::k_xflux_fxco<NN, 4>;
+                kernel<<<static_cast<unsigned>(units), 32 * dev::kFxCoWarps, dev::smem_xflux_co<NN>(), s>>>(
+                    d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
+            });
+            return true;
+        }
         const int warps = static_cast<int>(std::min<size_t>(dev::kFxXWarps, std::max<size_t>(1, (units + sms - 1) / sms)));
         const int grid = static_cast<int>(std::min<size_t>((units + warps - 1) / warps, sms));
         WV_FXW_SWITCH(p.Nx, {
@@ -217,10 +278,10 @@ bool fx_vinv(const Plan& p, const dev::DescDev& d, bool flux, double elapsed, co
         else dev::k_vinv_fxany<false><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
         return true;
     }
-    const int warps = fx_z_warps(p);
-    const dim3 grid(cdiv(p.Nkl, warps * (256 / p.fz.N)), d.members);
+    const int lines = flux ? 4 : 2, sets = fx_z_sets(p, lines), warps = sets * lines;
+    const dim3 grid(cdiv(p.Nkl, sets * (256 / p.fz.N)), d.members);
     WV_FXW_SWITCH(p.fz.N, {
-        const size_t sm = dev::smem_fx_vinv<NN>(warps);
+        const size_t sm = dev::smem_fx_z<NN>(lines, sets);
         if (flux) dev::k_vinv_fx<NN, true><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
         else dev::k_vinv_fx<NN, false><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
     });
@@ -241,10 +302,10 @@ bool fx_vfwd(const Plan& p, const dev::DescDev& d, bool flux, const double2* f, 
             dev::k_vfwd_fxany<false><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
         return true;
     }
-    const int warps = fx_z_warps(p);
-    const dim3 grid(cdiv(p.Nkl, warps * (256 / p.fz.N)), d.members);
+    const int sets = fx_z_sets(p, 2), warps = 2 * sets;
+    const dim3 grid(cdiv(p.Nkl, sets * (256 / p.fz.N)), d.members);
     WV_FXW_SWITCH(p.fz.N, {
-        const size_t sm = dev::smem_fx_vfwd<NN>(warps);
+        const size_t sm = dev::smem_fx_z<NN>(2, sets);
         if (flux)
             dev::k_vfwd_fx<NN, true><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
         else

@@ -38,4 +38,15 @@ bool fx_vfwd(const Plan& p, const dev::DescDev& d, bool flux, const double2* f, 
              const double* Am, const double* A0, const unsigned long long* speed, int damping, double* Fp, double* Fm,
              double* F0, cudaStream_t s);
 
+// The flux VJP's passes (fx_xadj: on kept rows of the x pass).
+cudaError_t fx_set_limits_adj(const Plan& p);
+bool fx_vfwd_adj(const Plan& p, const dev::DescDev& d, const double* Fpb, const double* Fmb, const double* F0b, double elapsed,
+                 double2* zadj, cudaStream_t s);
+bool fx_xadj(const Plan& p, const dev::DescDev& d, const FxRows& rows, const double2* yadj, double2* yout,
+             const double* rowsIn, cudaStream_t s);
+bool fx_yfwd_pair(const Plan& p, const dev::DescDev& d, const dev::YFwdPairMap& map, const double2* y, int nIn, double2* f,
+                  cudaStream_t s);
+bool fx_vinv_adj(const Plan& p, const dev::DescDev& d, const double2* fadj, double elapsed, double* Apb, double* Amb,
+                 double* A0b, cudaStream_t s);
+
 }  // namespace wvgpu

@@ -200,6 +200,154 @@ __device__ __forceinline__ unsigned fx_abs_hi(long long v) {
 }
 __device__ __forceinline__ int fx_pick(const int (&a)[3], int i) { return i == 0 ? a[0] : i == 1 ? a[1] : a[2]; }
 
+// Rows 2p and 2p + 1 of the x pass (0 u, 1 v, 2 w, then 3 + 3 t + (x, y, z derivative
+// of target t)) as the lane's entries of the line Z = A + i B.
+template <int N, int EK>
+__device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __restrict__ yrow, size_t cstride,
+                                             const double* __restrict__ rowK, unsigned wtop, int p, int nReal, fxc* __restrict__ x,
+                                             int t, fxc (&v)[8], int (&unit)[2]) {
+    constexpr int G = N / 8;
+    const int KX = d.kxColumns, nt = d.nt;
+    // rows 2p and 2p + 1: spectrum entries k = t + G i, both rows' loads in flight
+    double2 raw[2][EK];
+    int weighted = 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int r = 2 * p + q;
+        int ch = r;
+        if (r >= 3) {
+            const int tt = (r - 3) / 3, kind = (r - 3) - 3 * tt;
+            if (kind == 0) weighted |= 1 << q;
+            ch = kind == 0 ? d.tq[tt & 3] : kind == 1 ? 4 + tt : 4 + nt + tt;
+        }
+                        const double2* h = yrow + ch * cstride;
+    #pragma unroll
+                        for (int i = 0; i < EK; ++i) {
+                            const int k = t + G * i;
+                            raw[q][i] = k < KX && r < nReal ? h[k] : make_double2(0.0, 0.0);
+                        }
+                        if (t == 0) raw[q][0].y = 0.0;  // c2r semantics
+                    }
+                    fxc A[EK], B[EK];
+                    auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
+    #pragma unroll 1
+                    for (int q = 0; q < 2; ++q) {  // one copy of the code: it must stay in the instruction cache
+                        double2 a[EK];
+                        double w[EK];
+    #pragma unroll
+                        for (int i = 0; i < EK; ++i) {
+                            a[i] = q ? raw[1][i] : raw[0][i];
+                            A[i] = B[i];
+                        }
+                        int u;
+                        if ((weighted >> q) & 1) {
+    #pragma unroll
+                            for (int i = 0; i < EK; ++i) w[i] = t + G * i < KX ? rowK[t + G * i] : 0.0;
+                            fx_quantise_lane<EK, G, kFxImag>(a, w, wtop, 1, count, B, u);
+                        } else {
+                            fx_quantise_lane<EK, G, kFxPlain>(a, w, 0u, 1, count, B, u);
+                        }
+                        unit[0] = unit[1];
+                        unit[1] = u;
+                    }
+                    // Z = A + i B at k and its mirror at N - k; nothing between
+    #pragma unroll
+                    for (int i = 0; i < EK; ++i) {
+                        const fxc a = A[i], b = B[i];
+                        v[i] = fxc{a.x - b.y, a.y + b.x};
+                        const int k = t + G * i;
+                        const fxc m = {a.x + b.y, b.x - a.y};
+                        x[fx_pad(k == 0 ? N - G * EK : N - k)] = k == 0 ? fxc{0, 0} : m;
+                    }
+    #pragma unroll
+                    for (int e = EK; e < 8 - EK; ++e) v[e] = fxc{0, 0};
+                    __syncwarp();
+    #pragma unroll
+                    for (int e = 8 - EK; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+                    __syncwarp();
+}
+
+// Samples of an advecting velocity row (or the caller's doubles), normalised to 62
+// bits, into phys; returns the unit.
+template <int N>
+__device__ __forceinline__ int fx_velocity(const long long (&smp)[8], int unit, int t, long long* __restrict__ phys,
+                                           const double* __restrict__ advIn, double* __restrict__ advOut,
+                                           double* __restrict__ keep) {
+    constexpr int G = N / 8;
+    unsigned top = 0;
+    if (advIn) {
+        double a[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            a[e] = advIn[t + G * e];
+            top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
+        }
+        top = fx_group_max<G>(top);
+        const fxscale sc{static_cast<int>(top >> 20), 61};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            phys[t + G * e] = fx_from_double(a[e], sc);
+            if (keep) keep[t + G * e] = a[e];
+        }
+        return fx_unit(sc);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) top = max(top, fx_abs_hi(smp[e]));
+    top = fx_group_max<G>(top);
+    const int sh = max(0, __clz(static_cast<int>(top)) - 2);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const long long s = fx_round53(smp[e] << sh);
+        phys[t + G * e] = s;
+        if (advOut) advOut[t + G * e] = fx_to_double(s, unit - sh);
+        if (keep) keep[t + G * e] = fx_to_double(s, unit - sh);
+    }
+    return unit - sh;
+}
+
+// r2c of the products Sa, Sb (Sb null: none) of a row as one line; out[k], k < KX, and
+// out[cstride + k].
+template <int N>
+__device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa, const long long* __restrict__ Sb, int unitA,
+                                                int unitB, fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two,
+                                                int KX, double2* __restrict__ out, size_t cstride) {
+    constexpr int G = N / 8;
+    const bool both = Sb != nullptr;
+    fxc v[8];
+    int sh[2], u[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        unsigned sum = 0;
+        if (q == 0 || both)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum += (fx_abs_hi((q ? Sb : Sa)[t + G * e]) >> 9) + 1u;
+        sum = fx_group_add<G>(sum);
+        sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 59;  // sum |S| < 2^59 after the shift
+        u[q] = (q ? unitB : unitA) + sh[q] - 1;                 // the halves of the split below
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const long long a = Sa[t + G * e], b = both ? Sb[t + G * e] : 0;
+        v[e].x = sh[0] >= 0 ? a >> sh[0] : a << -sh[0];
+        v[e].y = sh[1] >= 0 ? b >> sh[1] : b << -sh[1];
+    }
+    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(unitA, both ? unitB : unitA)) ? 0 : two);
+    __syncwarp();
+#pragma unroll
+    for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+    __syncwarp();
+    const FxUnit o0 = fx_out(u[0]), o1 = fx_out(u[1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = t + G * i;
+        const fxc a = v[i], b = k == 0 ? v[0] : x[fx_pad(N - k)];
+        if (k < KX) {
+            out[k] = make_double2(fx_to_double(a.x + b.x, o0), fx_to_double(a.y - b.y, o0));
+            if (both) out[cstride + k] = make_double2(fx_to_double(a.y + b.y, o1), fx_to_double(b.x - a.x, o1));
+        }
+    }
+}
+
 // physOut / advOut / advIn / maxSpeedBits as k_xflux.
 // EK: spectrum entries of a lane (kx < EK N / 8; 3 under the 2/3 rule).
 template <int N, int EK>
@@ -239,65 +387,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
         for (int p = 0; 2 * p < nReal; ++p) {
             fxc v[8];
             int unit[2] = {kFxZero, kFxZero};
-            {
-                // rows 2p and 2p + 1: spectrum entries k = t + G i, both rows' loads in flight
-                double2 raw[2][EK];
-                int weighted = 0;
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int r = 2 * p + q;
-                    int ch = r;
-                    if (r >= 3) {
-                        const int tt = (r - 3) / 3, kind = (r - 3) - 3 * tt;
-                        if (kind == 0) weighted |= 1 << q;
-                        ch = kind == 0 ? d.tq[tt & 3] : kind == 1 ? 4 + tt : 4 + nt + tt;
-                    }
-                    const double2* h = yrow + ch * cstride;
-#pragma unroll
-                    for (int i = 0; i < EK; ++i) {
-                        const int k = t + G * i;
-                        raw[q][i] = k < KX && r < nReal ? h[k] : make_double2(0.0, 0.0);
-                    }
-                    if (t == 0) raw[q][0].y = 0.0;  // c2r semantics
-                }
-                fxc A[EK], B[EK];
-                auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
-#pragma unroll 1
-                for (int q = 0; q < 2; ++q) {  // one copy of the code: it must stay in the instruction cache
-                    double2 a[EK];
-                    double w[EK];
-#pragma unroll
-                    for (int i = 0; i < EK; ++i) {
-                        a[i] = q ? raw[1][i] : raw[0][i];
-                        A[i] = B[i];
-                    }
-                    int u;
-                    if ((weighted >> q) & 1) {
-#pragma unroll
-                        for (int i = 0; i < EK; ++i) w[i] = t + G * i < KX ? rowK[t + G * i] : 0.0;
-                        fx_quantise_lane<EK, G, kFxImag>(a, w, wtop, 1, count, B, u);
-                    } else {
-                        fx_quantise_lane<EK, G, kFxPlain>(a, w, 0u, 1, count, B, u);
-                    }
-                    unit[0] = unit[1];
-                    unit[1] = u;
-                }
-                // Z = A + i B at k and its mirror at N - k; nothing between
-#pragma unroll
-                for (int i = 0; i < EK; ++i) {
-                    const fxc a = A[i], b = B[i];
-                    v[i] = fxc{a.x - b.y, a.y + b.x};
-                    const int k = t + G * i;
-                    const fxc m = {a.x + b.y, b.x - a.y};
-                    x[fx_pad(k == 0 ? N - G * EK : N - k)] = k == 0 ? fxc{0, 0} : m;
-                }
-#pragma unroll
-                for (int e = EK; e < 8 - EK; ++e) v[e] = fxc{0, 0};
-                __syncwarp();
-#pragma unroll
-                for (int e = 8 - EK; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
-                __syncwarp();
-            }
+            fx_load_pair<N, EK>(d, yrow, cstride, rowK, wtop, p, nReal, x, t, v, unit);
             fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
             // samples x = t + G e: real part row 2p, imaginary part row 2p + 1
 #pragma unroll 1
@@ -314,42 +404,10 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
                     for (int e = 0; e < 8; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
                 }
                 if (r < 3) {
-                    // advecting velocity, normalised to 62 bits
                     const size_t g = static_cast<size_t>(r) * R3 + (static_cast<size_t>(z) * Ny + y) * N;
-                    int un;
-                    if (advIn) {
-                        double a[8];
-                        unsigned top = 0;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            a[e] = advIn[g + t + G * e];
-                            top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
-                        }
-                        top = fx_group_max<G>(top);
-                        const fxscale sc{static_cast<int>(top >> 20), 61};
-                        un = fx_unit(sc);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            phys[r * N + t + G * e] = fx_from_double(a[e], sc);
-                            if (physOut && live)
-                                physOut[((static_cast<size_t>(z) * nReal + r) * Ny + y) * N + t + G * e] = a[e];
-                        }
-                    } else {
-                        unsigned top = 0;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) top = max(top, fx_abs_hi(smp[e]));
-                        top = fx_group_max<G>(top);
-                        const int sh = max(0, __clz(static_cast<int>(top)) - 2);
-                        un = uq - sh;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const long long s = fx_round53(smp[e] << sh);
-                            phys[r * N + t + G * e] = s;
-                            if (advOut && live) advOut[g + t + G * e] = fx_to_double(s, un);
-                            if (physOut && live)
-                                physOut[((static_cast<size_t>(z) * nReal + r) * Ny + y) * N + t + G * e] = fx_to_double(s, un);
-                        }
-                    }
+                    double* keep = physOut && live ? physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N : nullptr;
+                    const int un = fx_velocity<N>(smp, uq, t, phys + r * N, advIn ? advIn + g : nullptr,
+                                                  advOut && live ? advOut + g : nullptr, keep);
                     if (r == 0) physUnit[0] = un;
                     else if (r == 1) physUnit[1] = un;
                     else physUnit[2] = un;
@@ -383,39 +441,8 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
             if (done > before && ((done & 1) == 0 || done == nt)) {
                 const bool both = (done & 1) == 0;
                 const int t0 = both ? done - 2 : done - 1;
-                int sh[2], u[2];
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    unsigned sum = 0;
-                    if (q == 0 || both)
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) sum += (fx_abs_hi(S[q * N + t + G * e]) >> 9) + 1u;
-                    sum = fx_group_add<G>(sum);
-                    sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 59;  // sum |S| < 2^59 after the shift
-                    u[q] = sUnit[q] + sh[q] - 1;                            // the halves of the split below
-                }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const long long a = S[t + G * e], b = both ? S[N + t + G * e] : 0;
-                    v[e].x = sh[0] >= 0 ? a >> sh[0] : a << -sh[0];
-                    v[e].y = sh[1] >= 0 ? b >> sh[1] : b << -sh[1];
-                }
-                fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(sUnit[0], both ? sUnit[1] : sUnit[0])) ? 0 : two);
-                __syncwarp();
-#pragma unroll
-                for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
-                __syncwarp();
                 double2* out = pspec + ((static_cast<size_t>(z) * nt + t0) * Ny + y) * KX;
-                const FxUnit o0 = fx_out(u[0]), o1 = fx_out(u[1]);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int k = t + G * i;
-                    const fxc a = v[i], b = k == 0 ? v[0] : x[fx_pad(N - k)];
-                    if (k < KX && live) {
-                        out[k] = make_double2(fx_to_double(a.x + b.x, o0), fx_to_double(a.y - b.y, o0));
-                        if (both) out[cstride + k] = make_double2(fx_to_double(a.y + b.y, o1), fx_to_double(b.x - a.x, o1));
-                    }
-                }
+                fx_forward_pair<N>(S, both ? S + N : nullptr, sUnit[0], sUnit[1], x, tw, t, two, live ? KX : 0, out, cstride);
                 __syncwarp();
             }
         }
@@ -432,6 +459,118 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
             for (int o = G / 2; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (t == 0) atomicMax(maxSpeedBits + z / d.Nz, (unsigned long long)__double_as_longlong(sqrt(m)));
         }
+    }
+}
+
+// The same pass for grids with too few rows to keep every SM busy with one warp a
+// row: a block takes one line-set of rows, a warp a pair of their c2r, all threads a
+// sample's products, a warp a pair of the r2c.  The arithmetic, to the bit, is
+// k_xflux_fx's.
+constexpr int kFxCoWarps = 8;  // (3 + 3 nt + 1) / 2 <= 8 pairs
+template <int N>
+inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * 256 * 8; }
+
+template <int N, int EK>
+__global__ void __launch_bounds__(32 * kFxCoWarps, 3)
+    k_xflux_fxco(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, double2* __restrict__ pspec,
+                 unsigned long long* __restrict__ maxSpeedBits, double* __restrict__ physOut, double* __restrict__ advOut,
+                 const double* __restrict__ advIn) {
+    using W = FxW<N>;
+    constexpr int G = W::G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int rowUnit[16][W::lines], sUnit[4][W::lines];
+    const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
+    const int nIn = 4 + 2 * nt, nReal = 3 + 3 * nt;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = lane % G, line = lane / G;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* buffers = reinterpret_cast<fxc*>(tw + W::twiddles);  // [pair][line][buffer]
+    fxc* x = buffers + static_cast<size_t>(warp * W::lines + line) * W::buffer;
+    long long* phys = reinterpret_cast<long long*>(buffers + kFxCoWarps * W::lines * W::buffer);  // [3][line][N]
+    long long* S = phys + 3 * 256;                                                               // [nt][line][N]
+    const int two = fx_two();
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
+    const double* rowK = row_k<double>(d);
+    const size_t cstride = static_cast<size_t>(Ny) * KX;
+    const size_t R3 = static_cast<size_t>(N) * Ny * d.Nz;
+    const int rows = Ny * d.zTotal;
+    const unsigned wtop = static_cast<unsigned>(__double2hiint(rowK[KX - 1]));
+    const int first = blockIdx.x * W::lines;
+    const bool live = first + line < rows;
+    const int row = min(first + line, rows - 1);
+    const int z = row / Ny, y = row - z * Ny;
+    const int p = warp;
+    __syncthreads();
+    if (2 * p < nReal) {
+        fxc v[8];
+        int unit[2] = {kFxZero, kFxZero};
+        fx_load_pair<N, EK>(d, yspec + (static_cast<size_t>(z) * nIn * Ny + y) * KX, cstride, rowK, wtop, p, nReal, x, t, v, unit);
+        fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[t + G * e] = v[e];
+#pragma unroll 1
+        for (int q = 0; q < 2; ++q) {
+            const int r = 2 * p + q;
+            if (r >= nReal) break;
+            int uq = q ? unit[1] : unit[0];
+            double* keep = physOut && live ? physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N : nullptr;
+            long long smp[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) smp[e] = q ? v[e].y : v[e].x;
+            if (r < 3) {
+                const size_t g = static_cast<size_t>(r) * R3 + (static_cast<size_t>(z) * Ny + y) * N;
+                uq = fx_velocity<N>(smp, uq, t, phys + (r * W::lines + line) * N, advIn ? advIn + g : nullptr,
+                                    advOut && live ? advOut + g : nullptr, keep);
+            } else if (keep) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
+            }
+            if (t == 0) rowUnit[r][line] = uq;
+        }
+    }
+    __syncthreads();
+    {
+        // one sample a thread
+        const int s = threadIdx.x, ln = s / N, xx = s - ln * N;
+        for (int tt = 0; tt < nt; ++tt) {
+            long long acc = 0;
+            int now = 0;
+#pragma unroll
+            for (int kind = 0; kind < 3; ++kind) {
+                const int r = 3 + 3 * tt + kind;
+                const fxc* b = buffers + static_cast<size_t>((r >> 1) * W::lines + ln) * W::buffer;
+                const long long q = (r & 1) ? b[xx].y : b[xx].x;
+                const int un = rowUnit[kind][ln] + rowUnit[r][ln] - 1023 + 62;
+                const long long pr = fx_prod(phys[kind * 256 + s], q);
+                if (kind == 0) {
+                    acc = -pr;
+                    now = un;
+                } else {
+                    const int next = max(now, un);
+                    acc = (acc >> min(63, next - now)) - (pr >> min(63, next - un));
+                    now = next;
+                }
+            }
+            S[tt * 256 + s] = acc;
+            if (xx == 0) sUnit[tt][ln] = now;
+        }
+        if (maxSpeedBits) {
+            const double U = fx_to_double(phys[s], rowUnit[0][ln]), V = fx_to_double(phys[256 + s], rowUnit[1][ln]);
+            double m = U * U + V * V;
+            constexpr int kSpan = N < 32 ? N : 32;
+#pragma unroll
+            for (int o = kSpan / 2; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+            m = fmax(m, 0.0);
+            const int zz = min(first + ln, rows - 1) / Ny;
+            if (lane % kSpan == 0) atomicMax(maxSpeedBits + zz / d.Nz, (unsigned long long)__double_as_longlong(sqrt(m)));
+        }
+    }
+    __syncthreads();
+    if (2 * p < nt) {
+        const bool both = 2 * p + 1 < nt;
+        const long long* Sa = S + 2 * p * 256 + line * N;
+        fx_forward_pair<N>(Sa, both ? Sa + 256 : nullptr, sUnit[2 * p][line], both ? sUnit[2 * p + 1][line] : 0, x, tw, t, two,
+                           live ? KX : 0, pspec + ((static_cast<size_t>(z) * nt + 2 * p) * Ny + y) * KX, cstride);
     }
 }
 

@@ -22,7 +22,7 @@ __device__ __forceinline__ int fx_tile(int y, int c, int cols) { return y * cols
 // Inverse FFTs along y of output channel blockIdx.z, columns blockIdx.x cols ...,
 // plane blockIdx.y: yspec[z][ch][y][kx] from zspec[src][z][pos] (times i l).
 template <int N>
-__global__ void __launch_bounds__(32 * kFxYWarps, 2)
+__global__ void __launch_bounds__(32 * kFxYWarps, 3)
     k_yinv_fx(DescDev d, YInvMap map, const double2* __restrict__ zspec, double2* __restrict__ yspec, unsigned ltop) {
     using W = FxW<N>;
     constexpr int G = W::G;
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
 // Forward FFTs along y of channel blockIdx.z, gathered to the active rows:
 // fspec[c][z][pos] from pspec[z][c][y][kx].
 template <int N>
-__global__ void __launch_bounds__(32 * kFxYWarps, 2)
+__global__ void __launch_bounds__(32 * kFxYWarps, 3)
     k_yfwd_fx(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec) {
     using W = FxW<N>;
     constexpr int G = W::G;
@@ -240,31 +240,31 @@ __device__ __forceinline__ void fx_project(const DescDev& d, int w, int j, doubl
 }
 
 constexpr int kFxZWarps = 8;
-// Per line: its buffer and the field spectra [4][N/2] of its mode.
+// Lines of one retained column: 4 (flux) or 2 in the inverse, 2 forward; each is a
+// warp's, so a column's lines run side by side (a small grid has few columns, and a
+// warp that walked them in turn took 24 us at 16x16x9).
+// A block holds 8 / lines sets of FxW<N>::lines columns.
 template <int N>
-inline size_t smem_fx_vinv(int warps) {
-    return static_cast<size_t>(FxW<N>::twiddles) * 16 +
-           static_cast<size_t>(warps) * FxW<N>::lines * (FxW<N>::buffer * 16 + 2 * N * 16);
-}
-template <int N>
-inline size_t smem_fx_vfwd(int warps) {
-    return static_cast<size_t>(FxW<N>::twiddles) * 16 + static_cast<size_t>(warps) * FxW<N>::lines * FxW<N>::buffer * 16;
+inline size_t smem_fx_z(int lines, int sets) {
+    const size_t columns = static_cast<size_t>(sets) * FxW<N>::lines;
+    return (FxW<N>::twiddles + columns * (lines * FxW<N>::buffer + 2 * N)) * 16;
 }
 
-// k_vinv_fft (wv_vfft.cuh) in fixed point, one retained column per line: the pairs
-// (u | w), (v | eta) and, for the flux, (m w | -m u), (m eta | -m v).  The two channels of a
-// pair keep their own scales (the even and the odd part separate them again), so
-// neither rounds at the other's magnitude.
+// k_vinv_fft (wv_vfft.cuh) in fixed point: the pairs (u | w), (v | eta) and, for the
+// flux, (m w | -m u), (m eta | -m v).  The two channels of a pair keep their own
+// scales (the even and the odd part separate them again), so neither rounds at the
+// other's magnitude.
 template <int N, bool FLUX>
-__global__ void __launch_bounds__(32 * kFxZWarps, 2)
+__global__ void __launch_bounds__(32 * kFxZWarps, 3)
     k_vinv_fx(DescDev d, const double* __restrict__ Ap, const double* __restrict__ Am, const double* __restrict__ A0,
               double elapsed, double2* __restrict__ zspec, unsigned long long* __restrict__ maxSpeedBits) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, kLines = FLUX ? 4 : 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nj = d.Nj, P = d.positions;
-    const int lane = threadIdx.x & 31, t = lane % G;
-    const int own = (threadIdx.x >> 5) * W::lines + lane / G, perBlock = (blockDim.x >> 5) * W::lines;
+    const int lane = threadIdx.x & 31, t = lane % G, warp = threadIdx.x >> 5;
+    const int set = warp / kLines, l = warp - set * kLines;
+    const int sets = (blockDim.x >> 5) / kLines;
     const int member = blockIdx.y;
     if (member > 0) {
         const long long o = member * d.memberStride;
@@ -273,106 +273,113 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && maxSpeedBits) maxSpeedBits[member] = 0ull;
     fxw* tw = reinterpret_cast<fxw*>(smem_raw);
-    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(own) * (W::buffer + 2 * N);
-    double2* fld = reinterpret_cast<double2*>(x + W::buffer);  // [4][N/2]
+    const int column = set * W::lines + lane / G;
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(column * kLines + l) * W::buffer;
+    double2* fld = reinterpret_cast<double2*>(reinterpret_cast<fxc*>(tw + W::twiddles) +
+                                              static_cast<size_t>(sets) * W::lines * kLines * W::buffer) +
+                   static_cast<size_t>(column) * 2 * N;  // field spectra [4][N/2]
     for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwZ[i];
-    __syncthreads();
-    const int want = blockIdx.x * perBlock + own;
+    const int want = blockIdx.x * sets * W::lines + column;
     const bool live = want < d.Nkl;
     const int mode = min(want, d.Nkl - 1);
-    const int w = d.modeWV[mode];
-    const unsigned char flags = d.modeFlags[mode];
     const double* mz = static_cast<const double*>(d.tMz);
     const unsigned mtop = static_cast<unsigned>(__double2hiint(mz[Nj - 1]));
+    {
+        const int w = d.modeWV[mode];
+        const unsigned char flags = d.modeFlags[mode];
 #pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-        const int j = t + G * i;
-        double2 f[4];
-        if (j < Nj) fx_field_spectra(d, Ap, Am, A0, elapsed, w, flags, j, f);
+        for (int i = l; i < 4; i += kLines) {  // the column's warps share its coefficients
+            const int j = t + G * i;
+            double2 f[4];
+            if (j < Nj) fx_field_spectra(d, Ap, Am, A0, elapsed, w, flags, j, f);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) fld[q * (N / 2) + j] = j < Nj ? f[q] : make_double2(0.0, 0.0);
+            for (int q = 0; q < 4; ++q) fld[q * (N / 2) + j] = j < Nj ? f[q] : make_double2(0.0, 0.0);
+        }
     }
-    int derivChan[4] = {-1, -1, -1, -1};
+    __syncthreads();
+    int derivC = -1, derivS = -1;  // channels of the z derivatives of targets l and l - 2
     if constexpr (FLUX)
-        for (int q = 0; q < d.nt; ++q) derivChan[d.tq[q]] = 4 + q;
+        for (int q = 0; q < d.nt; ++q) {
+            if (d.tq[q] == l) derivC = 4 + q;
+            if (d.tq[q] == l - 2) derivS = 4 + q;
+        }
     const int pos = d.modePos[mode], cpos = d.modeCompPos[mode];
     auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
-    constexpr int kLines = FLUX ? 4 : 2;
-#pragma unroll 1
-    for (int l = 0; l < kLines; ++l) {
-        // fld slots of the cosine and sine channels: (0|2) (1|3) (2|0) (3|1)
-        const int qc = l < 2 ? l : l, qs = l < 2 ? l + 2 : l - 2;
-        const int chC = l < 2 ? l : derivChan[l], chS = l < 2 ? l + 2 : derivChan[l - 2];
-        double2 a[4];
-        double wgt[4];
-        fxc C[4], D[4];
-        int uC, uD;
+    // fld slots of the cosine and sine channels: (0|2) (1|3) (2|0) (3|1)
+    const int qs = l < 2 ? l + 2 : l - 2;
+    const int chC = l < 2 ? l : derivC, chS = l < 2 ? l + 2 : derivS;
+    double2 a[4];
+    double wgt[4];
+    fxc C[4], D[4];
+    int uC, uD;
+    if (l < 2) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = fld[qc * (N / 2) + t + G * i];
-        if (l < 2) {
-            fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, C, uC);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) wgt[i] = t + G * i < Nj ? mz[t + G * i] : 0.0;
-            fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, C, uC);
-        }
+        for (int i = 0; i < 4; ++i) a[i] = fld[l * (N / 2) + t + G * i];
+        fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, C, uC);
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = fld[qs * (N / 2) + t + G * i];
-        if (l < 2) {
-            fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, D, uD);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) wgt[i] = -wgt[i];
-            fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, D, uD);
-        }
-        // 2 y[j] = C_j + i D_j, 2 y[N-j] = C_j - i D_j, 2 y[0] = C_0
-        fxc v[8];
+        fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, D, uD);
+    } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int j = t + G * i;
-            if (j == 0) D[i] = fxc{0, 0};
-            v[i] = fxc{C[i].x - D[i].y, C[i].y + D[i].x};
-            x[fx_pad(j == 0 ? N / 2 : N - j)] = j == 0 ? fxc{0, 0} : fxc{C[i].x + D[i].y, C[i].y - D[i].x};
+            a[i] = fld[l * (N / 2) + t + G * i];
+            wgt[i] = t + G * i < Nj ? mz[t + G * i] : 0.0;
         }
-        __syncwarp();
-#pragma unroll
-        for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
-        __syncwarp();
-        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uD)) ? 0 : fx_two());
-#pragma unroll
-        for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
-        __syncwarp();
-        // even part -> cosine channel, odd part -> sine channel, n = 0 .. N / 2
-        const FxUnit oC = fx_out(uC - 2), oD = fx_out(uD - 2);
-        auto put = [&](int n, fxc a1, fxc b1) {
-            const double2 ev = make_double2(fx_to_double(a1.x + b1.x, oC), fx_to_double(a1.y + b1.y, oC));
-            const double2 od = make_double2(fx_to_double(a1.x - b1.x, oD), fx_to_double(a1.y - b1.y, oD));
-            if (!live) return;
-            if (chC >= 0) {
-                double2* base = zspec + (static_cast<size_t>(chC) * d.zTotal + n) * P;
-                base[pos] = ev;
-                if (cpos >= 0) base[cpos] = make_double2(ev.x, -ev.y);
-            }
-            if (chS >= 0) {
-                double2* base = zspec + (static_cast<size_t>(chS) * d.zTotal + n) * P;
-                base[pos] = od;
-                if (cpos >= 0) base[cpos] = make_double2(od.x, -od.y);
-            }
-        };
+        fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, C, uC);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int n = t + G * i;
-            put(n, v[i], n == 0 ? v[0] : x[fx_pad(N - n)]);
+            a[i] = fld[qs * (N / 2) + t + G * i];
+            wgt[i] = -wgt[i];
         }
-        if (t == 0) put(N / 2, v[4], v[4]);
-        __syncwarp();
+        fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, D, uD);
     }
+    // 2 y[j] = C_j + i D_j, 2 y[N-j] = C_j - i D_j, 2 y[0] = C_0
+    fxc v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int j = t + G * i;
+        if (j == 0) D[i] = fxc{0, 0};
+        v[i] = fxc{C[i].x - D[i].y, C[i].y + D[i].x};
+        x[fx_pad(j == 0 ? N / 2 : N - j)] = j == 0 ? fxc{0, 0} : fxc{C[i].x + D[i].y, C[i].y - D[i].x};
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+    __syncwarp();
+    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uD)) ? 0 : fx_two());
+#pragma unroll
+    for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+    __syncwarp();
+    if (!live) return;
+    // even part -> cosine channel, odd part -> sine channel, n = 0 .. N / 2
+    const FxUnit oC = fx_out(uC - 2), oD = fx_out(uD - 2);
+    double2* baseC = zspec + static_cast<size_t>(chC) * d.zTotal * P;
+    double2* baseS = zspec + static_cast<size_t>(chS) * d.zTotal * P;
+    auto put = [&](int n, fxc a1, fxc b1) {
+        const size_t o = static_cast<size_t>(n) * P;
+        if (chC >= 0) {
+            const double2 ev = make_double2(fx_to_double(a1.x + b1.x, oC), fx_to_double(a1.y + b1.y, oC));
+            baseC[o + pos] = ev;
+            if (cpos >= 0) baseC[o + cpos] = make_double2(ev.x, -ev.y);
+        }
+        if (chS >= 0) {
+            const double2 od = make_double2(fx_to_double(a1.x - b1.x, oD), fx_to_double(a1.y - b1.y, oD));
+            baseS[o + pos] = od;
+            if (cpos >= 0) baseS[o + cpos] = make_double2(od.x, -od.y);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int n = t + G * i;
+        put(n, v[i], n == 0 ? v[0] : x[fx_pad(N - n)]);
+    }
+    if (t == 0) put(N / 2, v[4], v[4]);
 }
 
-// k_vfwd_fft in fixed point, one retained column per line: (u | w), then (v | eta);
-// lane t projects the coefficients j = t + G i it holds.
+// k_vfwd_fft in fixed point: lines (u | w) and (v | eta) of a column by two warps,
+// which then share its coefficients' projection.
 template <int N, bool FLUX>
-__global__ void __launch_bounds__(32 * kFxZWarps, 2)
+__global__ void __launch_bounds__(32 * kFxZWarps, 3)
     k_vfwd_fx(DescDev d, const double2* __restrict__ fspec, int nch, double elapsed, const double* __restrict__ Ap,
               const double* __restrict__ Am, const double* __restrict__ A0, const unsigned long long* __restrict__ maxSpeedBits,
               int applyDamping, double* __restrict__ Fp, double* __restrict__ Fm, double* __restrict__ F0) {
@@ -380,8 +387,8 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
     constexpr int G = W::G, L = N / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nj = d.Nj, P = d.positions;
-    const int lane = threadIdx.x & 31, t = lane % G;
-    const int own = (threadIdx.x >> 5) * W::lines + lane / G, perBlock = (blockDim.x >> 5) * W::lines;
+    const int lane = threadIdx.x & 31, t = lane % G, warp = threadIdx.x >> 5;
+    const int set = warp >> 1, l = warp & 1, sets = blockDim.x >> 6;
     const int member = blockIdx.y;
     if (member > 0) {
         const long long o = member * d.memberStride;
@@ -391,25 +398,25 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
         if (maxSpeedBits) maxSpeedBits += member;
     }
     fxw* tw = reinterpret_cast<fxw*>(smem_raw);
-    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(own) * W::buffer;
+    const int column = set * W::lines + lane / G;
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(column * 2 + l) * W::buffer;
+    double2* X = reinterpret_cast<double2*>(reinterpret_cast<fxc*>(tw + W::twiddles) +
+                                            static_cast<size_t>(sets) * W::lines * 2 * W::buffer) +
+                 static_cast<size_t>(column) * 2 * N;  // transformed slots [4][N/2]: 0 u, 1 v (cosine), 2 w, 3 eta (sine)
     for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwZ[i];
-    __syncthreads();
-    const int want = blockIdx.x * perBlock + own;
+    const int want = blockIdx.x * sets * W::lines + column;
     const bool live = want < d.Nkl;
     const int mode = min(want, d.Nkl - 1);
-    const int w = d.modeWV[mode];
-    const bool conj = d.modeFlags[mode] & 1;
-    const int pos = d.modePos[mode];
-    int chanOfQ[4] = {-1, -1, -1, -1};
-    for (int c = 0; c < nch; ++c) chanOfQ[FLUX ? d.tq[c] : ((d.hydrostatic && c == 2) ? 3 : c)] = c;
-    // X[q][i]: slots 0 u, 1 v (cosine), 2 w, 3 eta (sine) of j = t + G i
-    double2 X[4][4];
-    const double sc = 1.0 / (static_cast<double>(L) * static_cast<double>(d.Nx) * static_cast<double>(d.Ny));
-#pragma unroll
-    for (int l = 0; l < 2; ++l) {
-        const int cc = chanOfQ[l], cs = chanOfQ[2 + l];
-        const double2* hc = fspec + static_cast<size_t>(cc) * d.zTotal * P + pos;
-        const double2* hs = fspec + static_cast<size_t>(cs) * d.zTotal * P + pos;
+    int cc = -1, cs = -1;  // channels of slots l and 2 + l
+    for (int c = 0; c < nch; ++c) {
+        const int q = FLUX ? d.tq[c] : ((d.hydrostatic && c == 2) ? 3 : c);
+        if (q == l) cc = c;
+        if (q == 2 + l) cs = c;
+    }
+    {
+        const int pos = d.modePos[mode];
+        const double2* hc = fspec + static_cast<size_t>(max(cc, 0)) * d.zTotal * P + pos;
+        const double2* hs = fspec + static_cast<size_t>(max(cs, 0)) * d.zTotal * P + pos;
         double2 a[5], b[4];
         double none5[5], none4[4];
 #pragma unroll
@@ -422,6 +429,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
         int uC, uS;
         fx_quantise_lane<5, G, kFxPlain>(a, none5, 0u, 1, [&](int i) { return (i == 0 && t == 0) || i == 4 ? 1.0f : 2.0f; }, C, uC);
         fx_quantise_lane<4, G, kFxPlain>(b, none4, 0u, 1, [&](int) { return 2.0f; }, S, uS);
+        __syncthreads();  // twiddles
         // y[0] = c_0, y[L] = c_L, y[z] = c_z + s_z, y[N-z] = c_z - s_z
         fxc v[8];
 #pragma unroll
@@ -442,21 +450,25 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int j = t + G * i;
+            if (j >= Nj) continue;
             const fxc p = v[i], q = j == 0 ? v[0] : x[fx_pad(N - j)];
-            X[l][i] = make_double2(fx_to_double(p.x + q.x, oC), fx_to_double(p.y + q.y, oC));
+            X[l * L + j] = make_double2(fx_to_double(p.x + q.x, oC), fx_to_double(p.y + q.y, oC));
             // i times the odd part
-            X[2 + l][i] = make_double2(-fx_to_double(p.y - q.y, oS), fx_to_double(p.x - q.x, oS));
+            X[(2 + l) * L + j] = make_double2(-fx_to_double(p.y - q.y, oS), fx_to_double(p.x - q.x, oS));
         }
-        __syncwarp();
     }
+    __syncthreads();
     if (!live) return;
+    const int w = d.modeWV[mode];
+    const bool conj = d.modeFlags[mode] & 1;
+    const double sc = 1.0 / (static_cast<double>(L) * static_cast<double>(d.Nx) * static_cast<double>(d.Ny));
     double maxSpeed = 0.0;
     if (FLUX && applyDamping) maxSpeed = __longlong_as_double((long long)*maxSpeedBits);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
+#pragma unroll 1
+    for (int i = l; i < 4; i += 2) {
         const int j = t + G * i;
         if (j >= Nj) continue;
-        double2 U = X[0][i], V = X[1][i], Wv = X[2][i], E = X[3][i];
+        double2 U = X[j], V = X[L + j], Wv = X[2 * L + j], E = X[3 * L + j];
         if (conj) { U.y = -U.y; V.y = -V.y; Wv.y = -Wv.y; E.y = -E.y; }
         fx_project<FLUX>(d, w, j, U, V, Wv, E, sc, elapsed, maxSpeed, applyDamping, Ap, Am, A0, Fp, Fm, F0);
     }
