@@ -100,7 +100,15 @@ struct wv_handle {
     // F-grid scalar advection (built on first use): full-spectrum descriptor copy,
     // z-derivative matrix, per-position flags and scratch
     bool scalarReady = false;
-    wvgpu::FxRows fx{};  // FP64: lines of the x pass (length Nx, two rows per line)
+    // Fixed-point lines (FP64 handles always; FP32X2 handles while fxOn): lines of the
+    // x pass (length Nx, two rows per line) and the descriptor with their tables
+    wvgpu::FxRows fx{};
+    dev::DescDev fxd{};
+    // FP32X2: the fluxes, their VJP and the state transforms run on the fixed-point
+    // kernels -- more accurate than paired FP32 and, where every axis has lane-held
+    // lines, faster (2.03 against 2.34 ms a flux at 256x256x129; on the run-time
+    // stages 1.3 to 1.6 times slower) -- until a kernel is chosen explicitly
+    bool fxOn = false;
     dev::DescDev sd{};
     const void* scalarD = nullptr;
     const unsigned char* scalarFlags = nullptr;
@@ -122,6 +130,15 @@ namespace {
 // fails (-1: off), and the device bytes the handles hold right now.
 std::atomic<long long> g_failAllocationAfter{-1};
 std::atomic<long long> g_liveDeviceBytes{0};
+
+// Whether the handle's transforms run on the FP64 templates (fixed-point lines).
+bool fp64_path(const wv_handle* h) { return h->precision == WV_PRECISION_FP64 || h->fxOn; }
+// Descriptor of the working type T.
+template <typename T>
+const dev::DescDev& desc_of(const wv_handle* h) {
+    if constexpr (std::is_same<T, double>::value) return h->fxd;
+    else return h->dd;
+}
 
 bool injected_allocation_failure() {
     if (g_failAllocationAfter.load() < 0) return false;
@@ -526,7 +543,7 @@ template <typename T>
 void launch_yinv(wv_handle* h, const dev::YInvMap& map, const dev::cx<T>* z, dev::cx<T>* y, cudaStream_t s,
                  const dev::DescDev* over = nullptr) {
     const Plan& p = h->plan;
-    const dev::DescDev& dd = over ? *over : h->dd;
+    const dev::DescDev& dd = over ? *over : desc_of<T>(h);
     if constexpr (std::is_same<T, double>::value) {
         if (wvgpu::fx_yinv(p, dd, map, z, y, s)) return;
     }
@@ -543,15 +560,15 @@ template <typename T>
 void launch_yfwd(wv_handle* h, const dev::cx<T>* ps, int nch, dev::cx<T>* f, cudaStream_t s) {
     const Plan& p = h->plan;
     if constexpr (std::is_same<T, double>::value) {
-        if (wvgpu::fx_yfwd(p, h->dd, ps, nch, f, s)) return;
+        if (wvgpu::fx_yfwd(p, desc_of<T>(h), ps, nch, f, s)) return;
     }
     const int ry = warp_ry<T>(p);
     if (ry) {
-        const dim3 grid(cdiv(p.kxColumns, dev::kWG), h->dd.zTotal, nch);
-        WV_RSWITCH_Y(ry, (dev::k_yfwd_w<T, RR><<<grid, 256, smem_y_w<T>(p), s>>>(h->dd, ps, nch, f)));
+        const dim3 grid(cdiv(p.kxColumns, dev::kWG), desc_of<T>(h).zTotal, nch);
+        WV_RSWITCH_Y(ry, (dev::k_yfwd_w<T, RR><<<grid, 256, smem_y_w<T>(p), s>>>(desc_of<T>(h), ps, nch, f)));
         return;
     }
-    dev::k_yfwd<T><<<dim3(cdiv(p.kxColumns, dev::kYG), h->dd.zTotal, nch), 256, smem_y<T>(p), s>>>(h->dd, ps, nch, f);
+    dev::k_yfwd<T><<<dim3(cdiv(p.kxColumns, dev::kYG), desc_of<T>(h).zTotal, nch), 256, smem_y<T>(p), s>>>(desc_of<T>(h), ps, nch, f);
 }
 
 template <typename T>
@@ -559,17 +576,17 @@ void launch_xflux(wv_handle* h, const dev::cx<T>* y, dev::cx<T>* ps, unsigned lo
                   void* physOut = nullptr, double* advOut = nullptr, const double* advIn = nullptr) {
     const Plan& p = h->plan;
     if constexpr (std::is_same<T, double>::value) {
-        if (wvgpu::fx_xflux(p, h->dd, h->fx, y, ps, speed, static_cast<double*>(physOut), advOut, advIn, s)) return;
+        if (wvgpu::fx_xflux(p, desc_of<T>(h), h->fx, y, ps, speed, static_cast<double*>(physOut), advOut, advIn, s)) return;
     }
     const int rx = warp_rx<T>(p);
     if (rx) {
-        const dim3 grid(cdiv(p.Ny, dev::kWG), h->dd.zTotal);
-        WV_RSWITCH_X(T, rx, (dev::k_xflux_w<T, RR><<<grid, 256, smem_xflux_w<T>(p), s>>>(h->dd, y, ps, speed,
+        const dim3 grid(cdiv(p.Ny, dev::kWG), desc_of<T>(h).zTotal);
+        WV_RSWITCH_X(T, rx, (dev::k_xflux_w<T, RR><<<grid, 256, smem_xflux_w<T>(p), s>>>(desc_of<T>(h), y, ps, speed,
                                                                                            static_cast<dev::cx<T>*>(physOut),
                                                                                            advOut, advIn)));
         return;
     }
-    dev::k_xflux<T><<<dim3(p.Ny, h->dd.zTotal), 256, smem_xflux<T>(p), s>>>(h->dd, y, ps, speed, static_cast<T*>(physOut),
+    dev::k_xflux<T><<<dim3(p.Ny, desc_of<T>(h).zTotal), 256, smem_xflux<T>(p), s>>>(desc_of<T>(h), y, ps, speed, static_cast<T*>(physOut),
                                                                            advOut, advIn);
 }
 
@@ -577,7 +594,7 @@ template <typename T>
 void launch_xc2r(wv_handle* h, const dev::cx<T>* y, double* fields, cudaStream_t s, int nch = 4,
                  const dev::DescDev* over = nullptr) {
     const Plan& p = h->plan;
-    const dev::DescDev& dd = over ? *over : h->dd;
+    const dev::DescDev& dd = over ? *over : desc_of<T>(h);
     if constexpr (std::is_same<T, double>::value) {
         if (wvgpu::fx_xc2r(p, dd, h->fx, y, nch, fields, s)) return;
     }
@@ -594,15 +611,15 @@ template <typename T>
 void launch_xr2c(wv_handle* h, const double* fields, int nch, dev::cx<T>* ps, cudaStream_t s) {
     const Plan& p = h->plan;
     if constexpr (std::is_same<T, double>::value) {
-        if (wvgpu::fx_xr2c(p, h->dd, h->fx, fields, nch, ps, s)) return;
+        if (wvgpu::fx_xr2c(p, desc_of<T>(h), h->fx, fields, nch, ps, s)) return;
     }
     const int rx = warp_rx<T>(p);
     if (rx) {
-        const dim3 grid(cdiv(p.Ny, dev::kWG), h->dd.zTotal);
-        WV_RSWITCH_X(T, rx, (dev::k_xr2c_fields_w<T, RR><<<grid, 256, smem_xr2c_w<T>(p), s>>>(h->dd, fields, nch, ps)));
+        const dim3 grid(cdiv(p.Ny, dev::kWG), desc_of<T>(h).zTotal);
+        WV_RSWITCH_X(T, rx, (dev::k_xr2c_fields_w<T, RR><<<grid, 256, smem_xr2c_w<T>(p), s>>>(desc_of<T>(h), fields, nch, ps)));
         return;
     }
-    dev::k_xr2c_fields<T><<<dim3(p.Ny, h->dd.zTotal), 256, smem_xr2c<T>(p), s>>>(h->dd, fields, nch, ps);
+    dev::k_xr2c_fields<T><<<dim3(p.Ny, desc_of<T>(h).zTotal), 256, smem_xr2c<T>(p), s>>>(desc_of<T>(h), fields, nch, ps);
 }
 
 // The vertical transforms of FP64 handles on lane-held lines; false where the
@@ -611,7 +628,7 @@ template <typename T>
 bool launch_vinv_fx(wv_handle* h, bool flux, double elapsed, const double* Ap, const double* Am, const double* A0,
                     dev::cx<T>* z, unsigned long long* speed, cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value)
-        return wvgpu::fx_vinv(h->plan, h->dd, flux, elapsed, Ap, Am, A0, z, speed, s);
+        return wvgpu::fx_vinv(h->plan, desc_of<T>(h), flux, elapsed, Ap, Am, A0, z, speed, s);
     return false;
 }
 template <typename T>
@@ -619,7 +636,7 @@ bool launch_vfwd_fx(wv_handle* h, bool flux, const dev::cx<T>* f, int nch, doubl
                     const double* A0, const unsigned long long* speed, int damping, double* Fp, double* Fm, double* F0,
                     cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value)
-        return wvgpu::fx_vfwd(h->plan, h->dd, flux, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0, s);
+        return wvgpu::fx_vfwd(h->plan, desc_of<T>(h), flux, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0, s);
     return false;
 }
 
@@ -631,7 +648,7 @@ template <typename T>
 void launch_vinv_flux(wv_handle* h, double elapsed, const double* Ap, const double* Am, const double* A0, dev::cx<T>* z,
                       unsigned long long* speed, dev::cx<T>* yScratch, cudaStream_t s) {
     const Plan& p = h->plan;
-    const auto& d = h->dd;
+    const auto& d = desc_of<T>(h);
     auto* y = yScratch;
     if constexpr (sizeof(T) == 4) {
         if (h->vinvKind == WV_VERTICAL_TENSOR_CORES) {
@@ -682,7 +699,7 @@ cudaError_t launch_flux(wv_handle* h, double t, double t0, const double* Ap, con
                         double* Fp, double* Fm, double* F0, bool damping, cudaStream_t s, void* physOut = nullptr,
                         double* advOut = nullptr, const double* advIn = nullptr, const FluxScratch* scratch = nullptr) {
     const Plan& p = h->plan;
-    const auto& d = h->dd;
+    const auto& d = desc_of<T>(h);
     const double elapsed = t - t0;
     if (h->failLaunchAfter >= 0 && h->failLaunchAfter-- == 0) {  // test hook: fail before any launch
         h->injectedFailure = true;
@@ -978,7 +995,7 @@ template <typename T>
 cudaError_t launch_inverse(wv_handle* h, double t, double t0, const double* Ap, const double* Am, const double* A0,
                            double* fields, cudaStream_t s, int nch = 4) {
     const Plan& p = h->plan;
-    const auto& d = h->dd;
+    const auto& d = desc_of<T>(h);
     auto* z = static_cast<dev::cx<T>*>(h->zspec);
     auto* y = static_cast<dev::cx<T>*>(h->yspec);
     if (!launch_vinv_fx<T>(h, false, t - t0, Ap, Am, A0, z, nullptr, s))
@@ -996,7 +1013,7 @@ template <typename T>
 cudaError_t launch_forward(wv_handle* h, const double* fields, double t, double t0, double* Ap, double* Am, double* A0,
                            cudaStream_t s) {
     const Plan& p = h->plan;
-    const auto& d = h->dd;
+    const auto& d = desc_of<T>(h);
     const int nch = h->desc.c.is_hydrostatic ? 3 : 4;
     auto* ps = static_cast<dev::cx<T>*>(h->pspec);
     auto* f = static_cast<dev::cx<T>*>(h->fspec);
@@ -1085,6 +1102,10 @@ int ensure_adjoint(wv_handle* h) {
     const cudaError_t lim = h->precision == WV_PRECISION_FP64    ? set_smem_limits_adj<double>(p)
                             : h->precision == WV_PRECISION_MIXED ? set_smem_limits_adj<float>(p)
                                                                  : set_smem_limits_adj<dev::ff>(p);
+    if (lim == cudaSuccess && h->fxOn) {
+        const cudaError_t e = wvgpu::fx_set_limits_adj(p);
+        if (e != cudaSuccess) return cuda_fail(h, e, "adjoint set-up");
+    }
     if (lim == cudaErrorInvalidConfiguration)
         return fail(h, WV_UNSUPPORTED_OPERATION, "The adjoint kernels need more shared memory than one CTA has for this grid.");
     if (lim != cudaSuccess) return cuda_fail(h, lim, "adjoint set-up");
@@ -1096,7 +1117,7 @@ int ensure_adjoint(wv_handle* h) {
     if (e == cudaSuccess) e = alloc(h, nIn * p.Nz * p.positions * cb, &h->fadj);
     const size_t stateBytes = 6 * p.M * sizeof(double);
     void* tmp = nullptr;
-    if (e == cudaSuccess && h->precision == WV_PRECISION_FP64 && wvgpu::fx_has_rows(p)) {
+    if (e == cudaSuccess && fp64_path(h) && wvgpu::fx_has_rows(p)) {
         e = alloc(h, (3 + 3 * nt) * p.Nx * p.Ny * p.Nz * sizeof(double), &tmp);
         h->adjRows = static_cast<double*>(tmp);
     }
@@ -1139,7 +1160,7 @@ cudaError_t launch_flux_vjp(wv_handle* h, double t, double t0, const double* Ap,
                             const double* Fpb, const double* Fmb, const double* F0b, double* Apb, double* Amb, double* A0b,
                             cudaStream_t s, const void* physIn = nullptr) {
     const Plan& p = h->plan;
-    const auto& d = h->dd;
+    const auto& d = desc_of<T>(h);
     const double elapsed = t - t0;
     const int nt = p.targets.count, nIn = 4 + 2 * nt;
     auto* za = static_cast<dev::cx<T>*>(h->zadj);
@@ -1251,7 +1272,7 @@ cudaError_t launch_inverse_vjp(wv_handle* h, double t, double t0, const double* 
 cudaError_t flux_vjp_any(wv_handle* h, double t, double t0, const double* y, const double* yb, double* out, cudaStream_t s,
                          const void* physIn = nullptr) {
     const size_t M2 = 2 * h->plan.M;
-    return h->precision == WV_PRECISION_FP64
+    return fp64_path(h)
                ? launch_flux_vjp<double>(h, t, t0, y, y + M2, y + 2 * M2, yb, yb + M2, yb + 2 * M2, out, out + M2, out + 2 * M2, s, physIn)
                : h->precision == WV_PRECISION_MIXED ? launch_flux_vjp<float>(h, t, t0, y, y + M2, y + 2 * M2, yb, yb + M2, yb + 2 * M2, out, out + M2, out + 2 * M2, s, physIn)
                                                           : launch_flux_vjp<dev::ff>(h, t, t0, y, y + M2, y + 2 * M2, yb, yb + M2, yb + 2 * M2, out, out + M2, out + 2 * M2, s, physIn);
@@ -1260,7 +1281,7 @@ cudaError_t flux_vjp_any(wv_handle* h, double t, double t0, const double* y, con
 cudaError_t flux_any(wv_handle* h, double t, double t0, const double* Ap, const double* Am, const double* A0, double* Fp,
                      double* Fm, double* F0, bool damping, cudaStream_t s, void* physOut = nullptr, double* advOut = nullptr,
                      const double* advIn = nullptr) {
-    return h->precision == WV_PRECISION_FP64
+    return fp64_path(h)
                ? launch_flux<double>(h, t, t0, Ap, Am, A0, Fp, Fm, F0, damping, s, physOut, advOut, advIn)
                : h->precision == WV_PRECISION_MIXED ? launch_flux<float>(h, t, t0, Ap, Am, A0, Fp, Fm, F0, damping, s, physOut, advOut, advIn)
                                                           : launch_flux<dev::ff>(h, t, t0, Ap, Am, A0, Fp, Fm, F0, damping, s, physOut, advOut, advIn);
@@ -1567,34 +1588,6 @@ static int create_handle(const wv_config* config, int precision, int members, wv
     for (int i = 0; i < dev::kMaxStages; ++i) { dd.fx.radix[i] = p.fx.radix[i]; dd.fy.radix[i] = p.fy.radix[i]; }
     dd.fz.N = p.fz.N; dd.fz.nstages = p.fz.nstages;
     for (int i = 0; i < dev::kMaxStages; ++i) dd.fz.radix[i] = p.fz.radix[i];
-    if (precision == WV_PRECISION_FP64) {  // fixed-point lines: their own factors and twiddles
-        auto fixed_point_fft = [](size_t N) {
-            const wvgpu::FFTFactors q = wvgpu::factor_fixed_point(static_cast<int>(N));
-            dev::FFTDev f{};
-            f.N = q.N; f.nstages = q.nstages;
-            for (int i = 0; i < dev::kMaxStages; ++i) f.radix[i] = q.radix[i];
-            return f;
-        };
-        for (dev::FFTDev* f : {&dd.fx, &dd.fy, &dd.fz})
-            if (f->N) *f = fixed_point_fft(f->N);
-        h->fx.x = fixed_point_fft(p.Nx);
-        auto table = [&](const std::vector<int32_t>& v, const dev::fxw** dst) {
-            if (e != cudaSuccess || v.empty()) return;
-            const int32_t* q = nullptr;
-            e = upload(h, v, &q);
-            *dst = reinterpret_cast<const dev::fxw*>(q);
-        };
-        table(wvgpu::fixed_point_twiddles(static_cast<int>(p.Nx)), &h->fx.twX);
-        table(wvgpu::fx_lane_table(p.Nx), &h->fx.twXLane);
-        table(wvgpu::fx_lane_table(p.Ny), &dd.fxTwY);
-        table(wvgpu::fx_lane_table(p.fz.N), &dd.fxTwZ);
-        // exp(+2 pi i k / 256): the forward table read backwards
-        const std::vector<int32_t> forward = wvgpu::fixed_point_twiddles(256);
-        std::vector<int32_t> phases(forward.size());
-        for (int k = 0; k < 256; ++k)
-            std::copy_n(forward.begin() + 4 * ((256 - k) % 256), 4, phases.begin() + 4 * k);
-        table(phases, &dd.fxPhase);
-    }
     std::vector<int32_t> ymap(p.ymap);
     std::vector<int32_t> posKy(p.posKy), colStart(p.colStart), modeWV(p.modeWV), modePos(p.modePos), modeComp(p.modeCompPos);
     std::vector<double> inertial(d.inertialScale), apmw(d.apmWProjectionPrefactor);
@@ -1649,15 +1642,11 @@ static int create_handle(const wv_config* config, int precision, int members, wv
     };
     upT(p.Ccos, &dd.Ccos); upT(p.Csin, &dd.Csin); upT(p.CcosM, &dd.CcosM); upT(p.CsinM, &dd.CsinM);
     upT(p.Fcos, &dd.Fcos); upT(p.Fsin, &dd.Fsin); upT(p.twxN, &dd.twxN);
-    auto upTw = [&](const std::vector<double>& v, int N, const void** dst) {
-        if (precision != WV_PRECISION_FP64) { upT(v, dst); return; }
-        if (e != cudaSuccess) return;
-        const int32_t* q = nullptr;
-        e = upload(h, wvgpu::fixed_point_twiddles(N), &q);
-        *dst = q;
-    };
-    upTw(p.twx, p.fx.N, &dd.twx); upTw(p.twy, p.fy.N, &dd.twy);
-    if (p.fz.N > 0) { upTw(p.twz, p.fz.N, &dd.twz); upT(std::vector<double>(d.m.begin(), d.m.begin() + p.Nj), &dd.tMz); }
+    if (precision != WV_PRECISION_FP64) {  // (FP64: fixed-point tables below)
+        upT(p.twx, &dd.twx); upT(p.twy, &dd.twy);
+        if (p.fz.N > 0) upT(p.twz, &dd.twz);
+    }
+    if (p.fz.N > 0) upT(std::vector<double>(d.m.begin(), d.m.begin() + p.Nj), &dd.tMz);
     upT(p.rowK, &dd.tRowK); upT(p.rowL, &dd.tRowL);
     {
         auto transpose = [](const std::vector<double>& a, size_t rows, size_t cols) {
@@ -1769,6 +1758,55 @@ static int create_handle(const wv_config* config, int precision, int members, wv
             h->vfwdKind = fft ? WV_VERTICAL_FFT : WV_VERTICAL_CUDA_CORES;
         }
     }
+    // fixed-point lines: their own factors and twiddles, doubles where the working type has its copies
+    h->fxOn = precision == WV_PRECISION_FP32X2 && wvgpu::fx_all_lanes(p);
+    if (precision == WV_PRECISION_FP64 || h->fxOn) {
+        dev::DescDev& fd = h->fxd;
+        fd = dd;
+        auto fixed_point_fft = [](size_t N) {
+            const wvgpu::FFTFactors q = wvgpu::factor_fixed_point(static_cast<int>(N));
+            dev::FFTDev f{};
+            f.N = q.N; f.nstages = q.nstages;
+            for (int i = 0; i < dev::kMaxStages; ++i) f.radix[i] = q.radix[i];
+            return f;
+        };
+        for (dev::FFTDev* f : {&fd.fx, &fd.fy, &fd.fz})
+            if (f->N) *f = fixed_point_fft(f->N);
+        h->fx.x = fixed_point_fft(p.Nx);
+        auto table = [&](const std::vector<int32_t>& v, const dev::fxw** dst) {
+            if (e != cudaSuccess || v.empty()) return;
+            const int32_t* q = nullptr;
+            e = upload(h, v, &q);
+            *dst = reinterpret_cast<const dev::fxw*>(q);
+        };
+        table(wvgpu::fixed_point_twiddles(static_cast<int>(p.Nx)), &h->fx.twX);
+        table(wvgpu::fx_lane_table(p.Nx), &h->fx.twXLane);
+        auto words = [&](int N, const void** dst) {
+            const dev::fxw* q = nullptr;
+            table(wvgpu::fixed_point_twiddles(N), &q);
+            *dst = q;
+        };
+        words(fd.fx.N, &fd.twx);
+        words(fd.fy.N, &fd.twy);
+        if (fd.fz.N > 0) words(fd.fz.N, &fd.twz);
+        table(wvgpu::fx_lane_table(p.Ny), &fd.fxTwY);
+        table(wvgpu::fx_lane_table(p.fz.N), &fd.fxTwZ);
+        // exp(+2 pi i k / 256): the forward table read backwards
+        const std::vector<int32_t> forward = wvgpu::fixed_point_twiddles(256);
+        std::vector<int32_t> phases(forward.size());
+        for (int k = 0; k < 256; ++k)
+            std::copy_n(forward.begin() + 4 * ((256 - k) % 256), 4, phases.begin() + 4 * k);
+        table(phases, &fd.fxPhase);
+        if (h->fxOn) {
+            fd.tRowK = dd.rowK;
+            fd.tRowL = dd.rowL;
+            const double* m = nullptr;
+            if (e == cudaSuccess) e = upload(h, std::vector<double>(d.m.begin(), d.m.begin() + p.Nj), &m);
+            fd.tMz = m;
+        } else {
+            dd = fd;
+        }
+    }
     const auto ss = scratch_sizes(p);
     const size_t cb = 2 * elem_size(precision);
     const size_t R = p.Nx * p.Ny * p.Nz;
@@ -1792,6 +1830,7 @@ static int create_handle(const wv_config* config, int precision, int members, wv
     if (e == cudaSuccess)
         e = precision == WV_PRECISION_FP64 ? set_smem_limits_w<double>(p)
             : precision == WV_PRECISION_MIXED ? set_smem_limits_w<float>(p) : set_smem_limits_w<dev::ff>(p);
+    if (e == cudaSuccess && h->fxOn) e = wvgpu::fx_set_limits(p);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         const int code = e == cudaErrorMemoryAllocation ? WV_ALLOCATION_FAILURE : WV_FFT_PLAN_FAILURE;
@@ -1837,6 +1876,7 @@ int wv_set_vertical_kernels(wv_handle* h, int inverse_kind, int forward_kind) {
                     "The tensor-core forward vertical transform needs a mixed-precision handle with Nz <= 255.");
     h->vinvKind = inverse_kind;
     h->vfwdKind = forward_kind;
+    h->fxOn = false;
     return WV_SUCCESS;
 }
 
@@ -1867,6 +1907,7 @@ int wv_set_fft_variants(wv_handle* h, int y_variant, int x_variant) {
     if (!known(y_variant) || !known(x_variant)) return fail(h, WV_INVALID_CONFIGURATION, "Unknown FFT variant.");
     h->plan.stockhamY = y_variant == WV_FFT_STOCKHAM;
     h->plan.stockhamX = x_variant == WV_FFT_STOCKHAM;
+    h->fxOn = false;
     return WV_SUCCESS;
 }
 
@@ -2008,7 +2049,7 @@ int wv_inverse_device(wv_handle* h, double t, double t0, const double* Ap, const
     Guard g(h->busy);
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "Kernel operations are not reentrant.");
     cudaSetDevice(h->device);
-    const cudaError_t e = h->precision == WV_PRECISION_FP64
+    const cudaError_t e = fp64_path(h)
                               ? launch_inverse<double>(h, t, t0, Ap, Am, A0, fields, static_cast<cudaStream_t>(stream))
                               : h->precision == WV_PRECISION_MIXED ? launch_inverse<float>(h, t, t0, Ap, Am, A0, fields, static_cast<cudaStream_t>(stream))
                                                                          : launch_inverse<dev::ff>(h, t, t0, Ap, Am, A0, fields, static_cast<cudaStream_t>(stream));
@@ -2071,7 +2112,7 @@ int wv_inverse_uvw_device(wv_handle* h, double t, double t0, const double* Ap, c
     Guard g(h->busy);
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "Kernel operations are not reentrant.");
     cudaSetDevice(h->device);
-    const cudaError_t e = h->precision == WV_PRECISION_FP64
+    const cudaError_t e = fp64_path(h)
                               ? launch_inverse<double>(h, t, t0, Ap, Am, A0, fields, static_cast<cudaStream_t>(stream), 3)
                               : h->precision == WV_PRECISION_MIXED ? launch_inverse<float>(h, t, t0, Ap, Am, A0, fields, static_cast<cudaStream_t>(stream), 3)
                                                                          : launch_inverse<dev::ff>(h, t, t0, Ap, Am, A0, fields, static_cast<cudaStream_t>(stream), 3);
@@ -2134,7 +2175,7 @@ int wv_inverse_uvw(wv_handle* h, double t, double t0, const double* Ap, const do
     for (int c = 0; c < 3 && e == cudaSuccess; ++c)
         e = cudaMemcpyAsync(reinterpret_cast<char*>(h->state) + c * cb, in[c], cb, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = h->precision == WV_PRECISION_FP64
+        e = fp64_path(h)
                 ? launch_inverse<double>(h, t, t0, h->state, h->state + M2, h->state + 2 * M2, h->fields, s, 3)
                 : h->precision == WV_PRECISION_MIXED ? launch_inverse<float>(h, t, t0, h->state, h->state + M2, h->state + 2 * M2, h->fields, s, 3)
                                                            : launch_inverse<dev::ff>(h, t, t0, h->state, h->state + M2, h->state + 2 * M2, h->fields, s, 3);
@@ -2291,7 +2332,7 @@ int wv_forward_device(wv_handle* h, const double* fields, double t, double t0, d
     Guard g(h->busy);
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "Kernel operations are not reentrant.");
     cudaSetDevice(h->device);
-    const cudaError_t e = h->precision == WV_PRECISION_FP64
+    const cudaError_t e = fp64_path(h)
                               ? launch_forward<double>(h, fields, t, t0, Ap, Am, A0, static_cast<cudaStream_t>(stream))
                               : h->precision == WV_PRECISION_MIXED ? launch_forward<float>(h, fields, t, t0, Ap, Am, A0, static_cast<cudaStream_t>(stream))
                                                                          : launch_forward<dev::ff>(h, fields, t, t0, Ap, Am, A0, static_cast<cudaStream_t>(stream));
@@ -2483,7 +2524,7 @@ int wv_inverse(wv_handle* h, double t, double t0, const double* Ap, const double
     for (int c = 0; c < 3 && e == cudaSuccess; ++c)
         e = cudaMemcpyAsync(reinterpret_cast<char*>(h->state) + c * cb, in[c], cb, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = h->precision == WV_PRECISION_FP64
+        e = fp64_path(h)
                 ? launch_inverse<double>(h, t, t0, h->state, h->state + M2, h->state + 2 * M2, h->fields, s)
                 : h->precision == WV_PRECISION_MIXED ? launch_inverse<float>(h, t, t0, h->state, h->state + M2, h->state + 2 * M2, h->fields, s)
                                                            : launch_inverse<dev::ff>(h, t, t0, h->state, h->state + M2, h->state + 2 * M2, h->fields, s);
@@ -2506,7 +2547,7 @@ int wv_forward(wv_handle* h, const double* fields, double t, double t0, double* 
     auto s = h->stream;
     cudaError_t e = cudaMemcpyAsync(h->fields, fields, fb, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = h->precision == WV_PRECISION_FP64
+        e = fp64_path(h)
                 ? launch_forward<double>(h, h->fields, t, t0, h->flux, h->flux + M2, h->flux + 2 * M2, s)
                 : h->precision == WV_PRECISION_MIXED ? launch_forward<float>(h, h->fields, t, t0, h->flux, h->flux + M2, h->flux + 2 * M2, s)
                                                            : launch_forward<dev::ff>(h, h->fields, t, t0, h->flux, h->flux + M2, h->flux + 2 * M2, s);
@@ -2571,7 +2612,7 @@ int wv_flux_vjp_device(wv_handle* h, double t, double t0, const double* Ap, cons
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "Kernel operations are not reentrant.");
     rc = adjoint_preamble(h); if (rc) return rc;
     auto s = static_cast<cudaStream_t>(stream);
-    const cudaError_t e = h->precision == WV_PRECISION_FP64
+    const cudaError_t e = fp64_path(h)
         ? launch_flux_vjp<double>(h, t, t0, Ap, Am, A0, Fpb, Fmb, F0b, Apb, Amb, A0b, s)
         : h->precision == WV_PRECISION_MIXED ? launch_flux_vjp<float>(h, t, t0, Ap, Am, A0, Fpb, Fmb, F0b, Apb, Amb, A0b, s)
                                                    : launch_flux_vjp<dev::ff>(h, t, t0, Ap, Am, A0, Fpb, Fmb, F0b, Apb, Amb, A0b, s);
@@ -2791,7 +2832,7 @@ int wv_nonlinear_flux_device_noalloc(wv_handle* h, double t, double t0, const do
     const FluxScratch sc{sb + offs[0], sb + offs[1], sb + offs[2], sb + offs[3],
                          reinterpret_cast<unsigned long long*>(sb + offs[4])};
     // the same launch sequence (and kernel choice) as wv_nonlinear_flux_device, without damping
-    e = h->precision == WV_PRECISION_FP64
+    e = fp64_path(h)
             ? launch_flux<double>(h, t, t0, Ap, Am, A0, Fp, Fm, F0, false, s, nullptr, nullptr, nullptr, &sc)
         : h->precision == WV_PRECISION_MIXED
             ? launch_flux<float>(h, t, t0, Ap, Am, A0, Fp, Fm, F0, false, s, nullptr, nullptr, nullptr, &sc)
@@ -3039,6 +3080,7 @@ int wv_ensemble_set_vertical_kernel(wv_ensemble* e, int kind) {
                          "The tensor-core vertical transform needs mixed-precision (Nz <= 255) or FP32X2 (Nj <= 96) groups.");
     for (size_t g = 0; g < e->groups.size(); ++g) {
         wv_handle* h = e->groups[g];
+        h->fxOn = false;
         h->vinvKind = kind;
         h->vfwdKind = kind == WV_VERTICAL_TENSOR_CORES && !h->tcFwdAvailable ? WV_VERTICAL_CUDA_CORES : kind;
         e->tuning[g].vertical = h->vinvKind;

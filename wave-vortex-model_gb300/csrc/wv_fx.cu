@@ -16,22 +16,32 @@ namespace {
 
 unsigned cdiv(size_t a, size_t b) { return static_cast<unsigned>((a + b - 1) / b); }
 
-// Line lengths held by the lanes of a warp (wv_fxwarp.cuh).
-#define WV_FXW_SWITCH(N, ...)                             \
-    switch (N) {                                          \
-        case 16: { constexpr int NN = 16; __VA_ARGS__; } break;   \
-        case 32: { constexpr int NN = 32; __VA_ARGS__; } break;   \
-        case 64: { constexpr int NN = 64; __VA_ARGS__; } break;   \
-        case 128: { constexpr int NN = 128; __VA_ARGS__; } break; \
-        case 256: { constexpr int NN = 256; __VA_ARGS__; } break; \
-        default: break;                                   \
+// Line lengths held by the lanes of a warp (wv_fxwarp.cuh); NN: the length.
+#define WV_FXW_CASE(LEN, ...) case LEN: { constexpr int NN = LEN; __VA_ARGS__; } break
+#define WV_FXW_SWITCH(N, ...)          \
+    switch (N) {                       \
+        WV_FXW_CASE(16, __VA_ARGS__);  \
+        WV_FXW_CASE(24, __VA_ARGS__);  \
+        WV_FXW_CASE(32, __VA_ARGS__);  \
+        WV_FXW_CASE(48, __VA_ARGS__);  \
+        WV_FXW_CASE(64, __VA_ARGS__);  \
+        WV_FXW_CASE(96, __VA_ARGS__);  \
+        WV_FXW_CASE(128, __VA_ARGS__); \
+        WV_FXW_CASE(192, __VA_ARGS__); \
+        WV_FXW_CASE(256, __VA_ARGS__); \
+        default: break;                \
     }
-inline bool fx_lane_length(size_t N) { return N == 16 || N == 32 || N == 64 || N == 128 || N == 256; }
+// Lines of a warp; 0: no lane-held line of this length.
+inline size_t fx_lane_lines(size_t N) {
+    WV_FXW_SWITCH(N, return dev::FxW<NN>::lines);
+    return 0;
+}
+inline bool fx_lane_length(size_t N) { return fx_lane_lines(N) != 0; }
 template <int N>
 std::vector<int32_t> lane_table() {
     using W = dev::FxW<N>;
-    if (W::R3 > 1) return fixed_point_stage_twiddles(N, {8, W::R2, W::R3});
-    return fixed_point_stage_twiddles(N, {8, W::R2});
+    if (W::R3 > 1) return fixed_point_stage_twiddles(N, {W::R1, W::R2, W::R3});
+    return fixed_point_stage_twiddles(N, {W::R1, W::R2});
 }
 
 // The x pass: lane-held rows where the length allows (kx < Nx / 2 always holds on
@@ -39,13 +49,23 @@ std::vector<int32_t> lane_table() {
 // run-time stages; longer rows keep the block kernel.
 inline bool fx_x_lane(const Plan& p) { return fx_lane_length(p.Nx) && 2 * p.kxColumns <= p.Nx; }
 inline bool fx_x_any(const Plan& p) { return p.Nx <= 512 && p.kxColumns <= 256; }
+// Forms of the x pass at a length: spectrum entries of a lane under the 2/3 rule and at
+// most; whether the one-warp-a-row form exists.  That form is the faster one at 128
+// points with many rows (0.132 against 0.150 ms at 128x128x65, above 6 line-sets of rows
+// an SM) and loses at 256 (1.22 against 1.14 ms at 256x256x129) and on small grids
+// (0.037 against 0.022 ms at 64x64x33).
 constexpr size_t kFxCoUnits = 6;
 template <int N>
-size_t smem_xflux_fx() { return dev::FxW<N>::twiddles * sizeof(dev::fxw) + dev::kFxXWarps * dev::fx_xflux_warp_bytes(N); }
+struct XKernels {
+    static constexpr int few = dev::FxW<N>::E == 8 ? 3 : 5, all = dev::FxW<N>::H;
+    static constexpr bool rowForm = dev::FxW<N>::E == 8 && N < 256;
+};
+template <int N>
+size_t smem_xflux_fx() { return dev::FxW<N>::twiddles * sizeof(dev::fxw) + dev::kFxXWarps * dev::fx_xflux_warp_bytes<N>(); }
 // Warps of a y or z block: 8, fewer where the columns of a plane (the retained
 // columns) do not fill them; powers of two in y, as the tile's swizzle needs.
 inline int fx_y_warps(size_t Ny, size_t kxColumns) {
-    const size_t lines = 256 / Ny;
+    const size_t lines = fx_lane_lines(Ny);
     int warps = 1;
     while (warps < dev::kFxYWarps && warps * lines < kxColumns) warps *= 2;
     return warps;
@@ -53,7 +73,7 @@ inline int fx_y_warps(size_t Ny, size_t kxColumns) {
 // Column sets of a z block (its warps: sets x lines of a column): enough blocks for
 // every SM before the blocks grow to 8 warps.
 inline int fx_z_sets(const Plan& p, int lines) {
-    const size_t columns = 256 / p.fz.N, units = (p.Nkl + columns - 1) / columns, sms = grid_cap(1);
+    const size_t columns = fx_lane_lines(p.fz.N), units = (p.Nkl + columns - 1) / columns, sms = grid_cap(1);
     return static_cast<int>(std::min<size_t>(dev::kFxZWarps / lines, std::max<size_t>(1, units / sms)));
 }
 // Lines of any length along z: warps of a block, as shared memory allows.
@@ -107,8 +127,8 @@ cudaError_t fx_set_limits(const Plan& p) {
         if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(kernel), static_cast<int>(bytes));
     };
     WV_FXW_SWITCH(p.Ny, {
-        set(dev::k_yinv_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * (256 / NN)));
-        set(dev::k_yfwd_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * (256 / NN)));
+        set(dev::k_yinv_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * dev::FxW<NN>::lines));
+        set(dev::k_yfwd_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * dev::FxW<NN>::lines));
     });
     if (!fx_lane_length(p.Ny)) {
         // (the scalar pipeline has the most columns)
@@ -134,7 +154,17 @@ cudaError_t fx_set_limits(const Plan& p) {
         set(dev::k_vfwd_fx<NN, true>, dev::smem_fx_z<NN>(2, 4));
         set(dev::k_vfwd_fx<NN, false>, dev::smem_fx_z<NN>(2, 4));
     });
-    if (fx_x_lane(p)) { WV_FXW_SWITCH(p.Nx, set(dev::k_xflux_fx<NN, 3>, smem_xflux_fx<NN>()); set(dev::k_xflux_fx<NN, 4>, smem_xflux_fx<NN>()); set(dev::k_xflux_fxco<NN, 3>, dev::smem_xflux_co<NN>()); set(dev::k_xflux_fxco<NN, 4>, dev::smem_xflux_co<NN>())); }
+    if (fx_x_lane(p)) {
+        WV_FXW_SWITCH(p.Nx, {
+            using X = XKernels<NN>;
+            if constexpr (X::rowForm) {
+                set(dev::k_xflux_fx<NN, X::few>, smem_xflux_fx<NN>());
+                set(dev::k_xflux_fx<NN, X::all>, smem_xflux_fx<NN>());
+            }
+            set(dev::k_xflux_fxco<NN, X::few>, dev::smem_xflux_co<NN>());
+            set(dev::k_xflux_fxco<NN, X::all>, dev::smem_xflux_co<NN>());
+        });
+    }
     else if (fx_x_any(p)) { WV_FXX_SWITCH(p.kxColumns, set(dev::k_xflux_fxany<EK>, fx_x_launch(p, 1).smem)); }
     return e;
 }
@@ -148,7 +178,7 @@ cudaError_t fx_set_limits_adj(const Plan& p) {
         set(dev::k_vfwd_adj_fx<NN>, dev::smem_fx_z<NN>(2, 4));
         set(dev::k_vinv_adj_fx<NN>, dev::smem_fx_vinv_adj<NN>(2));
     });
-    WV_FXW_SWITCH(p.Ny, set(dev::k_yfwd_pair_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * (256 / NN))));
+    WV_FXW_SWITCH(p.Ny, set(dev::k_yfwd_pair_fx<NN>, dev::smem_fxy<NN>(dev::kFxYWarps * dev::FxW<NN>::lines)));
     if (fx_x_lane(p)) { WV_FXW_SWITCH(p.Nx, set(dev::k_xadj_fx<NN>, dev::smem_xadj_fx<NN>())); }
     return e;
 }
@@ -157,7 +187,7 @@ bool fx_vfwd_adj(const Plan& p, const dev::DescDev& d, const double* Fpb, const 
                  double2* zadj, cudaStream_t s) {
     if (!fx_lane_length(p.fz.N)) return false;
     const int sets = fx_z_sets(p, 2);
-    WV_FXW_SWITCH(p.fz.N, (dev::k_vfwd_adj_fx<NN><<<cdiv(p.Nkl, sets * (256 / NN)), 64 * sets, dev::smem_fx_z<NN>(2, sets), s>>>(
+    WV_FXW_SWITCH(p.fz.N, (dev::k_vfwd_adj_fx<NN><<<cdiv(p.Nkl, sets * dev::FxW<NN>::lines), 64 * sets, dev::smem_fx_z<NN>(2, sets), s>>>(
                               d, Fpb, Fmb, F0b, elapsed, zadj)));
     return true;
 }
@@ -166,7 +196,7 @@ bool fx_vinv_adj(const Plan& p, const dev::DescDev& d, const double2* fadj, doub
                  double* A0b, cudaStream_t s) {
     if (!fx_lane_length(p.fz.N)) return false;
     const int sets = fx_z_sets(p, 4);
-    WV_FXW_SWITCH(p.fz.N, (dev::k_vinv_adj_fx<NN><<<cdiv(p.Nkl, sets * (256 / NN)), 128 * sets, dev::smem_fx_vinv_adj<NN>(sets), s>>>(
+    WV_FXW_SWITCH(p.fz.N, (dev::k_vinv_adj_fx<NN><<<cdiv(p.Nkl, sets * dev::FxW<NN>::lines), 128 * sets, dev::smem_fx_vinv_adj<NN>(sets), s>>>(
                               d, fadj, elapsed, Apb, Amb, A0b)));
     return true;
 }
@@ -174,7 +204,7 @@ bool fx_vinv_adj(const Plan& p, const dev::DescDev& d, const double2* fadj, doub
 bool fx_yfwd_pair(const Plan& p, const dev::DescDev& d, const dev::YFwdPairMap& map, const double2* y, int nIn, double2* f,
                   cudaStream_t s) {
     if (!fx_lane_length(p.Ny)) return false;
-    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(256 / p.Ny);
+    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
     const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, map.nOut);
     WV_FXW_SWITCH(p.Ny, (dev::k_yfwd_pair_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(d, map, y, nIn, f)));
     return true;
@@ -183,33 +213,37 @@ bool fx_yfwd_pair(const Plan& p, const dev::DescDev& d, const dev::YFwdPairMap& 
 bool fx_xadj(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* yadj, double2* yout, const double* rowsIn,
              cudaStream_t s) {
     if (!fx_x_lane(p) || !rowsIn) return false;
-    const size_t rows = p.Ny * static_cast<size_t>(d.zTotal), lines = 256 / p.Nx;
+    const size_t rows = p.Ny * static_cast<size_t>(d.zTotal), lines = fx_lane_lines(p.Nx);
     WV_FXW_SWITCH(p.Nx, (dev::k_xadj_fx<NN><<<cdiv(rows, lines), 32 * dev::kFxCoWarps, dev::smem_xadj_fx<NN>(), s>>>(
                             d, r.twXLane, yadj, yout, rowsIn)));
     return true;
 }
+
+bool fx_all_lanes(const Plan& p) { return fx_x_lane(p) && fx_lane_length(p.Ny) && fx_lane_length(p.fz.N); }
 
 bool fx_has_rows(const Plan& p) { return fx_x_lane(p) || fx_x_any(p); }
 
 bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* y, double2* ps,
               unsigned long long* speed, double* physOut, double* advOut, const double* advIn, cudaStream_t s) {
     if (fx_x_lane(p)) {
-        // one block per SM; fewer warps a block where there are too few rows to fill it
-        const size_t rows = p.Ny * p.Nz * d.members, perWarp = 256 / p.Nx;
+        const size_t rows = p.Ny * p.Nz * d.members, perWarp = fx_lane_lines(p.Nx);
         const size_t units = (rows + perWarp - 1) / perWarp, sms = grid_cap(1);
-        if (p.Nx == 256 || units <= kFxCoUnits * sms) {
-            WV_FXW_SWITCH(p.Nx, {
-                auto* kernel = 8 * p.kxColumns <= 3 * p.Nx ? dev::k_xflux_fxco<NN, 3> : dev::k_xflux_fxco<NN, 4>;
-                kernel<<<static_cast<unsigned>(units), 32 * dev::kFxCoWarps, dev::smem_xflux_co<NN>(), s>>>(
-                    d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
-            });
-            return true;
-        }
-        const int warps = static_cast<int>(std::min<size_t>(dev::kFxXWarps, std::max<size_t>(1, (units + sms - 1) / sms)));
-        const int grid = static_cast<int>(std::min<size_t>((units + warps - 1) / warps, sms));
         WV_FXW_SWITCH(p.Nx, {
-            auto* kernel = 8 * p.kxColumns <= 3 * p.Nx ? dev::k_xflux_fx<NN, 3> : dev::k_xflux_fx<NN, 4>;
-            kernel<<<grid, 32 * warps, smem_xflux_fx<NN>(), s>>>(d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
+            using X = XKernels<NN>;
+            const bool few = p.kxColumns <= static_cast<size_t>(X::few) * dev::FxW<NN>::G;
+            if constexpr (X::rowForm) {
+                if (units > kFxCoUnits * sms) {
+                    // one block per SM
+                    const int warps = dev::kFxXWarps;
+                    const int grid = static_cast<int>(std::min<size_t>((units + warps - 1) / warps, sms));
+                    auto* kernel = few ? dev::k_xflux_fx<NN, X::few> : dev::k_xflux_fx<NN, X::all>;
+                    kernel<<<grid, 32 * warps, smem_xflux_fx<NN>(), s>>>(d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
+                    return true;
+                }
+            }
+            auto* kernel = few ? dev::k_xflux_fxco<NN, X::few> : dev::k_xflux_fxco<NN, X::all>;
+            kernel<<<static_cast<unsigned>(units), 32 * dev::kFxCoWarps, dev::smem_xflux_co<NN>(), s>>>(
+                d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
         });
         return true;
     }
@@ -228,7 +262,7 @@ bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, cons
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, map, z, y, cols);
         return true;
     }
-    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * (256 / Ny);
+    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
     const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, map.nOut);
     double ltop = 0.0;
     for (double l : p.rowL) ltop = std::max(ltop, std::fabs(l));
@@ -247,7 +281,7 @@ bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, d
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, ps, nch, f, cols);
         return true;
     }
-    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * (256 / Ny);
+    const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
     const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, nch);
     WV_FXW_SWITCH(p.Ny, (dev::k_yfwd_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(d, ps, nch, f)));
     return true;
@@ -279,7 +313,7 @@ bool fx_vinv(const Plan& p, const dev::DescDev& d, bool flux, double elapsed, co
         return true;
     }
     const int lines = flux ? 4 : 2, sets = fx_z_sets(p, lines), warps = sets * lines;
-    const dim3 grid(cdiv(p.Nkl, sets * (256 / p.fz.N)), d.members);
+    const dim3 grid(cdiv(p.Nkl, sets * fx_lane_lines(p.fz.N)), d.members);
     WV_FXW_SWITCH(p.fz.N, {
         const size_t sm = dev::smem_fx_z<NN>(lines, sets);
         if (flux) dev::k_vinv_fx<NN, true><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
@@ -303,7 +337,7 @@ bool fx_vfwd(const Plan& p, const dev::DescDev& d, bool flux, const double2* f, 
         return true;
     }
     const int sets = fx_z_sets(p, 2), warps = 2 * sets;
-    const dim3 grid(cdiv(p.Nkl, sets * (256 / p.fz.N)), d.members);
+    const dim3 grid(cdiv(p.Nkl, sets * fx_lane_lines(p.fz.N)), d.members);
     WV_FXW_SWITCH(p.fz.N, {
         const size_t sm = dev::smem_fx_z<NN>(2, sets);
         if (flux)

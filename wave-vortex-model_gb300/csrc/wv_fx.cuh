@@ -163,13 +163,36 @@ WV_HD void fx_dft8(fxc (&v)[8]) {
     v[2] = fx_add(e2, o2); v[6] = fx_sub(e2, o2);
     v[3] = fx_add(e3, o3); v[7] = fx_sub(e3, o3);
 }
+// 12 = 4 x 3 by coprime index maps (no twiddles): n = 4 n1 + 3 n2, k = 4 k1 + 9 k2 mod 12
+template <bool INV>
+WV_HD void fx_dft12(fxc (&v)[12]) {
+    fx_dft4<INV>(v[0], v[3], v[6], v[9]);
+    fx_dft4<INV>(v[4], v[7], v[10], v[1]);
+    fx_dft4<INV>(v[8], v[11], v[2], v[5]);
+    fx_dft3<INV>(v[0], v[4], v[8]);
+    fx_dft3<INV>(v[3], v[7], v[11]);
+    fx_dft3<INV>(v[6], v[10], v[2]);
+    fx_dft3<INV>(v[9], v[1], v[5]);
+    // v[4 n1 + 3 n2] now holds (k1, k2) = (n1, n2), output 4 k1 + 9 k2
+    const fxc t3 = v[3], t1 = v[1], t6 = v[6], t7 = v[7], t9 = v[9], t11 = v[11], t5 = v[5], t2 = v[2], t10 = v[10];
+    v[9] = t3;              // (0, 1)
+    v[6] = t6;              // (0, 2)
+    v[3] = t9;              // (0, 3): 27 mod 12
+    v[1] = t7;              // (1, 1): 13 mod 12
+    v[10] = t10;            // (1, 2): 22 mod 12
+    v[7] = t1;              // (1, 3): 31 mod 12
+    v[5] = t11;             // (2, 1): 17 mod 12
+    v[2] = t2;              // (2, 2): 26 mod 12
+    v[11] = t5;             // (2, 3): 35 mod 12
+}
 template <int R, bool INV>
 WV_HD void fx_dft(fxc (&v)[R]) {
     if constexpr (R == 2) fx_dft2<INV>(v[0], v[1]);
     else if constexpr (R == 3) fx_dft3<INV>(v[0], v[1], v[2]);
     else if constexpr (R == 4) fx_dft4<INV>(v[0], v[1], v[2], v[3]);
     else if constexpr (R == 5) fx_dft5<INV>(v[0], v[1], v[2], v[3], v[4]);
-    else fx_dft8<INV>(v);
+    else if constexpr (R == 8) fx_dft8<INV>(v);
+    else fx_dft12<INV>(v);
 }
 
 // ---- doubles to and from the line's fixed point -----------------------------------

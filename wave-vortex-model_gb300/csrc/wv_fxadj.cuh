@@ -70,11 +70,11 @@ __device__ __forceinline__ void fx_vinv_adj_store(const DescDev& d, int idx, dou
 // k_vfwd_adj_fft: lines (u | w), (v | eta) of a column by two warps;
 // y[0] = X_0, y[j] = (X_j + i Y_j) / 2, y[N-j] = (X_j - i Y_j) / 2.
 template <int N>
-__global__ void __launch_bounds__(32 * kFxZWarps, 3)
+__global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
     k_vfwd_adj_fx(DescDev d, const double* __restrict__ Fpb, const double* __restrict__ Fmb, const double* __restrict__ F0b,
                   double elapsed, double2* __restrict__ zadj) {
     using W = FxW<N>;
-    constexpr int G = W::G, L = N / 2;
+    constexpr int G = W::G, E = W::E, H = W::H, L = N / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nj = d.Nj, P = d.positions;
     const int lane = threadIdx.x & 31, t = lane % G, warp = threadIdx.x >> 5;
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
     const bool live = want < d.Nkl;
     const int mode = min(want, d.Nkl - 1);
 #pragma unroll 1
-    for (int i = l; i < 4; i += 2) {
+    for (int i = l; i < H; i += 2) {
         const int j = t + G * i;
         double2 f[4];
         if (j < Nj) fx_vfwd_adj_values(d, Fpb, Fmb, F0b, elapsed, d.modeWV[mode], j, f);
@@ -103,19 +103,19 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
         if (d.tq[q] == l) tc = q;
         if (d.tq[q] == 2 + l) ts = q;
     }
-    double2 a[4];
-    double none[4];
-    fxc C[4], D[4];
+    double2 a[H];
+    double none[H];
+    fxc C[H], D[H];
     int uC, uD;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = tc >= 0 ? fld[l * L + t + G * i] : make_double2(0.0, 0.0);
-    fx_quantise_lane<4, G, kFxPlain>(a, none, 0u, 1, [](int) { return 2.0f; }, C, uC);
+    for (int i = 0; i < H; ++i) a[i] = tc >= 0 ? fld[l * L + t + G * i] : make_double2(0.0, 0.0);
+    fx_quantise_lane<H, G, kFxPlain>(a, none, 0u, 1, [](int) { return 2.0f; }, C, uC);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = ts >= 0 ? fld[(2 + l) * L + t + G * i] : make_double2(0.0, 0.0);
-    fx_quantise_lane<4, G, kFxPlain>(a, none, 0u, 1, [](int) { return 2.0f; }, D, uD);
-    fxc v[8];
+    for (int i = 0; i < H; ++i) a[i] = ts >= 0 ? fld[(2 + l) * L + t + G * i] : make_double2(0.0, 0.0);
+    fx_quantise_lane<H, G, kFxPlain>(a, none, 0u, 1, [](int) { return 2.0f; }, D, uD);
+    fxc v[E];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {  // 2 y
+    for (int i = 0; i < H; ++i) {  // 2 y
         const int j = t + G * i;
         if (j == 0) {
             v[i] = fxc{2 * C[i].x, 2 * C[i].y};
@@ -127,11 +127,11 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
     }
     __syncwarp();
 #pragma unroll
-    for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+    for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
     __syncwarp();
     fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uD)) ? 0 : fx_two());
 #pragma unroll
-    for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+    for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
     __syncwarp();
     if (!live) return;
     const double sc = 1.0 / (static_cast<double>(L) * static_cast<double>(d.Nx) * static_cast<double>(d.Ny));
@@ -151,11 +151,11 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
         }
     };
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < H; ++i) {
         const int n = t + G * i;
         put(n, v[i], n == 0 ? v[0] : x[fx_pad(N - n)], n == 0 ? oC0 : oC);  // w_z = 1 at the ends, 2 inside
     }
-    if (t == 0) put(L, v[4], v[4], oC0);
+    if (t == 0) put(L, v[H], v[H], oC0);
 }
 
 // Shared memory of k_vinv_adj_fx: line buffers and the parts [8][N/2] of each column.
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
     k_vinv_adj_fx(DescDev d, const double2* __restrict__ fadj, double elapsed, double* __restrict__ Apb,
                   double* __restrict__ Amb, double* __restrict__ A0b) {
     using W = FxW<N>;
-    constexpr int G = W::G, L = N / 2;
+    constexpr int G = W::G, E = W::E, H = W::H, L = N / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nj = d.Nj, Nz = d.Nz, P = d.positions;
     const int lane = threadIdx.x & 31, t = lane % G, warp = threadIdx.x >> 5;
@@ -204,26 +204,26 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
             if (flags & 1) v.y = -v.y;
             return v;
         };
-        double2 a[5], b[4];
-        double none5[5], none4[4];
+        double2 a[H + 1], b[H];
+        double none5[H + 1], none4[H];
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
+        for (int i = 0; i < H + 1; ++i) {
             const int z = t + G * i;
-            a[i] = chC >= 0 && (i < 4 || t == 0) ? colval(chC, z) : make_double2(0.0, 0.0);
-            if (i < 4) b[i] = chS >= 0 && z != 0 ? colval(chS, z) : make_double2(0.0, 0.0);
+            a[i] = chC >= 0 && (i < H || t == 0) ? colval(chC, z) : make_double2(0.0, 0.0);
+            if (i < H) b[i] = chS >= 0 && z != 0 ? colval(chS, z) : make_double2(0.0, 0.0);
         }
-        fxc C[5], S[4];
+        fxc C[H + 1], S[H];
         int uC, uS;
-        fx_quantise_lane<5, G, kFxPlain>(a, none5, 0u, 1, [](int) { return 2.0f; }, C, uC);
-        fx_quantise_lane<4, G, kFxPlain>(b, none4, 0u, 1, [](int) { return 2.0f; }, S, uS);
+        fx_quantise_lane<H + 1, G, kFxPlain>(a, none5, 0u, 1, [](int) { return 2.0f; }, C, uC);
+        fx_quantise_lane<H, G, kFxPlain>(b, none4, 0u, 1, [](int) { return 2.0f; }, S, uS);
         __syncthreads();  // twiddles
-        fxc v[8];
+        fxc v[E];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {  // 2 y
+        for (int i = 0; i < H; ++i) {  // 2 y
             const int z = t + G * i;
             if (z == 0) {
                 v[i] = fxc{2 * C[i].x, 2 * C[i].y};
-                x[fx_pad(L)] = fxc{2 * C[4].x, 2 * C[4].y};
+                x[fx_pad(L)] = fxc{2 * C[H].x, 2 * C[H].y};
             } else {
                 v[i] = fxc{C[i].x - S[i].y, C[i].y + S[i].x};
                 x[fx_pad(N - z)] = fxc{C[i].x + S[i].y, C[i].y - S[i].x};
@@ -231,15 +231,15 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
         }
         __syncwarp();
 #pragma unroll
-        for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+        for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
         fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two());
 #pragma unroll
-        for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+        for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();
         const FxUnit oC = fx_out(uC - 2), oC0 = fx_out(uC - 3), oS = fx_out(uS - 2);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             const int j = t + G * i;
             if (j >= Nj) continue;
             const fxc p = v[i], q = j == 0 ? v[0] : x[fx_pad(N - j)];
@@ -249,8 +249,11 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
         }
     }
     __syncthreads();
-    const int j = t + G * l;
-    if (!live || j >= Nj) return;
+    if (!live) return;
+#pragma unroll 1
+    for (int i = l; i < H; i += 4) {
+    const int j = t + G * i;
+    if (j >= Nj) continue;
     const double m = static_cast<const double*>(d.tMz)[j];
     // u_bar = Ccos^T U + (-m) Csin^T u_z;  w_bar = Csin^T W + m Ccos^T w_z; likewise v, eta
     const double2 e0 = X[j], o0 = X[L + j], e1 = X[2 * L + j], o1 = X[3 * L + j];
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
     fx_vinv_adj_store(d, j + Nj * d.modeWV[mode], elapsed, make_double2(e0.x - m * o2.x, e0.y - m * o2.y),
                       make_double2(e1.x - m * o3.x, e1.y - m * o3.y), make_double2(o0.x + m * e2.x, o0.y + m * e2.y),
                       make_double2(o1.x + m * e3.x, o1.y + m * e3.y), Apb, Amb, A0b);
+    }
 }
 
 // k_yfwd_pair: FFT_y(srcA) + (-i l) FFT_y(srcB), gathered to the active rows.
@@ -265,7 +269,7 @@ template <int N>
 __global__ void __launch_bounds__(32 * kFxYWarps, 2)
     k_yfwd_pair_fx(DescDev d, YFwdPairMap map, const double2* __restrict__ yin, int nIn, double2* __restrict__ fout) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = d.positions, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
@@ -277,9 +281,9 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
     for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwY[i];
     const int g = min(cols, KX - kx0);
     const double* rowL = row_l<double>(d);
-    double2 sum[8];
+    double2 sum[E];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) sum[e] = make_double2(0.0, 0.0);
+    for (int e = 0; e < E; ++e) sum[e] = make_double2(0.0, 0.0);
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
         const int src = part == 0 ? map.srcA[ch] : map.srcB[ch];
@@ -290,18 +294,18 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
             tile[fx_tile(y, c, cols)] = c < g ? in[static_cast<size_t>(y) * KX + c] : make_double2(0.0, 0.0);
         }
         __syncthreads();
-        double2 a[8];
+        double2 a[E];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
+        for (int e = 0; e < E; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
         __syncthreads();
-        fxc v[8];
+        fxc v[E];
         int unit;
-        double none[8];
-        fx_quantise_lane<8, G, kFxPlain>(a, none, 0u, 0, [](int) { return 1.0f; }, v, unit);
+        double none[E];
+        fx_quantise_lane<E, G, kFxPlain>(a, none, 0u, 0, [](int) { return 1.0f; }, v, unit);
         fx_fft_warp<N, false>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
         const FxUnit o = fx_out(unit);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
+        for (int e = 0; e < E; ++e) {
             const double re = fx_to_double(v[e].x, o), im = fx_to_double(v[e].y, o);
             if (part == 0) {
                 sum[e] = make_double2(re, im);
@@ -316,18 +320,18 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
     if (kx >= KX) return;
     double2* out = fout + (static_cast<size_t>(ch) * d.zTotal + z) * P;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < E; ++e) {
         const int pos = d.ymap[static_cast<size_t>(kx) * N + t + G * e];
         if (pos >= 0) out[pos] = sum[e];
     }
 }
 
-// Real values of a lane (8 a row) in the fixed point of their row, for two rows to a line.
-template <int G>
-__device__ __forceinline__ void fx_quantise_real(const double (&a)[8], long long (&out)[8], int& unit) {
+// Real values of a lane (E a row) in the fixed point of their row, for two rows to a line.
+template <int E, int G>
+__device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long (&out)[E], int& unit) {
     float sum = 0.f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) sum += fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
+    for (int e = 0; e < E; ++e) sum += fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
     sum = fx_group_sum<G>(sum);
     fxscale sc = fx_scale(sum);
     bool zero = false;
@@ -335,11 +339,11 @@ __device__ __forceinline__ void fx_quantise_real(const double (&a)[8], long long
     if (__any_sync(0xffffffffu, odd)) {
         unsigned top = 0;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
+        for (int e = 0; e < E; ++e) top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
         top = fx_group_max<G>(top);
         float rel = 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) rel += fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
+        for (int e = 0; e < E; ++e) rel += fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
         rel = fx_group_sum<G>(rel);
         if (odd) {
             zero = top == 0;
@@ -349,7 +353,7 @@ __device__ __forceinline__ void fx_quantise_real(const double (&a)[8], long long
     sc.bit -= 2;
     unit = zero ? kFxZero : fx_unit(sc);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) out[e] = fx_from_double(a[e], sc);
+    for (int e = 0; e < E; ++e) out[e] = fx_from_double(a[e], sc);
 }
 
 // k_xadj on kept rows: a block takes one line-set of rows, as k_xflux_fxco.  Two warps
@@ -357,14 +361,14 @@ __device__ __forceinline__ void fx_quantise_real(const double (&a)[8], long long
 // (24 operations), a warp each transforms two of the 3 + 3 nt gradient rows.
 template <int N>
 inline size_t smem_xadj_fx() {
-    return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + 4 * 256 * 8 + 7 * 128 * 16;
+    return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + 4 * FxW<N>::samples * 8 + 7 * (FxW<N>::samples / 2) * 16;
 }
 template <int N>
 __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
     k_xadj_fx(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yadj, double2* __restrict__ yout,
               const double* __restrict__ physIn) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
     const int nIn = 4 + 2 * nt, nReal = 3 + 3 * nt;
@@ -374,8 +378,8 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
     fxc* buffers = reinterpret_cast<fxc*>(tw + W::twiddles);  // [pair][line][buffer]
     fxc* x = buffers + static_cast<size_t>(p * W::lines + line) * W::buffer;
     double* Sb = reinterpret_cast<double*>(buffers + kFxCoWarps * W::lines * W::buffer);  // adjoint rows [nt][line][N]
-    double2* specV = reinterpret_cast<double2*>(Sb + 4 * 256);                             // U, V, W [3][line][N/2]
-    double2* specX = specV + 3 * 128;                                                      // x derivatives [nt][line][N/2]
+    double2* specV = reinterpret_cast<double2*>(Sb + 4 * W::samples);                             // U, V, W [3][line][N/2]
+    double2* specX = specV + 3 * (W::samples / 2);                                                      // x derivatives [nt][line][N/2]
     const int two = fx_two();
     for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
     const size_t cstride = static_cast<size_t>(Ny) * KX;
@@ -387,25 +391,25 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
     __syncthreads();
     if (2 * p < nt) {
         // c2r of the adjoint spectra, interior kx at weight 1/2 (adjoint of r2c)
-        fxc AB[2][4], v[8];
+        fxc AB[2][H], v[E];
         int unit[2] = {kFxZero, kFxZero};
         auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
-        double none[4];
+        double none[H];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const bool has = 2 * p + q < nt;
             const double2* h = yadj + ((static_cast<size_t>(z) * nt + 2 * p + (has ? q : 0)) * Ny + y) * KX;
-            double2 a[4];
+            double2 a[H];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < H; ++i) {
                 const int k = t + G * i;
                 const double2 s = has && k < KX ? h[k] : make_double2(0.0, 0.0);
                 a[i] = k == 0 ? make_double2(s.x, 0.0) : make_double2(0.5 * s.x, 0.5 * s.y);
             }
-            fx_quantise_lane<4, G, kFxPlain>(a, none, 0u, 1, count, AB[q], unit[q]);
+            fx_quantise_lane<H, G, kFxPlain>(a, none, 0u, 1, count, AB[q], unit[q]);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             const fxc a = AB[0][i], b = AB[1][i];
             const int k = t + G * i;
             v[i] = fxc{a.x - b.y, a.y + b.x};
@@ -413,20 +417,20 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
         }
         __syncwarp();
 #pragma unroll
-        for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+        for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
         fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
         const FxUnit oa = fx_out(unit[0]), ob = fx_out(unit[1]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            Sb[2 * p * 256 + line * N + t + G * e] = fx_to_double(v[e].x, oa);
-            if (2 * p + 1 < nt) Sb[(2 * p + 1) * 256 + line * N + t + G * e] = fx_to_double(v[e].y, ob);
+        for (int e = 0; e < E; ++e) {
+            Sb[2 * p * W::samples + line * N + t + G * e] = fx_to_double(v[e].x, oa);
+            if (2 * p + 1 < nt) Sb[(2 * p + 1) * W::samples + line * N + t + G * e] = fx_to_double(v[e].y, ob);
         }
     }
     __syncthreads();
-    {
-        // one sample a thread: g_U = -sum S q_x ..., and -S (U, V, W) for the derivative rows
-        const int s = threadIdx.x, ln = s / N, xx = s - ln * N;
+    for (int s = threadIdx.x; s < W::samples; s += 32 * kFxCoWarps) {
+        // a sample a thread: g_U = -sum S q_x ..., and -S (U, V, W) for the derivative rows
+        const int ln = s / N, xx = s - ln * N;
         const int rr = min(first + ln, rows - 1), zz = rr / Ny, yy = rr - zz * Ny;
         const double* ph = physIn + (static_cast<size_t>(zz) * nReal * Ny + yy) * N + xx;
         const size_t rs = static_cast<size_t>(Ny) * N;
@@ -436,7 +440,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
             return reinterpret_cast<double*>(buffers + static_cast<size_t>((r >> 1) * W::lines + ln) * W::buffer + xx) + (r & 1);
         };
         for (int tt = 0; tt < nt; ++tt) {
-            const double sb = Sb[tt * 256 + s];
+            const double sb = Sb[tt * W::samples + s];
 #pragma unroll
             for (int kind = 0; kind < 3; ++kind) {
                 const int r = 3 + 3 * tt + kind;
@@ -450,24 +454,24 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
     }
     __syncthreads();
     if (2 * p < nReal) {
-        double ra[8], rb[8];
+        double ra[E], rb[E];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
+        for (int e = 0; e < E; ++e) {
             const double2 s = reinterpret_cast<const double2*>(x)[t + G * e];
             ra[e] = s.x;
             rb[e] = s.y;
         }
         __syncwarp();
-        long long ia[8], ib[8];
+        long long ia[E], ib[E];
         int ua, ub;
-        fx_quantise_real<G>(ra, ia, ua);
-        fx_quantise_real<G>(rb, ib, ub);
-        fxc v[8];
+        fx_quantise_real<E, G>(ra, ia, ua);
+        fx_quantise_real<E, G>(rb, ib, ub);
+        fxc v[E];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = fxc{ia[e], ib[e]};
+        for (int e = 0; e < E; ++e) v[e] = fxc{ia[e], ib[e]};
         fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(ua, ub)) ? 0 : two);
 #pragma unroll
-        for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+        for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();
         const double* rowK = row_k<double>(d);
         // interior kx doubled (adjoint of c2r); the split's halves cancel it there
@@ -484,7 +488,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
             if (live) yout[(static_cast<size_t>(z) * nIn + c) * cstride + static_cast<size_t>(y) * KX + k] = val;
         };
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             const int k = t + G * i;
             if (k >= KX) continue;
             const fxc a = v[i], b = k == 0 ? v[0] : x[fx_pad(N - k)];

@@ -1,8 +1,9 @@
 // Fixed-point FFT lines (wv_fx.cuh) of 16 to 256 points held by lanes: a line of N
-// points belongs to N / 8 lanes of one warp, lane t holding points t + (N/8) e, e <
-// 8, before and after the transform; 32 / (N/8) lines ride in a warp.  The stages
-// are 8 x 2, 8 x 4, 8 x 8, 8 x 4 x 4 or 8 x 8 x 4 points of registers with one
-// exchange through shared memory between two stages (warp barriers only).
+// = E G points (E = 8, or 12 for three times a power of two) belongs to G lanes of
+// one warp, lane t holding points t + G e, e < E, before and after the transform; 32 / G
+// lines ride in a warp.  The stages (8 x 2, 8 x 4, 8 x 8, 8 x 4 x 4, 8 x 8 x 4; 2 x 12,
+// 4 x 12, 4 x 2 x 12, 4 x 4 x 12) work on registers, with one exchange through shared
+// memory between two of them (warp barriers only).
 //
 // What bounds these lines is the number of instructions issued: against the
 // run-time Stockham stages of wv_fx.cuh every index is a constant here, the first
@@ -17,26 +18,31 @@ namespace wvgpu {
 namespace dev {
 
 template <int N> struct FxW {
-    static constexpr int G = N / 8;         // lanes of a line
-    static constexpr int lines = 32 / G;    // lines of a warp
-    static constexpr int buffer = N + N / 8;  // padded line buffer
-    static constexpr int R2 = N == 16 ? 2 : (N == 32 || N == 128) ? 4 : 8;
-    static constexpr int R3 = N >= 128 ? 4 : 1;
-    static constexpr int twiddles = (R2 - 1) * 8 + (R3 - 1) * 8 * R2;
+    static constexpr int E = N % 3 == 0 ? 12 : 8;  // points of a lane
+    static constexpr int H = E / 2;
+    static constexpr int G = N / E;                // lanes of a line
+    static constexpr int lines = 32 / G;           // lines of a warp
+    static constexpr int samples = lines * N;      // points of a warp: 32 E
+    static constexpr int buffer = N + N / 8;       // padded line buffer
+    // radices of the stages (their products end with N; R3 = 1: two stages)
+    static constexpr int R1 = E == 8 ? 8 : N == 24 ? 2 : 4;
+    static constexpr int R2 = E == 8 ? (N == 16 ? 2 : (N == 32 || N == 128) ? 4 : 8) : N == 96 ? 2 : N == 192 ? 4 : 12;
+    static constexpr int R3 = N / (R1 * R2);
+    static constexpr int twiddles = (R2 - 1) * R1 + (R3 - 1) * R1 * R2;
 };
 __device__ __forceinline__ int fx_pad(int i) { return i + (i >> 3); }
 
 // Stage of radix R behind Ns points already combined; tw[(r - 1) Ns + k].
 template <int N, int R, int Ns, bool INV>
-__device__ __forceinline__ void fx_wstage(fxc (&v)[8], const fxw* __restrict__ tw, int t, int two) {
-    constexpr int G = N / 8, B = 8 / R;
+__device__ __forceinline__ void fx_wstage(fxc (&v)[FxW<N>::E], const fxw* __restrict__ tw, int t, int two) {
+    constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
 #pragma unroll
     for (int b = 0; b < B; ++b) {
-        const int k = (t + G * b) & (Ns - 1);
+        const int k = (t + G * b) & (Ns - 1);  // (Ns is a power of two)
         fxc u[R];
         u[0] = v[b];
 #pragma unroll
-        for (int r = 1; r < R; ++r) u[r] = fx_cmul60<INV>(v[b + B * r], tw[(r - 1) * Ns + k], two);
+        for (int r = 1; r < R; ++r) u[r] = Ns == 1 ? v[b + B * r] : fx_cmul60<INV>(v[b + B * r], tw[(r - 1) * Ns + k], two);
         fx_dft<R, INV>(u);
 #pragma unroll
         for (int r = 0; r < R; ++r) v[b + B * r] = u[r];
@@ -44,8 +50,8 @@ __device__ __forceinline__ void fx_wstage(fxc (&v)[8], const fxw* __restrict__ t
 }
 // v[b + B r], the outputs of a stage of radix R, to their places and back to lane order
 template <int N, int R, int Ns>
-__device__ __forceinline__ void fx_wexchange(fxc (&v)[8], fxc* __restrict__ x, int t) {
-    constexpr int G = N / 8, B = 8 / R;
+__device__ __forceinline__ void fx_wexchange(fxc (&v)[FxW<N>::E], fxc* __restrict__ x, int t) {
+    constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
 #pragma unroll
     for (int b = 0; b < B; ++b) {
         const int j = t + G * b, k = j & (Ns - 1), jq = j / Ns;
@@ -54,19 +60,19 @@ __device__ __forceinline__ void fx_wexchange(fxc (&v)[8], fxc* __restrict__ x, i
     }
     __syncwarp();
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+    for (int e = 0; e < FxW<N>::E; ++e) v[e] = x[fx_pad(t + G * e)];
     __syncwarp();
 }
 // The whole line (sum of moduli below 2^60); x: this line's buffer, tw: the stage twiddles in shared memory.
 template <int N, bool INV>
-__device__ __forceinline__ void fx_fft_warp(fxc (&v)[8], fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two) {
+__device__ __forceinline__ void fx_fft_warp(fxc (&v)[FxW<N>::E], fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two) {
     using W = FxW<N>;
-    fx_dft8<INV>(v);
-    fx_wexchange<N, 8, 1>(v, x, t);
-    fx_wstage<N, W::R2, 8, INV>(v, tw, t, two);
+    fx_wstage<N, W::R1, 1, INV>(v, tw, t, two);
+    fx_wexchange<N, W::R1, 1>(v, x, t);
+    fx_wstage<N, W::R2, W::R1, INV>(v, tw, t, two);
     if constexpr (W::R3 > 1) {
-        fx_wexchange<N, W::R2, 8>(v, x, t);
-        fx_wstage<N, W::R3, 8 * W::R2, INV>(v, tw + (W::R2 - 1) * 8, t, two);
+        fx_wexchange<N, W::R2, W::R1>(v, x, t);
+        fx_wstage<N, W::R3, W::R1 * W::R2, INV>(v, tw + (W::R2 - 1) * W::R1, t, two);
     }
 }
 
@@ -176,7 +182,8 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
 // (a b) >> 62 on velocities normalised to 62 bits and added at the largest unit of
 // a target's three.
 
-inline size_t fx_xflux_warp_bytes(int N) { return static_cast<size_t>(256 / N) * ((N + N / 8) * 16 + 40 * N); }
+template <int N>
+inline size_t fx_xflux_warp_bytes() { return static_cast<size_t>(FxW<N>::lines) * (FxW<N>::buffer * 16 + 40 * N); }
 constexpr int kFxXWarps = 15;  // 14.8 KB of shared memory and 32 x 128 registers each fill an SM
 
 // (a b) >> 62 rounded, |a| < 2^62, |b| < 2^61
@@ -205,8 +212,8 @@ __device__ __forceinline__ int fx_pick(const int (&a)[3], int i) { return i == 0
 template <int N, int EK>
 __device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __restrict__ yrow, size_t cstride,
                                              const double* __restrict__ rowK, unsigned wtop, int p, int nReal, fxc* __restrict__ x,
-                                             int t, fxc (&v)[8], int (&unit)[2]) {
-    constexpr int G = N / 8;
+                                             int t, fxc (&v)[FxW<N>::E], int (&unit)[2]) {
+    constexpr int G = FxW<N>::G, E = FxW<N>::E, H = E / 2;
     const int KX = d.kxColumns, nt = d.nt;
     // rows 2p and 2p + 1: spectrum entries k = t + G i, both rows' loads in flight
     double2 raw[2][EK];
@@ -260,43 +267,43 @@ __device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __
                         x[fx_pad(k == 0 ? N - G * EK : N - k)] = k == 0 ? fxc{0, 0} : m;
                     }
     #pragma unroll
-                    for (int e = EK; e < 8 - EK; ++e) v[e] = fxc{0, 0};
+                    for (int e = EK; e < E - EK; ++e) v[e] = fxc{0, 0};
                     __syncwarp();
     #pragma unroll
-                    for (int e = 8 - EK; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+                    for (int e = E - EK; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
                     __syncwarp();
 }
 
 // Samples of an advecting velocity row (or the caller's doubles), normalised to 62
 // bits, into phys; returns the unit.
 template <int N>
-__device__ __forceinline__ int fx_velocity(const long long (&smp)[8], int unit, int t, long long* __restrict__ phys,
+__device__ __forceinline__ int fx_velocity(const long long (&smp)[FxW<N>::E], int unit, int t, long long* __restrict__ phys,
                                            const double* __restrict__ advIn, double* __restrict__ advOut,
                                            double* __restrict__ keep) {
-    constexpr int G = N / 8;
+    constexpr int G = FxW<N>::G, E = FxW<N>::E, H = E / 2;
     unsigned top = 0;
     if (advIn) {
-        double a[8];
+        double a[E];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
+        for (int e = 0; e < E; ++e) {
             a[e] = advIn[t + G * e];
             top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
         }
         top = fx_group_max<G>(top);
         const fxscale sc{static_cast<int>(top >> 20), 61};
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
+        for (int e = 0; e < E; ++e) {
             phys[t + G * e] = fx_from_double(a[e], sc);
             if (keep) keep[t + G * e] = a[e];
         }
         return fx_unit(sc);
     }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) top = max(top, fx_abs_hi(smp[e]));
+    for (int e = 0; e < E; ++e) top = max(top, fx_abs_hi(smp[e]));
     top = fx_group_max<G>(top);
     const int sh = max(0, __clz(static_cast<int>(top)) - 2);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < E; ++e) {
         const long long s = fx_round53(smp[e] << sh);
         phys[t + G * e] = s;
         if (advOut) advOut[t + G * e] = fx_to_double(s, unit - sh);
@@ -311,22 +318,22 @@ template <int N>
 __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa, const long long* __restrict__ Sb, int unitA,
                                                 int unitB, fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two,
                                                 int KX, double2* __restrict__ out, size_t cstride) {
-    constexpr int G = N / 8;
+    constexpr int G = FxW<N>::G, E = FxW<N>::E, H = E / 2;
     const bool both = Sb != nullptr;
-    fxc v[8];
+    fxc v[E];
     int sh[2], u[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         unsigned sum = 0;
         if (q == 0 || both)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) sum += (fx_abs_hi((q ? Sb : Sa)[t + G * e]) >> 9) + 1u;
+            for (int e = 0; e < E; ++e) sum += (fx_abs_hi((q ? Sb : Sa)[t + G * e]) >> 9) + 1u;
         sum = fx_group_add<G>(sum);
         sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 59;  // sum |S| < 2^59 after the shift
         u[q] = (q ? unitB : unitA) + sh[q] - 1;                 // the halves of the split below
     }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < E; ++e) {
         const long long a = Sa[t + G * e], b = both ? Sb[t + G * e] : 0;
         v[e].x = sh[0] >= 0 ? a >> sh[0] : a << -sh[0];
         v[e].y = sh[1] >= 0 ? b >> sh[1] : b << -sh[1];
@@ -334,11 +341,11 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
     fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(unitA, both ? unitB : unitA)) ? 0 : two);
     __syncwarp();
 #pragma unroll
-    for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+    for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
     __syncwarp();
     const FxUnit o0 = fx_out(u[0]), o1 = fx_out(u[1]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < H; ++i) {
         const int k = t + G * i;
         const fxc a = v[i], b = k == 0 ? v[0] : x[fx_pad(N - k)];
         if (k < KX) {
@@ -349,14 +356,14 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
 }
 
 // physOut / advOut / advIn / maxSpeedBits as k_xflux.
-// EK: spectrum entries of a lane (kx < EK N / 8; 3 under the 2/3 rule).
+// EK: spectrum entries of a lane (kx < EK G; E / 2 at most, fewer under the 2/3 rule).
 template <int N, int EK>
 __global__ void __launch_bounds__(32 * kFxXWarps, 1)
     k_xflux_fx(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, double2* __restrict__ pspec,
                unsigned long long* __restrict__ maxSpeedBits, double* __restrict__ physOut, double* __restrict__ advOut,
                const double* __restrict__ advIn) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
     const int nIn = 4 + 2 * nt, nReal = 3 + 3 * nt;
@@ -381,11 +388,11 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
         const int z = row / Ny, y = row - z * Ny;
         const double2* yrow = yspec + (static_cast<size_t>(z) * nIn * Ny + y) * KX;
         int physUnit[3] = {0, 0, 0}, sUnit[2] = {0, 0}, unitNow = 0;  // (as fx_unit)
-        long long acc[8];  // products of the current target
+        long long acc[E];  // products of the current target
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] = 0;
+        for (int e = 0; e < E; ++e) acc[e] = 0;
         for (int p = 0; 2 * p < nReal; ++p) {
-            fxc v[8];
+            fxc v[E];
             int unit[2] = {kFxZero, kFxZero};
             fx_load_pair<N, EK>(d, yrow, cstride, rowK, wtop, p, nReal, x, t, v, unit);
             fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
@@ -395,13 +402,13 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
                 const int r = 2 * p + q;
                 if (r >= nReal) break;
                 const int uq = q ? unit[1] : unit[0];
-                long long smp[8];
+                long long smp[E];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) smp[e] = q ? v[e].y : v[e].x;
+                for (int e = 0; e < E; ++e) smp[e] = q ? v[e].y : v[e].x;
                 if (physOut && live && r >= 3) {
                     double* keep = physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
+                    for (int e = 0; e < E; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
                 }
                 if (r < 3) {
                     const size_t g = static_cast<size_t>(r) * R3 + (static_cast<size_t>(z) * Ny + y) * N;
@@ -419,18 +426,18 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
                 if (kind == 0) {
                     unitNow = un;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[e] = -fx_prod(vel[t + G * e], smp[e]);
+                    for (int e = 0; e < E; ++e) acc[e] = -fx_prod(vel[t + G * e], smp[e]);
                 } else {
                     const int now = max(unitNow, un);
                     const int shS = min(63, now - unitNow), shP = min(63, now - un);
                     unitNow = now;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
+                    for (int e = 0; e < E; ++e)
                         acc[e] = (acc[e] >> shS) - (fx_prod(vel[t + G * e], smp[e]) >> shP);
                 }
                 if (kind == 2) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) S[(tt & 1) * N + t + G * e] = acc[e];
+                    for (int e = 0; e < E; ++e) S[(tt & 1) * N + t + G * e] = acc[e];
                     sUnit[0] = (tt & 1) ? sUnit[0] : unitNow;
                     sUnit[1] = (tt & 1) ? unitNow : sUnit[1];
                 }
@@ -450,7 +457,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
         if (maxSpeedBits) {
             double m = 0.0;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
+            for (int e = 0; e < E; ++e) {
                 const double U = fx_to_double(phys[t + G * e], physUnit[0]);
                 const double V = fx_to_double(phys[N + t + G * e], physUnit[1]);
                 m = fmax(m, U * U + V * V);
@@ -468,15 +475,15 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
 // k_xflux_fx's.
 constexpr int kFxCoWarps = 8;  // (3 + 3 nt + 1) / 2 <= 8 pairs
 template <int N>
-inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * 256 * 8; }
+inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * FxW<N>::samples * 8; }
 
 template <int N, int EK>
-__global__ void __launch_bounds__(32 * kFxCoWarps, 3)
+__global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
     k_xflux_fxco(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, double2* __restrict__ pspec,
                  unsigned long long* __restrict__ maxSpeedBits, double* __restrict__ physOut, double* __restrict__ advOut,
                  const double* __restrict__ advIn) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int rowUnit[16][W::lines], sUnit[4][W::lines];
     const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
@@ -487,7 +494,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 3)
     fxc* buffers = reinterpret_cast<fxc*>(tw + W::twiddles);  // [pair][line][buffer]
     fxc* x = buffers + static_cast<size_t>(warp * W::lines + line) * W::buffer;
     long long* phys = reinterpret_cast<long long*>(buffers + kFxCoWarps * W::lines * W::buffer);  // [3][line][N]
-    long long* S = phys + 3 * 256;                                                               // [nt][line][N]
+    long long* S = phys + 3 * W::samples;                                                               // [nt][line][N]
     const int two = fx_two();
     for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
     const double* rowK = row_k<double>(d);
@@ -502,36 +509,37 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 3)
     const int p = warp;
     __syncthreads();
     if (2 * p < nReal) {
-        fxc v[8];
+        fxc v[E];
         int unit[2] = {kFxZero, kFxZero};
         fx_load_pair<N, EK>(d, yspec + (static_cast<size_t>(z) * nIn * Ny + y) * KX, cstride, rowK, wtop, p, nReal, x, t, v, unit);
         fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[t + G * e] = v[e];
+        for (int e = 0; e < E; ++e) x[t + G * e] = v[e];
 #pragma unroll 1
         for (int q = 0; q < 2; ++q) {
             const int r = 2 * p + q;
             if (r >= nReal) break;
             int uq = q ? unit[1] : unit[0];
             double* keep = physOut && live ? physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N : nullptr;
-            long long smp[8];
+            long long smp[E];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) smp[e] = q ? v[e].y : v[e].x;
+            for (int e = 0; e < E; ++e) smp[e] = q ? v[e].y : v[e].x;
             if (r < 3) {
                 const size_t g = static_cast<size_t>(r) * R3 + (static_cast<size_t>(z) * Ny + y) * N;
                 uq = fx_velocity<N>(smp, uq, t, phys + (r * W::lines + line) * N, advIn ? advIn + g : nullptr,
                                     advOut && live ? advOut + g : nullptr, keep);
             } else if (keep) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
+                for (int e = 0; e < E; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
             }
             if (t == 0) rowUnit[r][line] = uq;
         }
     }
     __syncthreads();
     {
-        // one sample a thread
-        const int s = threadIdx.x, ln = s / N, xx = s - ln * N;
+        // a sample a thread
+        for (int s = threadIdx.x; s < W::samples; s += 32 * kFxCoWarps) {
+        const int ln = s / N, xx = s - ln * N;
         for (int tt = 0; tt < nt; ++tt) {
             long long acc = 0;
             int now = 0;
@@ -541,7 +549,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 3)
                 const fxc* b = buffers + static_cast<size_t>((r >> 1) * W::lines + ln) * W::buffer;
                 const long long q = (r & 1) ? b[xx].y : b[xx].x;
                 const int un = rowUnit[kind][ln] + rowUnit[r][ln] - 1023 + 62;
-                const long long pr = fx_prod(phys[kind * 256 + s], q);
+                const long long pr = fx_prod(phys[kind * W::samples + s], q);
                 if (kind == 0) {
                     acc = -pr;
                     now = un;
@@ -551,25 +559,27 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 3)
                     now = next;
                 }
             }
-            S[tt * 256 + s] = acc;
+            S[tt * W::samples + s] = acc;
             if (xx == 0) sUnit[tt][ln] = now;
         }
         if (maxSpeedBits) {
-            const double U = fx_to_double(phys[s], rowUnit[0][ln]), V = fx_to_double(phys[256 + s], rowUnit[1][ln]);
+            const double U = fx_to_double(phys[s], rowUnit[0][ln]), V = fx_to_double(phys[W::samples + s], rowUnit[1][ln]);
             double m = U * U + V * V;
-            constexpr int kSpan = N < 32 ? N : 32;
+            // samples of one row among a warp's 32: the power of two that divides N
+            constexpr int kSpan = (N & -N) < 32 ? (N & -N) : 32;
 #pragma unroll
             for (int o = kSpan / 2; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
             m = fmax(m, 0.0);
             const int zz = min(first + ln, rows - 1) / Ny;
             if (lane % kSpan == 0) atomicMax(maxSpeedBits + zz / d.Nz, (unsigned long long)__double_as_longlong(sqrt(m)));
         }
+        }
     }
     __syncthreads();
     if (2 * p < nt) {
         const bool both = 2 * p + 1 < nt;
-        const long long* Sa = S + 2 * p * 256 + line * N;
-        fx_forward_pair<N>(Sa, both ? Sa + 256 : nullptr, sUnit[2 * p][line], both ? sUnit[2 * p + 1][line] : 0, x, tw, t, two,
+        const long long* Sa = S + 2 * p * W::samples + line * N;
+        fx_forward_pair<N>(Sa, both ? Sa + W::samples : nullptr, sUnit[2 * p][line], both ? sUnit[2 * p + 1][line] : 0, x, tw, t, two,
                            live ? KX : 0, pspec + ((static_cast<size_t>(z) * nt + 2 * p) * Ny + y) * KX, cstride);
     }
 }

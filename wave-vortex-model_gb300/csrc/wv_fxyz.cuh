@@ -22,10 +22,10 @@ __device__ __forceinline__ int fx_tile(int y, int c, int cols) { return y * cols
 // Inverse FFTs along y of output channel blockIdx.z, columns blockIdx.x cols ...,
 // plane blockIdx.y: yspec[z][ch][y][kx] from zspec[src][z][pos] (times i l).
 template <int N>
-__global__ void __launch_bounds__(32 * kFxYWarps, 3)
+__global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     k_yinv_fx(DescDev d, YInvMap map, const double2* __restrict__ zspec, double2* __restrict__ yspec, unsigned ltop) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = d.positions, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
@@ -36,23 +36,23 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 3)
     for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = d.fxTwY[i];
     const double2* in = zspec + (static_cast<size_t>(map.src[oc]) * d.zTotal + z) * P;
     const int kx = kx0 + own;
-    double2 a[8];
+    double2 a[E];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < E; ++e) {
         const int pos = kx < KX ? d.ymap[static_cast<size_t>(kx) * N + t + G * e] : -1;
         a[e] = pos >= 0 ? in[pos] : make_double2(0.0, 0.0);
     }
-    fxc v[8];
+    fxc v[E];
     int unit;
-    double w[8];
+    double w[E];
     auto count = [](int) { return 1.0f; };
     if (map.mulL[oc]) {
         const double* rowL = row_l<double>(d);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = rowL[t + G * e];
-        fx_quantise_lane<8, G, kFxImag>(a, w, ltop, 0, count, v, unit);
+        for (int e = 0; e < E; ++e) w[e] = rowL[t + G * e];
+        fx_quantise_lane<E, G, kFxImag>(a, w, ltop, 0, count, v, unit);
     } else {
-        fx_quantise_lane<8, G, kFxPlain>(a, w, 0u, 0, count, v, unit);
+        fx_quantise_lane<E, G, kFxPlain>(a, w, 0u, 0, count, v, unit);
     }
     __syncthreads();  // twiddles
     fx_fft_warp<N, true>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 3)
     double2* tile = reinterpret_cast<double2*>(tw + W::twiddles);
     const FxUnit o = fx_out(unit);
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
+    for (int e = 0; e < E; ++e)
         tile[fx_tile(t + G * e, own, cols)] = make_double2(fx_to_double(v[e].x, o), fx_to_double(v[e].y, o));
     __syncthreads();
     double2* out = yspec + (static_cast<size_t>(z) * map.nOut + oc) * N * KX + kx0;
@@ -74,10 +74,10 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 3)
 // Forward FFTs along y of channel blockIdx.z, gathered to the active rows:
 // fspec[c][z][pos] from pspec[z][c][y][kx].
 template <int N>
-__global__ void __launch_bounds__(32 * kFxYWarps, 3)
+__global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     k_yfwd_fx(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec) {
     using W = FxW<N>;
-    constexpr int G = W::G;
+    constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = d.positions, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
@@ -94,21 +94,21 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 3)
         tile[fx_tile(y, c, cols)] = c < g ? in[static_cast<size_t>(y) * KX + c] : make_double2(0.0, 0.0);
     }
     __syncthreads();
-    double2 a[8];
+    double2 a[E];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
+    for (int e = 0; e < E; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
     __syncthreads();  // the line buffers take the tile's place
-    fxc v[8];
+    fxc v[E];
     int unit;
-    double w[8];
-    fx_quantise_lane<8, G, kFxPlain>(a, w, 0u, 0, [](int) { return 1.0f; }, v, unit);
+    double w[E];
+    fx_quantise_lane<E, G, kFxPlain>(a, w, 0u, 0, [](int) { return 1.0f; }, v, unit);
     fx_fft_warp<N, false>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
     const int kx = kx0 + own;
     if (kx >= KX) return;
     double2* out = fspec + (static_cast<size_t>(ch) * d.zTotal + z) * P;
     const FxUnit o = fx_out(unit);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < E; ++e) {
         const int pos = d.ymap[static_cast<size_t>(kx) * N + t + G * e];
         if (pos >= 0) out[pos] = make_double2(fx_to_double(v[e].x, o), fx_to_double(v[e].y, o));
     }
@@ -255,11 +255,11 @@ inline size_t smem_fx_z(int lines, int sets) {
 // scales (the even and the odd part separate them again), so neither rounds at the
 // other's magnitude.
 template <int N, bool FLUX>
-__global__ void __launch_bounds__(32 * kFxZWarps, 3)
+__global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
     k_vinv_fx(DescDev d, const double* __restrict__ Ap, const double* __restrict__ Am, const double* __restrict__ A0,
               double elapsed, double2* __restrict__ zspec, unsigned long long* __restrict__ maxSpeedBits) {
     using W = FxW<N>;
-    constexpr int G = W::G, kLines = FLUX ? 4 : 2;
+    constexpr int G = W::G, E = W::E, H = W::H, kLines = FLUX ? 4 : 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nj = d.Nj, P = d.positions;
     const int lane = threadIdx.x & 31, t = lane % G, warp = threadIdx.x >> 5;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
         const int w = d.modeWV[mode];
         const unsigned char flags = d.modeFlags[mode];
 #pragma unroll 1
-        for (int i = l; i < 4; i += kLines) {  // the column's warps share its coefficients
+        for (int i = l; i < H; i += kLines) {  // the column's warps share its coefficients
             const int j = t + G * i;
             double2 f[4];
             if (j < Nj) fx_field_spectra(d, Ap, Am, A0, elapsed, w, flags, j, f);
@@ -308,35 +308,35 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
     // fld slots of the cosine and sine channels: (0|2) (1|3) (2|0) (3|1)
     const int qs = l < 2 ? l + 2 : l - 2;
     const int chC = l < 2 ? l : derivC, chS = l < 2 ? l + 2 : derivS;
-    double2 a[4];
-    double wgt[4];
-    fxc C[4], D[4];
+    double2 a[H];
+    double wgt[H];
+    fxc C[H], D[H];
     int uC, uD;
     if (l < 2) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = fld[l * (N / 2) + t + G * i];
-        fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, C, uC);
+        for (int i = 0; i < H; ++i) a[i] = fld[l * (N / 2) + t + G * i];
+        fx_quantise_lane<H, G, kFxPlain>(a, wgt, 0u, 1, count, C, uC);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = fld[qs * (N / 2) + t + G * i];
-        fx_quantise_lane<4, G, kFxPlain>(a, wgt, 0u, 1, count, D, uD);
+        for (int i = 0; i < H; ++i) a[i] = fld[qs * (N / 2) + t + G * i];
+        fx_quantise_lane<H, G, kFxPlain>(a, wgt, 0u, 1, count, D, uD);
     } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             a[i] = fld[l * (N / 2) + t + G * i];
             wgt[i] = t + G * i < Nj ? mz[t + G * i] : 0.0;
         }
-        fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, C, uC);
+        fx_quantise_lane<H, G, kFxReal>(a, wgt, mtop, 1, count, C, uC);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             a[i] = fld[qs * (N / 2) + t + G * i];
             wgt[i] = -wgt[i];
         }
-        fx_quantise_lane<4, G, kFxReal>(a, wgt, mtop, 1, count, D, uD);
+        fx_quantise_lane<H, G, kFxReal>(a, wgt, mtop, 1, count, D, uD);
     }
     // 2 y[j] = C_j + i D_j, 2 y[N-j] = C_j - i D_j, 2 y[0] = C_0
-    fxc v[8];
+    fxc v[E];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < H; ++i) {
         const int j = t + G * i;
         if (j == 0) D[i] = fxc{0, 0};
         v[i] = fxc{C[i].x - D[i].y, C[i].y + D[i].x};
@@ -344,11 +344,11 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
     }
     __syncwarp();
 #pragma unroll
-    for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+    for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
     __syncwarp();
     fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uD)) ? 0 : fx_two());
 #pragma unroll
-    for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+    for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
     __syncwarp();
     if (!live) return;
     // even part -> cosine channel, odd part -> sine channel, n = 0 .. N / 2
@@ -369,22 +369,22 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
         }
     };
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < H; ++i) {
         const int n = t + G * i;
         put(n, v[i], n == 0 ? v[0] : x[fx_pad(N - n)]);
     }
-    if (t == 0) put(N / 2, v[4], v[4]);
+    if (t == 0) put(N / 2, v[H], v[H]);
 }
 
 // k_vfwd_fft in fixed point: lines (u | w) and (v | eta) of a column by two warps,
 // which then share its coefficients' projection.
 template <int N, bool FLUX>
-__global__ void __launch_bounds__(32 * kFxZWarps, 3)
+__global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
     k_vfwd_fx(DescDev d, const double2* __restrict__ fspec, int nch, double elapsed, const double* __restrict__ Ap,
               const double* __restrict__ Am, const double* __restrict__ A0, const unsigned long long* __restrict__ maxSpeedBits,
               int applyDamping, double* __restrict__ Fp, double* __restrict__ Fm, double* __restrict__ F0) {
     using W = FxW<N>;
-    constexpr int G = W::G, L = N / 2;
+    constexpr int G = W::G, E = W::E, H = W::H, L = N / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nj = d.Nj, P = d.positions;
     const int lane = threadIdx.x & 31, t = lane % G, warp = threadIdx.x >> 5;
@@ -417,38 +417,38 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
         const int pos = d.modePos[mode];
         const double2* hc = fspec + static_cast<size_t>(max(cc, 0)) * d.zTotal * P + pos;
         const double2* hs = fspec + static_cast<size_t>(max(cs, 0)) * d.zTotal * P + pos;
-        double2 a[5], b[4];
-        double none5[5], none4[4];
+        double2 a[H + 1], b[H];
+        double none5[H + 1], none4[H];
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
+        for (int i = 0; i < H + 1; ++i) {
             const int zz = t + G * i;
-            a[i] = cc >= 0 && (i < 4 || t == 0) ? hc[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
-            if (i < 4) b[i] = cs >= 0 && zz != 0 ? hs[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
+            a[i] = cc >= 0 && (i < H || t == 0) ? hc[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
+            if (i < H) b[i] = cs >= 0 && zz != 0 ? hs[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
         }
-        fxc C[5], S[4];
+        fxc C[H + 1], S[H];
         int uC, uS;
-        fx_quantise_lane<5, G, kFxPlain>(a, none5, 0u, 1, [&](int i) { return (i == 0 && t == 0) || i == 4 ? 1.0f : 2.0f; }, C, uC);
-        fx_quantise_lane<4, G, kFxPlain>(b, none4, 0u, 1, [&](int) { return 2.0f; }, S, uS);
+        fx_quantise_lane<H + 1, G, kFxPlain>(a, none5, 0u, 1, [&](int i) { return (i == 0 && t == 0) || i == H ? 1.0f : 2.0f; }, C, uC);
+        fx_quantise_lane<H, G, kFxPlain>(b, none4, 0u, 1, [&](int) { return 2.0f; }, S, uS);
         __syncthreads();  // twiddles
         // y[0] = c_0, y[L] = c_L, y[z] = c_z + s_z, y[N-z] = c_z - s_z
-        fxc v[8];
+        fxc v[E];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             const int zz = t + G * i;
             v[i] = fx_add(C[i], S[i]);
-            x[fx_pad(zz == 0 ? L : N - zz)] = zz == 0 ? C[4] : fx_sub(C[i], S[i]);
+            x[fx_pad(zz == 0 ? L : N - zz)] = zz == 0 ? C[H] : fx_sub(C[i], S[i]);
         }
         __syncwarp();
 #pragma unroll
-        for (int e = 4; e < 8; ++e) v[e] = x[fx_pad(t + G * e)];
+        for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
         fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two());
         const FxUnit oC = fx_out(uC - 1), oS = fx_out(uS - 1);
 #pragma unroll
-        for (int e = 4; e < 8; ++e) x[fx_pad(t + G * e)] = v[e];
+        for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < H; ++i) {
             const int j = t + G * i;
             if (j >= Nj) continue;
             const fxc p = v[i], q = j == 0 ? v[0] : x[fx_pad(N - j)];
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 3)
     double maxSpeed = 0.0;
     if (FLUX && applyDamping) maxSpeed = __longlong_as_double((long long)*maxSpeedBits);
 #pragma unroll 1
-    for (int i = l; i < 4; i += 2) {
+    for (int i = l; i < H; i += 2) {
         const int j = t + G * i;
         if (j >= Nj) continue;
         double2 U = X[j], V = X[L + j], Wv = X[2 * L + j], E = X[3 * L + j];
