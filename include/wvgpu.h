@@ -64,11 +64,11 @@ typedef struct wv_config {
  * flux accumulation and RK4 stage accumulation.
  * FP32X2: the xy transforms, products and vertical contractions in paired FP32
  * ("float-float", about 48 significand bits) on the FP32 pipe, FP64 phases,
- * projections and RK4 -- FP64-class flux accuracy without the FP64 pipe.  Fluxes,
- * their VJP and the state transforms run on the 64-bit fixed-point kernels of FP64
- * handles (more accurate, and faster) where Nx, Ny and 2 (Nz - 1) are all 16 to 256
- * and one or three times a power of two, until wv_set_vertical_kernel(s) or
- * wv_set_fft_variants chooses paired-FP32 kernels.
+ * projections and RK4 -- FP64-class flux accuracy without the FP64 pipe.  Fluxes and
+ * the state transforms (not the adjoint) run on the 64-bit fixed-point kernels of FP64
+ * handles, more accurate and faster, where Nx, Ny and 2 (Nz - 1) are all 16 to 256 and
+ * one or three times a power of two (Nx and Ny not 192), until
+ * wv_set_vertical_kernel(s) or wv_set_fft_variants chooses paired-FP32 kernels.
  * FP32X2 handles serve every entry point (kernel operations, adjoint, ensembles). */
 enum { WV_PRECISION_FP64 = 0, WV_PRECISION_MIXED = 1, WV_PRECISION_FP32X2 = 2 };
 

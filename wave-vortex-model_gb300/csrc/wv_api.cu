@@ -152,6 +152,16 @@ struct Guard {
     ~Guard() { if (entered) flag.store(false); }
 };
 
+// The adjoint entry points of FP32X2 handles, forward sweeps included, run on the
+// paired-FP32 kernels: their lane-held VJP lines are the faster ones at powers of two
+// (flux VJP 128x128x65 0.608 ms, fixed point 0.659; 192x96x49 0.488 and 0.616).
+struct PairedAdjoint {
+    bool& on;
+    const bool was;
+    explicit PairedAdjoint(wv_handle* h) : on(h->fxOn), was(h->fxOn) { on = false; }
+    ~PairedAdjoint() { on = was; }
+};
+
 int fail(wv_handle* h, int code, const std::string& message) {
     if (h) h->message = message;
     return code;
@@ -864,7 +874,7 @@ int ensure_scalar(wv_handle* h) {
         e = h->precision == WV_PRECISION_FP64    ? raise_smem_limit(dev::k_xc2r_fields<double>, static_cast<int>(smC2R))
             : h->precision == WV_PRECISION_MIXED ? raise_smem_limit(dev::k_xc2r_fields<float>, static_cast<int>(smC2R))
                                                  : raise_smem_limit(dev::k_xc2r_fields<dev::ff>, static_cast<int>(smC2R));
-    const size_t smD = Nz * dev::kScalarCols * cb;
+    const size_t smD = Nz * 32 * cb;
     if (e == cudaSuccess)
         e = h->precision == WV_PRECISION_FP64    ? raise_smem_limit(dev::k_scalar_derivs<double>, static_cast<int>(smD))
             : h->precision == WV_PRECISION_MIXED ? raise_smem_limit(dev::k_scalar_derivs<float>, static_cast<int>(smD))
@@ -913,7 +923,7 @@ cudaError_t launch_scalar_advection(wv_handle* h, const double* scalar, const do
     r2c(scalar, sp);
     dev::cx<T>* sf3 = sf + (size_t)3 * Nz * P;
     yfwd(sf3);
-    dev::k_scalar_derivs<T><<<cdiv(P, dev::kScalarCols), 256, Nz * dev::kScalarCols * cb, s>>>(sd, sf3, D, h->scalarFlags, hs, sf);
+    dev::k_scalar_derivs<T><<<cdiv(P, dev::ScalarCols<T>::value), 256, Nz * dev::ScalarCols<T>::value * cb, s>>>(sd, sf3, D, h->scalarFlags, hs, sf);
     dev::YInvMap map{};
     map.nOut = 3;
     for (int c = 0; c < 3; ++c) { map.src[c] = c; map.mulL[c] = 0; }
@@ -1102,10 +1112,6 @@ int ensure_adjoint(wv_handle* h) {
     const cudaError_t lim = h->precision == WV_PRECISION_FP64    ? set_smem_limits_adj<double>(p)
                             : h->precision == WV_PRECISION_MIXED ? set_smem_limits_adj<float>(p)
                                                                  : set_smem_limits_adj<dev::ff>(p);
-    if (lim == cudaSuccess && h->fxOn) {
-        const cudaError_t e = wvgpu::fx_set_limits_adj(p);
-        if (e != cudaSuccess) return cuda_fail(h, e, "adjoint set-up");
-    }
     if (lim == cudaErrorInvalidConfiguration)
         return fail(h, WV_UNSUPPORTED_OPERATION, "The adjoint kernels need more shared memory than one CTA has for this grid.");
     if (lim != cudaSuccess) return cuda_fail(h, lim, "adjoint set-up");
@@ -1117,7 +1123,7 @@ int ensure_adjoint(wv_handle* h) {
     if (e == cudaSuccess) e = alloc(h, nIn * p.Nz * p.positions * cb, &h->fadj);
     const size_t stateBytes = 6 * p.M * sizeof(double);
     void* tmp = nullptr;
-    if (e == cudaSuccess && fp64_path(h) && wvgpu::fx_has_rows(p)) {
+    if (e == cudaSuccess && h->precision == WV_PRECISION_FP64 && wvgpu::fx_has_rows(p)) {
         e = alloc(h, (3 + 3 * nt) * p.Nx * p.Ny * p.Nz * sizeof(double), &tmp);
         h->adjRows = static_cast<double*>(tmp);
     }
@@ -1759,7 +1765,7 @@ static int create_handle(const wv_config* config, int precision, int members, wv
         }
     }
     // fixed-point lines: their own factors and twiddles, doubles where the working type has its copies
-    h->fxOn = precision == WV_PRECISION_FP32X2 && wvgpu::fx_all_lanes(p);
+    h->fxOn = precision == WV_PRECISION_FP32X2 && wvgpu::fx_beats_paired(p);
     if (precision == WV_PRECISION_FP64 || h->fxOn) {
         dev::DescDev& fd = h->fxd;
         fd = dd;
@@ -2610,6 +2616,7 @@ int wv_flux_vjp_device(wv_handle* h, double t, double t0, const double* Ap, cons
     for (const void* q : ptrs) if (!q) return fail(h, WV_INVALID_POINTER, "Flux VJP received a null pointer.");
     Guard g(h->busy);
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "Kernel operations are not reentrant.");
+    const PairedAdjoint paired(h);
     rc = adjoint_preamble(h); if (rc) return rc;
     auto s = static_cast<cudaStream_t>(stream);
     const cudaError_t e = fp64_path(h)
@@ -2660,6 +2667,7 @@ int wv_rk4_step_vjp_device(wv_handle* h, const double* Ap, const double* Am, con
     if (!(dt > 0.0) || !std::isfinite(dt)) return fail(h, WV_INVALID_CONFIGURATION, "RK4 step size must be finite and positive.");
     Guard g(h->busy);
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "RK4 stepping is not reentrant.");
+    const PairedAdjoint paired(h);
     rc = adjoint_preamble(h); if (rc) return rc;
     auto s = static_cast<cudaStream_t>(stream);
     cudaError_t e = gather3(h, h->state, Ap, Am, A0, s);
@@ -2678,6 +2686,7 @@ int wv_rk4_adjoint_device(wv_handle* h, const double* Ap, const double* Am, cons
     if (n < 0 || K < 1) return fail(h, WV_INVALID_CONFIGURATION, "Step count must be nonnegative and the checkpoint interval positive.");
     Guard g(h->busy);
     if (!g.entered) return fail(h, WV_REENTRANT_EXECUTION, "RK4 stepping is not reentrant.");
+    const PairedAdjoint paired(h);
     rc = adjoint_preamble(h); if (rc) return rc;
     auto s = static_cast<cudaStream_t>(stream);
     const size_t stateBytes = 6 * h->plan.M * sizeof(double);

@@ -89,9 +89,18 @@ inline FxFieldLaunch fx_field_launch(size_t Nx, size_t rows, int nch) {
     const int lines = (nch + 1) / 2;
     const size_t each = 2 * static_cast<size_t>(lines) * Nx * 16;
     l.warps = static_cast<int>(std::min<size_t>(dev::kFxAnyWarps, std::max<size_t>(1, (104 * 1024 - Nx * 16) / each)));
+    while (l.warps > 1 && rows < l.warps * static_cast<size_t>(grid_cap(1))) l.warps /= 2;
     l.smem = dev::smem_fx_any_x(static_cast<int>(Nx), lines, l.warps);
     l.grid = static_cast<int>(std::min<size_t>((rows + l.warps - 1) / l.warps, grid_cap(2)));
     return l;
+}
+// Grid and warps of the lane-held field kernels (a warp per line-set and channel pair;
+// single warps while they don't fill every SM).
+struct FxLaneField { unsigned grid; int warps; };
+FxLaneField fx_lane_field(const Plan& p, const dev::DescDev& d, int nch) {
+    const size_t sets = (p.Ny * d.zTotal + fx_lane_lines(p.Nx) - 1) / fx_lane_lines(p.Nx), units = sets * ((nch + 1) / 2);
+    const int warps = units < dev::kFxFieldWarps * static_cast<size_t>(grid_cap(1)) ? 1 : dev::kFxFieldWarps;
+    return {cdiv(units, warps), warps};
 }
 struct FxXLaunch { int warps, grid, pairs; size_t smem; };
 inline FxXLaunch fx_x_launch(const Plan& p, int members) {
@@ -132,13 +141,17 @@ cudaError_t fx_set_limits(const Plan& p) {
     });
     if (!fx_lane_length(p.Ny)) {
         // (the scalar pipeline has the most columns)
-        const size_t sm = dev::smem_fx_any_y(static_cast<int>(p.Ny), dev::fx_any_cols(static_cast<int>(p.Ny), 1 << 20));
+        const size_t sm = dev::smem_fx_any_y(static_cast<int>(p.Ny), dev::fx_any_cols(static_cast<int>(p.Ny), 1 << 20, 1, 1));
         set(dev::k_yinv_fxany<0>, sm);
         set(dev::k_yfwd_fxany<0>, sm);
     }
-    if (fx_x_any(p)) {
+    WV_FXW_SWITCH(p.Nx, {
+        set(dev::k_xc2r_fx<NN>, dev::smem_fx_field<NN>(dev::kFxFieldWarps));
+        set(dev::k_xr2c_fx<NN>, dev::smem_fx_field<NN>(dev::kFxFieldWarps));
+    });
+    if (fx_x_any(p) && !fx_lane_length(p.Nx)) {
         for (int nch = 1; nch <= 4; nch += 2) {
-            const FxFieldLaunch l = fx_field_launch(p.Nx, 1, nch);
+            const FxFieldLaunch l = fx_field_launch(p.Nx, SIZE_MAX / 2, nch);
             set(dev::k_xc2r_fxany<2>, l.smem); set(dev::k_xc2r_fxany<4>, l.smem); set(dev::k_xc2r_fxany<8>, l.smem);
             set(dev::k_xr2c_fxany<0>, l.smem);
         }
@@ -219,7 +232,13 @@ bool fx_xadj(const Plan& p, const dev::DescDev& d, const FxRows& r, const double
     return true;
 }
 
-bool fx_all_lanes(const Plan& p) { return fx_x_lane(p) && fx_lane_length(p.Ny) && fx_lane_length(p.fz.N); }
+// Against the paired-FP32 kernels per flux: 1.05 to 1.7 times as fast where every axis
+// has lane-held lines (64x64x97 158 -> 144 us, 96x96x49 221 -> 189, RK4 step at
+// 256x256x129 9.41 -> 8.35 ms), but not with x or y lines of 192 points (RK4 step at
+// 192x192x97 4.23 -> 4.33 ms) nor on the run-time stages (0.6 to 0.8 times as fast).
+bool fx_beats_paired(const Plan& p) {
+    return fx_x_lane(p) && fx_lane_length(p.Ny) && fx_lane_length(p.fz.N) && p.Nx != 192 && p.Ny != 192;
+}
 
 bool fx_has_rows(const Plan& p) { return fx_x_lane(p) || fx_x_any(p); }
 
@@ -257,7 +276,7 @@ bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& r, const doubl
 bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, const double2* z, double2* y, cudaStream_t s) {
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
-        const int cols = dev::fx_any_cols(Ny, d.kxColumns);
+        const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * map.nOut, grid_cap(1));
         dev::k_yinv_fxany<0><<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps,
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, map, z, y, cols);
         return true;
@@ -276,7 +295,7 @@ bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, cons
 bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, double2* f, cudaStream_t s) {
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
-        const int cols = dev::fx_any_cols(Ny, d.kxColumns);
+        const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * nch, grid_cap(1));
         dev::k_yfwd_fxany<0><<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps,
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, ps, nch, f, cols);
         return true;
@@ -288,6 +307,12 @@ bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, d
 }
 
 bool fx_xc2r(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* y, int nch, double* fields, cudaStream_t s) {
+    if (fx_lane_length(p.Nx)) {
+        const FxLaneField l = fx_lane_field(p, d, nch);
+        WV_FXW_SWITCH(p.Nx, (dev::k_xc2r_fx<NN><<<l.grid, 32 * l.warps, dev::smem_fx_field<NN>(l.warps), s>>>(
+                                d, r.twXLane, y, nch, fields)));
+        return true;
+    }
     if (p.Nx > 512 || d.kxColumns > 256) return false;
     const FxFieldLaunch l = fx_field_launch(p.Nx, p.Ny * d.zTotal, nch);
     WV_FXX_SWITCH(d.kxColumns, (dev::k_xc2r_fxany<EK><<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, y, nch, fields)));
@@ -295,6 +320,12 @@ bool fx_xc2r(const Plan& p, const dev::DescDev& d, const FxRows& r, const double
 }
 
 bool fx_xr2c(const Plan& p, const dev::DescDev& d, const FxRows& r, const double* fields, int nch, double2* ps, cudaStream_t s) {
+    if (fx_lane_length(p.Nx)) {
+        const FxLaneField l = fx_lane_field(p, d, nch);
+        WV_FXW_SWITCH(p.Nx, (dev::k_xr2c_fx<NN><<<l.grid, 32 * l.warps, dev::smem_fx_field<NN>(l.warps), s>>>(
+                                d, r.twXLane, fields, nch, ps)));
+        return true;
+    }
     if (p.Nx > 512 || d.kxColumns > 256) return false;
     const FxFieldLaunch l = fx_field_launch(p.Nx, p.Ny * d.zTotal, nch);
     dev::k_xr2c_fxany<0><<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, fields, nch, ps);

@@ -22,8 +22,8 @@ std::vector<int32_t> fx_lane_table(size_t N);
 // Shared-memory limits of every kernel a handle of this plan launches.
 cudaError_t fx_set_limits(const Plan& p);
 
-// Whether the x, y and z lines all have lane-held lengths.
-bool fx_all_lanes(const Plan& p);
+// Whether the fixed-point kernels beat the paired-FP32 ones of FP32X2 handles.
+bool fx_beats_paired(const Plan& p);
 // Whether fx_xflux serves the plan's rows.
 bool fx_has_rows(const Plan& p);
 bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& rows, const double2* y, double2* ps,

@@ -326,36 +326,6 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
     }
 }
 
-// Real values of a lane (E a row) in the fixed point of their row, for two rows to a line.
-template <int E, int G>
-__device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long (&out)[E], int& unit) {
-    float sum = 0.f;
-#pragma unroll
-    for (int e = 0; e < E; ++e) sum += fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
-    sum = fx_group_sum<G>(sum);
-    fxscale sc = fx_scale(sum);
-    bool zero = false;
-    const bool odd = !fx_plain_sum(sum);
-    if (__any_sync(0xffffffffu, odd)) {
-        unsigned top = 0;
-#pragma unroll
-        for (int e = 0; e < E; ++e) top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
-        top = fx_group_max<G>(top);
-        float rel = 0.f;
-#pragma unroll
-        for (int e = 0; e < E; ++e) rel += fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
-        rel = fx_group_sum<G>(rel);
-        if (odd) {
-            zero = top == 0;
-            sc = fx_scale(top, rel);
-        }
-    }
-    sc.bit -= 2;
-    unit = zero ? kFxZero : fx_unit(sc);
-#pragma unroll
-    for (int e = 0; e < E; ++e) out[e] = fx_from_double(a[e], sc);
-}
-
 // k_xadj on kept rows: a block takes one line-set of rows, as k_xflux_fxco.  Two warps
 // transform the adjoint spectra, every thread forms a sample's gradients in FP64
 // (24 operations), a warp each transforms two of the 3 + 3 nt gradient rows.

@@ -45,12 +45,14 @@ __device__ __forceinline__ fxscale fx_warp_scale(int n, int lane, At at, Count c
 // ---- y ------------------------------------------------------------------------------
 
 constexpr int kFxAnyWarps = 8;
-// Columns of a block: about 2048 entries, at least one line per warp where the plane
-// has them.
-inline int fx_any_cols(int Ny, int kxColumns) {
+// Columns of a block of `planes` (z, channel) planes: about 2048 entries, but down to a
+// line per warp while the blocks don't reach every SM twice.
+inline int fx_any_cols(int Ny, int kxColumns, size_t planes, size_t sms) {
     int c = 2048 / Ny;
     if (c > 32 * kFxAnyWarps) c = 32 * kFxAnyWarps;  // (a lane keeps one line's unit)
-    return c < 1 ? 1 : c > kxColumns ? kxColumns : c;
+    if (c > kxColumns) c = kxColumns;
+    while (c > kFxAnyWarps && (kxColumns + c - 1) / c * planes < 2 * sms) c = (c + 1) / 2;
+    return c < 1 ? 1 : c;
 }
 inline size_t smem_fx_any_y(int Ny, int cols) {
     return (static_cast<size_t>(Ny) + 2 * static_cast<size_t>(cols) * fx_any_ld(Ny)) * 16;

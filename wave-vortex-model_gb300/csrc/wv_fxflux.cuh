@@ -36,7 +36,7 @@ __device__ __forceinline__ void fx_load_row(const double2* __restrict__ h, int K
     }
     auto count = [&](int i) { const int k = lane + 32 * i; return k == 0 || 2 * k == Nx ? 1.0f : 2.0f; };
     if (useK) {
-        fx_quantise_lane<EK, 32, kFxImag, 0>(v, w, static_cast<unsigned>(__double2hiint(rowK[KX - 1])), 1, count, row, unit);
+        fx_quantise_lane<EK, 32, kFxImag, 0>(v, w, fx_row_k_top(rowK, KX), 1, count, row, unit);
 #pragma unroll
         for (int i = 0; i < EK; ++i)
             if (2 * (lane + 32 * i) == Nx) row[i].y = 0;

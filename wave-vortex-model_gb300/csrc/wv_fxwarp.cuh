@@ -108,6 +108,11 @@ __device__ __forceinline__ unsigned long long fx_mantissa(double v, int& e) {
 // What a line's entries are multiplied by: nothing, real weights w, or i w.
 enum FxWeight { kFxPlain, kFxReal, kFxImag };
 
+// High word of the largest k (a full half spectrum ends with a zero weight).
+__device__ __forceinline__ unsigned fx_row_k_top(const double* __restrict__ rowK, int KX) {
+    return static_cast<unsigned>(max(__double2hiint(rowK[KX - 1]), __double2hiint(rowK[max(KX - 2, 0)])));
+}
+
 // C doubles of a lane, weighted, in the fixed point of their line.  count(c): how
 // often entry c enters the line's sum of moduli; spare: bits kept free (1 when two
 // rows share the line); wtop: high word of the largest |w|.
@@ -144,8 +149,8 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
         }
         rel = fx_group_sum<G>(rel);
         if (odd) {
-            zero = top == 0;
             sc = fx_scale(top, rel);
+            zero = top == 0 || (MODE != kFxPlain && wtop == 0 && sc.e0 < 0x7ff);
             if (MODE != kFxPlain) wexp = static_cast<int>((wtop >> 20) & 0x7ffu) - 1023;
         }
     }
@@ -381,7 +386,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
     const size_t cstride = static_cast<size_t>(Ny) * KX;
     const size_t R3 = static_cast<size_t>(N) * Ny * d.Nz;
     const int rows = Ny * d.zTotal;
-    const unsigned wtop = static_cast<unsigned>(__double2hiint(rowK[KX - 1]));
+    const unsigned wtop = fx_row_k_top(rowK, KX);
     for (int first = (blockIdx.x * warps + warp) * W::lines; first < rows; first += gridDim.x * warps * W::lines) {
         const bool live = first + line < rows;
         const int row = min(first + line, rows - 1);
@@ -501,7 +506,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
     const size_t cstride = static_cast<size_t>(Ny) * KX;
     const size_t R3 = static_cast<size_t>(N) * Ny * d.Nz;
     const int rows = Ny * d.zTotal;
-    const unsigned wtop = static_cast<unsigned>(__double2hiint(rowK[KX - 1]));
+    const unsigned wtop = fx_row_k_top(rowK, KX);
     const int first = blockIdx.x * W::lines;
     const bool live = first + line < rows;
     const int row = min(first + line, rows - 1);

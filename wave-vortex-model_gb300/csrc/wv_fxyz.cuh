@@ -114,6 +114,170 @@ __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     }
 }
 
+// Real values of a lane (E a row) in the fixed point of their row, for two rows to a line.
+template <int E, int G>
+__device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long (&out)[E], int& unit) {
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) sum += fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
+    sum = fx_group_sum<G>(sum);
+    fxscale sc = fx_scale(sum);
+    bool zero = false;
+    const bool odd = !fx_plain_sum(sum);
+    if (__any_sync(0xffffffffu, odd)) {
+        unsigned top = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
+        top = fx_group_max<G>(top);
+        float rel = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) rel += fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
+        rel = fx_group_sum<G>(rel);
+        if (odd) {
+            zero = top == 0;
+            sc = fx_scale(top, rel);
+        }
+    }
+    sc.bit -= 2;
+    unit = zero ? kFxZero : fx_unit(sc);
+#pragma unroll
+    for (int e = 0; e < E; ++e) out[e] = fx_from_double(a[e], sc);
+}
+
+// ---- field rows along x -----------------------------------------------------------------
+
+constexpr int kFxFieldWarps = 4;
+template <int N>
+inline size_t smem_fx_field(int warps) { return (FxW<N>::twiddles + warps * FxW<N>::lines * FxW<N>::buffer) * 16; }
+
+// k_xc2r_fields: a warp takes two channels of a line-set of rows as one line.  KX may
+// reach N / 2 + 1 (the scalar pipeline's full half spectrum).
+template <int N>
+__global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
+    k_xc2r_fx(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, int nch, double* __restrict__ fields) {
+    using W = FxW<N>;
+    constexpr int G = W::G, E = W::E, H = W::H;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int Ny = d.Ny, KX = d.kxColumns;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = lane % G, line = lane / G;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(warp * W::lines + line) * W::buffer;
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
+    const int rows = Ny * d.zTotal, pairs = (nch + 1) / 2;
+    const int unitOfWork = blockIdx.x * (blockDim.x >> 5) + warp;
+    const int p = unitOfWork % pairs, first = unitOfWork / pairs * W::lines;
+    const bool live = first + line < rows;
+    const int row = min(first + line, rows - 1);
+    const int z = row / Ny, y = row - z * Ny;
+    const double* rowK = row_k<double>(d);
+    const unsigned wtop = fx_row_k_top(rowK, KX);
+    // entries k = t + G i of both channels, and k = N / 2 on lane 0
+    fxc AB[2][H + 1];
+    int unit[2] = {kFxZero, kFxZero};
+    auto count = [&](int i) { return (i == 0 && t == 0) || i == H ? 1.0f : 2.0f; };
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int c = 2 * p + q;
+        const double2* h = yspec + ((static_cast<size_t>(z) * nch + min(c, nch - 1)) * Ny + y) * KX;
+        double2 a[H + 1];
+        double w[H + 1];
+        const bool useK = ((d.c2rUseK >> c) & 1) != 0;
+#pragma unroll
+        for (int i = 0; i < H + 1; ++i) {
+            const int k = t + G * i;
+            const bool has = c < nch && k < KX && (i < H || t == 0);
+            a[i] = has ? h[k] : make_double2(0.0, 0.0);
+            w[i] = useK && has ? rowK[k] : 0.0;
+            if (k == 0 || i == H) a[i].y = 0.0;  // c2r semantics
+        }
+        if (useK) {
+            fx_quantise_lane<H + 1, G, kFxImag>(a, w, wtop, 1, count, AB[q], unit[q]);
+            AB[q][H].y = 0;
+        } else {
+            fx_quantise_lane<H + 1, G, kFxPlain>(a, w, 0u, 1, count, AB[q], unit[q]);
+        }
+    }
+    __syncthreads();  // twiddles
+    fxc v[E];
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const fxc a = AB[0][i], b = AB[1][i];
+        const int k = t + G * i;
+        v[i] = fxc{a.x - b.y, a.y + b.x};
+        x[fx_pad(k == 0 ? N / 2 : N - k)] = k == 0 ? fxc{AB[0][H].x, AB[1][H].x} : fxc{a.x + b.y, b.x - a.y};
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
+    __syncwarp();
+    fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : fx_two());
+    if (!live) return;
+    const FxUnit oa = fx_out(unit[0]), ob = fx_out(unit[1]);
+    const size_t R = static_cast<size_t>(N) * Ny * d.Nz;
+    double* o = fields + static_cast<size_t>(2 * p) * R + (static_cast<size_t>(z) * Ny + y) * N;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        o[t + G * e] = fx_to_double(v[e].x, oa);
+        if (2 * p + 1 < nch) o[R + t + G * e] = fx_to_double(v[e].y, ob);
+    }
+}
+
+// k_xr2c_fields: a warp takes two channels of a line-set of rows as one line.
+template <int N>
+__global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
+    k_xr2c_fx(DescDev d, const fxw* __restrict__ twg, const double* __restrict__ fields, int nch, double2* __restrict__ pspec) {
+    using W = FxW<N>;
+    constexpr int G = W::G, E = W::E, H = W::H;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int Ny = d.Ny, KX = d.kxColumns;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = lane % G, line = lane / G;
+    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
+    fxc* x = reinterpret_cast<fxc*>(tw + W::twiddles) + static_cast<size_t>(warp * W::lines + line) * W::buffer;
+    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
+    const int rows = Ny * d.zTotal, pairs = (nch + 1) / 2;
+    const int unitOfWork = blockIdx.x * (blockDim.x >> 5) + warp;
+    const int p = unitOfWork % pairs, first = unitOfWork / pairs * W::lines;
+    const bool live = first + line < rows, both = 2 * p + 1 < nch;
+    const int row = min(first + line, rows - 1);
+    const int z = row / Ny, y = row - z * Ny;
+    const size_t R = static_cast<size_t>(N) * Ny * d.Nz;
+    const double* in = fields + static_cast<size_t>(2 * p) * R + (static_cast<size_t>(z) * Ny + y) * N;
+    double ra[E], rb[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        ra[e] = in[t + G * e];
+        rb[e] = both ? in[R + t + G * e] : 0.0;
+    }
+    long long ia[E], ib[E];
+    int ua, ub;
+    fx_quantise_real<E, G>(ra, ia, ua);
+    fx_quantise_real<E, G>(rb, ib, ub);
+    fxc v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = fxc{ia[e], ib[e]};
+    __syncthreads();  // twiddles
+    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(ua, ub)) ? 0 : fx_two());
+#pragma unroll
+    for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
+    __syncwarp();
+    if (!live) return;
+    const FxUnit oa = fx_out(ua - 1), ob = fx_out(ub - 1);  // the halves of the split
+    double2* out = pspec + ((static_cast<size_t>(z) * nch + 2 * p) * Ny + y) * KX;
+    const size_t cstride = static_cast<size_t>(Ny) * KX;
+    auto store = [&](int k, fxc a, fxc b) {
+        out[k] = make_double2(fx_to_double(a.x + b.x, oa), fx_to_double(a.y - b.y, oa));
+        if (both) out[cstride + k] = make_double2(fx_to_double(a.y + b.y, ob), fx_to_double(b.x - a.x, ob));
+    };
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const int k = t + G * i;
+        if (k < KX) store(k, v[i], k == 0 ? v[0] : x[fx_pad(N - k)]);
+    }
+    if (t == 0 && N / 2 < KX) store(N / 2, v[H], v[H]);
+}
+
 // ---- phases ----------------------------------------------------------------------------
 
 // exp(i angle) rounded from fixed point: the angle in turns is the exact product of

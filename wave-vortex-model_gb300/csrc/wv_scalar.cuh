@@ -11,7 +11,10 @@
 namespace wvgpu {
 namespace dev {
 
-constexpr int kScalarCols = 32;  // positions per CTA of k_scalar_derivs
+// Positions per CTA of k_scalar_derivs.  FP64's dense z contraction is bound by the
+// FP64 pipe: eight positions spread a small grid's columns over every SM (96x64x33:
+// 392 blocks instead of 98 on 152 SMs).
+template <typename T> struct ScalarCols { static constexpr int value = sizeof(T) == 8 && std::is_same<T, double>::value ? 8 : 32; };
 
 // in: channel spectra [z][pos] of the scalar after the y forward FFT (unscaled).
 // out: [3][z][pos] = i k v, i l v, D v with v = hs * in; self-conjugate rows real.
@@ -20,6 +23,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_scalar_derivs(DescDev d, const cx<T>* __restrict__ in, const T* __restrict__ D,
                                                       const unsigned char* __restrict__ flags, double hs,
                                                       cx<T>* __restrict__ out) {
+    constexpr int kScalarCols = ScalarCols<T>::value;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<T>* v = reinterpret_cast<cx<T>*>(smem_raw);  // [Nz][kScalarCols]
     const int P = d.positions, Nz = d.Nz, Ny = d.Ny;
