@@ -82,16 +82,15 @@ inline int fx_z_any_warps(const Plan& p, int lines) {
     const size_t room = std::max<size_t>(1, (100 * 1024) / each);
     return static_cast<int>(std::min<size_t>({room, dev::kFxAnyWarps, std::max<size_t>(1, (p.Nkl + sms - 1) / sms)}));
 }
-// The field kernels along x: one warp per row.
+// The run-time field kernels along x: a warp per row and channel pair.
 struct FxFieldLaunch { int warps, grid; size_t smem; };
 inline FxFieldLaunch fx_field_launch(size_t Nx, size_t rows, int nch) {
     FxFieldLaunch l{};
-    const int lines = (nch + 1) / 2;
-    const size_t each = 2 * static_cast<size_t>(lines) * Nx * 16;
+    const size_t units = rows * ((nch + 1) / 2), each = 2 * Nx * 16;
     l.warps = static_cast<int>(std::min<size_t>(dev::kFxAnyWarps, std::max<size_t>(1, (104 * 1024 - Nx * 16) / each)));
-    while (l.warps > 1 && rows < l.warps * static_cast<size_t>(grid_cap(1))) l.warps /= 2;
-    l.smem = dev::smem_fx_any_x(static_cast<int>(Nx), lines, l.warps);
-    l.grid = static_cast<int>(std::min<size_t>((rows + l.warps - 1) / l.warps, grid_cap(2)));
+    while (l.warps > 1 && units < l.warps * static_cast<size_t>(grid_cap(1))) l.warps /= 2;
+    l.smem = dev::smem_fx_any_x(static_cast<int>(Nx), l.warps);
+    l.grid = static_cast<int>(std::min<size_t>((units + l.warps - 1) / l.warps, grid_cap(2)));
     return l;
 }
 // Grid and warps of the lane-held field kernels (a warp per line-set and channel pair;
@@ -142,19 +141,17 @@ cudaError_t fx_set_limits(const Plan& p) {
     if (!fx_lane_length(p.Ny)) {
         // (the scalar pipeline has the most columns)
         const size_t sm = dev::smem_fx_any_y(static_cast<int>(p.Ny), dev::fx_any_cols(static_cast<int>(p.Ny), 1 << 20, 1, 1));
-        set(dev::k_yinv_fxany<0>, sm);
-        set(dev::k_yfwd_fxany<0>, sm);
+        set(dev::k_yinv_fxany, sm);
+        set(dev::k_yfwd_fxany, sm);
     }
     WV_FXW_SWITCH(p.Nx, {
         set(dev::k_xc2r_fx<NN>, dev::smem_fx_field<NN>(dev::kFxFieldWarps));
         set(dev::k_xr2c_fx<NN>, dev::smem_fx_field<NN>(dev::kFxFieldWarps));
     });
     if (fx_x_any(p) && !fx_lane_length(p.Nx)) {
-        for (int nch = 1; nch <= 4; nch += 2) {
-            const FxFieldLaunch l = fx_field_launch(p.Nx, SIZE_MAX / 2, nch);
-            set(dev::k_xc2r_fxany<2>, l.smem); set(dev::k_xc2r_fxany<4>, l.smem); set(dev::k_xc2r_fxany<8>, l.smem);
-            set(dev::k_xr2c_fxany<0>, l.smem);
-        }
+        const FxFieldLaunch l = fx_field_launch(p.Nx, SIZE_MAX / 4, 1);
+        set(dev::k_xc2r_fxany<2>, l.smem); set(dev::k_xc2r_fxany<4>, l.smem); set(dev::k_xc2r_fxany<8>, l.smem);
+        set(dev::k_xr2c_fxany, l.smem);
     }
     if (p.fz.N > 0 && !fx_lane_length(p.fz.N)) {
         const size_t inv = dev::smem_fx_any_z(p.fz.N, 4, fx_z_any_warps(p, 4)), two = dev::smem_fx_any_z(p.fz.N, 2, fx_z_any_warps(p, 2));
@@ -277,7 +274,7 @@ bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, cons
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
         const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * map.nOut, grid_cap(1));
-        dev::k_yinv_fxany<0><<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps,
+        dev::k_yinv_fxany<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps,
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, map, z, y, cols);
         return true;
     }
@@ -296,7 +293,7 @@ bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, d
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
         const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * nch, grid_cap(1));
-        dev::k_yfwd_fxany<0><<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps,
+        dev::k_yfwd_fxany<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps,
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, ps, nch, f, cols);
         return true;
     }
@@ -328,7 +325,7 @@ bool fx_xr2c(const Plan& p, const dev::DescDev& d, const FxRows& r, const double
     }
     if (p.Nx > 512 || d.kxColumns > 256) return false;
     const FxFieldLaunch l = fx_field_launch(p.Nx, p.Ny * d.zTotal, nch);
-    dev::k_xr2c_fxany<0><<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, fields, nch, ps);
+    dev::k_xr2c_fxany<<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, fields, nch, ps);
     return true;
 }
 

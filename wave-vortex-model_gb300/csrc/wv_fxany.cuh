@@ -63,7 +63,6 @@ __device__ __forceinline__ void fx_any_twiddles(fxw* tw, const fxw* __restrict__
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = twg[i];
     __syncthreads();
 }
-template <int kUnused>
 __global__ void __launch_bounds__(32 * kFxAnyWarps)
     k_yinv_fxany(DescDev d, YInvMap map, const double2* __restrict__ zspec, double2* __restrict__ yspec, int cols) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -122,7 +121,6 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
 }
 
 // k_yfwd, channel blockIdx.z.
-template <int kUnused>
 __global__ void __launch_bounds__(32 * kFxAnyWarps)
     k_yfwd_fxany(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec, int cols) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -170,13 +168,11 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
 
 // ---- field rows along x -----------------------------------------------------------------
 
-// Shared memory of the field kernels: twiddles [Nx], per warp two buffers of
-// `lines` lines.
-inline size_t smem_fx_any_x(int Nx, int lines, int warps) {
-    return (static_cast<size_t>(Nx) + static_cast<size_t>(warps) * 2 * lines * Nx) * 16;
-}
+// Shared memory of the field kernels: twiddles [Nx], per warp two buffers of one line.
+inline size_t smem_fx_any_x(int Nx, int warps) { return (static_cast<size_t>(Nx) + static_cast<size_t>(warps) * 2 * Nx) * 16; }
 
-// k_xc2r_fields: one warp per (y, z) row, two channels to a line.
+// k_xc2r_fields: a warp takes two channels of a (y, z) row as one line.  A warp per
+// row with all its channels leaves small grids to a few long-running warps.
 template <int EK>
 __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
     k_xc2r_fxany(DescDev d, FFTDev f, const fxw* __restrict__ twg, const double2* __restrict__ yspec, int nch,
@@ -184,86 +180,72 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nx = d.Nx, Ny = d.Ny, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const int lines = (nch + 1) / 2;
     fxw* tw = reinterpret_cast<fxw*>(smem_raw);
-    fxc* bufA = reinterpret_cast<fxc*>(tw + Nx) + static_cast<size_t>(warp) * 2 * lines * Nx;
-    fxc* bufB = bufA + lines * Nx;
+    fxc* bufA = reinterpret_cast<fxc*>(tw + Nx) + static_cast<size_t>(warp) * 2 * Nx;
+    fxc* bufB = bufA + Nx;
     fx_any_twiddles(tw, twg, Nx);
     const size_t R = static_cast<size_t>(Nx) * Ny * d.Nz;
-    const int rows = Ny * d.zTotal;
-    for (int row = blockIdx.x * warps + warp; row < rows; row += gridDim.x * warps) {
+    const int pairs = (nch + 1) / 2, units = Ny * d.zTotal * pairs;
+    for (int unit = blockIdx.x * warps + warp; unit < units; unit += gridDim.x * warps) {
+        const int row = unit / pairs, ca = 2 * (unit - row * pairs), cb = ca + 1;
         const int z = row / Ny, y = row - z * Ny;
-        const double2* h = yspec + (static_cast<size_t>(z) * nch * Ny + y) * KX;
-        int units = 0;
-        for (int l = 0; l < lines; ++l) {
-            fxc A[EK], B[EK];
-            int uA, uB = 0;
-            const int ca = 2 * l, cb = 2 * l + 1;
-            fx_load_row<EK>(h + static_cast<size_t>(ca) * Ny * KX, KX, Nx, lane, ((d.c2rUseK >> ca) & 1) != 0, row_k<double>(d), A, uA);
-            if (cb < nch) {
-                fx_load_row<EK>(h + static_cast<size_t>(cb) * Ny * KX, KX, Nx, lane, ((d.c2rUseK >> cb) & 1) != 0, row_k<double>(d), B, uB);
-            } else {
+        const double2* h = yspec + ((static_cast<size_t>(z) * nch + ca) * Ny + y) * KX;
+        fxc A[EK], B[EK];
+        int uA, uB = 0;
+        fx_load_row<EK>(h, KX, Nx, lane, ((d.c2rUseK >> ca) & 1) != 0, row_k<double>(d), A, uA);
+        if (cb < nch) {
+            fx_load_row<EK>(h + static_cast<size_t>(Ny) * KX, KX, Nx, lane, ((d.c2rUseK >> cb) & 1) != 0, row_k<double>(d), B, uB);
+        } else {
 #pragma unroll
-                for (int e = 0; e < EK; ++e) B[e] = fxc{0, 0};
-            }
-            if (lane == ca) units = uA;
-            if (lane == cb) units = uB;
-            fx_pack_rows<EK>(A, B, bufA + l * Nx, KX, Nx, lane);
+            for (int e = 0; e < EK; ++e) B[e] = fxc{0, 0};
         }
+        fx_pack_rows<EK>(A, B, bufA, KX, Nx, lane);
         __syncwarp();
-        const fxc* r = fx_lines<true, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, lines, Nx, tw);
-        for (int c = 0; c < nch; ++c) {
-            const int u = __shfl_sync(0xffffffffu, units, c);
-            double* o = fields + static_cast<size_t>(c) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
-            const fxc* s = r + (c >> 1) * Nx;
-            for (int x = lane; x < Nx; x += 32) o[x] = fx_to_double((c & 1) ? s[x].y : s[x].x, fx_out(u));
+        const fxc* r = fx_lines<true, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, Nx, tw);
+        double* o = fields + static_cast<size_t>(ca) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
+        for (int x = lane; x < Nx; x += 32) {
+            o[x] = fx_to_double(r[x].x, fx_out(uA));
+            if (cb < nch) o[R + x] = fx_to_double(r[x].y, fx_out(uB));
         }
         __syncwarp();
     }
 }
 
-// k_xr2c_fields: one warp per (y, z) row, two channels to a line.
-template <int kUnused>
+// k_xr2c_fields: a warp takes two channels of a (y, z) row as one line.
 __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
     k_xr2c_fxany(DescDev d, FFTDev f, const fxw* __restrict__ twg, const double* __restrict__ fields, int nch,
                  double2* __restrict__ pspec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Nx = d.Nx, Ny = d.Ny, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const int lines = (nch + 1) / 2;
     fxw* tw = reinterpret_cast<fxw*>(smem_raw);
-    fxc* bufA = reinterpret_cast<fxc*>(tw + Nx) + static_cast<size_t>(warp) * 2 * lines * Nx;
-    fxc* bufB = bufA + lines * Nx;
+    fxc* bufA = reinterpret_cast<fxc*>(tw + Nx) + static_cast<size_t>(warp) * 2 * Nx;
+    fxc* bufB = bufA + Nx;
     fx_any_twiddles(tw, twg, Nx);
     const size_t R = static_cast<size_t>(Nx) * Ny * d.Nz;
-    const int rows = Ny * d.zTotal;
-    for (int row = blockIdx.x * warps + warp; row < rows; row += gridDim.x * warps) {
+    const int pairs = (nch + 1) / 2, units = Ny * d.zTotal * pairs;
+    for (int unit = blockIdx.x * warps + warp; unit < units; unit += gridDim.x * warps) {
+        const int row = unit / pairs, c = 2 * (unit - row * pairs);
         const int z = row / Ny, y = row - z * Ny;
-        int units = 0;
-        for (int c = 0; c < 2 * lines; ++c) {
-            double2* raw = reinterpret_cast<double2*>(bufB + (c >> 1) * Nx);  // the samples, in their fixed-point slots
-            const double* s = fields + static_cast<size_t>(min(c, nch - 1)) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
-            for (int x = lane; x < Nx; x += 32) raw[x].x = c < nch ? s[x] : 0.0;
-            fxscale sc = fx_warp_scale(Nx, lane, [&](int x) { return make_double2(raw[x].x, 0.0); }, [](int) { return 1.0f; });
-            sc.bit -= 1;
-            for (int x = lane; x < Nx; x += 32) {
-                const long long v = fx_from_double(raw[x].x, sc);
-                fxc* q = bufA + (c >> 1) * Nx + x;
-                if (c & 1) q->y = v; else q->x = v;
-            }
-            if (lane == c) units = fx_unit(sc) - 1;  // the halves of the split below
-        }
+        const bool both = c + 1 < nch;
+        double2* raw = reinterpret_cast<double2*>(bufB);  // the samples, in their fixed-point slots
+        const double* s = fields + static_cast<size_t>(c) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
+        for (int x = lane; x < Nx; x += 32) raw[x] = make_double2(s[x], both ? s[R + x] : 0.0);
+        auto one = [](int) { return 1.0f; };
+        fxscale sa = fx_warp_scale(Nx, lane, [&](int x) { return make_double2(raw[x].x, 0.0); }, one);
+        fxscale sb = fx_warp_scale(Nx, lane, [&](int x) { return make_double2(raw[x].y, 0.0); }, one);
+        sa.bit -= 1;
+        sb.bit -= 1;
+        for (int x = lane; x < Nx; x += 32) bufA[x] = fxc{fx_from_double(raw[x].x, sa), fx_from_double(raw[x].y, sb)};
+        const int ua = fx_unit(sa) - 1, ub = fx_unit(sb) - 1;  // the halves of the split below
         __syncwarp();
-        const fxc* r = fx_lines<false, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, lines, Nx, tw);
-        for (int l = 0; l < lines; ++l) {
-            const int ua = __shfl_sync(0xffffffffu, units, 2 * l), ub = __shfl_sync(0xffffffffu, units, 2 * l + 1);
-            double2* o = pspec + ((static_cast<size_t>(z) * nch + 2 * l) * Ny + y) * KX;
-            for (int k = lane; k < KX; k += 32) {
-                const fxc a = r[l * Nx + k], b = r[l * Nx + (k == 0 ? 0 : Nx - k)];
-                o[k] = make_double2(fx_to_double(a.x + b.x, fx_out(ua)), fx_to_double(a.y - b.y, fx_out(ua)));
-                if (2 * l + 1 < nch)
-                    o[static_cast<size_t>(Ny) * KX + k] = make_double2(fx_to_double(a.y + b.y, fx_out(ub)), fx_to_double(b.x - a.x, fx_out(ub)));
-            }
+        const fxc* r = fx_lines<false, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, Nx, tw);
+        double2* o = pspec + ((static_cast<size_t>(z) * nch + c) * Ny + y) * KX;
+        for (int k = lane; k < KX; k += 32) {
+            const fxc a = r[k], b = r[k == 0 ? 0 : Nx - k];
+            o[k] = make_double2(fx_to_double(a.x + b.x, fx_out(ua)), fx_to_double(a.y - b.y, fx_out(ua)));
+            if (both)
+                o[static_cast<size_t>(Ny) * KX + k] = make_double2(fx_to_double(a.y + b.y, fx_out(ub)), fx_to_double(b.x - a.x, fx_out(ub)));
         }
         __syncwarp();
     }
