@@ -427,22 +427,33 @@ cudaError_t set_smem_limits(const Plan& p) {
     if (e != cudaSuccess) return e;
     WV_SET((dev::k_vinv<T, true>), smem_vinv<T>(p));
     WV_SET((dev::k_vinv<T, false>), smem_vinv<T>(p));
-    WV_SET((dev::k_yinv<T>), smem_y<T>(p));
-    WV_SET((dev::k_yfwd<T>), smem_y<T>(p));
+    if constexpr (std::is_same<T, double>::value) {
+        // (FP64 lines along y and z run in fixed point; grids are refused where they
+        // outgrow the block transforms of the other forms)
+        int device = 0, room = 0;
+        e = cudaGetDevice(&device);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        if (e != cudaSuccess) return e;
+        const size_t zb = p.fz.N > 0 ? std::max({dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, true>::modes),
+                                                 dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, false>::modes),
+                                                 dev::smem_vfwd_fft<T>(p.fz.N)}) : 0;
+        if (std::max(smem_y<T>(p), zb) > static_cast<size_t>(room)) return cudaErrorInvalidConfiguration;
+        e = wvgpu::fx_set_limits(p);
+        if (e != cudaSuccess) return e;
+    } else {
+        WV_SET((dev::k_yinv<T>), smem_y<T>(p));
+        WV_SET((dev::k_yfwd<T>), smem_y<T>(p));
+        if (p.fz.N > 0) {
+            WV_SET((dev::k_vinv_fft<T, true>), dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, true>::modes));
+            WV_SET((dev::k_vinv_fft<T, false>), dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, false>::modes));
+            WV_SET((dev::k_vfwd_fft<T, true>), dev::smem_vfwd_fft<T>(p.fz.N));
+        }
+    }
     WV_SET((dev::k_xflux<T>), smem_xflux<T>(p));
     WV_SET((dev::k_xc2r_fields<T>), smem_xc2r<T>(p, 4));
     WV_SET((dev::k_xr2c_fields<T>), smem_xr2c<T>(p));
     WV_SET((dev::k_vfwd<T, true>), smem_vfwd<T>(p, 4));
     WV_SET((dev::k_vfwd<T, false>), smem_vfwd<T>(p, 4));
-    if constexpr (std::is_same<T, double>::value) {
-        e = wvgpu::fx_set_limits(p);
-        if (e != cudaSuccess) return e;
-    }
-    if (p.fz.N > 0) {
-        WV_SET((dev::k_vinv_fft<T, true>), dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, true>::modes));
-        WV_SET((dev::k_vinv_fft<T, false>), dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, dev::VzShape<T, false>::modes));
-        WV_SET((dev::k_vfwd_fft<T, true>), dev::smem_vfwd_fft<T>(p.fz.N));
-    }
 #undef WV_SET
     return cudaSuccess;
 }
@@ -555,30 +566,33 @@ void launch_yinv(wv_handle* h, const dev::YInvMap& map, const dev::cx<T>* z, dev
     const Plan& p = h->plan;
     const dev::DescDev& dd = over ? *over : desc_of<T>(h);
     if constexpr (std::is_same<T, double>::value) {
-        if (wvgpu::fx_yinv(p, dd, map, z, y, s)) return;
+        wvgpu::fx_yinv(p, dd, map, z, y, s);
+    } else {
+        const int ry = warp_ry<T>(p);
+        if (ry) {
+            const dim3 grid(cdiv(p.kxColumns, dev::kWG), dd.zTotal, map.nOut);
+            WV_RSWITCH_Y(ry, (dev::k_yinv_w<T, RR><<<grid, 256, smem_y_w<T>(p), s>>>(dd, map, z, y)));
+            return;
+        }
+        dev::k_yinv<T><<<dim3(cdiv(p.kxColumns, dev::kYG), dd.zTotal), 256, smem_y<T>(p), s>>>(dd, map, z, 0, y);
     }
-    const int ry = warp_ry<T>(p);
-    if (ry) {
-        const dim3 grid(cdiv(p.kxColumns, dev::kWG), dd.zTotal, map.nOut);
-        WV_RSWITCH_Y(ry, (dev::k_yinv_w<T, RR><<<grid, 256, smem_y_w<T>(p), s>>>(dd, map, z, y)));
-        return;
-    }
-    dev::k_yinv<T><<<dim3(cdiv(p.kxColumns, dev::kYG), dd.zTotal), 256, smem_y<T>(p), s>>>(dd, map, z, 0, y);
 }
 
 template <typename T>
 void launch_yfwd(wv_handle* h, const dev::cx<T>* ps, int nch, dev::cx<T>* f, cudaStream_t s) {
     const Plan& p = h->plan;
+    const dev::DescDev& dd = desc_of<T>(h);
     if constexpr (std::is_same<T, double>::value) {
-        if (wvgpu::fx_yfwd(p, desc_of<T>(h), ps, nch, f, s)) return;
+        wvgpu::fx_yfwd(p, dd, ps, nch, f, s);
+    } else {
+        const int ry = warp_ry<T>(p);
+        if (ry) {
+            const dim3 grid(cdiv(p.kxColumns, dev::kWG), dd.zTotal, nch);
+            WV_RSWITCH_Y(ry, (dev::k_yfwd_w<T, RR><<<grid, 256, smem_y_w<T>(p), s>>>(dd, ps, nch, f)));
+            return;
+        }
+        dev::k_yfwd<T><<<dim3(cdiv(p.kxColumns, dev::kYG), dd.zTotal, nch), 256, smem_y<T>(p), s>>>(dd, ps, nch, f);
     }
-    const int ry = warp_ry<T>(p);
-    if (ry) {
-        const dim3 grid(cdiv(p.kxColumns, dev::kWG), desc_of<T>(h).zTotal, nch);
-        WV_RSWITCH_Y(ry, (dev::k_yfwd_w<T, RR><<<grid, 256, smem_y_w<T>(p), s>>>(desc_of<T>(h), ps, nch, f)));
-        return;
-    }
-    dev::k_yfwd<T><<<dim3(cdiv(p.kxColumns, dev::kYG), desc_of<T>(h).zTotal, nch), 256, smem_y<T>(p), s>>>(desc_of<T>(h), ps, nch, f);
 }
 
 template <typename T>
@@ -632,24 +646,6 @@ void launch_xr2c(wv_handle* h, const double* fields, int nch, dev::cx<T>* ps, cu
     dev::k_xr2c_fields<T><<<dim3(p.Ny, desc_of<T>(h).zTotal), 256, smem_xr2c<T>(p), s>>>(desc_of<T>(h), fields, nch, ps);
 }
 
-// The vertical transforms of FP64 handles on lane-held lines; false where the
-// length has none.
-template <typename T>
-bool launch_vinv_fx(wv_handle* h, bool flux, double elapsed, const double* Ap, const double* Am, const double* A0,
-                    dev::cx<T>* z, unsigned long long* speed, cudaStream_t s) {
-    if constexpr (std::is_same<T, double>::value)
-        return wvgpu::fx_vinv(h->plan, desc_of<T>(h), flux, elapsed, Ap, Am, A0, z, speed, s);
-    return false;
-}
-template <typename T>
-bool launch_vfwd_fx(wv_handle* h, bool flux, const dev::cx<T>* f, int nch, double elapsed, const double* Ap, const double* Am,
-                    const double* A0, const unsigned long long* speed, int damping, double* Fp, double* Fm, double* F0,
-                    cudaStream_t s) {
-    if constexpr (std::is_same<T, double>::value)
-        return wvgpu::fx_vfwd(h->plan, desc_of<T>(h), flux, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0, s);
-    return false;
-}
-
 // The flux's vertical inverse transform with the handle's kernel choice: the
 // tensor-core kernels (mixed: split-BF16; FP32X2: digit slices, with the
 // y-spectra buffer yScratch as its scratch), the FFTs of the even / odd
@@ -679,11 +675,14 @@ void launch_vinv_flux(wv_handle* h, double elapsed, const double* Ap, const doub
             const size_t sm = dev::smem_vinv_wfft<T>(static_cast<int>(p.Nj), p.fz.N);
             WV_RSWITCH_Y(warp_rz<T>(p), (dev::k_vinv_wfft<T, RR><<<grid, 256, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed)));
         }
-    } else if (h->vinvKind == WV_VERTICAL_FFT && launch_vinv_fx<T>(h, true, elapsed, Ap, Am, A0, z, speed, s)) {
     } else if (h->vinvKind == WV_VERTICAL_FFT) {
-        constexpr int modes = dev::VzShape<T, true>::modes;
-        dev::k_vinv_fft<T, true><<<dim3(cdiv(p.Nkl, modes), d.members), 256,
-                                    dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, modes), s>>>(d, Ap, Am, A0, elapsed, z, speed);
+        if constexpr (std::is_same<T, double>::value) {
+            wvgpu::fx_vinv(p, d, true, elapsed, Ap, Am, A0, z, speed, s);
+        } else {
+            constexpr int modes = dev::VzShape<T, true>::modes;
+            dev::k_vinv_fft<T, true><<<dim3(cdiv(p.Nkl, modes), d.members), 256,
+                                        dev::smem_vinv_fft<T>(static_cast<int>(p.Nj), p.fz.N, modes), s>>>(d, Ap, Am, A0, elapsed, z, speed);
+        }
     } else {
         dev::k_vinv<T, true><<<dim3(cdiv(p.Nkl, dev::kVinvModes), d.members), 256, smem_vinv<T>(p), s>>>(d, Ap, Am, A0, elapsed, z, speed);
     }
@@ -757,11 +756,12 @@ cudaError_t launch_flux(wv_handle* h, double t, double t0, const double* Ap, con
         }
         fwdTC = true;
     }
-    if (!fwdTC && h->vfwdKind == WV_VERTICAL_FFT)
-        fwdTC = launch_vfwd_fx<T>(h, true, f, nt, elapsed, Ap, Am, A0, speed, damping ? 1 : 0, Fp, Fm, F0, s);
     if (!fwdTC && h->vfwdKind == WV_VERTICAL_FFT) {
-        dev::k_vfwd_fft<T, true><<<dim3(cdiv(p.Nkl, dev::vf_modes<T>()), d.members), 256, dev::smem_vfwd_fft<T>(p.fz.N), s>>>(
-            d, f, nt, elapsed, Ap, Am, A0, speed, damping ? 1 : 0, Fp, Fm, F0);
+        if constexpr (std::is_same<T, double>::value)
+            wvgpu::fx_vfwd(p, d, true, f, nt, elapsed, Ap, Am, A0, speed, damping ? 1 : 0, Fp, Fm, F0, s);
+        else
+            dev::k_vfwd_fft<T, true><<<dim3(cdiv(p.Nkl, dev::vf_modes<T>()), d.members), 256, dev::smem_vfwd_fft<T>(p.fz.N), s>>>(
+                d, f, nt, elapsed, Ap, Am, A0, speed, damping ? 1 : 0, Fp, Fm, F0);
         fwdTC = true;  // forward transform launched
     }
     if (!fwdTC)
@@ -908,12 +908,12 @@ cudaError_t launch_scalar_advection(wv_handle* h, const double* scalar, const do
         dev::k_xr2c_fields<T><<<dim3(Ny, Nz), 256, smR2C, s>>>(sd, in, 1, out);
     };
     auto yfwd = [&](dev::cx<T>* out) {
-        if constexpr (fp64) if (wvgpu::fx_yfwd(p, sd, sp, 1, out, s)) return;
-        dev::k_yfwd<T><<<dim3(cdiv(KX, dev::kYG), Nz, 1), 256, smem_y<T>(p), s>>>(sd, sp, 1, out);
+        if constexpr (fp64) wvgpu::fx_yfwd(p, sd, sp, 1, out, s);
+        else dev::k_yfwd<T><<<dim3(cdiv(KX, dev::kYG), Nz, 1), 256, smem_y<T>(p), s>>>(sd, sp, 1, out);
     };
     auto yinv = [&](const dev::YInvMap& m) {
-        if constexpr (fp64) if (wvgpu::fx_yinv(p, sd, m, sf, sp, s)) return;
-        dev::k_yinv<T><<<dim3(cdiv(KX, dev::kYG), Nz), 256, smem_y<T>(p), s>>>(sd, m, sf, 0, sp);
+        if constexpr (fp64) wvgpu::fx_yinv(p, sd, m, sf, sp, s);
+        else dev::k_yinv<T><<<dim3(cdiv(KX, dev::kYG), Nz), 256, smem_y<T>(p), s>>>(sd, m, sf, 0, sp);
     };
     auto c2r = [&](int nch, double* out, size_t sm) {
         if constexpr (fp64) if (wvgpu::fx_xc2r(p, sd, h->fx, sp, nch, out, s)) return;
@@ -1008,7 +1008,9 @@ cudaError_t launch_inverse(wv_handle* h, double t, double t0, const double* Ap, 
     const auto& d = desc_of<T>(h);
     auto* z = static_cast<dev::cx<T>*>(h->zspec);
     auto* y = static_cast<dev::cx<T>*>(h->yspec);
-    if (!launch_vinv_fx<T>(h, false, t - t0, Ap, Am, A0, z, nullptr, s))
+    bool done = false;
+    if constexpr (std::is_same<T, double>::value) done = wvgpu::fx_vinv(p, d, false, t - t0, Ap, Am, A0, z, nullptr, s);
+    if (!done)
         dev::k_vinv<T, false><<<dim3(cdiv(p.Nkl, dev::kVinvModes), d.members), 256, smem_vinv<T>(p), s>>>(d, Ap, Am, A0, t - t0, z, nullptr);
     dev::YInvMap map{};
     map.nOut = nch;
@@ -1029,7 +1031,10 @@ cudaError_t launch_forward(wv_handle* h, const double* fields, double t, double 
     auto* f = static_cast<dev::cx<T>*>(h->fspec);
     launch_xr2c<T>(h, fields, nch, ps, s);
     launch_yfwd<T>(h, ps, nch, f, s);
-    if (!launch_vfwd_fx<T>(h, false, f, nch, t - t0, nullptr, nullptr, nullptr, nullptr, 0, Ap, Am, A0, s))
+    bool done = false;
+    if constexpr (std::is_same<T, double>::value)
+        done = wvgpu::fx_vfwd(p, d, false, f, nch, t - t0, nullptr, nullptr, nullptr, nullptr, 0, Ap, Am, A0, s);
+    if (!done)
         dev::k_vfwd<T, false><<<dim3(cdiv(p.Nkl, dev::kVfwdModes), d.members), 256, smem_vfwd<T>(p, nch), s>>>(
             d, f, nch, t - t0, nullptr, nullptr, nullptr, nullptr, 0, Ap, Am, A0);
     h->metrics.kernel_launches += 3;

@@ -270,13 +270,13 @@ bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& r, const doubl
     return true;
 }
 
-bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, const double2* z, double2* y, cudaStream_t s) {
+void fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, const double2* z, double2* y, cudaStream_t s) {
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
         const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * map.nOut, grid_cap(1));
         dev::k_yinv_fxany<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps,
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, map, z, y, cols);
-        return true;
+        return;
     }
     const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
     const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, map.nOut);
@@ -286,21 +286,19 @@ bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, cons
     std::memcpy(&bits, &ltop, 8);
     WV_FXW_SWITCH(p.Ny, (dev::k_yinv_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(
                             d, map, z, y, static_cast<unsigned>(bits >> 32))));
-    return true;
 }
 
-bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, double2* f, cudaStream_t s) {
+void fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, double2* f, cudaStream_t s) {
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
         const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * nch, grid_cap(1));
         dev::k_yfwd_fxany<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps,
                                dev::smem_fx_any_y(Ny, cols), s>>>(d, ps, nch, f, cols);
-        return true;
+        return;
     }
     const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
     const dim3 grid(cdiv(d.kxColumns, cols), d.zTotal, nch);
     WV_FXW_SWITCH(p.Ny, (dev::k_yfwd_fx<NN><<<grid, 32 * warps, dev::smem_fxy<NN>(cols), s>>>(d, ps, nch, f)));
-    return true;
 }
 
 bool fx_xc2r(const Plan& p, const dev::DescDev& d, const FxRows& r, const double2* y, int nch, double* fields, cudaStream_t s) {

@@ -2,10 +2,10 @@
 //
 // The FP64 pipe of this GPU retires about 1.7 operations per SM and clock
 // (measured; 1/64 of the FP32 rate), which bounded every FP64 transform.  The
-// integer pipes add 62 64-bit values per SM and clock and run 16-18 32 x 32 ->
-// 64-bit multiply-adds, so a butterfly costs 10 to 30 times less there.  A line
-// of doubles is scaled by one power of two to 64-bit integers, transformed
-// exactly in its sums and to one unit in its products, and scaled back.
+// integer pipes add 63 64-bit values per SM and clock and run 32 32 x 32 -> 64-bit
+// multiplies, so a butterfly costs about 10 times less there.  A line of doubles is
+// scaled by one power of two to 64-bit integers, transformed exactly in its sums and
+// to one unit in its products, and scaled back.  Flux at 256x256x129: 9.6 -> 2.05 ms.
 //
 // Range: with B = sum |x_k| over the line (every partial sum of a DFT is at most
 // B in magnitude, twiddles having modulus 1), the scale puts B into
@@ -78,9 +78,9 @@ WV_HD fxc fx_cmul(fxc a, fxw w) {
 }
 #ifdef __CUDACC__
 // x w for |x| < 2^60 (1 - 2^-9): the middle terms as four high halves (32-bit sums;
-// each cuts its last bit, `two` gives the mean back), 25 instructions against 37.
+// each cuts half a unit on average, `two` gives it back), 27 instructions against 37.
 // two: the value 2 in a register the compiler cannot rebuild (fx_two); 0 on all-zero
-// lines, which stay exactly zero.
+// lines, which stay exactly zero.  Twiddles +-1 and +-i (no low words) cut nothing.
 template <bool INV>
 __device__ __forceinline__ fxc fx_cmul60(fxc a, fxw w, int two) {
     const long long x4 = a.x << 2, y4 = a.y << 2;
@@ -89,8 +89,9 @@ __device__ __forceinline__ fxc fx_cmul60(fxc a, fxw w, int two) {
     const int sh = INV ? nh : w.sh, sl = INV ? nl : w.sl, mh = INV ? w.sh : nh, ml = INV ? w.sl : nl;
     auto mad = [](int p, int q, int c) { int r; asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(p), "r"(q), "r"(c)); return r; };
     auto mul = [](int p, int q) { long long r; asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(p), "r"(q)); return r; };
-    const int m = mad(xh, w.cl, mad(xl, w.ch, mad(yh, ml, mad(yl, mh, two))));
-    const int n = mad(xh, sl, mad(xl, sh, mad(yh, w.cl, mad(yl, w.ch, two))));
+    const int mean = static_cast<int>(min(static_cast<unsigned>(w.cl | w.sl), static_cast<unsigned>(two)));
+    const int m = mad(xh, w.cl, mad(xl, w.ch, mad(yh, ml, mad(yl, mh, mean))));
+    const int n = mad(xh, sl, mad(xl, sh, mad(yh, w.cl, mad(yl, w.ch, mean))));
     return fxc{mul(xh, w.ch) + mul(yh, mh) + static_cast<long long>(m), mul(xh, sh) + mul(yh, w.ch) + static_cast<long long>(n)};
 }
 __device__ __forceinline__ int fx_two() {
@@ -121,7 +122,8 @@ template <bool INV>
 WV_HD void fx_dft3(fxc& v0, fxc& v1, fxc& v2) {
     constexpr long long q = 3993837246235628775ll;
     const fxc t = fx_add(v1, v2), e = fx_sub(v1, v2);
-    const fxc m = {v0.x - (t.x >> 1), v0.y - (t.y >> 1)};
+    // (the last bit of v0 decides halves: their mean is zero)
+    const fxc m = {v0.x - ((t.x + (v0.x & 1)) >> 1), v0.y - ((t.y + (v0.y & 1)) >> 1)};
     const fxc s = {fx_rmul(e.x, fx_qh(q), fx_ql(q)), fx_rmul(e.y, fx_qh(q), fx_ql(q))};
     const fxc i = INV ? fxc{-s.y, s.x} : fxc{s.y, -s.x};  // -/+ i sin(60) (v1 - v2)
     v0 = fx_add(v0, t); v1 = fx_add(m, i); v2 = fx_sub(m, i);
@@ -135,7 +137,7 @@ WV_HD void fx_dft5(fxc& v0, fxc& v1, fxc& v2, fxc& v3, fxc& v4) {
     const fxc a = fx_add(v1, v4), b = fx_add(v2, v3), c = fx_sub(v1, v4), d = fx_sub(v2, v3);
     const fxc t = fx_add(a, b), u = fx_sub(a, b);
     const fxc du = {fx_rmul(u.x, fx_qh(qd), fx_ql(qd)), fx_rmul(u.y, fx_qh(qd), fx_ql(qd))};
-    const fxc m = {v0.x - (t.x >> 2), v0.y - (t.y >> 2)};
+    const fxc m = {v0.x - ((t.x + (v0.x & 3)) >> 2), v0.y - ((t.y + (v0.y & 3)) >> 2)};
     const fxc m1 = fx_add(m, du), m2 = fx_sub(m, du);
     const fxc s1 = {fx_rmul(c.x, fx_qh(q1), fx_ql(q1)) + fx_rmul(d.x, fx_qh(q2), fx_ql(q2)),
                     fx_rmul(c.y, fx_qh(q1), fx_ql(q1)) + fx_rmul(d.y, fx_qh(q2), fx_ql(q2))};
@@ -274,11 +276,17 @@ WV_HD fxscale fx_scale(float l1) {
     const int el = static_cast<int>(fx_float_bits(l1 * 1.0025f) >> 23) - 126;
     return {1023, 61 - el};
 }
-// m (2^e at bit 62) shifted right by rs + 1 with the last bit rounded (up), negated
-// if asked
+// m (2^e at bit 62) shifted right by rs + 1 and rounded to nearest, negated if asked.
+// Roundings here have mean zero on both signs: a mean of a fraction of a unit, the same
+// in every line, would add up in the lowest modes of the passes that follow (0.25 units
+// here put 2e-12 instead of 2e-13 on the flux VJP's largest scales at 96x64x49).
 WV_HD long long fx_shift_in(unsigned long long m, int rs, int sign) {
-    const long long s = sign >> 31;  // 0 or -1
-    return ((static_cast<long long>(m >> (rs > 63 ? 63 : rs)) ^ s) + (1 - s)) >> 1;
+    const long long s = sign >> 31;  // 0 or -1; one's complement + 1 is the negative
+    return ((static_cast<long long>(m >> (rs > 63 ? 63 : rs)) ^ s) + 1) >> 1;
+}
+// x 2^-sh, rounded
+WV_HD long long fx_shift_round(long long x, int sh) {
+    return sh > 0 ? ((x >> (sh - 1)) + 1) >> 1 : x << -sh;
 }
 // (zeros and denormals leave through the shift: fx_scale keeps e0 far above them)
 WV_HD long long fx_from_double(double v, fxscale sc) {
@@ -329,8 +337,7 @@ WV_HD double fx_to_double(long long x, int unit) {
 
 #ifdef __CUDACC__
 // fx_to_double for a line's unit taken apart once: values of lines in the middle of
-// the exponent range need no checks of their own.  Magnitudes are one's complements
-// (one unit low below zero), rounded to 53 bits.
+// the exponent range need no checks of their own.
 struct FxUnit {
     int unit;
     unsigned keep, set;  // masks of the high word: 0 flushes the line, set makes it NaN
@@ -342,8 +349,9 @@ __device__ __forceinline__ FxUnit fx_out(int unit) {
 __device__ __forceinline__ double fx_to_double(long long x, FxUnit o) {
     unsigned lo = static_cast<unsigned>(x), hi = static_cast<unsigned>(static_cast<unsigned long long>(x) >> 32);
     const unsigned s = static_cast<unsigned>(static_cast<int>(hi) >> 31);
-    lo ^= s;
-    hi ^= s;
+    const unsigned long long a = (static_cast<unsigned long long>(hi ^ s) << 32 | (lo ^ s)) + (s & 1u);
+    lo = static_cast<unsigned>(a);
+    hi = static_cast<unsigned>(a >> 32);
     int base = o.unit + 62;
     if (hi == 0) { hi = lo; lo = 0; base -= 32; }
     const int lz = __clz(static_cast<int>(hi));

@@ -32,8 +32,8 @@ bool fx_xc2r(const Plan& p, const dev::DescDev& d, const FxRows& rows, const dou
              cudaStream_t s);
 bool fx_xr2c(const Plan& p, const dev::DescDev& d, const FxRows& rows, const double* fields, int nch, double2* ps,
              cudaStream_t s);
-bool fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, const double2* z, double2* y, cudaStream_t s);
-bool fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, double2* f, cudaStream_t s);
+void fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, const double2* z, double2* y, cudaStream_t s);
+void fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, double2* f, cudaStream_t s);
 bool fx_vinv(const Plan& p, const dev::DescDev& d, bool flux, double elapsed, const double* Ap, const double* Am,
              const double* A0, double2* z, unsigned long long* speed, cudaStream_t s);
 bool fx_vfwd(const Plan& p, const dev::DescDev& d, bool flux, const double2* f, int nch, double elapsed, const double* Ap,

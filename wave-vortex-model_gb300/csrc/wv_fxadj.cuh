@@ -67,6 +67,9 @@ __device__ __forceinline__ void fx_vinv_adj_store(const DescDev& d, int idx, dou
     zstore(A0b + 2 * idx, zd{u0 * ub.y + v0 * vb.y + na0 * nb.x, -u0 * ub.x - v0 * vb.x + na0 * nb.y});
 }
 
+// The VJP's four kernels, 128x128x65: 2.06 ms on the FP64 pipe (forward fields
+// included) -> 0.66 ms; all bound by integer issue.
+//
 // k_vfwd_adj_fft: lines (u | w), (v | eta) of a column by two warps;
 // y[0] = X_0, y[j] = (X_j + i Y_j) / 2, y[N-j] = (X_j - i Y_j) / 2.
 template <int N>

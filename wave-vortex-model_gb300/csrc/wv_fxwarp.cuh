@@ -340,8 +340,8 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const long long a = Sa[t + G * e], b = both ? Sb[t + G * e] : 0;
-        v[e].x = sh[0] >= 0 ? a >> sh[0] : a << -sh[0];
-        v[e].y = sh[1] >= 0 ? b >> sh[1] : b << -sh[1];
+        v[e].x = fx_shift_round(a, sh[0]);
+        v[e].y = fx_shift_round(b, sh[1]);
     }
     fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(unitA, both ? unitB : unitA)) ? 0 : two);
     __syncwarp();
@@ -360,6 +360,9 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
     }
 }
 
+// The x pass, a warp per line-set of rows with all its transforms, products and sums in
+// registers.  Bound by integer issue.  128x128x65: 0.132 ms (0.150 in the
+// block form below).
 // physOut / advOut / advIn / maxSpeedBits as k_xflux.
 // EK: spectrum entries of a lane (kx < EK G; E / 2 at most, fewer under the 2/3 rule).
 template <int N, int EK>
@@ -477,7 +480,9 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
 // The same pass for grids with too few rows to keep every SM busy with one warp a
 // row: a block takes one line-set of rows, a warp a pair of their c2r, all threads a
 // sample's products, a warp a pair of the r2c.  The arithmetic, to the bit, is
-// k_xflux_fx's.
+// k_xflux_fx's.  At 256 points it is the faster form on every grid: its warps hold one
+// pair of rows at a time, so three blocks fit an SM.  256x256x129: 5.92 (FP64 pipe)
+// -> 1.05 ms, 57 % of the issue slots; 192x192x97 1.00 -> 0.53 ms (run-time stages -> lanes).
 constexpr int kFxCoWarps = 8;  // (3 + 3 nt + 1) / 2 <= 8 pairs
 template <int N>
 inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * FxW<N>::samples * 8; }
