@@ -466,10 +466,7 @@ inline unsigned cdiv(size_t a, size_t b) { return static_cast<unsigned>((a + b -
 
 template <typename T>
 inline int warp_ry(const Plan& p, bool ignoreChoice = false) {
-    // FP64 stays on the shared-memory radix-4 Stockham kernels: on the FP64 pipe
-    // the radix-2 shuffle stages (64-bit shuffles, the twiddle product evaluated
-    // in every lane) cost more than the smem round trips they replace.  Paired
-    // FP32 takes the register lines up to 256 points (8 values per lane; 2.7 %
+    // FP64 lines run in fixed point (wv_fx.cu).  Paired FP32 takes the register lines up to 256 points (8 values per lane; 2.7 %
     // faster per flux at 256x256x129, 14 % at 128x128x65) and the Stockham
     // kernel for 512 (16 values per lane: 3 % slower there).
     if (std::is_same<T, double>::value || (p.stockhamY && !ignoreChoice) || p.Ny % 32 != 0) return 0;

@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(32 * kFxXWarps, 1)
 // sample's products, a warp a pair of the r2c.  The arithmetic, to the bit, is
 // k_xflux_fx's.  At 256 points it is the faster form on every grid: its warps hold one
 // pair of rows at a time, so three blocks fit an SM.  256x256x129: 5.92 (FP64 pipe)
-// -> 1.05 ms, 57 % of the issue slots; 192x192x97 1.00 -> 0.53 ms (run-time stages -> lanes).
+// -> 1.06 ms, 57 % of the issue slots; 192x192x97 1.00 -> 0.55 ms (run-time stages -> lanes).
 constexpr int kFxCoWarps = 8;  // (3 + 3 nt + 1) / 2 <= 8 pairs
 template <int N>
 inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * FxW<N>::samples * 8; }
