@@ -67,7 +67,8 @@ typedef struct wv_config {
  * projections and RK4 -- FP64-class flux accuracy without the FP64 pipe.  Fluxes and
  * the state transforms (not the adjoint) run on the 64-bit fixed-point kernels of FP64
  * handles, more accurate and faster, where Nx, Ny and 2 (Nz - 1) are all 16 to 256 and
- * one or three times a power of two (Nx and Ny not 192), until
+ * one or three times a power of two (Nx and Ny not 192; not on small grids whose y and
+ * z lines fit warp registers), until
  * wv_set_vertical_kernel(s) or wv_set_fft_variants chooses paired-FP32 kernels.
  * FP32X2 handles serve every entry point (kernel operations, adjoint, ensembles). */
 enum { WV_PRECISION_FP64 = 0, WV_PRECISION_MIXED = 1, WV_PRECISION_FP32X2 = 2 };

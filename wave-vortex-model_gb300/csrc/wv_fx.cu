@@ -51,10 +51,11 @@ inline bool fx_x_lane(const Plan& p) { return fx_lane_length(p.Nx) && 2 * p.kxCo
 inline bool fx_x_any(const Plan& p) { return p.Nx <= 512 && p.kxColumns <= 256; }
 // Forms of the x pass at a length: spectrum entries of a lane under the 2/3 rule and at
 // most; whether the one-warp-a-row form exists.  That form is the faster one at 128
-// points with many rows (0.132 against 0.150 ms at 128x128x65, above 6 line-sets of rows
-// an SM) and loses at 256 (1.22 against 1.14 ms at 256x256x129) and on small grids
+// points with many rows (0.132 against 0.150 ms at 128x128x65; flux at 128x128x33, 14
+// line-sets of rows an SM, 0.159 against 0.167 ms), loses where its 15 warps an SM have
+// too few (flux at 128x64x33, 7 an SM, 0.134 against 0.109 ms) and loses at 256 (1.22 against 1.14 ms at 256x256x129) and on small grids
 // (0.037 against 0.022 ms at 64x64x33).
-constexpr size_t kFxCoUnits = 6;
+constexpr size_t kFxCoUnits = 12;
 template <int N>
 struct XKernels {
     static constexpr int few = dev::FxW<N>::E == 8 ? 3 : 5, all = dev::FxW<N>::H;
@@ -232,9 +233,12 @@ bool fx_xadj(const Plan& p, const dev::DescDev& d, const FxRows& r, const double
 // Against the paired-FP32 kernels per flux: 1.05 to 1.7 times as fast where every axis
 // has lane-held lines (64x64x97 158 -> 144 us, 96x96x49 221 -> 189, RK4 step at
 // 256x256x129 9.41 -> 8.35 ms), but not with x or y lines of 192 points (RK4 step at
-// 192x192x97 4.23 -> 4.33 ms) nor on the run-time stages (0.6 to 0.8 times as fast).
+// 192x192x97 4.23 -> 4.33 ms), on the run-time stages (0.6 to 0.8 times as fast), nor
+// on small grids whose y and z lines the paired form holds in warp registers
+// (32x32x17 hydrostatic 38.9 -> 44.2 us).
 bool fx_beats_paired(const Plan& p) {
-    return fx_x_lane(p) && fx_lane_length(p.Ny) && fx_lane_length(p.fz.N) && p.Nx != 192 && p.Ny != 192;
+    const bool small = p.Ny % 32 == 0 && p.fz.N % 32 == 0 && p.Nx * p.Ny * p.Nz < 65536;
+    return fx_x_lane(p) && fx_lane_length(p.Ny) && fx_lane_length(p.fz.N) && p.Nx != 192 && p.Ny != 192 && !small;
 }
 
 bool fx_has_rows(const Plan& p) { return fx_x_lane(p) || fx_x_any(p); }
