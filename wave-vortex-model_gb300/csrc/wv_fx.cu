@@ -49,20 +49,11 @@ std::vector<int32_t> lane_table() {
 // run-time stages; longer rows keep the block kernel.
 inline bool fx_x_lane(const Plan& p) { return fx_lane_length(p.Nx) && 2 * p.kxColumns <= p.Nx; }
 inline bool fx_x_any(const Plan& p) { return p.Nx <= 512 && p.kxColumns <= 256; }
-// Forms of the x pass at a length: spectrum entries of a lane under the 2/3 rule and at
-// most; whether the one-warp-a-row form exists.  That form is the faster one at 128
-// points with many rows (0.132 against 0.150 ms at 128x128x65; flux at 128x128x33, 14
-// line-sets of rows an SM, 0.159 against 0.167 ms), loses where its 15 warps an SM have
-// too few (flux at 128x64x33, 7 an SM, 0.134 against 0.109 ms) and loses at 256 (1.22 against 1.14 ms at 256x256x129) and on small grids
-// (0.037 against 0.022 ms at 64x64x33).
-constexpr size_t kFxCoUnits = 12;
+// Spectrum entries of a lane in the x pass under the 2/3 rule, and at most.
 template <int N>
 struct XKernels {
     static constexpr int few = dev::FxW<N>::E == 8 ? 3 : 5, all = dev::FxW<N>::H;
-    static constexpr bool rowForm = dev::FxW<N>::E == 8 && N < 256;
 };
-template <int N>
-size_t smem_xflux_fx() { return dev::FxW<N>::twiddles * sizeof(dev::fxw) + dev::kFxXWarps * dev::fx_xflux_warp_bytes<N>(); }
 // Warps of a y or z block: 8, fewer where the columns of a plane (the retained
 // columns) do not fill them; powers of two in y, as the tile's swizzle needs.
 inline int fx_y_warps(size_t Ny, size_t kxColumns) {
@@ -168,10 +159,6 @@ cudaError_t fx_set_limits(const Plan& p) {
     if (fx_x_lane(p)) {
         WV_FXW_SWITCH(p.Nx, {
             using X = XKernels<NN>;
-            if constexpr (X::rowForm) {
-                set(dev::k_xflux_fx<NN, X::few>, smem_xflux_fx<NN>());
-                set(dev::k_xflux_fx<NN, X::all>, smem_xflux_fx<NN>());
-            }
             set(dev::k_xflux_fxco<NN, X::few>, dev::smem_xflux_co<NN>());
             set(dev::k_xflux_fxco<NN, X::all>, dev::smem_xflux_co<NN>());
         });
@@ -247,20 +234,10 @@ bool fx_xflux(const Plan& p, const dev::DescDev& d, const FxRows& r, const doubl
               unsigned long long* speed, double* physOut, double* advOut, const double* advIn, cudaStream_t s) {
     if (fx_x_lane(p)) {
         const size_t rows = p.Ny * p.Nz * d.members, perWarp = fx_lane_lines(p.Nx);
-        const size_t units = (rows + perWarp - 1) / perWarp, sms = grid_cap(1);
+        const size_t units = (rows + perWarp - 1) / perWarp;
         WV_FXW_SWITCH(p.Nx, {
             using X = XKernels<NN>;
             const bool few = p.kxColumns <= static_cast<size_t>(X::few) * dev::FxW<NN>::G;
-            if constexpr (X::rowForm) {
-                if (units > kFxCoUnits * sms) {
-                    // one block per SM
-                    const int warps = dev::kFxXWarps;
-                    const int grid = static_cast<int>(std::min<size_t>((units + warps - 1) / warps, sms));
-                    auto* kernel = few ? dev::k_xflux_fx<NN, X::few> : dev::k_xflux_fx<NN, X::all>;
-                    kernel<<<grid, 32 * warps, smem_xflux_fx<NN>(), s>>>(d, r.twXLane, y, ps, speed, physOut, advOut, advIn);
-                    return true;
-                }
-            }
             auto* kernel = few ? dev::k_xflux_fxco<NN, X::few> : dev::k_xflux_fxco<NN, X::all>;
             kernel<<<static_cast<unsigned>(units), 32 * dev::kFxCoWarps, dev::smem_xflux_co<NN>(), s>>>(
                 d, r.twXLane, y, ps, speed, physOut, advOut, advIn);

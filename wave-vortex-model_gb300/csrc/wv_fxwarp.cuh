@@ -180,16 +180,11 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
 
 // ---------------------------------------------------------------------------
 // x pass of the FP64 flux: c2r of the velocities and of every derivative, the
-// quadratic products and their r2c, one (y, z) row per line of the warp and no
-// block barrier.  Two real rows share one complex line (Z = A + i B for the c2r,
+// quadratic products and their r2c.  Two real rows share one complex line (Z = A + i B for the c2r,
 // S_a + i S_b for the r2c); each row keeps its own scale, so its rounding stays
 // relative to its own magnitude whatever its partner holds.  Products are formed as
 // (a b) >> 62 on velocities normalised to 62 bits and added at the largest unit of
 // a target's three.
-
-template <int N>
-inline size_t fx_xflux_warp_bytes() { return static_cast<size_t>(FxW<N>::lines) * (FxW<N>::buffer * 16 + 40 * N); }
-constexpr int kFxXWarps = 15;  // 14.8 KB of shared memory and 32 x 128 registers each fill an SM
 
 // (a b) >> 62 rounded, |a| < 2^62, |b| < 2^61
 __device__ __forceinline__ long long fx_prod(long long a, long long b) {
@@ -360,129 +355,15 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
     }
 }
 
-// The x pass, a warp per line-set of rows with all its transforms, products and sums in
-// registers.  Bound by integer issue.  128x128x65: 0.132 ms (0.150 in the
-// block form below).
+// The x pass: a block takes one line-set of rows, a warp a pair of their c2r, all threads
+// a sample's products, a warp a pair of the r2c.  A warp holds one pair of rows at a
+// time, so three blocks fit an SM.  (A warp per row with all its transforms in registers
+// gained 2 to 4 % on 12 to 40 line-sets an SM of 16 or 128 points and lost 4 to 7 % on
+// more, 10 to 30 % on fewer: flux 128x128x65 290 against 295 us, 128x256x129 1137 against
+// 1064, 128x64x33 133 against 109.)  256x256x129: 5.92 (FP64 pipe) -> 1.06 ms, 57 % of
+// the issue slots; 192x192x97 1.00 -> 0.55 ms (run-time stages -> lanes).
 // physOut / advOut / advIn / maxSpeedBits as k_xflux.
 // EK: spectrum entries of a lane (kx < EK G; E / 2 at most, fewer under the 2/3 rule).
-template <int N, int EK>
-__global__ void __launch_bounds__(32 * kFxXWarps, 1)
-    k_xflux_fx(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, double2* __restrict__ pspec,
-               unsigned long long* __restrict__ maxSpeedBits, double* __restrict__ physOut, double* __restrict__ advOut,
-               const double* __restrict__ advIn) {
-    using W = FxW<N>;
-    constexpr int G = W::G, E = W::E, H = W::H;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
-    const int nIn = 4 + 2 * nt, nReal = 3 + 3 * nt;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const int t = lane % G, line = lane / G;
-    fxw* tw = reinterpret_cast<fxw*>(smem_raw);
-    for (int i = threadIdx.x; i < W::twiddles; i += blockDim.x) tw[i] = twg[i];
-    __syncthreads();
-    unsigned char* mine = smem_raw + W::twiddles * 16 + static_cast<size_t>(warp * W::lines + line) * (W::buffer * 16 + 40 * N);
-    fxc* x = reinterpret_cast<fxc*>(mine);                         // line buffer
-    long long* phys = reinterpret_cast<long long*>(x + W::buffer);  // u, v, w [3][N]
-    long long* S = phys + 3 * N;                                    // products of two targets [2][N]
-    const int two = fx_two();
-    const double* rowK = row_k<double>(d);
-    const size_t cstride = static_cast<size_t>(Ny) * KX;
-    const size_t R3 = static_cast<size_t>(N) * Ny * d.Nz;
-    const int rows = Ny * d.zTotal;
-    const unsigned wtop = fx_row_k_top(rowK, KX);
-    for (int first = (blockIdx.x * warps + warp) * W::lines; first < rows; first += gridDim.x * warps * W::lines) {
-        const bool live = first + line < rows;
-        const int row = min(first + line, rows - 1);
-        const int z = row / Ny, y = row - z * Ny;
-        const double2* yrow = yspec + (static_cast<size_t>(z) * nIn * Ny + y) * KX;
-        int physUnit[3] = {0, 0, 0}, sUnit[2] = {0, 0}, unitNow = 0;  // (as fx_unit)
-        long long acc[E];  // products of the current target
-#pragma unroll
-        for (int e = 0; e < E; ++e) acc[e] = 0;
-        for (int p = 0; 2 * p < nReal; ++p) {
-            fxc v[E];
-            int unit[2] = {kFxZero, kFxZero};
-            fx_load_pair<N, EK>(d, yrow, cstride, rowK, wtop, p, nReal, x, t, v, unit);
-            fx_fft_warp<N, true>(v, x, tw, t, fx_silent(max(unit[0], unit[1])) ? 0 : two);
-            // samples x = t + G e: real part row 2p, imaginary part row 2p + 1
-#pragma unroll 1
-            for (int q = 0; q < 2; ++q) {
-                const int r = 2 * p + q;
-                if (r >= nReal) break;
-                const int uq = q ? unit[1] : unit[0];
-                long long smp[E];
-#pragma unroll
-                for (int e = 0; e < E; ++e) smp[e] = q ? v[e].y : v[e].x;
-                if (physOut && live && r >= 3) {
-                    double* keep = physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N;
-#pragma unroll
-                    for (int e = 0; e < E; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
-                }
-                if (r < 3) {
-                    const size_t g = static_cast<size_t>(r) * R3 + (static_cast<size_t>(z) * Ny + y) * N;
-                    double* keep = physOut && live ? physOut + ((static_cast<size_t>(z) * nReal + r) * Ny + y) * N : nullptr;
-                    const int un = fx_velocity<N>(smp, uq, t, phys + r * N, advIn ? advIn + g : nullptr,
-                                                  advOut && live ? advOut + g : nullptr, keep);
-                    if (r == 0) physUnit[0] = un;
-                    else if (r == 1) physUnit[1] = un;
-                    else physUnit[2] = un;
-                    continue;  // phys is read back by the lane that wrote it
-                }
-                const int tt = (r - 3) / 3, kind = (r - 3) - 3 * tt;
-                const int un = fx_pick(physUnit, kind) + uq - 1023 + 62;
-                const long long* vel = phys + kind * N;
-                if (kind == 0) {
-                    unitNow = un;
-#pragma unroll
-                    for (int e = 0; e < E; ++e) acc[e] = -fx_prod(vel[t + G * e], smp[e]);
-                } else {
-                    const int now = max(unitNow, un);
-                    const int shS = min(63, now - unitNow), shP = min(63, now - un);
-                    unitNow = now;
-#pragma unroll
-                    for (int e = 0; e < E; ++e)
-                        acc[e] = (acc[e] >> shS) - (fx_prod(vel[t + G * e], smp[e]) >> shP);
-                }
-                if (kind == 2) {
-#pragma unroll
-                    for (int e = 0; e < E; ++e) S[(tt & 1) * N + t + G * e] = acc[e];
-                    sUnit[0] = (tt & 1) ? sUnit[0] : unitNow;
-                    sUnit[1] = (tt & 1) ? unitNow : sUnit[1];
-                }
-            }
-            // targets finished so far: a full pair, or the last one, goes forward
-            const int done = min(nt, (2 * p + 2 - 3) / 3);
-            const int before = p == 0 ? 0 : min(nt, max(0, (2 * p - 3) / 3));
-            if (done > before && ((done & 1) == 0 || done == nt)) {
-                const bool both = (done & 1) == 0;
-                const int t0 = both ? done - 2 : done - 1;
-                double2* out = pspec + ((static_cast<size_t>(z) * nt + t0) * Ny + y) * KX;
-                fx_forward_pair<N>(S, both ? S + N : nullptr, sUnit[0], sUnit[1], x, tw, t, two, live ? KX : 0, out, cstride);
-                __syncwarp();
-            }
-        }
-        // max |u_h| (only when adaptive damping consumes it)
-        if (maxSpeedBits) {
-            double m = 0.0;
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const double U = fx_to_double(phys[t + G * e], physUnit[0]);
-                const double V = fx_to_double(phys[N + t + G * e], physUnit[1]);
-                m = fmax(m, U * U + V * V);
-            }
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (t == 0) atomicMax(maxSpeedBits + z / d.Nz, (unsigned long long)__double_as_longlong(sqrt(m)));
-        }
-    }
-}
-
-// The same pass for grids with too few rows to keep every SM busy with one warp a
-// row: a block takes one line-set of rows, a warp a pair of their c2r, all threads a
-// sample's products, a warp a pair of the r2c.  The arithmetic, to the bit, is
-// k_xflux_fx's.  At 256 points it is the faster form on every grid: its warps hold one
-// pair of rows at a time, so three blocks fit an SM.  256x256x129: 5.92 (FP64 pipe)
-// -> 1.06 ms, 57 % of the issue slots; 192x192x97 1.00 -> 0.55 ms (run-time stages -> lanes).
 constexpr int kFxCoWarps = 8;  // (3 + 3 nt + 1) / 2 <= 8 pairs
 template <int N>
 inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * FxW<N>::samples * 8; }
