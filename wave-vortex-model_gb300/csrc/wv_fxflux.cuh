@@ -169,11 +169,12 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                 long long* s = S + t * Nx;
                 const int before = t == 0 ? sUnit[0] : t == 1 ? sUnit[1] : t == 2 ? sUnit[2] : sUnit[3];
                 const int now = kind == 0 ? un : max(before, un);
-                const int shS = min(63, now - before), shP = min(63, now - un);
+                const int shS = kind == 0 ? 0 : min(63, now - before), shP = min(63, now - un);
+                const long long hS = fx_half(shS, lane & 1), hP = fx_half(shP, lane & 1);
                 for (int x = lane; x < Nx; x += 32) {
                     const long long v = a[2 * x];
-                    const long long pr = fx_prod(vel[x], v) >> shP;
-                    s[x] = kind == 0 ? -pr : (s[x] >> shS) - pr;
+                    const long long pr = (fx_prod(vel[x], v) + hP) >> shP;
+                    s[x] = kind == 0 ? -pr : ((s[x] + hS) >> shS) - pr;
                     if (keep) keep[x] = fx_to_double(v, unit);
                 }
                 if (t == 0) sUnit[0] = now; else if (t == 1) sUnit[1] = now; else if (t == 2) sUnit[2] = now; else sUnit[3] = now;

@@ -364,6 +364,8 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
 // the issue slots; 192x192x97 1.00 -> 0.55 ms (run-time stages -> lanes).
 // physOut / advOut / advIn / maxSpeedBits as k_xflux.
 // EK: spectrum entries of a lane (kx < EK G; E / 2 at most, fewer under the 2/3 rule).
+// How a product comes to its target's unit: (p + half) >> shift (fx_half).
+struct alignas(16) FxAlign { long long half; int shift; };
 constexpr int kFxCoWarps = 8;  // (3 + 3 nt + 1) / 2 <= 8 pairs
 template <int N>
 inline size_t smem_xflux_co() { return (FxW<N>::twiddles + kFxCoWarps * FxW<N>::lines * FxW<N>::buffer) * 16 + (3 + 4) * FxW<N>::samples * 8; }
@@ -377,6 +379,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
     constexpr int G = W::G, E = W::E, H = W::H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int rowUnit[16][W::lines], sUnit[4][W::lines];
+    __shared__ FxAlign align[2][12][W::lines];  // [odd sample][target, kind][line]
     const int Ny = d.Ny, KX = d.kxColumns, nt = d.nt;
     const int nIn = 4 + 2 * nt, nReal = 3 + 3 * nt;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -427,31 +430,35 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
         }
     }
     __syncthreads();
-    {
-        // a sample a thread
-        for (int s = threadIdx.x; s < W::samples; s += 32 * kFxCoWarps) {
+    // a target's products are added at the largest unit of its three
+    for (int i = threadIdx.x; i < 2 * nt * W::lines; i += 32 * kFxCoWarps) {
+        const int ln = i % W::lines, odd = (i / W::lines) & 1, tt = i / (2 * W::lines);
+        int un[3];
+#pragma unroll
+        for (int kind = 0; kind < 3; ++kind) un[kind] = rowUnit[kind][ln] + rowUnit[3 + 3 * tt + kind][ln] - 1023 + 62;
+        const int most = max(un[0], max(un[1], un[2]));
+#pragma unroll
+        for (int kind = 0; kind < 3; ++kind) {
+            const int sh = min(63, most - un[kind]);
+            align[odd][3 * tt + kind][ln] = FxAlign{fx_half(sh, odd), sh};
+        }
+        if (odd == 0) sUnit[tt][ln] = most;
+    }
+    __syncthreads();
+    // a sample a thread
+    for (int s = threadIdx.x; s < W::samples; s += 32 * kFxCoWarps) {
         const int ln = s / N, xx = s - ln * N;
         for (int tt = 0; tt < nt; ++tt) {
             long long acc = 0;
-            int now = 0;
 #pragma unroll
             for (int kind = 0; kind < 3; ++kind) {
                 const int r = 3 + 3 * tt + kind;
                 const fxc* b = buffers + static_cast<size_t>((r >> 1) * W::lines + ln) * W::buffer;
                 const long long q = (r & 1) ? b[xx].y : b[xx].x;
-                const int un = rowUnit[kind][ln] + rowUnit[r][ln] - 1023 + 62;
-                const long long pr = fx_prod(phys[kind * W::samples + s], q);
-                if (kind == 0) {
-                    acc = -pr;
-                    now = un;
-                } else {
-                    const int next = max(now, un);
-                    acc = (acc >> min(63, next - now)) - (pr >> min(63, next - un));
-                    now = next;
-                }
+                const FxAlign a = align[s & 1][r - 3][ln];
+                acc -= (fx_prod(phys[kind * W::samples + s], q) + a.half) >> a.shift;
             }
             S[tt * W::samples + s] = acc;
-            if (xx == 0) sUnit[tt][ln] = now;
         }
         if (maxSpeedBits) {
             const double U = fx_to_double(phys[s], rowUnit[0][ln]), V = fx_to_double(phys[W::samples + s], rowUnit[1][ln]);
@@ -463,7 +470,6 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
             m = fmax(m, 0.0);
             const int zz = min(first + ln, rows - 1) / Ny;
             if (lane % kSpan == 0) atomicMax(maxSpeedBits + zz / d.Nz, (unsigned long long)__double_as_longlong(sqrt(m)));
-        }
         }
     }
     __syncthreads();
