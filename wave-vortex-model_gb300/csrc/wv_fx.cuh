@@ -263,13 +263,14 @@ WV_HD bool fx_plain_sum(float l1) { return l1 > 1e-30f && l1 < 1e30f; }
 struct fxscale {
     int e0;   // biased exponent at bit `bit`
     int bit;
+    bool zero = false;  // no entry but zeros
 };
 WV_HD fxscale fx_scale(unsigned top, float l1) {
     const float s = l1 * 1.0025f;
     int el = static_cast<int>(fx_float_bits(s) >> 23) - 126;  // s < 2^el
     if (el < -40) el = -40;                                   // (weighted rows of one dominant, weightless entry)
     const int e0 = static_cast<int>(top >> 20);
-    return {e0 < 200 ? 200 : e0, 61 - el};
+    return {e0 < 200 ? 200 : e0, 61 - el, top == 0};
 }
 // the same from a sum of fx_mag moduli
 WV_HD fxscale fx_scale(float l1) {
@@ -308,7 +309,7 @@ constexpr int kFxBad = 1 << 28;
 // unit of an all-zero line (fx_silent); units derived from it stay below half of it
 constexpr int kFxZero = -(1 << 24);
 WV_HD bool fx_silent(int unit) { return unit < kFxZero / 2; }
-WV_HD int fx_unit(fxscale sc) { return sc.e0 >= 0x7ff ? kFxBad : sc.e0 - sc.bit; }
+WV_HD int fx_unit(fxscale sc) { return sc.zero ? kFxZero : sc.e0 >= 0x7ff ? kFxBad : sc.e0 - sc.bit; }
 WV_HD int fx_clz(unsigned long long v) {
 #ifdef __CUDA_ARCH__
     return __clzll(static_cast<long long>(v));

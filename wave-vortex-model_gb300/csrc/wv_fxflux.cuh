@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                         for (int x = lane; x < Nx; x += 32)
                             top = max(top, static_cast<unsigned>(__double2hiint(advIn[g + x])) & 0x7fffffffu);
                         top = __reduce_max_sync(0xffffffffu, top);
-                        const fxscale sc{static_cast<int>(top >> 20), 61};
+                        const fxscale sc = fx_velocity_scale(top);
                         for (int x = lane; x < Nx; x += 32) {
                             const double v = advIn[g + x];
                             phys[r * Nx + x] = fx_from_double(v, sc);

@@ -274,6 +274,10 @@ __device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __
                     __syncwarp();
 }
 
+// Scale of a caller's velocity row, largest high word `top`: its leading bit at 61.  (The
+// scale stops at 2^-823: zeros have to leave through the shift.)
+__device__ __forceinline__ fxscale fx_velocity_scale(unsigned top) { return {max(static_cast<int>(top >> 20), 200), 61, top == 0}; }
+
 // Samples of an advecting velocity row (or the caller's doubles), normalised to 62
 // bits, into phys; returns the unit.
 template <int N>
@@ -290,7 +294,7 @@ __device__ __forceinline__ int fx_velocity(const long long (&smp)[FxW<N>::E], in
             top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
         }
         top = fx_group_max<G>(top);
-        const fxscale sc{static_cast<int>(top >> 20), 61};
+        const fxscale sc = fx_velocity_scale(top);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             phys[t + G * e] = fx_from_double(a[e], sc);
