@@ -59,7 +59,13 @@ typedef struct wv_config {
     uint8_t should_antialias;
 } wv_config;
 
-/* Arithmetic of a handle.  FP64: the plain drop-in, every stage in double.
+/* Arithmetic of a handle.  FP64: the drop-in.  Coefficients, phases, projections and
+ * RK4 in double; the transforms and products of the flux, the state transforms, the
+ * scalar advection and the VJP in 64-bit block fixed point.  There a value is held to
+ * 2^-58 or finer of the sum of moduli of its line (one transform along x, y or z), not
+ * to 2^-53 of itself.  Lines whose largest value is 5e-277 or more and whose sum of
+ * moduli is at most 2e307 keep that; larger ones come out as NaN, smaller ones lose
+ * digits and are zeros below 5e-290.  A NaN or an infinity makes its whole line NaN.
  * MIXED: FP32 xy transforms and quadratic products, FP64 phases, projections,
  * flux accumulation and RK4 stage accumulation.
  * FP32X2: the xy transforms, products and vertical contractions in paired FP32

@@ -1,5 +1,6 @@
 """Where the fixed-point lines of FP64 handles could lose what plain doubles keep:
-advecting velocities that are identically zero."""
+advecting velocities that are identically zero, and values near both ends of a double's
+range."""
 import numpy as np
 import pytest
 
@@ -41,4 +42,38 @@ def test_still_velocity_component_advects_nothing(wv, shape):
     assert not adv[2].any() and adv[0].any()
     for a, b in zip(k.nonlinearFluxUsingAdvectionFields(50.0, 0.0, *A, adv), F):
         assert np.array_equal(a, b)
+    k.close()
+
+
+@pytest.mark.parametrize("shape", [(32, 48, 17), (20, 18, 11), (516, 8, 7)])
+@pytest.mark.parametrize("power", [-900, 960])
+def test_values_near_the_ends_of_the_range(wv, shape, power):
+    """A power of two moves only exponents (tolerances of
+    test_scaled_states_give_scaled_fields): lines bounded by 2^-892 and less or by
+    2^938 and more keep their values; the flux is quadratic, so half the power there."""
+    import torch
+    c, d, A, k = _setup(wv, shape)
+    s, h = 2.0 ** power, 2.0 ** (power // 2)
+    f = k.transformWaveVortexToUVWEta(300.0, 0.0, *A)
+    g = k.transformWaveVortexToUVWEta(300.0, 0.0, *[s * x for x in A])
+    for a, b in zip(g, f):
+        assert np.max(np.abs(a / s - b)) <= 2e-14 * np.max(np.abs(b))
+    for a, b in zip(k.nonlinearFlux(300.0, 0.0, *[h * x for x in A]), k.nonlinearFlux(300.0, 0.0, *A)):
+        assert np.max(np.abs(a / h / h - b)) <= 1e-13 * np.max(np.abs(b))
+    rng = np.random.default_rng(6)
+    R = (shape[2], shape[1], shape[0])
+    f = rng.standard_normal((4,) + R)
+    B = k.transformUVWEtaToWaveVortex(f, 300.0, 0.0)
+    S = k.transformUVWEtaToWaveVortex(s * f, 300.0, 0.0)
+    for a, b in zip(S, B):
+        assert np.max(np.abs(a / s - b)) <= 1e-13 * np.max(np.abs(b))
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    q, adv = rng.standard_normal(R), 0.1 * rng.standard_normal((3,) + R)
+    one = k.advectFGridScalar(dev(q), dev(adv), True).cpu().numpy()
+    big = k.advectFGridScalar(dev(s * q), dev(adv), True).cpu().numpy()
+    assert np.max(np.abs(big / s - one)) <= 1e-13 * np.max(np.abs(one))
+    u = [dev(s * x) for x in A]  # the VJP is linear in the cotangents
+    for a, b in zip(k.flux_vjp(300.0, 0.0, *map(dev, A), *u), k.flux_vjp(300.0, 0.0, *map(dev, A), *map(dev, A))):
+        a, b = a.cpu().numpy(), b.cpu().numpy()
+        assert np.max(np.abs(a / s - b)) <= 1e-13 * np.max(np.abs(b))
     k.close()

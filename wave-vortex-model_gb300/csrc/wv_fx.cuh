@@ -258,6 +258,9 @@ WV_HD float fx_mag(unsigned hi) {
 // zero, tiny, huge or non-finite) take their scale from their largest entry.
 WV_HD bool fx_plain_sum(float l1) { return l1 > 1e-30f && l1 < 1e30f; }
 
+// Lowest exponent of a scale (2^-919): zeros carry an implied leading bit that has to leave
+// through the shift, 61 - bit + e0 >= 63 with bit <= 101.  Lines below lose digits.
+constexpr int kFxLowest = 104;
 // Scale of a line: the bit position of 2^e0.  l1: the sum of fx_modulus over the
 // line (its words were cut after 20 bits, hence the factor).
 struct fxscale {
@@ -270,7 +273,7 @@ WV_HD fxscale fx_scale(unsigned top, float l1) {
     int el = static_cast<int>(fx_float_bits(s) >> 23) - 126;  // s < 2^el
     if (el < -40) el = -40;                                   // (weighted rows of one dominant, weightless entry)
     const int e0 = static_cast<int>(top >> 20);
-    return {e0 < 200 ? 200 : e0, 61 - el, top == 0};
+    return {e0 < kFxLowest ? kFxLowest : e0, 61 - el, top == 0};
 }
 // the same from a sum of fx_mag moduli
 WV_HD fxscale fx_scale(float l1) {
@@ -295,7 +298,7 @@ WV_HD long long fx_shift_round(long long x, int sh) {
 WV_HD long long fx_half(int sh, int odd) {
     return static_cast<long long>(((1ull << sh) - static_cast<unsigned long long>(odd)) >> 1);
 }
-// (zeros and denormals leave through the shift: fx_scale keeps e0 far above them)
+// v in the line's fixed point (zeros and denormals leave through the shift)
 WV_HD long long fx_from_double(double v, fxscale sc) {
     unsigned hi, lo;
     fx_words(v, hi, lo);
@@ -310,50 +313,25 @@ constexpr int kFxBad = 1 << 28;
 constexpr int kFxZero = -(1 << 24);
 WV_HD bool fx_silent(int unit) { return unit < kFxZero / 2; }
 WV_HD int fx_unit(fxscale sc) { return sc.zero ? kFxZero : sc.e0 >= 0x7ff ? kFxBad : sc.e0 - sc.bit; }
-WV_HD int fx_clz(unsigned long long v) {
+WV_HD int fx_clz(unsigned v) {
 #ifdef __CUDA_ARCH__
-    return __clzll(static_cast<long long>(v));
+    return __clz(static_cast<int>(v));
 #else
-    return v ? __builtin_clzll(v) : 64;
+    return v ? __builtin_clz(v) : 32;
 #endif
 }
-// integer * 2^(unit - 1023) rounded to the nearest double (0 below the normal range, inf above)
-WV_HD double fx_to_double(long long x, int unit) {
-    const long long s = x >> 63;
-    const unsigned long long a = static_cast<unsigned long long>((x ^ s) - s);
-    unsigned h = static_cast<unsigned>(a >> 32), l = static_cast<unsigned>(a);
-    const bool low = h == 0;  // the leading bit is in the low word
-    if (low) { h = l; l = 0; }
-#ifdef __CUDA_ARCH__
-    const int lz = __clz(static_cast<int>(h));
-#else
-    const int lz = h ? __builtin_clz(h) : 32;
-#endif
-    // leading bit to bit 62, half a unit of the 53 bits added, cut; the hidden bit
-    // and a carry past it add to the exponent field
-    unsigned long long m = (static_cast<unsigned long long>(h) << 32 | l) >> 1;
-    m <<= (lz & 31);
-    m = (m + 512) >> 10;
-    const int e = unit + (low ? 30 : 62) - lz;
-    unsigned long long bits = m + (static_cast<unsigned long long>(static_cast<unsigned>(e)) << 52);
-    if (e < 0 || h == 0) bits = 0;
-    if (e >= 0x7fe && h != 0) bits = unit >= kFxBad / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull;
-    if (unit >= kFxBad / 2) bits = 0x7ff8000000000000ull;
-    return fx_double(bits | (static_cast<unsigned long long>(x) & 0x8000000000000000ull));
-}
-
-#ifdef __CUDACC__
-// fx_to_double for a line's unit taken apart once: values of lines in the middle of
-// the exponent range need no checks of their own.
+// integer * 2^(unit - 1023) rounded to the nearest double, for a line's unit taken apart
+// once.  Units 1 to 1983 (bounds of the line's sum of moduli from 2^-961 to 2^1021) make
+// every value a normal double; a line below comes out as zeros, one above as NaN.
 struct FxUnit {
     int unit;
     unsigned keep, set;  // masks of the high word: 0 flushes the line, set makes it NaN
 };
-__device__ __forceinline__ FxUnit fx_out(int unit) {
-    const bool huge = unit > 1900, tiny = unit < 70;
+WV_HD FxUnit fx_out(int unit) {
+    const bool huge = unit > 1983, tiny = unit < 1;
     return FxUnit{huge || tiny ? 1000 : unit, tiny ? 0u : 0xffffffffu, huge ? 0x7ff80000u : 0u};
 }
-__device__ __forceinline__ double fx_to_double(long long x, FxUnit o) {
+WV_HD double fx_to_double(long long x, FxUnit o) {
     unsigned lo = static_cast<unsigned>(x), hi = static_cast<unsigned>(static_cast<unsigned long long>(x) >> 32);
     const unsigned s = static_cast<unsigned>(static_cast<int>(hi) >> 31);
     const unsigned long long a = (static_cast<unsigned long long>(hi ^ s) << 32 | (lo ^ s)) + (s & 1u);
@@ -361,14 +339,27 @@ __device__ __forceinline__ double fx_to_double(long long x, FxUnit o) {
     hi = static_cast<unsigned>(a >> 32);
     int base = o.unit + 62;
     if (hi == 0) { hi = lo; lo = 0; base -= 32; }
-    const int lz = __clz(static_cast<int>(hi));
-    const unsigned th = __funnelshift_l(lo, hi, lz), tl = lo << (lz & 31);
-    const unsigned long long m = (((static_cast<unsigned long long>(th) << 32 | tl) >> 1) + 512) >> 10;
+    const int lz = fx_clz(hi);
+    // leading bit to bit 62, half a unit of the 53 bits added, cut; the hidden bit and a
+    // carry past it add to the exponent field
+#ifdef __CUDA_ARCH__
+    const unsigned long long top = static_cast<unsigned long long>(__funnelshift_l(lo, hi, lz)) << 32 | lo << (lz & 31);
+#else
+    const unsigned long long top = (static_cast<unsigned long long>(hi) << 32 | lo) << (lz & 31);
+#endif
+    const unsigned long long m = ((top >> 1) + 512) >> 10;
     unsigned h = static_cast<unsigned>(m >> 32) + (static_cast<unsigned>(base - lz) << 20);
     if (hi == 0) h = 0;
     h = ((h & o.keep) | (s & 0x80000000u)) | o.set;
+#ifdef __CUDA_ARCH__
     return __hiloint2double(static_cast<int>(h), static_cast<int>(m));
+#else
+    return fx_double(static_cast<unsigned long long>(h) << 32 | static_cast<unsigned>(m));
+#endif
 }
+WV_HD double fx_to_double(long long x, int unit) { return fx_to_double(x, fx_out(unit)); }
+
+#ifdef __CUDACC__
 // One stage over `lines` lines (as fft_stage): radix R from src to dst.
 template <int R, bool INV>
 __device__ __forceinline__ void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int Ns, int lines,

@@ -151,11 +151,12 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                             top = max(top, static_cast<unsigned>(static_cast<unsigned long long>(fx_abs(a[2 * x])) >> 32));
                         top = __reduce_max_sync(0xffffffffu, top);
                         const int sh = max(0, __clz(static_cast<int>(top)) - 2);
+                        const FxUnit o = fx_out(unit - sh);
                         for (int x = lane; x < Nx; x += 32) {
                             const long long v = fx_round53(a[2 * x] << sh);
                             phys[r * Nx + x] = v;
-                            if (advOut) advOut[g + x] = fx_to_double(v, unit - sh);
-                            if (keep) keep[x] = fx_to_double(v, unit - sh);
+                            if (advOut) advOut[g + x] = fx_to_double(v, o);
+                            if (keep) keep[x] = fx_to_double(v, o);
                         }
                         const int un = unit - sh;
                         if (r == 0) physUnit[0] = un; else if (r == 1) physUnit[1] = un; else physUnit[2] = un;
@@ -170,12 +171,13 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                 const int before = t == 0 ? sUnit[0] : t == 1 ? sUnit[1] : t == 2 ? sUnit[2] : sUnit[3];
                 const int now = kind == 0 ? un : max(before, un);
                 const int shS = kind == 0 ? 0 : min(63, now - before), shP = min(63, now - un);
+                const FxUnit o = fx_out(unit);
                 const long long hS = fx_half(shS, lane & 1), hP = fx_half(shP, lane & 1);
                 for (int x = lane; x < Nx; x += 32) {
                     const long long v = a[2 * x];
                     const long long pr = (fx_prod(vel[x], v) + hP) >> shP;
                     s[x] = kind == 0 ? -pr : ((s[x] + hS) >> shS) - pr;
-                    if (keep) keep[x] = fx_to_double(v, unit);
+                    if (keep) keep[x] = fx_to_double(v, o);
                 }
                 if (t == 0) sUnit[0] = now; else if (t == 1) sUnit[1] = now; else if (t == 2) sUnit[2] = now; else sUnit[3] = now;
             }
@@ -192,8 +194,9 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                 speedMember = member;
                 vmax2 = 0.0;
             }
+            const FxUnit oU = fx_out(physUnit[0]), oV = fx_out(physUnit[1]);
             for (int x = lane; x < Nx; x += 32) {
-                const double U = fx_to_double(phys[x], physUnit[0]), V = fx_to_double(phys[Nx + x], physUnit[1]);
+                const double U = fx_to_double(phys[x], oU), V = fx_to_double(phys[Nx + x], oV);
                 vmax2 = fmax(vmax2, U * U + V * V);
             }
         }

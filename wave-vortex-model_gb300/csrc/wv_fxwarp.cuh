@@ -274,9 +274,8 @@ __device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __
                     __syncwarp();
 }
 
-// Scale of a caller's velocity row, largest high word `top`: its leading bit at 61.  (The
-// scale stops at 2^-823: zeros have to leave through the shift.)
-__device__ __forceinline__ fxscale fx_velocity_scale(unsigned top) { return {max(static_cast<int>(top >> 20), 200), 61, top == 0}; }
+// Scale of a caller's velocity row, largest high word `top`: its leading bit at 61.
+__device__ __forceinline__ fxscale fx_velocity_scale(unsigned top) { return {max(static_cast<int>(top >> 20), kFxLowest), 61, top == 0}; }
 
 // Samples of an advecting velocity row (or the caller's doubles), normalised to 62
 // bits, into phys; returns the unit.
@@ -306,12 +305,13 @@ __device__ __forceinline__ int fx_velocity(const long long (&smp)[FxW<N>::E], in
     for (int e = 0; e < E; ++e) top = max(top, fx_abs_hi(smp[e]));
     top = fx_group_max<G>(top);
     const int sh = max(0, __clz(static_cast<int>(top)) - 2);
+    const FxUnit o = fx_out(unit - sh);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const long long s = fx_round53(smp[e] << sh);
         phys[t + G * e] = s;
-        if (advOut) advOut[t + G * e] = fx_to_double(s, unit - sh);
-        if (keep) keep[t + G * e] = fx_to_double(s, unit - sh);
+        if (advOut) advOut[t + G * e] = fx_to_double(s, o);
+        if (keep) keep[t + G * e] = fx_to_double(s, o);
     }
     return unit - sh;
 }
@@ -427,8 +427,9 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
                 uq = fx_velocity<N>(smp, uq, t, phys + (r * W::lines + line) * N, advIn ? advIn + g : nullptr,
                                     advOut && live ? advOut + g : nullptr, keep);
             } else if (keep) {
+                const FxUnit o = fx_out(uq);
 #pragma unroll
-                for (int e = 0; e < E; ++e) keep[t + G * e] = fx_to_double(smp[e], uq);
+                for (int e = 0; e < E; ++e) keep[t + G * e] = fx_to_double(smp[e], o);
             }
             if (t == 0) rowUnit[r][line] = uq;
         }

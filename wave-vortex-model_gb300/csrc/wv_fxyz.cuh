@@ -126,7 +126,6 @@ __device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long
     for (int e = 0; e < E; ++e) sum += fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
     sum = fx_group_sum<G>(sum);
     fxscale sc = fx_scale(sum);
-    bool zero = false;
     const bool odd = !fx_plain_sum(sum);
     if (__any_sync(0xffffffffu, odd)) {
         unsigned top = 0;
@@ -137,13 +136,10 @@ __device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long
 #pragma unroll
         for (int e = 0; e < E; ++e) rel += fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
         rel = fx_group_sum<G>(rel);
-        if (odd) {
-            zero = top == 0;
-            sc = fx_scale(top, rel);
-        }
+        if (odd) sc = fx_scale(top, rel);
     }
     sc.bit -= 2;
-    unit = zero ? kFxZero : fx_unit(sc);
+    unit = fx_unit(sc);
 #pragma unroll
     for (int e = 0; e < E; ++e) out[e] = fx_from_double(a[e], sc);
 }
