@@ -8,6 +8,11 @@ using namespace wvgpu::dev;
 
 extern "C" {
 
+// out[i] = the product x[i] as the r2c takes it in
+void shift_products(const long long* x, size_t n, int sh, long long* out) {
+    for (size_t i = 0; i < n; ++i) out[i] = fx_shift_round(x[i], sh, static_cast<int>(i & 1));
+}
+
 // out[i] = (x[i] + fx_half(sh, i & 1)) >> sh: a product aligned to a larger unit
 void align_products(const long long* x, size_t n, int sh, long long* out) {
     for (size_t i = 0; i < n; ++i) out[i] = (x[i] + fx_half(sh, static_cast<int>(i & 1))) >> sh;

@@ -42,3 +42,20 @@ def test_aligned_products_round_without_a_mean(lib, sh):
     error = (out.astype(object) * (1 << sh) - x.astype(object)).astype(np.float64) / (1 << sh)
     assert np.max(np.abs(error)) <= 0.5
     assert abs(np.mean(error)) <= 5 * 0.29 / 2 ** 10 + (0.25 * 5 / 2 ** 10 if sh == 1 else 0.0)
+
+
+@pytest.mark.parametrize("sh", [-9, 0, 1, 2, 3, 5, 9])
+def test_shifted_products_round_without_a_mean(lib, sh):
+    """As above: one tie in 2^sh rounded up every time was 2^-(sh + 1) units of mean, which
+    put 5.7e-13 instead of 2e-14 on F0 of the horizontal mean at 16x384x9."""
+    rng = np.random.default_rng(4)
+    n = 1 << 20
+    x = rng.integers(-(1 << 48), 1 << 48, n, dtype=np.int64)
+    out = np.empty_like(x)
+    lib.shift_products(_p(x), ctypes.c_size_t(n), ctypes.c_int(sh), _p(out))
+    if sh <= 0:
+        assert np.array_equal(out, x << -sh)
+        return
+    error = (out * (1 << sh) - x) / (1 << sh)
+    assert np.max(np.abs(error)) <= 0.5
+    assert abs(np.mean(error)) <= 5 * 0.36 / 2 ** 10

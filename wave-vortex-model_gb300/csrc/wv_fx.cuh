@@ -288,16 +288,14 @@ WV_HD long long fx_shift_in(unsigned long long m, int rs, int sign) {
     const long long s = sign >> 31;  // 0 or -1; one's complement + 1 is the negative
     return ((static_cast<long long>(m >> (rs > 63 ? 63 : rs)) ^ s) + 1) >> 1;
 }
-// x 2^-sh, rounded
-WV_HD long long fx_shift_round(long long x, int sh) {
-    return sh > 0 ? ((x >> (sh - 1)) + 1) >> 1 : x << -sh;
-}
 // Half of 2^sh, less one on odd places: (x + fx_half(sh, odd)) >> sh rounds to nearest and
 // decides ties up and down in turn.  (A plain shift cuts half a unit, the same in every
 // sample of a row, which adds up in the row's mean.)  sh <= 63, |x| < 2^62; 63 gives 0.
 WV_HD long long fx_half(int sh, int odd) {
     return static_cast<long long>(((1ull << sh) - static_cast<unsigned long long>(odd)) >> 1);
 }
+// x 2^-sh at an odd or even place, rounded
+WV_HD long long fx_shift_round(long long x, int sh, int odd) { return sh > 0 ? (x + fx_half(sh, odd)) >> sh : x << -sh; }
 // v in the line's fixed point (zeros and denormals leave through the shift)
 WV_HD long long fx_from_double(double v, fxscale sc) {
     unsigned hi, lo;

@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                 const bool both = t0 + 2 * i + 1 < nt;
                 for (int x = lane; x < Nx; x += 32) {
                     fxc v;
-                    v.x = fx_shift_round(a[x], sh[0]);
-                    v.y = both ? fx_shift_round(a[Nx + x], sh[1]) : 0;
+                    v.x = fx_shift_round(a[x], sh[0], lane & 1);
+                    v.y = both ? fx_shift_round(a[Nx + x], sh[1], lane & 1) : 0;
                     bufA[i * Nx + x] = v;
                 }
             }

@@ -339,8 +339,8 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const long long a = Sa[t + G * e], b = both ? Sb[t + G * e] : 0;
-        v[e].x = fx_shift_round(a, sh[0]);
-        v[e].y = fx_shift_round(b, sh[1]);
+        v[e].x = fx_shift_round(a, sh[0], t & 1);
+        v[e].y = fx_shift_round(b, sh[1], t & 1);
     }
     fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(unitA, both ? unitB : unitA)) ? 0 : two);
     __syncwarp();
