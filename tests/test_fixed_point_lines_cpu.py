@@ -6,6 +6,7 @@ import subprocess
 
 import numpy as np
 import pytest
+import scipy.fft
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -59,3 +60,67 @@ def test_shifted_products_round_without_a_mean(lib, sh):
     error = (out * (1 << sh) - x) / (1 << sh)
     assert np.max(np.abs(error)) <= 0.5
     assert abs(np.mean(error)) <= 5 * 0.36 / 2 ** 10
+
+
+LANES = [16, 24, 32, 48, 64, 96, 128, 192, 256]
+ANY = [15, 60, 192, 198, 200, 243, 250, 256, 300, 384, 500, 512, 640, 720, 768, 1000, 1024]
+
+
+def _rows(kind, n, rng):
+    if kind == "equal":
+        return 1.2345678901 * rng.choice([-1.0, 1.0], (2, n))
+    x = rng.standard_normal((2, n))
+    if kind == "smooth":
+        x = np.fft.irfft(np.fft.rfft(x) / (1.0 + np.arange(n // 2 + 1)), n)
+    return np.ascontiguousarray(x)
+
+
+def _error(got, ref):
+    return float(np.sqrt(np.sum(np.abs(got - ref) ** 2) / np.sum(np.abs(ref) ** 2)))
+
+
+@pytest.mark.parametrize("lanes,n", [(1, n) for n in LANES] + [(0, n) for n in ANY])
+@pytest.mark.parametrize("kind", ["smooth", "white", "equal"])
+def test_long_lines_are_as_exact_as_short_ones(lib, lanes, n, kind):
+    """Relative L2 error against long double at most 1.7e-16, where mixed-radix FFTs in
+    doubles leave 1.4e-16 to 2.5e-16: real rows in pairs, and complex lines both ways."""
+    if not np.finfo(np.longdouble).eps < 1e-18:
+        pytest.skip("no long double")
+    rng = np.random.default_rng(n)
+    ld = np.longdouble
+    worst = 0.0
+    for _ in range(4):
+        rows = _rows(kind, n, rng)
+        out = np.empty(2 * (n // 2 + 1))
+        lib.real_pair(_p(rows[0]), _p(rows[1]), n, lanes, _p(out))
+        worst = max(worst, _error(out[0::2].astype(ld) + 1j * out[1::2], scipy.fft.rfft(rows[0].astype(ld))))
+        z = np.ascontiguousarray(rows[0] + 1j * _rows(kind, n, rng)[0])
+        if kind == "equal":
+            z = np.exp(2j * np.pi * rng.random(n))
+        if kind == "smooth":  # a spectrum: the inverse's input
+            z = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+            z = np.ascontiguousarray(z / (1.0 + np.abs(np.fft.fftfreq(n, 1.0 / n))))
+        got = np.empty(2 * n)
+        lib.complex_line(_p(z), n, int(kind == "smooth"), lanes, _p(got))
+        ref = scipy.fft.ifft(z.astype(np.clongdouble), norm="forward") if kind == "smooth" else scipy.fft.fft(z.astype(np.clongdouble))
+        worst = max(worst, _error(got[0::2].astype(ld) + 1j * got[1::2], ref))
+    assert worst <= 1.7e-16, worst
+
+
+@pytest.mark.parametrize("n", [127, 509])
+@pytest.mark.parametrize("kind", ["smooth", "white", "equal"])
+def test_prime_lines_are_no_further_off_than_sums_of_doubles(lib, n, kind):
+    """A prime length is one stage of O(n) sums: against the same sums in doubles."""
+    if not np.finfo(np.longdouble).eps < 1e-18:
+        pytest.skip("no long double")
+    rng = np.random.default_rng(n)
+    m = np.arange(n)
+    tw = np.exp(-2j * np.pi * m / n)
+    rows = _rows(kind, n, rng)
+    ref = scipy.fft.rfft(rows[0].astype(np.longdouble))
+    out = np.empty(2 * (n // 2 + 1))
+    lib.real_pair(_p(rows[0]), _p(rows[1]), n, 0, _p(out))
+    plain = np.zeros(n // 2 + 1, complex)
+    for i in range(n):
+        plain += rows[0][i] * tw[i * m[:n // 2 + 1] % n]
+    assert _error(out[0::2].astype(np.longdouble) + 1j * out[1::2], ref) <= _error(plain, ref)

@@ -1,10 +1,11 @@
 """Where the fixed-point lines of FP64 handles could lose what plain doubles keep:
-advecting velocities that are identically zero, and values near both ends of a double's
-range."""
+advecting velocities that are identically zero, values near both ends of a double's
+range, and lines of several hundred points."""
 import numpy as np
 import pytest
 
 import wv_oracle as O
+from test_gpu_fixed_point import extended  # noqa: F401 (a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -76,4 +77,29 @@ def test_values_near_the_ends_of_the_range(wv, shape, power):
     for a, b in zip(k.flux_vjp(300.0, 0.0, *map(dev, A), *u), k.flux_vjp(300.0, 0.0, *map(dev, A), *map(dev, A))):
         a, b = a.cpu().numpy(), b.cpu().numpy()
         assert np.max(np.abs(a / s - b)) <= 1e-13 * np.max(np.abs(b))
+    k.close()
+
+
+# y, x and z lines (2 (Nz - 1) points) past 192, on run-time and block-wide stages, and lane-held 256
+@pytest.mark.parametrize("shape", [(16, 384, 9), (12, 640, 7), (420, 10, 9), (1000, 8, 7), (10, 12, 161), (8, 10, 257),
+                                   (256, 12, 9), (12, 256, 9), (10, 12, 129)])
+def test_long_lines_against_long_double(wv, extended, shape):  # noqa: F811
+    """Largest error against the oracle in long double at most twice that of the oracle
+    in doubles, whose FFTs round alike (1e-16 to 2e-16 of a line), plus 1e-15."""
+    c, d, A, k = _setup(wv, shape)
+    wide = [a.astype(np.clongdouble) for a in A]
+    rng = np.random.default_rng(8)
+    fields = rng.standard_normal((4, shape[2], shape[1], shape[0]))
+
+    def check(got, plain, ref):
+        for a, b, r in zip(got, plain, ref):
+            scale = np.max(np.abs(r))
+            far = lambda x: float(np.max(np.abs(np.asarray(x).astype(r.dtype) - r)) / scale)
+            assert far(a) <= 2.0 * far(b) + 1e-15, (far(a), far(b))
+
+    check(k.nonlinearFlux(123.0, 0.0, *A), O.nonlinear_flux(d, *A, 123.0, 0.0), extended.nonlinear_flux(d, *wide, 123.0, 0.0))
+    check(k.transformWaveVortexToUVWEta(123.0, 0.0, *A), O.inverse_uvweta(d, *A, 123.0, 0.0),
+          extended.inverse_uvweta(d, *wide, 123.0, 0.0))
+    check(k.transformUVWEtaToWaveVortex(fields, 123.0, 0.0), O.forward(d, fields, 123.0, 0.0),
+          extended.forward(d, fields.astype(np.longdouble), 123.0, 0.0))
     k.close()

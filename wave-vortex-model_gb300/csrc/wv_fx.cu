@@ -133,8 +133,9 @@ cudaError_t fx_set_limits(const Plan& p) {
     if (!fx_lane_length(p.Ny)) {
         // (the scalar pipeline has the most columns)
         const size_t sm = dev::smem_fx_any_y(static_cast<int>(p.Ny), dev::fx_any_cols(static_cast<int>(p.Ny), 1 << 20, 1, 1));
-        set(dev::k_yinv_fxany, sm);
-        set(dev::k_yfwd_fxany, sm);
+        const bool late = p.Ny > dev::kFxLateFrom;
+        set(late ? dev::k_yinv_fxany<true> : dev::k_yinv_fxany<false>, sm);
+        set(late ? dev::k_yfwd_fxany<true> : dev::k_yfwd_fxany<false>, sm);
     }
     WV_FXW_SWITCH(p.Nx, {
         set(dev::k_xc2r_fx<NN>, dev::smem_fx_field<NN>(dev::kFxFieldWarps));
@@ -143,12 +144,17 @@ cudaError_t fx_set_limits(const Plan& p) {
     if (fx_x_any(p) && !fx_lane_length(p.Nx)) {
         const FxFieldLaunch l = fx_field_launch(p.Nx, SIZE_MAX / 4, 1);
         set(dev::k_xc2r_fxany<2>, l.smem); set(dev::k_xc2r_fxany<4>, l.smem); set(dev::k_xc2r_fxany<8>, l.smem);
-        set(dev::k_xr2c_fxany, l.smem);
+        set(p.Nx > dev::kFxLateFrom ? dev::k_xr2c_fxany<true> : dev::k_xr2c_fxany<false>, l.smem);
     }
     if (p.fz.N > 0 && !fx_lane_length(p.fz.N)) {
         const size_t inv = dev::smem_fx_any_z(p.fz.N, 4, fx_z_any_warps(p, 4)), two = dev::smem_fx_any_z(p.fz.N, 2, fx_z_any_warps(p, 2));
-        set(dev::k_vinv_fxany<true>, inv); set(dev::k_vinv_fxany<false>, two);
-        set(dev::k_vfwd_fxany<true>, two); set(dev::k_vfwd_fxany<false>, two);
+        if (p.fz.N > dev::kFxLateFrom) {
+            set(dev::k_vinv_fxany<true, true>, inv); set(dev::k_vinv_fxany<false, true>, two);
+            set(dev::k_vfwd_fxany<true, true>, two); set(dev::k_vfwd_fxany<false, true>, two);
+        } else {
+            set(dev::k_vinv_fxany<true, false>, inv); set(dev::k_vinv_fxany<false, false>, two);
+            set(dev::k_vfwd_fxany<true, false>, two); set(dev::k_vfwd_fxany<false, false>, two);
+        }
     }
     WV_FXW_SWITCH(p.fz.N, {
         set(dev::k_vinv_fx<NN, true>, dev::smem_fx_z<NN>(4, 2));
@@ -255,8 +261,9 @@ void fx_yinv(const Plan& p, const dev::DescDev& d, const dev::YInvMap& map, cons
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
         const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * map.nOut, grid_cap(1));
-        dev::k_yinv_fxany<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps,
-                               dev::smem_fx_any_y(Ny, cols), s>>>(d, map, z, y, cols);
+        auto* kernel = Ny > dev::kFxLateFrom ? dev::k_yinv_fxany<true> : dev::k_yinv_fxany<false>;
+        kernel<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, map.nOut), 32 * dev::kFxAnyWarps, dev::smem_fx_any_y(Ny, cols), s>>>(
+            d, map, z, y, cols);
         return;
     }
     const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
@@ -273,8 +280,9 @@ void fx_yfwd(const Plan& p, const dev::DescDev& d, const double2* ps, int nch, d
     const int Ny = static_cast<int>(p.Ny);
     if (!fx_lane_length(p.Ny)) {
         const int cols = dev::fx_any_cols(Ny, d.kxColumns, static_cast<size_t>(d.zTotal) * nch, grid_cap(1));
-        dev::k_yfwd_fxany<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps,
-                               dev::smem_fx_any_y(Ny, cols), s>>>(d, ps, nch, f, cols);
+        auto* kernel = Ny > dev::kFxLateFrom ? dev::k_yfwd_fxany<true> : dev::k_yfwd_fxany<false>;
+        kernel<<<dim3(cdiv(d.kxColumns, cols), d.zTotal, nch), 32 * dev::kFxAnyWarps, dev::smem_fx_any_y(Ny, cols), s>>>(
+            d, ps, nch, f, cols);
         return;
     }
     const int warps = fx_y_warps(p.Ny, d.kxColumns), cols = warps * static_cast<int>(fx_lane_lines(p.Ny));
@@ -304,7 +312,8 @@ bool fx_xr2c(const Plan& p, const dev::DescDev& d, const FxRows& r, const double
     }
     if (p.Nx > 512 || d.kxColumns > 256) return false;
     const FxFieldLaunch l = fx_field_launch(p.Nx, p.Ny * d.zTotal, nch);
-    dev::k_xr2c_fxany<<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, fields, nch, ps);
+    auto* kernel = p.Nx > dev::kFxLateFrom ? dev::k_xr2c_fxany<true> : dev::k_xr2c_fxany<false>;
+    kernel<<<l.grid, 32 * l.warps, l.smem, s>>>(d, r.x, r.twX, fields, nch, ps);
     return true;
 }
 
@@ -315,8 +324,10 @@ bool fx_vinv(const Plan& p, const dev::DescDev& d, bool flux, double elapsed, co
         const int lines = flux ? 4 : 2, warps = fx_z_any_warps(p, lines);
         const dim3 grid(cdiv(p.Nkl, warps), d.members);
         const size_t sm = dev::smem_fx_any_z(p.fz.N, lines, warps);
-        if (flux) dev::k_vinv_fxany<true><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
-        else dev::k_vinv_fxany<false><<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
+        const bool late = p.fz.N > dev::kFxLateFrom;
+        auto* kernel = flux ? (late ? dev::k_vinv_fxany<true, true> : dev::k_vinv_fxany<true, false>)
+                            : (late ? dev::k_vinv_fxany<false, true> : dev::k_vinv_fxany<false, false>);
+        kernel<<<grid, 32 * warps, sm, s>>>(d, Ap, Am, A0, elapsed, z, speed);
         return true;
     }
     const int lines = flux ? 4 : 2, sets = fx_z_sets(p, lines), warps = sets * lines;
@@ -337,10 +348,10 @@ bool fx_vfwd(const Plan& p, const dev::DescDev& d, bool flux, const double2* f, 
         const int warps = fx_z_any_warps(p, 2);
         const dim3 grid(cdiv(p.Nkl, warps), d.members);
         const size_t sm = dev::smem_fx_any_z(p.fz.N, 2, warps);
-        if (flux)
-            dev::k_vfwd_fxany<true><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
-        else
-            dev::k_vfwd_fxany<false><<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
+        const bool late = p.fz.N > dev::kFxLateFrom;
+        auto* kernel = flux ? (late ? dev::k_vfwd_fxany<true, true> : dev::k_vfwd_fxany<true, false>)
+                            : (late ? dev::k_vfwd_fxany<false, true> : dev::k_vfwd_fxany<false, false>);
+        kernel<<<grid, 32 * warps, sm, s>>>(d, f, nch, elapsed, Ap, Am, A0, speed, damping, Fp, Fm, F0);
         return true;
     }
     const int sets = fx_z_sets(p, 2), warps = 2 * sets;

@@ -11,9 +11,14 @@
 // B in magnitude, twiddles having modulus 1), the scale puts B into
 // (2^59, 2^61): no sum overflows 63 bits and no product its accumulator.
 // Precision: the unit is 2^-60 B at worst; quantisation contributes 0.29 units
-// per entry and each twiddle product at most about one, so a 256-point line ends
-// near 7 units rms against the FP64 FFT's 2 x 2^-53 of the line's rms -- smaller
-// for every spectrum between flat (B = 18 rms) and steep (B = 4 rms).
+// per entry and each twiddle product at most about one.  B / rms and the early
+// stages' noise both grow with sqrt(N) on flat lines, so long lines start finer: an
+// output of the first s stages is a sum of P_s = R_1 ... R_s entries, at most P_s max|x|,
+// and while that is below B the line is held on a scale finer by the difference
+// (fx_gap) and shifted down stage by stage: run-time lines past 192 points, and lane-held
+// ones of 128 and more whose input is samples (spectra fall off; flat ones of 85 of 256
+// entries stay at 1.7e-16).  Errors then stay at 0.5 to 1.6e-16 of the line at every
+// length, those of mixed-radix FFTs in doubles at 1.4 to 2.5e-16 (without it 3.3e-16 at 1024).
 #pragma once
 
 #include <cstdint>
@@ -23,8 +28,10 @@
 
 #ifdef __CUDACC__
 #define WV_HD __host__ __device__ __forceinline__
+#define WV_DEV __device__ __forceinline__
 #else
 #define WV_HD inline
+#define WV_DEV inline
 #endif
 
 namespace wvgpu {
@@ -76,24 +83,31 @@ WV_HD fxc fx_cmul(fxc a, fxw w) {
     r = fx_mad(yh4, mh, r);   i = fx_mad(yh4, w.ch, i);
     return fxc{r, i};
 }
-#ifdef __CUDACC__
 // x w for |x| < 2^60 (1 - 2^-9): the middle terms as four high halves (32-bit sums;
 // each cuts half a unit on average, `two` gives it back), 27 instructions against 37.
 // two: the value 2 in a register the compiler cannot rebuild (fx_two); 0 on all-zero
 // lines, which stay exactly zero.  Twiddles +-1 and +-i (no low words) cut nothing.
-template <bool INV>
-__device__ __forceinline__ fxc fx_cmul60(fxc a, fxw w, int two) {
-    const long long x4 = a.x << 2, y4 = a.y << 2;
+// SHIFT: x 2^-sh w; the operand carries two more bits, so a shift cuts at a quarter unit.
+template <bool INV, bool SHIFT>
+WV_HD fxc fx_cmul60(fxc a, fxw w, int two, int sh) {
+    const long long x4 = SHIFT ? (a.x << 2) >> sh : a.x << 2, y4 = SHIFT ? (a.y << 2) >> sh : a.y << 2;
     const int xl = fx_lo(x4), yl = fx_lo(y4), xh = fx_hi(x4), yh = fx_hi(y4);
     const int nh = -w.sh, nl = -w.sl;
-    const int sh = INV ? nh : w.sh, sl = INV ? nl : w.sl, mh = INV ? w.sh : nh, ml = INV ? w.sl : nl;
+    const int sih = INV ? nh : w.sh, sil = INV ? nl : w.sl, mh = INV ? w.sh : nh, ml = INV ? w.sl : nl;
+#ifdef __CUDA_ARCH__
     auto mad = [](int p, int q, int c) { int r; asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(p), "r"(q), "r"(c)); return r; };
     auto mul = [](int p, int q) { long long r; asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(p), "r"(q)); return r; };
-    const int mean = static_cast<int>(min(static_cast<unsigned>(w.cl | w.sl), static_cast<unsigned>(two)));
+#else
+    auto mad = [](int p, int q, int c) { return static_cast<int>((static_cast<long long>(p) * q) >> 32) + c; };
+    auto mul = [](int p, int q) { return static_cast<long long>(p) * q; };
+#endif
+    const unsigned low = static_cast<unsigned>(w.cl | w.sl);
+    const int mean = static_cast<int>(low < static_cast<unsigned>(two) ? low : static_cast<unsigned>(two));
     const int m = mad(xh, w.cl, mad(xl, w.ch, mad(yh, ml, mad(yl, mh, mean))));
-    const int n = mad(xh, sl, mad(xl, sh, mad(yh, w.cl, mad(yl, w.ch, mean))));
-    return fxc{mul(xh, w.ch) + mul(yh, mh) + static_cast<long long>(m), mul(xh, sh) + mul(yh, w.ch) + static_cast<long long>(n)};
+    const int n = mad(xh, sil, mad(xl, sih, mad(yh, w.cl, mad(yl, w.ch, mean))));
+    return fxc{mul(xh, w.ch) + mul(yh, mh) + static_cast<long long>(m), mul(xh, sih) + mul(yh, w.ch) + static_cast<long long>(n)};
 }
+#ifdef __CUDACC__
 __device__ __forceinline__ int fx_two() {
     int r;
     asm volatile("mov.u32 %0, 2;" : "=r"(r));
@@ -267,6 +281,7 @@ struct fxscale {
     int e0;   // biased exponent at bit `bit`
     int bit;
     bool zero = false;  // no entry but zeros
+    int gap = 0;        // bits by which the line may start finer (fx_gap)
 };
 WV_HD fxscale fx_scale(unsigned top, float l1) {
     const float s = l1 * 1.0025f;
@@ -280,6 +295,12 @@ WV_HD fxscale fx_scale(float l1) {
     const int el = static_cast<int>(fx_float_bits(l1 * 1.0025f) >> 23) - 126;
     return {1023, 61 - el};
 }
+// Bits between a line's sum of moduli and `radix` times its largest modulus.
+WV_HD int fx_gap(float l1, float most, int radix) {
+    const int g = static_cast<int>(fx_float_bits(l1 * 1.0025f) >> 23) - static_cast<int>(fx_float_bits(most * radix * 1.0025f) >> 23);
+    return g > 0 ? g : 0;
+}
+constexpr int kFxAnyGap = 31;  // of an all-zero line, which limits no partner
 // m (2^e at bit 62) shifted right by rs + 1 and rounded to nearest, negated if asked.
 // Roundings here have mean zero on both signs: a mean of a fraction of a unit, the same
 // in every line, would add up in the lowest modes of the passes that follow (0.25 units
@@ -357,15 +378,120 @@ WV_HD double fx_to_double(long long x, FxUnit o) {
 }
 WV_HD double fx_to_double(long long x, int unit) { return fx_to_double(x, fx_out(unit)); }
 
-#ifdef __CUDACC__
+// ---- lines of 16 to 256 points held by lanes (wv_fxwarp.cuh) ------------------------------
+
+template <int N> struct FxW {
+    static constexpr int E = N % 3 == 0 ? 12 : 8;  // points of a lane
+    static constexpr int H = E / 2;
+    static constexpr int G = N / E;                // lanes of a line
+    static constexpr int lines = 32 / G;           // lines of a warp
+    static constexpr int samples = lines * N;      // points of a warp: 32 E
+    static constexpr int buffer = N + N / 8;       // padded line buffer
+    // radices of the stages (their products end with N; R3 = 1: two stages)
+    static constexpr int R1 = E == 8 ? 8 : N == 24 ? 2 : 4;
+    static constexpr int R2 = E == 8 ? (N == 16 ? 2 : (N == 32 || N == 128) ? 4 : 8) : N == 96 ? 2 : N == 192 ? 4 : 12;
+    static constexpr int R3 = N / (R1 * R2);
+    static constexpr int twiddles = (R2 - 1) * R1 + (R3 - 1) * R1 * R2;
+    // stages before which a line of samples is shifted down (fx_gap), for two rows or
+    // channels to a line and for one: as many as keep the error below a double FFT's
+    static constexpr int latePair = N == 256 ? 2 : N >= 128 ? 1 : 0;
+    static constexpr int lateOne = N == 256 ? 1 : 0;
+};
+WV_HD int fx_pad(int i) { return i + (i >> 3); }
+
+// Stage of radix R behind Ns points already combined; tw[(r - 1) Ns + k].  SHIFT: the
+// inputs come down by sh bits, rounded by the half unit that the stage before added to
+// its outputs (`half` on its first input; NEXT), ties in turn over the lanes.
+template <int N, int R, int Ns, bool INV, bool SHIFT, bool NEXT>
+WV_HD void fx_wstage(fxc (&v)[FxW<N>::E], const fxw* tw, int t, int two, int sh, long long half) {
+    constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        const int k = (t + G * b) & (Ns - 1);  // (Ns is a power of two)
+        fxc u[R];
+        u[0] = v[b];
+        if (SHIFT) u[0] = fxc{(((u[0].x << 2) >> sh) + 1 + (t & 1)) >> 2, (((u[0].y << 2) >> sh) + 1 + (t & 1)) >> 2};
+        if (NEXT) u[0] = fxc{u[0].x + half, u[0].y + half};
+#pragma unroll
+        for (int r = 1; r < R; ++r)
+            u[r] = Ns == 1 ? v[b + B * r] : fx_cmul60<INV, SHIFT>(v[b + B * r], tw[(r - 1) * Ns + k], two, sh);
+        fx_dft<R, INV>(u);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[b + B * r] = u[r];
+    }
+}
+// v[b + B r], the outputs of a stage of radix R, to their places, and back in lane order
+template <int N, int R, int Ns>
+WV_HD void fx_wscatter(const fxc (&v)[FxW<N>::E], fxc* x, int t) {
+    constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        const int j = t + G * b, k = j & (Ns - 1), jq = j / Ns;
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[fx_pad(jq * Ns * R + k + r * Ns)] = v[b + B * r];
+    }
+}
+template <int N>
+WV_HD void fx_wgather(fxc (&v)[FxW<N>::E], const fxc* x, int t) {
+#pragma unroll
+    for (int e = 0; e < FxW<N>::E; ++e) v[e] = x[fx_pad(t + FxW<N>::G * e)];
+}
+// The whole line (sum of moduli below 2^60, 2^gap times that in the first stage); x: this
+// line's buffer, tw: the stage twiddles; LATE: FxW's latePair or lateOne, `gap` its bits.
+// each(f): f(v, t) for every lane of the line, a barrier after it (fx_fft_warp; a host
+// test walks the lanes).
+template <int N, bool INV, int LATE, typename Each>
+WV_DEV void fx_line_stages(fxc* x, const fxw* tw, int two, int gap, Each each) {
+    using W = FxW<N>;
+    constexpr bool three = W::R3 > 1, second = LATE >= 1, third = LATE >= 2 && three;
+    constexpr int most2 = W::R2 == 8 ? 3 : W::R2 == 4 ? 2 : W::R2 == 2 ? 1 : 4;  // ceil log2 R2
+    const int sh2 = third && gap > most2 ? most2 : gap, sh3 = gap - sh2;
+    const long long half2 = static_cast<long long>((1ull << sh2) >> 3), half3 = static_cast<long long>((1ull << sh3) >> 3);
+    each([=](fxc (&v)[W::E], int t) {
+        fx_wstage<N, W::R1, 1, INV, false, second>(v, tw, t, two, 0, half2);
+        fx_wscatter<N, W::R1, 1>(v, x, t);
+    });
+    each([=](fxc (&v)[W::E], int t) { fx_wgather<N>(v, x, t); });
+    each([=](fxc (&v)[W::E], int t) {
+        fx_wstage<N, W::R2, W::R1, INV, second, third>(v, tw, t, two, sh2, half3);
+        if constexpr (three) fx_wscatter<N, W::R2, W::R1>(v, x, t);
+    });
+    if constexpr (three) {
+        each([=](fxc (&v)[W::E], int t) { fx_wgather<N>(v, x, t); });
+        each([=](fxc (&v)[W::E], int t) {
+            fx_wstage<N, W::R3, W::R1 * W::R2, INV, third, false>(v, tw + (W::R2 - 1) * W::R1, t, two, sh3, 0);
+        });
+    }
+}
+
+// ---- lines of any length, run-time stages -----------------------------------------------
+
+// How far a line is shifted down before a stage: its gap (one for all lines, or one each)
+// as far as the stage's span needs it, `before` bits of which went with earlier stages.
+struct FxLate {
+    const int* gaps;
+    int gap, before, after;
+    WV_HD int operator()(int line) const {
+        const int g = gaps ? gaps[line] : gap;
+        return (g < after ? g : after) - (g < before ? g : before);
+    }
+};
+constexpr int kFxLateFrom = 192;  // longer run-time lines start finer
+WV_HD int fx_ceil_log2(int n) { return n <= 1 ? 0 : 32 - fx_clz(static_cast<unsigned>(n - 1)); }
+// entry at place j, shifted down
+WV_HD fxc fx_late(fxc a, int sh, int j) {
+    if (sh == 0) return a;
+    const long long h = fx_half(sh, j & 1);
+    return fxc{(a.x + h) >> sh, (a.y + h) >> sh};
+}
 // One stage over `lines` lines (as fft_stage): radix R from src to dst.
-template <int R, bool INV>
-__device__ __forceinline__ void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int Ns, int lines,
-                                         int ld, const fxw* __restrict__ tw, int tid, int nt) {
+template <int R, bool INV, bool LATE>
+WV_HD void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int Ns, int lines, int ld,
+                    const fxw* __restrict__ tw, FxLate late, int tid, int nt) {
     const int nb = N / R;
     const int tstride = N / (Ns * R);
     const bool p2 = (N & (N - 1)) == 0;
-    const int nbShift = __ffs(nb) - 1, nsShift = __ffs(Ns) - 1;
+    const int nbShift = 31 - fx_clz(static_cast<unsigned>(nb)), nsShift = 31 - fx_clz(static_cast<unsigned>(Ns));
     for (int it = tid; it < lines * nb; it += nt) {
         int line, j, k, jq;
         if (p2) {
@@ -374,9 +500,10 @@ __device__ __forceinline__ void fx_stage(const fxc* __restrict__ src, fxc* __res
             line = it / nb; j = it - line * nb; jq = j / Ns; k = j - jq * Ns;
         }
         const fxc* in = src + line * ld + j;
+        const int sh = LATE ? late(line) : 0;
         fxc v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = in[r * nb];
+        for (int r = 0; r < R; ++r) v[r] = LATE ? fx_late(in[r * nb], sh, j) : in[r * nb];
         if (Ns > 1) {
             const int ts = k * tstride;
 #pragma unroll
@@ -388,10 +515,11 @@ __device__ __forceinline__ void fx_stage(const fxc* __restrict__ src, fxc* __res
         for (int r = 0; r < R; ++r) out[r * Ns] = v[r];
     }
 }
-// Any other radix: one output per work item, an O(R) sum.
+// Any other radix: one output per work item, an O(R) sum.  (fx_shift_lines before it: R
+// items read each entry.)
 template <bool INV>
-__device__ __forceinline__ void fx_stage_any(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int R, int Ns,
-                                             int lines, int ld, const fxw* __restrict__ tw, int tid, int nt) {
+WV_HD void fx_stage_any(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int R, int Ns, int lines, int ld,
+                        const fxw* __restrict__ tw, int tid, int nt) {
     const int nb = N / R;
     const int tstride = N / (Ns * R);
     for (int it = tid; it < lines * N; it += nt) {
@@ -412,11 +540,37 @@ __device__ __forceinline__ void fx_stage_any(const fxc* __restrict__ src, fxc* _
 }
 
 struct FxFactors { int N, nstages; const int* radix; };
+WV_HD void fx_shift_lines(fxc* lines_, int N, int lines, int ld, FxLate late, int tid, int nt) {
+    for (int it = tid; it < lines * N; it += nt) {
+        const int line = it / N, i = it - line * N;
+        lines_[line * ld + i] = fx_late(lines_[line * ld + i], late(line), i);
+    }
+}
+WV_HD bool fx_any_radix(int R) { return R != 2 && R != 3 && R != 4 && R != 5 && R != 8; }
+// What the lines are shifted down by before stage s > 0, which follows Ns points combined.
+WV_HD FxLate fx_late_of(const FxFactors& f, int s, int Ns, const int* gaps, int gap) {
+    return {gaps, gap, fx_ceil_log2(Ns / f.radix[0]), fx_ceil_log2(Ns * f.radix[s] / f.radix[0])};
+}
+// Stage s of the lines, work items tid, tid + nt ...  LATE: lines past kFxLateFrom.
+template <bool INV, bool LATE>
+WV_HD void fx_run_stage(const fxc* a, fxc* b, const FxFactors& f, int s, int Ns, int lines, int ld, const fxw* tw, const int* gaps,
+                        int gap, int tid, int nt) {
+    const int R = f.radix[s];
+    const FxLate late = LATE && s > 0 ? fx_late_of(f, s, Ns, gaps, gap) : FxLate{nullptr, 0, 0, 0};
+    if (R == 8) fx_stage<8, INV, LATE>(a, b, f.N, Ns, lines, ld, tw, late, tid, nt);
+    else if (R == 4) fx_stage<4, INV, LATE>(a, b, f.N, Ns, lines, ld, tw, late, tid, nt);
+    else if (R == 2) fx_stage<2, INV, LATE>(a, b, f.N, Ns, lines, ld, tw, late, tid, nt);
+    else if (R == 3) fx_stage<3, INV, LATE>(a, b, f.N, Ns, lines, ld, tw, late, tid, nt);
+    else if (R == 5) fx_stage<5, INV, LATE>(a, b, f.N, Ns, lines, ld, tw, late, tid, nt);
+    else fx_stage_any<INV>(a, b, f.N, R, Ns, lines, ld, tw, tid, nt);
+}
 
+#ifdef __CUDACC__
 // Lines of doubles (re, im) in place to fixed point: one group of warps per line
-// sums the moduli, then every entry is scaled.  unit[line] receives fx_unit.
+// sums the moduli, then every entry is scaled.  unit[line] receives fx_unit, gaps[line]
+// the bits by which long lines start finer (radix: that of the first stage).
 // Called by all threads of the block.
-__device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, int* unit) {
+__device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, int radix, int* unit, int* gaps) {
     __shared__ unsigned redTop[32];
     __shared__ float redSum[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -440,15 +594,31 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
             }
             return sum;
         };
-        float sum = 0.f;
+        auto largest = [&](float m) {  // over the warps of the line
+            unsigned bits = __reduce_max_sync(0xffffffffu, fx_float_bits(m));
+            if (per > 1) {
+                __syncthreads();  // (redTop may still be read)
+                if (lane == 0) redTop[warp] = bits;
+                __syncthreads();
+                if (has)
+                    for (int w = 0; w < per; ++w) bits = max(bits, redTop[g * per + w]);
+                __syncthreads();
+            }
+            return fx_float(bits);
+        };
+        float sum = 0.f, most = 0.f;
         if (has)
             for (int i = t; i < N; i += step) {
                 const double2 v = row[i];
-                sum += fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))),
-                                  fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
+                const float m = fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))),
+                                           fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
+                sum += m;
+                most = m > most ? m : most;
             }
         sum = total(sum);
         fxscale sc = fx_scale(sum);
+        int gap = 0;
+        if (N > kFxLateFrom) gap = fx_gap(sum, largest(most), radix);
         const bool odd = has && !fx_plain_sum(sum);
         if (per > 1 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) {
             unsigned top = 0;
@@ -465,18 +635,25 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
                 if (has)
                     for (int w = 0; w < per; ++w) top = max(top, redTop[g * per + w]);
             }
-            float rel = 0.f;
+            float rel = 0.f, relMost = 0.f;
             if (has)
                 for (int i = t; i < N; i += step) {
                     const double2 v = row[i];
-                    rel += fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
-                                      fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
+                    const float m = fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
+                                               fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
+                    rel += m;
+                    relMost = m > relMost ? m : relMost;
                 }
             rel = total(rel);
-            if (odd) sc = fx_scale(top, rel);
+            const int relGap = N > kFxLateFrom ? fx_gap(rel, largest(relMost), radix) : 0;
+            if (odd) {
+                sc = fx_scale(top, rel);
+                gap = relGap;
+            }
         }
         if (has) {
-            if (t == 0) unit[line] = fx_unit(sc);
+            if (t == 0) { unit[line] = fx_unit(sc); gaps[line] = gap; }
+            sc.bit += gap;
             for (int i = t; i < N; i += step) {
                 const double2 v = row[i];
                 out[line * ld + i] = fxc{fx_from_double(v.x, sc), fx_from_double(v.y, sc)};
@@ -487,33 +664,33 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
     __syncthreads();
 }
 
-// All stages over fixed-point lines; returns the buffer holding the result.
+// All stages over fixed-point lines; returns the buffer holding the result.  gaps: bits by
+// which each line starts finer (null: `gap` for every line), LATE only.
 // WARP: the lines belong to one warp (no block barrier), else to the block.
-template <bool INV, bool WARP>
-__device__ inline fxc* fx_lines(fxc* a, fxc* b, const FxFactors f, int lines, int ld, const fxw* tw) {
+template <bool INV, bool WARP, bool LATE>
+__device__ inline fxc* fx_all_stages(fxc* a, fxc* b, const FxFactors f, int lines, int ld, const fxw* tw, const int* gaps, int gap) {
     const int tid = WARP ? (threadIdx.x & 31) : threadIdx.x, nt = WARP ? 32 : blockDim.x;
     int Ns = 1;
     for (int s = 0; s < f.nstages; ++s) {
-        const int R = f.radix[s];
-        if (R == 8) fx_stage<8, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
-        else if (R == 4) fx_stage<4, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
-        else if (R == 2) fx_stage<2, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
-        else if (R == 3) fx_stage<3, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
-        else if (R == 5) fx_stage<5, INV>(a, b, f.N, Ns, lines, ld, tw, tid, nt);
-        else fx_stage_any<INV>(a, b, f.N, R, Ns, lines, ld, tw, tid, nt);
+        if (LATE && s > 0 && fx_any_radix(f.radix[s])) {
+            fx_shift_lines(a, f.N, lines, ld, fx_late_of(f, s, Ns, gaps, gap), tid, nt);
+            if (WARP) __syncwarp(); else __syncthreads();
+        }
+        fx_run_stage<INV, LATE>(a, b, f, s, Ns, lines, ld, tw, gaps, gap, tid, nt);
         if (WARP) __syncwarp(); else __syncthreads();
-        Ns *= R;
+        Ns *= f.radix[s];
         fxc* t = a; a = b; b = t;
     }
     return a;
 }
-
 // fft_lines of FP64 lines: scaled, transformed and scaled back in place.
 template <bool INV>
 __device__ inline double2* fx_fft_lines(double2* a, double2* b, const FxFactors f, int lines, int ld, const fxw* tw) {
-    __shared__ int unit[16];
-    fx_quantise(a, f.N, lines, ld, unit);
-    fxc* r = fx_lines<INV, false>(reinterpret_cast<fxc*>(a), reinterpret_cast<fxc*>(b), f, lines, ld, tw);
+    __shared__ int unit[16], gaps[16];
+    fx_quantise(a, f.N, lines, ld, f.radix[0], unit, gaps);
+    fxc *fa = reinterpret_cast<fxc*>(a), *fb = reinterpret_cast<fxc*>(b);
+    fxc* r = f.N > kFxLateFrom ? fx_all_stages<INV, false, true>(fa, fb, f, lines, ld, tw, gaps, 0)
+                               : fx_all_stages<INV, false, false>(fa, fb, f, lines, ld, tw, nullptr, 0);
     double2* out = reinterpret_cast<double2*>(r);
     for (int i = threadIdx.x; i < lines * f.N; i += blockDim.x) {
         const int line = i / f.N, k = i - line * f.N, u = unit[line];

@@ -216,9 +216,12 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
             if (i < H) b[i] = chS >= 0 && z != 0 ? colval(chS, z) : make_double2(0.0, 0.0);
         }
         fxc C[H + 1], S[H];
-        int uC, uS;
-        fx_quantise_lane<H + 1, G, kFxPlain>(a, none5, 0u, 1, [](int) { return 2.0f; }, C, uC);
-        fx_quantise_lane<H, G, kFxPlain>(b, none4, 0u, 1, [](int) { return 2.0f; }, S, uS);
+        constexpr int radix = W::latePair ? W::R1 : 0;
+        auto twice = [](int) { return 2.0f; };
+        const FxLine lC = fx_line<H + 1, G, kFxPlain, radix>(a, none5, 0u, 1, twice), lS = fx_line<H, G, kFxPlain, radix>(b, none4, 0u, 1, twice);
+        const int gap = fx_shared_gap(lC.gap, lS.gap), uC = lC.unit, uS = lS.unit;
+        fx_fixed<H + 1, kFxPlain>(a, none5, lC.base - gap, C);
+        fx_fixed<H, kFxPlain>(b, none4, lS.base - gap, S);
         __syncthreads();  // twiddles
         fxc v[E];
 #pragma unroll
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
 #pragma unroll
         for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
-        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two());
+        fx_fft_warp<N, false, W::latePair>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two(), gap);
 #pragma unroll
         for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();
@@ -272,7 +275,7 @@ template <int N>
 __global__ void __launch_bounds__(32 * kFxYWarps, 2)
     k_yfwd_pair_fx(DescDev d, YFwdPairMap map, const double2* __restrict__ yin, int nIn, double2* __restrict__ fout) {
     using W = FxW<N>;
-    constexpr int G = W::G, E = W::E, H = W::H;
+    constexpr int G = W::G, E = W::E;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = d.positions, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
@@ -302,11 +305,11 @@ __global__ void __launch_bounds__(32 * kFxYWarps, 2)
         for (int e = 0; e < E; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
         __syncthreads();
         fxc v[E];
-        int unit;
         double none[E];
-        fx_quantise_lane<E, G, kFxPlain>(a, none, 0u, 0, [](int) { return 1.0f; }, v, unit);
-        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
-        const FxUnit o = fx_out(unit);
+        const FxLine l = fx_line<E, G, kFxPlain, W::lateOne ? W::R1 : 0>(a, none, 0u, 0, [](int) { return 1.0f; });
+        fx_fixed<E, kFxPlain>(a, none, l.base - l.gap, v);
+        fx_fft_warp<N, false, W::lateOne>(v, x, tw, t, fx_silent(l.unit) ? 0 : fx_two(), l.gap);
+        const FxUnit o = fx_out(l.unit);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const double re = fx_to_double(v[e].x, o), im = fx_to_double(v[e].y, o);
@@ -435,14 +438,10 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, 2)
             rb[e] = s.y;
         }
         __syncwarp();
-        long long ia[E], ib[E];
-        int ua, ub;
-        fx_quantise_real<E, G>(ra, ia, ua);
-        fx_quantise_real<E, G>(rb, ib, ub);
         fxc v[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) v[e] = fxc{ia[e], ib[e]};
-        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(ua, ub)) ? 0 : two);
+        int ua, ub, gap;
+        fx_real_pair<N>(ra, rb, v, ua, ub, gap);
+        fx_fft_warp<N, false, W::latePair>(v, x, tw, t, fx_silent(max(ua, ub)) ? 0 : two, gap);
 #pragma unroll
         for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
         __syncwarp();

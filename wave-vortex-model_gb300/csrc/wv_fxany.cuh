@@ -15,17 +15,23 @@ namespace dev {
 __host__ __device__ inline int fx_any_ld(int N) { return N | 1; }
 
 // Scale of a line whose entry i (0 <= i < n) is at(i), counted count(i) times in the
-// sum of moduli; the warp's lanes share the entries.
+// sum of moduli; the warp's lanes share the entries.  radix > 0: with the bits by which
+// the line may start finer.
 template <typename At, typename Count>
-__device__ __forceinline__ fxscale fx_warp_scale(int n, int lane, At at, Count count) {
-    float sum = 0.f;
+__device__ __forceinline__ fxscale fx_warp_scale(int n, int lane, int radix, At at, Count count) {
+    float sum = 0.f, most = 0.f;
     for (int i = lane; i < n; i += 32) {
         const double2 v = at(i);
-        sum += count(i) * fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))),
-                                     fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
+        const float m = fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))), fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
+        sum += count(i) * m;
+        most = fmaxf(most, m);
     }
     sum = fx_group_sum<32>(sum);
-    if (fx_plain_sum(sum)) return fx_scale(sum);
+    if (fx_plain_sum(sum)) {
+        fxscale sc = fx_scale(sum);
+        if (radix > 0) sc.gap = fx_gap(sum, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most))), radix);
+        return sc;
+    }
     unsigned top = 0;
     for (int i = lane; i < n; i += 32) {
         const double2 v = at(i);
@@ -34,14 +40,21 @@ __device__ __forceinline__ fxscale fx_warp_scale(int n, int lane, At at, Count c
     }
     top = __reduce_max_sync(0xffffffffu, top);
     float rel = 0.f;
+    most = 0.f;
     for (int i = lane; i < n; i += 32) {
         const double2 v = at(i);
-        rel += count(i) * fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
-                                     fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
+        const float m = fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
+                                   fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
+        rel += count(i) * m;
+        most = fmaxf(most, m);
     }
-    return fx_scale(top, fx_group_sum<32>(rel));
+    rel = fx_group_sum<32>(rel);
+    most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most)));
+    fxscale sc = fx_scale(top, rel);
+    if (radix > 0) sc.gap = sc.zero ? kFxAnyGap : fx_gap(rel, most, radix);
+    return sc;
 }
-
+// LATE in the kernels below: the lines are longer than kFxLateFrom and may start finer.
 // ---- y ------------------------------------------------------------------------------
 
 constexpr int kFxAnyWarps = 8;
@@ -64,6 +77,7 @@ __device__ __forceinline__ void fx_any_twiddles(fxw* tw, const fxw* __restrict__
 }
 // k_yinv, channel blockIdx.z.  Bound by shared memory: a stage reads and writes every
 // entry.  60x50x31 hydrostatic, all five passes: 268 (FP64 pipe) -> 111 us.
+template <bool LATE>
 __global__ void __launch_bounds__(32 * kFxAnyWarps)
     k_yinv_fxany(DescDev d, YInvMap map, const double2* __restrict__ zspec, double2* __restrict__ yspec, int cols) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -80,6 +94,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
     const bool mulL = map.mulL[oc] != 0;
     const int each = (cols + warps - 1) / warps;  // lines of a warp
     const int c0 = warp * each, nl = min(each, g - c0);
+    __shared__ int gaps[kFxAnyWarps][LATE ? 32 : 1];  // of the warp's lines
     int units = 0;  // lane l keeps the unit of line c0 + l (each <= 32)
     for (int l = 0; l < nl; ++l) {
         double2* row = bufA + (c0 + l) * ld;
@@ -90,19 +105,21 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
             if (mulL) v = make_double2(-rowL[i] * v.y, rowL[i] * v.x);
             row[i] = v;
         }
-        const fxscale sc = fx_warp_scale(Ny, lane, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
+        fxscale sc = fx_warp_scale(Ny, lane, LATE ? d.fy.radix[0] : 0, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
+        if (lane == l) units = fx_unit(sc);
+        if (LATE && lane == 0) gaps[warp][l] = sc.gap;
+        sc.bit += sc.gap;
         fxc* q = reinterpret_cast<fxc*>(row);
         for (int i = lane; i < Ny; i += 32) {
             const double2 v = row[i];
             q[i] = fxc{fx_from_double(v.x, sc), fx_from_double(v.y, sc)};
         }
-        if (lane == l) units = fx_unit(sc);
     }
     __syncwarp();
     double2* res = bufA;
     if (nl > 0) {
-        fxc* r = fx_lines<true, true>(reinterpret_cast<fxc*>(bufA + c0 * ld), reinterpret_cast<fxc*>(bufB + c0 * ld),
-                                      FxFactors{d.fy.N, d.fy.nstages, d.fy.radix}, nl, ld, tw);
+        fxc* r = fx_all_stages<true, true, LATE>(reinterpret_cast<fxc*>(bufA + c0 * ld), reinterpret_cast<fxc*>(bufB + c0 * ld),
+                                                 FxFactors{d.fy.N, d.fy.nstages, d.fy.radix}, nl, ld, tw, gaps[warp], 0);
         for (int l = 0; l < nl; ++l) {
             const int u = __shfl_sync(0xffffffffu, units, l);
             double2* o = reinterpret_cast<double2*>(r + l * ld);
@@ -122,6 +139,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
 }
 
 // k_yfwd, channel blockIdx.z.
+template <bool LATE>
 __global__ void __launch_bounds__(32 * kFxAnyWarps)
     k_yfwd_fxany(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec, int cols) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -141,20 +159,23 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
     const int each = (cols + warps - 1) / warps;
     const int c0 = warp * each, nl = min(each, g - c0);
     if (nl <= 0) return;
+    __shared__ int gaps[kFxAnyWarps][LATE ? 32 : 1];
     int units = 0;
     for (int l = 0; l < nl; ++l) {
         double2* row = bufA + (c0 + l) * ld;
-        const fxscale sc = fx_warp_scale(Ny, lane, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
+        fxscale sc = fx_warp_scale(Ny, lane, LATE ? d.fy.radix[0] : 0, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
+        if (lane == l) units = fx_unit(sc);
+        if (LATE && lane == 0) gaps[warp][l] = sc.gap;
+        sc.bit += sc.gap;
         fxc* q = reinterpret_cast<fxc*>(row);
         for (int i = lane; i < Ny; i += 32) {
             const double2 v = row[i];
             q[i] = fxc{fx_from_double(v.x, sc), fx_from_double(v.y, sc)};
         }
-        if (lane == l) units = fx_unit(sc);
     }
     __syncwarp();
-    const fxc* r = fx_lines<false, true>(reinterpret_cast<fxc*>(bufA + c0 * ld), reinterpret_cast<fxc*>(bufB + c0 * ld),
-                                         FxFactors{d.fy.N, d.fy.nstages, d.fy.radix}, nl, ld, tw);
+    const fxc* r = fx_all_stages<false, true, LATE>(reinterpret_cast<fxc*>(bufA + c0 * ld), reinterpret_cast<fxc*>(bufB + c0 * ld),
+                                                    FxFactors{d.fy.N, d.fy.nstages, d.fy.radix}, nl, ld, tw, gaps[warp], 0);
     double2* out = fspec + (static_cast<size_t>(ch) * d.zTotal + z) * P;
     for (int l = 0; l < nl; ++l) {
         const int u = __shfl_sync(0xffffffffu, units, l);
@@ -192,17 +213,12 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
         const int z = row / Ny, y = row - z * Ny;
         const double2* h = yspec + ((static_cast<size_t>(z) * nch + ca) * Ny + y) * KX;
         fxc A[EK], B[EK];
-        int uA, uB = 0;
-        fx_load_row<EK>(h, KX, Nx, lane, ((d.c2rUseK >> ca) & 1) != 0, row_k<double>(d), A, uA);
-        if (cb < nch) {
-            fx_load_row<EK>(h + static_cast<size_t>(Ny) * KX, KX, Nx, lane, ((d.c2rUseK >> cb) & 1) != 0, row_k<double>(d), B, uB);
-        } else {
-#pragma unroll
-            for (int e = 0; e < EK; ++e) B[e] = fxc{0, 0};
-        }
+        int uA, uB, gap;
+        fx_load_rows<EK>(h, cb < nch ? h + static_cast<size_t>(Ny) * KX : nullptr, ((d.c2rUseK >> ca) & 1) != 0,
+                         cb < nch && ((d.c2rUseK >> cb) & 1) != 0, KX, Nx, f.radix[0], lane, row_k<double>(d), A, B, uA, uB, gap);
         fx_pack_rows<EK>(A, B, bufA, KX, Nx, lane);
         __syncwarp();
-        const fxc* r = fx_lines<true, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, Nx, tw);
+        const fxc* r = fx_row_stages<EK, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, tw, gap);
         double* o = fields + static_cast<size_t>(ca) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
         for (int x = lane; x < Nx; x += 32) {
             o[x] = fx_to_double(r[x].x, fx_out(uA));
@@ -213,6 +229,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
 }
 
 // k_xr2c_fields: a warp takes two channels of a (y, z) row as one line.
+template <bool LATE>
 __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
     k_xr2c_fxany(DescDev d, FFTDev f, const fxw* __restrict__ twg, const double* __restrict__ fields, int nch,
                  double2* __restrict__ pspec) {
@@ -233,14 +250,18 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
         const double* s = fields + static_cast<size_t>(c) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
         for (int x = lane; x < Nx; x += 32) raw[x] = make_double2(s[x], both ? s[R + x] : 0.0);
         auto one = [](int) { return 1.0f; };
-        fxscale sa = fx_warp_scale(Nx, lane, [&](int x) { return make_double2(raw[x].x, 0.0); }, one);
-        fxscale sb = fx_warp_scale(Nx, lane, [&](int x) { return make_double2(raw[x].y, 0.0); }, one);
+        const int radix = LATE ? f.radix[0] : 0;
+        fxscale sa = fx_warp_scale(Nx, lane, radix, [&](int x) { return make_double2(raw[x].x, 0.0); }, one);
+        fxscale sb = fx_warp_scale(Nx, lane, radix, [&](int x) { return make_double2(raw[x].y, 0.0); }, one);
         sa.bit -= 1;
         sb.bit -= 1;
-        for (int x = lane; x < Nx; x += 32) bufA[x] = fxc{fx_from_double(raw[x].x, sa), fx_from_double(raw[x].y, sb)};
         const int ua = fx_unit(sa) - 1, ub = fx_unit(sb) - 1;  // the halves of the split below
+        const int gap = fx_shared_gap(sa.gap, sb.gap);
+        sa.bit += gap;
+        sb.bit += gap;
+        for (int x = lane; x < Nx; x += 32) bufA[x] = fxc{fx_from_double(raw[x].x, sa), fx_from_double(raw[x].y, sb)};
         __syncwarp();
-        const fxc* r = fx_lines<false, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, Nx, tw);
+        const fxc* r = fx_all_stages<false, true, LATE>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, Nx, tw, nullptr, gap);
         double2* o = pspec + ((static_cast<size_t>(z) * nch + c) * Ny + y) * KX;
         for (int k = lane; k < KX; k += 32) {
             const fxc a = r[k], b = r[k == 0 ? 0 : Nx - k];
@@ -260,7 +281,7 @@ inline size_t smem_fx_any_z(int N, int lines, int warps) {
 }
 
 // k_vinv_fx for any length, one retained column per warp.
-template <bool FLUX>
+template <bool FLUX, bool LATE>
 __global__ void __launch_bounds__(32 * kFxAnyWarps)
     k_vinv_fxany(DescDev d, const double* __restrict__ Ap, const double* __restrict__ Am, const double* __restrict__ A0,
                  double elapsed, double2* __restrict__ zspec, unsigned long long* __restrict__ maxSpeedBits) {
@@ -295,15 +316,20 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
     if constexpr (FLUX)
         for (int q = 0; q < d.nt; ++q) derivChan[d.tq[q]] = 4 + q;
     auto count = [](int j) { return j == 0 ? 1.0f : 2.0f; };
+    __shared__ int gaps[kFxAnyWarps][kLines];
     int uC[kLines], uD[kLines];
 #pragma unroll
     for (int l = 0; l < kLines; ++l) {
         const int qc = l, qs = l < 2 ? l + 2 : l - 2;
         auto atC = [&](int j) { const double2 v = fld[qc * Nj + j]; const double m = l < 2 ? 1.0 : mz[j]; return make_double2(m * v.x, m * v.y); };
         auto atD = [&](int j) { const double2 v = fld[qs * Nj + j]; const double m = l < 2 ? 1.0 : -mz[j]; return make_double2(m * v.x, m * v.y); };
-        fxscale sC = fx_warp_scale(Nj, lane, atC, count), sD = fx_warp_scale(Nj, lane, atD, count);
+        const int radix = LATE ? d.fz.radix[0] : 0;
+        fxscale sC = fx_warp_scale(Nj, lane, radix, atC, count), sD = fx_warp_scale(Nj, lane, radix, atD, count);
         sC.bit -= 1; sD.bit -= 1;
         uC[l] = fx_unit(sC); uD[l] = fx_unit(sD);
+        const int gap = fx_shared_gap(sC.gap, sD.gap);
+        if (LATE && lane == 0) gaps[warp][l] = gap;
+        sC.bit += gap; sD.bit += gap;
         // 2 y[j] = C_j + i D_j, 2 y[N-j] = C_j - i D_j, 2 y[0] = C_0; nothing between
         fxc* y = bufA + l * N;
         for (int j = lane; j < Nj; j += 32) {
@@ -317,7 +343,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         for (int k = Nj + lane; k <= N - Nj; k += 32) y[k] = fxc{0, 0};
     }
     __syncwarp();
-    const fxc* F = fx_lines<false, true>(bufA, bufB, FxFactors{d.fz.N, d.fz.nstages, d.fz.radix}, kLines, N, tw);
+    const fxc* F = fx_all_stages<false, true, LATE>(bufA, bufB, FxFactors{d.fz.N, d.fz.nstages, d.fz.radix}, kLines, N, tw, gaps[warp], 0);
     const int pos = d.modePos[mode], cpos = d.modeCompPos[mode];
 #pragma unroll
     for (int l = 0; l < kLines; ++l) {
@@ -342,7 +368,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
 }
 
 // k_vfwd_fx for any length, one retained column per warp.
-template <bool FLUX>
+template <bool FLUX, bool LATE>
 __global__ void __launch_bounds__(32 * kFxAnyWarps)
     k_vfwd_fxany(DescDev d, const double2* __restrict__ fspec, int nch, double elapsed, const double* __restrict__ Ap,
                  const double* __restrict__ Am, const double* __restrict__ A0, const unsigned long long* __restrict__ maxSpeedBits,
@@ -370,6 +396,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
     int chanOfQ[4] = {-1, -1, -1, -1};
     for (int c = 0; c < nch; ++c) chanOfQ[FLUX ? d.tq[c] : ((d.hydrostatic && c == 2) ? 3 : c)] = c;
     auto count = [L](int z) { return z == 0 || z == L ? 1.0f : 2.0f; };
+    __shared__ int gaps[kFxAnyWarps][2];
     int uC[2], uS[2];
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
@@ -381,10 +408,14 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         for (int z = 1 + lane; z < L; z += 32)
             rs[z] = cs >= 0 ? fspec[(static_cast<size_t>(cs) * d.zTotal + z) * P + pos] : make_double2(0.0, 0.0);
         __syncwarp();
-        fxscale sC = fx_warp_scale(L + 1, lane, [&](int z) { return rc[z]; }, count);
-        fxscale sS = fx_warp_scale(L, lane, [&](int z) { return z == 0 ? make_double2(0.0, 0.0) : rs[z]; }, count);
+        const int radix = LATE ? d.fz.radix[0] : 0;
+        fxscale sC = fx_warp_scale(L + 1, lane, radix, [&](int z) { return rc[z]; }, count);
+        fxscale sS = fx_warp_scale(L, lane, radix, [&](int z) { return z == 0 ? make_double2(0.0, 0.0) : rs[z]; }, count);
         sC.bit -= 1; sS.bit -= 1;
         uC[l] = fx_unit(sC); uS[l] = fx_unit(sS);
+        const int gap = fx_shared_gap(sC.gap, sS.gap);
+        if (LATE && lane == 0) gaps[warp][l] = gap;
+        sC.bit += gap; sS.bit += gap;
         fxc* y = bufA + l * N;
         for (int z = lane; z <= L; z += 32) {
             const double2 cv = rc[z];
@@ -397,7 +428,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         }
     }
     __syncwarp();
-    const fxc* F = fx_lines<false, true>(bufA, bufB, FxFactors{d.fz.N, d.fz.nstages, d.fz.radix}, 2, N, tw);
+    const fxc* F = fx_all_stages<false, true, LATE>(bufA, bufB, FxFactors{d.fz.N, d.fz.nstages, d.fz.radix}, 2, N, tw, gaps[warp], 0);
     double maxSpeed = 0.0;
     if (FLUX && applyDamping) maxSpeed = __longlong_as_double((long long)*maxSpeedBits);
     const double sc = 1.0 / (static_cast<double>(L) * static_cast<double>(d.Nx) * static_cast<double>(d.Ny));

@@ -1,5 +1,5 @@
 // The x pass of the FP64 flux in fixed point for row lengths without a lane-held
-// line (wv_fxwarp.cuh): the same arithmetic with run-time stages (fx_lines) over
+// line (wv_fxwarp.cuh): the same arithmetic with run-time stages (fx_all_stages) over
 // one warp's lines in shared memory, one warp per (y, z) row.
 #pragma once
 
@@ -20,31 +20,65 @@ __host__ __device__ inline size_t fx_xany_warp_bytes(int Nx, int nt, int pairs) 
     return (static_cast<size_t>(Nx) * (32 * pairs + 24 + 8 * nt) + 15) / 16 * 16;
 }
 
-// One spectrum row in fixed point, held by a warp: entries k = lane + 32 i (0
-// from KX on); unit as fx_unit.
+// Two spectrum rows in fixed point, held by a warp: entries k = lane + 32 i (0 from KX
+// on; a null row: zeros), units as fx_unit, `gap` the bits by which their line starts finer.
 template <int EK>
-__device__ __forceinline__ void fx_load_row(const double2* __restrict__ h, int KX, int Nx, int lane, bool useK,
-                                            const double* __restrict__ rowK, fxc (&row)[EK], int& unit) {
-    double2 v[EK];
+__device__ __forceinline__ void fx_load_rows(const double2* __restrict__ hA, const double2* __restrict__ hB, bool kA, bool kB,
+                                             int KX, int Nx, int radix, int lane, const double* __restrict__ rowK, fxc (&A)[EK],
+                                             fxc (&B)[EK], int& unitA, int& unitB, int& gap) {
+    constexpr int radix1 = EK > 2 ? 1 : 0;  // (64 columns and fewer: no rows past kFxLateFrom)
+    double2 v[2][EK];
     double w[EK];
-#pragma unroll
-    for (int i = 0; i < EK; ++i) {
-        const int k = lane + 32 * i;
-        v[i] = k < KX ? h[k] : make_double2(0.0, 0.0);
-        if (k == 0 || 2 * k == Nx) v[i].y = 0.0;  // c2r semantics
-        w[i] = useK && k < KX ? rowK[k] : 0.0;
-    }
+    FxLine l[2];
     auto count = [&](int i) { const int k = lane + 32 * i; return k == 0 || 2 * k == Nx ? 1.0f : 2.0f; };
-    if (useK) {
-        fx_quantise_lane<EK, 32, kFxImag, 0>(v, w, fx_row_k_top(rowK, KX), 1, count, row, unit);
+    auto weights = [&]() {
 #pragma unroll
-        for (int i = 0; i < EK; ++i)
-            if (2 * (lane + 32 * i) == Nx) row[i].y = 0;
-    } else {
-        fx_quantise_lane<EK, 32, kFxPlain, 0>(v, w, 0u, 1, count, row, unit);
+        for (int i = 0; i < EK; ++i) w[i] = lane + 32 * i < KX ? rowK[lane + 32 * i] : 0.0;
+    };
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const double2* h = q ? hB : hA;
+#pragma unroll
+        for (int i = 0; i < EK; ++i) {
+            const int k = lane + 32 * i;
+            v[q][i] = h && k < KX ? h[k] : make_double2(0.0, 0.0);
+            if (k == 0 || 2 * k == Nx) v[q][i].y = 0.0;  // c2r semantics
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if (q ? kB : kA) {
+            weights();
+            l[q] = fx_line<EK, 32, kFxImag, radix1, 0>(v[q], w, fx_row_k_top(rowK, KX), 1, count);
+        } else {
+            l[q] = fx_line<EK, 32, kFxPlain, radix1, 0>(v[q], w, 0u, 1, count);
+        }
+    }
+    // (fx_line's gap is against one entry; the first stage adds `radix` of them)
+    gap = radix1 && Nx > kFxLateFrom ? max(0, fx_shared_gap(l[0].gap, l[1].gap) - fx_ceil_log2(radix)) : 0;
+    unitA = l[0].unit;
+    unitB = l[1].unit;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        fxc(&row)[EK] = q ? B : A;
+        if (q ? kB : kA) {
+            weights();
+            fx_fixed<EK, kFxImag>(v[q], w, l[q].base - gap, row);
+#pragma unroll
+            for (int i = 0; i < EK; ++i)
+                if (2 * (lane + 32 * i) == Nx) row[i].y = 0;
+        } else {
+            fx_fixed<EK, kFxPlain>(v[q], w, l[q].base - gap, row);
+        }
     }
 }
 
+// Rows of x past kFxLateFrom points have more than 64 columns (EK > 2) or keep no gap.
+template <int EK, bool INV>
+__device__ inline fxc* fx_row_stages(fxc* a, fxc* b, const FxFactors f, int lines, const fxw* tw, int gap) {
+    if (EK > 2 && f.N > kFxLateFrom) return fx_all_stages<INV, true, (EK > 2)>(a, b, f, lines, f.N, tw, nullptr, gap);
+    return fx_all_stages<INV, true, false>(a, b, f, lines, f.N, tw, nullptr, 0);
+}
 // Z = A + i B and its mirror into the line (every entry of it written).
 template <int EK>
 __device__ __forceinline__ void fx_pack_rows(const fxc (&A)[EK], const fxc (&B)[EK], fxc* __restrict__ line, int KX, int Nx,
@@ -96,33 +130,30 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
         for (int p0 = 0; 2 * p0 < nReal; p0 += pairs) {
             const int np = min(pairs, (nReal + 1) / 2 - p0);
             int units = 0;  // lane 2 i (2 i + 1) keeps the unit of row A (B) of pair i
+            int gap = 0;    // (rows past kFxLateFrom: one pair a batch)
             for (int i = 0; i < np; ++i) {
                 fxc A[EK], B[EK];
                 int uA, uB;
-                auto load = [&](int r, fxc (&out)[EK], int& u) {
-                    if (r >= nReal) {
-#pragma unroll
-                        for (int e = 0; e < EK; ++e) out[e] = fxc{0, 0};
-                        u = 0;
-                        return;
-                    }
+                bool useK[2] = {false, false};
+                auto spectrum = [&](int q) -> const double2* {
+                    const int r = 2 * (p0 + i) + q;
+                    if (r >= nReal) return nullptr;
                     int ch = r;
-                    bool useK = false;
                     if (r >= 3) {
                         const int t = (r - 3) / 3, kind = (r - 3) - 3 * t;
-                        useK = kind == 0;
+                        useK[q] = kind == 0;
                         ch = kind == 0 ? d.tq[t] : kind == 1 ? 4 + t : 4 + nt + t;
                     }
-                    fx_load_row<EK>(yrow + ch * cstride, KX, Nx, lane, useK, rowK, out, u);
+                    return yrow + ch * cstride;
                 };
-                load(2 * (p0 + i), A, uA);
-                load(2 * (p0 + i) + 1, B, uB);
+                const double2 *hA = spectrum(0), *hB = spectrum(1);
+                fx_load_rows<EK>(hA, hB, useK[0], useK[1], KX, Nx, f.radix[0], lane, rowK, A, B, uA, uB, gap);
                 if (lane == 2 * i) units = uA;
                 if (lane == 2 * i + 1) units = uB;
                 fx_pack_rows<EK>(A, B, bufA + i * Nx, KX, Nx, lane);
             }
             __syncwarp();
-            const fxc* res = fx_lines<true, true>(bufA, bufB, fac, np, Nx, tw);
+            const fxc* res = fx_row_stages<EK, true>(bufA, bufB, fac, np, tw, gap);
             const long long* real = reinterpret_cast<const long long*>(res);
             for (int i = 0; i < 2 * np; ++i) {
                 const int r = 2 * p0 + i;
@@ -203,21 +234,30 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
         // r2c of the products, two targets to a line
         for (int t0 = 0; t0 < nt; t0 += 2 * pairs) {
             const int nl = min(pairs, (nt - t0 + 1) / 2);
-            int units = 0;
+            int units = 0, gap = 0;
             for (int i = 0; i < nl; ++i) {
                 int sh[2] = {0, 0};
+                gap = EK > 2 && Nx > kFxLateFrom ? kFxAnyGap : 0;
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int t = t0 + 2 * i + q;
                     if (t >= nt) continue;
-                    unsigned sum = 0;
-                    for (int x = lane; x < Nx; x += 32)
-                        sum += static_cast<unsigned>(static_cast<unsigned long long>(fx_abs(S[t * Nx + x])) >> 41) + 1u;
+                    unsigned sum = 0, most = 0;
+                    for (int x = lane; x < Nx; x += 32) {
+                        const unsigned m = static_cast<unsigned>(static_cast<unsigned long long>(fx_abs(S[t * Nx + x])) >> 41) + 1u;
+                        sum += m;
+                        most = max(most, m);
+                    }
                     sum = __reduce_add_sync(0xffffffffu, sum);
-                    sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 60;  // sum |S| < 2^60 after the shift
+                    most = __reduce_max_sync(0xffffffffu, most);
+                    const int bits = 32 - __clz(static_cast<int>(sum));
+                    sh[q] = 41 + bits - 60;  // sum |S| < 2^60 after the shift
+                    gap = min(gap, max(0, bits - (32 - __clz(static_cast<int>(most))) - fx_ceil_log2(f.radix[0])));
                     const int u = (t == 0 ? sUnit[0] : t == 1 ? sUnit[1] : t == 2 ? sUnit[2] : sUnit[3]) + sh[q] - 1;
                     if (lane == 2 * i + q) units = u;
                 }
+                sh[0] -= gap;
+                sh[1] -= gap;
                 const long long* a = S + (t0 + 2 * i) * Nx;
                 const bool both = t0 + 2 * i + 1 < nt;
                 for (int x = lane; x < Nx; x += 32) {
@@ -228,7 +268,7 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                 }
             }
             __syncwarp();
-            const fxc* res = fx_lines<false, true>(bufA, bufB, fac, nl, Nx, tw);
+            const fxc* res = fx_row_stages<EK, false>(bufA, bufB, fac, nl, tw, gap);
             for (int i = 0; i < nl; ++i) {
                 const int t = t0 + 2 * i;
                 const int ua = __shfl_sync(0xffffffffu, units, 2 * i), ub = __shfl_sync(0xffffffffu, units, 2 * i + 1);

@@ -17,63 +17,14 @@
 namespace wvgpu {
 namespace dev {
 
-template <int N> struct FxW {
-    static constexpr int E = N % 3 == 0 ? 12 : 8;  // points of a lane
-    static constexpr int H = E / 2;
-    static constexpr int G = N / E;                // lanes of a line
-    static constexpr int lines = 32 / G;           // lines of a warp
-    static constexpr int samples = lines * N;      // points of a warp: 32 E
-    static constexpr int buffer = N + N / 8;       // padded line buffer
-    // radices of the stages (their products end with N; R3 = 1: two stages)
-    static constexpr int R1 = E == 8 ? 8 : N == 24 ? 2 : 4;
-    static constexpr int R2 = E == 8 ? (N == 16 ? 2 : (N == 32 || N == 128) ? 4 : 8) : N == 96 ? 2 : N == 192 ? 4 : 12;
-    static constexpr int R3 = N / (R1 * R2);
-    static constexpr int twiddles = (R2 - 1) * R1 + (R3 - 1) * R1 * R2;
-};
-__device__ __forceinline__ int fx_pad(int i) { return i + (i >> 3); }
-
-// Stage of radix R behind Ns points already combined; tw[(r - 1) Ns + k].
-template <int N, int R, int Ns, bool INV>
-__device__ __forceinline__ void fx_wstage(fxc (&v)[FxW<N>::E], const fxw* __restrict__ tw, int t, int two) {
-    constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-        const int k = (t + G * b) & (Ns - 1);  // (Ns is a power of two)
-        fxc u[R];
-        u[0] = v[b];
-#pragma unroll
-        for (int r = 1; r < R; ++r) u[r] = Ns == 1 ? v[b + B * r] : fx_cmul60<INV>(v[b + B * r], tw[(r - 1) * Ns + k], two);
-        fx_dft<R, INV>(u);
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[b + B * r] = u[r];
-    }
-}
-// v[b + B r], the outputs of a stage of radix R, to their places and back to lane order
-template <int N, int R, int Ns>
-__device__ __forceinline__ void fx_wexchange(fxc (&v)[FxW<N>::E], fxc* __restrict__ x, int t) {
-    constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-        const int j = t + G * b, k = j & (Ns - 1), jq = j / Ns;
-#pragma unroll
-        for (int r = 0; r < R; ++r) x[fx_pad(jq * Ns * R + k + r * Ns)] = v[b + B * r];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < FxW<N>::E; ++e) v[e] = x[fx_pad(t + G * e)];
-    __syncwarp();
-}
-// The whole line (sum of moduli below 2^60); x: this line's buffer, tw: the stage twiddles in shared memory.
-template <int N, bool INV>
-__device__ __forceinline__ void fx_fft_warp(fxc (&v)[FxW<N>::E], fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two) {
-    using W = FxW<N>;
-    fx_wstage<N, W::R1, 1, INV>(v, tw, t, two);
-    fx_wexchange<N, W::R1, 1>(v, x, t);
-    fx_wstage<N, W::R2, W::R1, INV>(v, tw, t, two);
-    if constexpr (W::R3 > 1) {
-        fx_wexchange<N, W::R2, W::R1>(v, x, t);
-        fx_wstage<N, W::R3, W::R1 * W::R2, INV>(v, tw + (W::R2 - 1) * W::R1, t, two);
-    }
+// A line by its lanes (fx_line_stages).
+template <int N, bool INV, int LATE = 0>
+__device__ __forceinline__ void fx_fft_warp(fxc (&v)[FxW<N>::E], fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two,
+                                            int gap = 0) {
+    fx_line_stages<N, INV, LATE>(x, tw, two, gap, [&](auto step) {
+        step(v, t);
+        __syncwarp();
+    });
 }
 
 // maxima and sums over the lanes of a line
@@ -113,21 +64,27 @@ __device__ __forceinline__ unsigned fx_row_k_top(const double* __restrict__ rowK
     return static_cast<unsigned>(max(__double2hiint(rowK[KX - 1]), __double2hiint(rowK[max(KX - 2, 0)])));
 }
 
-// C doubles of a lane, weighted, in the fixed point of their line.  count(c): how
-// often entry c enters the line's sum of moduli; spare: bits kept free (1 when two
-// rows share the line); wtop: high word of the largest |w|.
-template <int C, int G, FxWeight MODE, int FRAME = 1, typename Count>
-__device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const double (&w)[C], unsigned wtop, int spare,
-                                                 Count count, fxc (&out)[C], int& unit) {
-    float sum = 0.f;
+// How a line's entries become fixed point: shift base less the entry's exponents (less
+// `gap` where the line starts finer), and the unit they end with.
+struct FxLine { int base, unit, gap; };
+
+// Of the line whose C entries a lane holds, weighted.  count(c): how often entry c enters
+// the sum of moduli; spare: bits kept free (1 when two rows share the line); wtop: high
+// word of the largest |w|; RADIX: that of the first stage where the line may start finer.
+template <int C, int G, FxWeight MODE, int RADIX = 0, int FRAME = 1, typename Count>
+__device__ __forceinline__ FxLine fx_line(const double2 (&v)[C], const double (&w)[C], unsigned wtop, int spare, Count count) {
+    float sum = 0.f, most = 0.f;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         float m = fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v[c].x))),
                              fx_mag(static_cast<unsigned>(__double2hiint(v[c].y))));
         if (MODE != kFxPlain) m *= fx_mag(static_cast<unsigned>(__double2hiint(w[c])));
         sum += count(c) * m;
+        if (RADIX) most = fmaxf(most, m);
     }
     sum = fx_group_sum<G>(sum);
+    int gap = 0;
+    if (RADIX) gap = fx_gap(sum, __uint_as_float(fx_group_max<G>(__float_as_uint(most))), RADIX);
     fxscale sc = fx_scale(sum);
     int wexp = 0;
     bool zero = false;
@@ -139,24 +96,30 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
             top = max(top, max(static_cast<unsigned>(__double2hiint(v[c].x)) & 0x7fffffffu,
                                static_cast<unsigned>(__double2hiint(v[c].y)) & 0x7fffffffu));
         top = fx_group_max<G>(top);
-        float rel = 0.f;
+        float rel = 0.f, relMost = 0.f;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             float m = fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v[c].x)), top),
                                  fx_rel(static_cast<unsigned>(__double2hiint(v[c].y)), top));
             if (MODE != kFxPlain) m *= fx_rel(static_cast<unsigned>(__double2hiint(w[c])), wtop) * 1.00001f;
             rel += count(c) * m;
+            if (RADIX) relMost = fmaxf(relMost, m);
         }
         rel = fx_group_sum<G>(rel);
+        if (RADIX) relMost = __uint_as_float(fx_group_max<G>(__float_as_uint(relMost)));
         if (odd) {
             sc = fx_scale(top, rel);
             zero = top == 0 || (MODE != kFxPlain && wtop == 0 && sc.e0 < 0x7ff);
+            gap = zero ? kFxAnyGap : RADIX ? fx_gap(rel, relMost, RADIX) : 0;
             if (MODE != kFxPlain) wexp = static_cast<int>((wtop >> 20) & 0x7ffu) - 1023;
         }
     }
     sc.bit -= spare + FRAME;
-    unit = zero ? kFxZero : sc.e0 >= 0x7ff ? kFxBad : sc.e0 + wexp - sc.bit;
-    const int base = 61 - sc.bit + sc.e0;
+    return {61 - sc.bit + sc.e0 + (MODE != kFxPlain ? wexp + 1022 : 0),
+            zero ? kFxZero : sc.e0 >= 0x7ff ? kFxBad : sc.e0 + wexp - sc.bit, gap};
+}
+template <int C, FxWeight MODE>
+__device__ __forceinline__ void fx_fixed(const double2 (&v)[C], const double (&w)[C], int base, fxc (&out)[C]) {
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         int ex, ey;
@@ -168,8 +131,7 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
             const int sw = __double2hiint(w[c]);
             mx = __umul64hi(mx, mw);  // 2^(e + ew - 1022) at bit 62
             my = __umul64hi(my, mw);
-            const int b2 = base + wexp + 1022 - ew;
-            const long long wx = fx_shift_in(mx, b2 - ex, sx ^ sw), wy = fx_shift_in(my, b2 - ey, sy ^ sw);
+            const long long wx = fx_shift_in(mx, base - ew - ex, sx ^ sw), wy = fx_shift_in(my, base - ew - ey, sy ^ sw);
             out[c] = MODE == kFxImag ? fxc{-wy, wx} : fxc{wx, wy};
         } else {
             out[c].x = fx_shift_in(mx, base - ex, sx);
@@ -177,11 +139,21 @@ __device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const do
         }
     }
 }
+// Both for a line that doesn't start finer.
+template <int C, int G, FxWeight MODE, typename Count>
+__device__ __forceinline__ void fx_quantise_lane(const double2 (&v)[C], const double (&w)[C], unsigned wtop, int spare, Count count,
+                                                 fxc (&out)[C], int& unit) {
+    const FxLine l = fx_line<C, G, MODE>(v, w, wtop, spare, count);
+    fx_fixed<C, MODE>(v, w, l.base, out);
+    unit = l.unit;
+}
+// Two rows or channels of a line: both start finer by the smaller gap.
+__device__ __forceinline__ int fx_shared_gap(int a, int b) { return min(a, b); }
 
 // ---------------------------------------------------------------------------
 // x pass of the FP64 flux: c2r of the velocities and of every derivative, the
-// quadratic products and their r2c.  Two real rows share one complex line (Z = A + i B for the c2r,
-// S_a + i S_b for the r2c); each row keeps its own scale, so its rounding stays
+// quadratic products and their r2c.  Two real rows share one complex line (Z = A + i B
+// for the c2r, S_a + i S_b for the r2c); each row keeps its own scale, so its rounding stays
 // relative to its own magnitude whatever its partner holds.  Products are formed as
 // (a b) >> 62 on velocities normalised to 62 bits and added at the largest unit of
 // a target's three.
@@ -213,7 +185,7 @@ template <int N, int EK>
 __device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __restrict__ yrow, size_t cstride,
                                              const double* __restrict__ rowK, unsigned wtop, int p, int nReal, fxc* __restrict__ x,
                                              int t, fxc (&v)[FxW<N>::E], int (&unit)[2]) {
-    constexpr int G = FxW<N>::G, E = FxW<N>::E, H = E / 2;
+    constexpr int G = FxW<N>::G, E = FxW<N>::E;
     const int KX = d.kxColumns, nt = d.nt;
     // rows 2p and 2p + 1: spectrum entries k = t + G i, both rows' loads in flight
     double2 raw[2][EK];
@@ -227,51 +199,51 @@ __device__ __forceinline__ void fx_load_pair(const DescDev& d, const double2* __
             if (kind == 0) weighted |= 1 << q;
             ch = kind == 0 ? d.tq[tt & 3] : kind == 1 ? 4 + tt : 4 + nt + tt;
         }
-                        const double2* h = yrow + ch * cstride;
-    #pragma unroll
-                        for (int i = 0; i < EK; ++i) {
-                            const int k = t + G * i;
-                            raw[q][i] = k < KX && r < nReal ? h[k] : make_double2(0.0, 0.0);
-                        }
-                        if (t == 0) raw[q][0].y = 0.0;  // c2r semantics
-                    }
-                    fxc A[EK], B[EK];
-                    auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
-    #pragma unroll 1
-                    for (int q = 0; q < 2; ++q) {  // one copy of the code: it must stay in the instruction cache
-                        double2 a[EK];
-                        double w[EK];
-    #pragma unroll
-                        for (int i = 0; i < EK; ++i) {
-                            a[i] = q ? raw[1][i] : raw[0][i];
-                            A[i] = B[i];
-                        }
-                        int u;
-                        if ((weighted >> q) & 1) {
-    #pragma unroll
-                            for (int i = 0; i < EK; ++i) w[i] = t + G * i < KX ? rowK[t + G * i] : 0.0;
-                            fx_quantise_lane<EK, G, kFxImag>(a, w, wtop, 1, count, B, u);
-                        } else {
-                            fx_quantise_lane<EK, G, kFxPlain>(a, w, 0u, 1, count, B, u);
-                        }
-                        unit[0] = unit[1];
-                        unit[1] = u;
-                    }
-                    // Z = A + i B at k and its mirror at N - k; nothing between
-    #pragma unroll
-                    for (int i = 0; i < EK; ++i) {
-                        const fxc a = A[i], b = B[i];
-                        v[i] = fxc{a.x - b.y, a.y + b.x};
-                        const int k = t + G * i;
-                        const fxc m = {a.x + b.y, b.x - a.y};
-                        x[fx_pad(k == 0 ? N - G * EK : N - k)] = k == 0 ? fxc{0, 0} : m;
-                    }
-    #pragma unroll
-                    for (int e = EK; e < E - EK; ++e) v[e] = fxc{0, 0};
-                    __syncwarp();
-    #pragma unroll
-                    for (int e = E - EK; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
-                    __syncwarp();
+        const double2* h = yrow + ch * cstride;
+#pragma unroll
+        for (int i = 0; i < EK; ++i) {
+            const int k = t + G * i;
+            raw[q][i] = k < KX && r < nReal ? h[k] : make_double2(0.0, 0.0);
+        }
+        if (t == 0) raw[q][0].y = 0.0;  // c2r semantics
+    }
+    fxc A[EK], B[EK];
+    auto count = [&](int i) { return i == 0 && t == 0 ? 1.0f : 2.0f; };
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {  // one copy of the code: it must stay in the instruction cache
+        double2 a[EK];
+        double w[EK];
+#pragma unroll
+        for (int i = 0; i < EK; ++i) {
+            a[i] = q ? raw[1][i] : raw[0][i];
+            A[i] = B[i];
+        }
+        int u;
+        if ((weighted >> q) & 1) {
+#pragma unroll
+            for (int i = 0; i < EK; ++i) w[i] = t + G * i < KX ? rowK[t + G * i] : 0.0;
+            fx_quantise_lane<EK, G, kFxImag>(a, w, wtop, 1, count, B, u);
+        } else {
+            fx_quantise_lane<EK, G, kFxPlain>(a, w, 0u, 1, count, B, u);
+        }
+        unit[0] = unit[1];
+        unit[1] = u;
+    }
+    // Z = A + i B at k and its mirror at N - k; nothing between
+#pragma unroll
+    for (int i = 0; i < EK; ++i) {
+        const fxc a = A[i], b = B[i];
+        v[i] = fxc{a.x - b.y, a.y + b.x};
+        const int k = t + G * i;
+        const fxc m = {a.x + b.y, b.x - a.y};
+        x[fx_pad(k == 0 ? N - G * EK : N - k)] = k == 0 ? fxc{0, 0} : m;
+    }
+#pragma unroll
+    for (int e = EK; e < E - EK; ++e) v[e] = fxc{0, 0};
+    __syncwarp();
+#pragma unroll
+    for (int e = E - EK; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
+    __syncwarp();
 }
 
 // Scale of a caller's velocity row, largest high word `top`: its leading bit at 61.
@@ -283,7 +255,7 @@ template <int N>
 __device__ __forceinline__ int fx_velocity(const long long (&smp)[FxW<N>::E], int unit, int t, long long* __restrict__ phys,
                                            const double* __restrict__ advIn, double* __restrict__ advOut,
                                            double* __restrict__ keep) {
-    constexpr int G = FxW<N>::G, E = FxW<N>::E, H = E / 2;
+    constexpr int G = FxW<N>::G, E = FxW<N>::E;
     unsigned top = 0;
     if (advIn) {
         double a[E];
@@ -323,26 +295,37 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
                                                 int unitB, fxc* __restrict__ x, const fxw* __restrict__ tw, int t, int two,
                                                 int KX, double2* __restrict__ out, size_t cstride) {
     constexpr int G = FxW<N>::G, E = FxW<N>::E, H = E / 2;
+    using W = FxW<N>;
     const bool both = Sb != nullptr;
     fxc v[E];
-    int sh[2], u[2];
+    int sh[2], u[2], gap = kFxAnyGap;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-        unsigned sum = 0;
+        unsigned sum = 0, most = 0;
         if (q == 0 || both)
 #pragma unroll
-            for (int e = 0; e < E; ++e) sum += (fx_abs_hi((q ? Sb : Sa)[t + G * e]) >> 9) + 1u;
+            for (int e = 0; e < E; ++e) {
+                const unsigned m = (fx_abs_hi((q ? Sb : Sa)[t + G * e]) >> 9) + 1u;
+                sum += m;
+                if (W::latePair) most = max(most, m);
+            }
         sum = fx_group_add<G>(sum);
-        sh[q] = 41 + (32 - __clz(static_cast<int>(sum))) - 59;  // sum |S| < 2^59 after the shift
-        u[q] = (q ? unitB : unitA) + sh[q] - 1;                 // the halves of the split below
+        const int bits = 32 - __clz(static_cast<int>(sum));
+        sh[q] = 41 + bits - 59;                  // sum |S| < 2^59 after the shift
+        u[q] = (q ? unitB : unitA) + sh[q] - 1;  // the halves of the split below
+        if (W::latePair && (q == 0 || both))
+            gap = fx_shared_gap(gap, max(0, bits - (32 - __clz(static_cast<int>(fx_group_max<G>(most) * W::R1)))));
     }
+    if (!W::latePair) gap = 0;
+    sh[0] -= gap;
+    sh[1] -= gap;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const long long a = Sa[t + G * e], b = both ? Sb[t + G * e] : 0;
         v[e].x = fx_shift_round(a, sh[0], t & 1);
         v[e].y = fx_shift_round(b, sh[1], t & 1);
     }
-    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(unitA, both ? unitB : unitA)) ? 0 : two);
+    fx_fft_warp<N, false, W::latePair>(v, x, tw, t, fx_silent(max(unitA, both ? unitB : unitA)) ? 0 : two, gap);
     __syncwarp();
 #pragma unroll
     for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
@@ -380,7 +363,7 @@ __global__ void __launch_bounds__(32 * kFxCoWarps, FxW<N>::E == 8 ? 3 : 2)
                  unsigned long long* __restrict__ maxSpeedBits, double* __restrict__ physOut, double* __restrict__ advOut,
                  const double* __restrict__ advIn) {
     using W = FxW<N>;
-    constexpr int G = W::G, E = W::E, H = W::H;
+    constexpr int G = W::G, E = W::E;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int rowUnit[16][W::lines], sUnit[4][W::lines];
     __shared__ FxAlign align[2][12][W::lines];  // [odd sample][target, kind][line]

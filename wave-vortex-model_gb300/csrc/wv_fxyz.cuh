@@ -28,7 +28,7 @@ template <int N>
 __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     k_yinv_fx(DescDev d, YInvMap map, const double2* __restrict__ zspec, double2* __restrict__ yspec, unsigned ltop) {
     using W = FxW<N>;
-    constexpr int G = W::G, E = W::E, H = W::H;
+    constexpr int G = W::G, E = W::E;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = d.positions, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
@@ -81,7 +81,7 @@ template <int N>
 __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     k_yfwd_fx(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec) {
     using W = FxW<N>;
-    constexpr int G = W::G, E = W::E, H = W::H;
+    constexpr int G = W::G, E = W::E;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = d.positions, KX = d.kxColumns;
     const int lane = threadIdx.x & 31, t = lane % G, own = (threadIdx.x >> 5) * W::lines + lane / G;
@@ -103,10 +103,11 @@ __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     for (int e = 0; e < E; ++e) a[e] = tile[fx_tile(t + G * e, own, cols)];
     __syncthreads();  // the line buffers take the tile's place
     fxc v[E];
-    int unit;
     double w[E];
-    fx_quantise_lane<E, G, kFxPlain>(a, w, 0u, 0, [](int) { return 1.0f; }, v, unit);
-    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two());
+    const FxLine l = fx_line<E, G, kFxPlain, W::lateOne ? W::R1 : 0>(a, w, 0u, 0, [](int) { return 1.0f; });
+    fx_fixed<E, kFxPlain>(a, w, l.base - l.gap, v);
+    const int unit = l.unit;
+    fx_fft_warp<N, false, W::lateOne>(v, x, tw, t, fx_silent(unit) ? 0 : fx_two(), l.gap);
     const int kx = kx0 + own;
     if (kx >= KX) return;
     double2* out = fspec + (static_cast<size_t>(ch) * d.zTotal + z) * P;
@@ -118,13 +119,19 @@ __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     }
 }
 
-// Real values of a lane (E a row) in the fixed point of their row, for two rows to a line.
-template <int E, int G>
-__device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long (&out)[E], int& unit) {
-    float sum = 0.f;
+// Real values of a lane (E a row), for two rows to a line (as fx_line and fx_fixed).
+template <int E, int G, int RADIX>
+__device__ __forceinline__ FxLine fx_real_line(const double (&a)[E]) {
+    float sum = 0.f, most = 0.f;
 #pragma unroll
-    for (int e = 0; e < E; ++e) sum += fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
+    for (int e = 0; e < E; ++e) {
+        const float m = fx_mag(static_cast<unsigned>(__double2hiint(a[e])));
+        sum += m;
+        if (RADIX) most = fmaxf(most, m);
+    }
     sum = fx_group_sum<G>(sum);
+    int gap = 0;
+    if (RADIX) gap = fx_gap(sum, __uint_as_float(fx_group_max<G>(__float_as_uint(most))), RADIX);
     fxscale sc = fx_scale(sum);
     const bool odd = !fx_plain_sum(sum);
     if (__any_sync(0xffffffffu, odd)) {
@@ -132,16 +139,46 @@ __device__ __forceinline__ void fx_quantise_real(const double (&a)[E], long long
 #pragma unroll
         for (int e = 0; e < E; ++e) top = max(top, static_cast<unsigned>(__double2hiint(a[e])) & 0x7fffffffu);
         top = fx_group_max<G>(top);
-        float rel = 0.f;
+        float rel = 0.f, relMost = 0.f;
 #pragma unroll
-        for (int e = 0; e < E; ++e) rel += fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
+        for (int e = 0; e < E; ++e) {
+            const float m = fx_rel(static_cast<unsigned>(__double2hiint(a[e])), top);
+            rel += m;
+            relMost = fmaxf(relMost, m);
+        }
         rel = fx_group_sum<G>(rel);
-        if (odd) sc = fx_scale(top, rel);
+        if (RADIX) relMost = __uint_as_float(fx_group_max<G>(__float_as_uint(relMost)));
+        if (odd) {
+            sc = fx_scale(top, rel);
+            gap = top == 0 ? kFxAnyGap : RADIX ? fx_gap(rel, relMost, RADIX) : 0;
+        }
     }
     sc.bit -= 2;
-    unit = fx_unit(sc);
+    return {61 - sc.bit + sc.e0, fx_unit(sc), gap};
+}
+template <int E>
+__device__ __forceinline__ void fx_real_fixed(const double (&a)[E], int base, long long (&out)[E]) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) out[e] = fx_from_double(a[e], sc);
+    for (int e = 0; e < E; ++e) {
+        int ex;
+        const unsigned long long m = fx_mantissa(a[e], ex);
+        out[e] = fx_shift_in(m, base - ex, __double2hiint(a[e]));
+    }
+}
+// Two real rows of a lane as the line ra + i rb.
+template <int N>
+__device__ __forceinline__ void fx_real_pair(const double (&ra)[FxW<N>::E], const double (&rb)[FxW<N>::E], fxc (&v)[FxW<N>::E],
+                                             int& ua, int& ub, int& gap) {
+    constexpr int E = FxW<N>::E, G = FxW<N>::G, radix = FxW<N>::latePair ? FxW<N>::R1 : 0;
+    long long ia[E], ib[E];
+    const FxLine la = fx_real_line<E, G, radix>(ra), lb = fx_real_line<E, G, radix>(rb);
+    gap = fx_shared_gap(la.gap, lb.gap);
+    ua = la.unit;
+    ub = lb.unit;
+    fx_real_fixed<E>(ra, la.base - gap, ia);
+    fx_real_fixed<E>(rb, lb.base - gap, ib);
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = fxc{ia[e], ib[e]};
 }
 
 // ---- field rows along x -----------------------------------------------------------------
@@ -253,15 +290,11 @@ __global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
         ra[e] = in[t + G * e];
         rb[e] = both ? in[R + t + G * e] : 0.0;
     }
-    long long ia[E], ib[E];
-    int ua, ub;
-    fx_quantise_real<E, G>(ra, ia, ua);
-    fx_quantise_real<E, G>(rb, ib, ub);
     fxc v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = fxc{ia[e], ib[e]};
+    int ua, ub, gap;
+    fx_real_pair<N>(ra, rb, v, ua, ub, gap);
     __syncthreads();  // twiddles
-    fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(ua, ub)) ? 0 : fx_two());
+    fx_fft_warp<N, false, W::latePair>(v, x, tw, t, fx_silent(max(ua, ub)) ? 0 : fx_two(), gap);
 #pragma unroll
     for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
     __syncwarp();
@@ -595,9 +628,12 @@ __global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
             if (i < H) b[i] = cs >= 0 && zz != 0 ? hs[static_cast<size_t>(zz) * P] : make_double2(0.0, 0.0);
         }
         fxc C[H + 1], S[H];
-        int uC, uS;
-        fx_quantise_lane<H + 1, G, kFxPlain>(a, none5, 0u, 1, [&](int i) { return (i == 0 && t == 0) || i == H ? 1.0f : 2.0f; }, C, uC);
-        fx_quantise_lane<H, G, kFxPlain>(b, none4, 0u, 1, [&](int) { return 2.0f; }, S, uS);
+        constexpr int radix = W::latePair ? W::R1 : 0;
+        const FxLine lC = fx_line<H + 1, G, kFxPlain, radix>(a, none5, 0u, 1, [&](int i) { return (i == 0 && t == 0) || i == H ? 1.0f : 2.0f; });
+        const FxLine lS = fx_line<H, G, kFxPlain, radix>(b, none4, 0u, 1, [&](int) { return 2.0f; });
+        const int gap = fx_shared_gap(lC.gap, lS.gap), uC = lC.unit, uS = lS.unit;
+        fx_fixed<H + 1, kFxPlain>(a, none5, lC.base - gap, C);
+        fx_fixed<H, kFxPlain>(b, none4, lS.base - gap, S);
         __syncthreads();  // twiddles
         // y[0] = c_0, y[L] = c_L, y[z] = c_z + s_z, y[N-z] = c_z - s_z
         fxc v[E];
@@ -611,7 +647,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
 #pragma unroll
         for (int e = H; e < E; ++e) v[e] = x[fx_pad(t + G * e)];
         __syncwarp();
-        fx_fft_warp<N, false>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two());
+        fx_fft_warp<N, false, W::latePair>(v, x, tw, t, fx_silent(max(uC, uS)) ? 0 : fx_two(), gap);
         const FxUnit oC = fx_out(uC - 1), oS = fx_out(uS - 1);
 #pragma unroll
         for (int e = H; e < E; ++e) x[fx_pad(t + G * e)] = v[e];
