@@ -1,6 +1,6 @@
 """Where the fixed-point lines of FP64 handles could lose what plain doubles keep:
 advecting velocities that are identically zero, values near both ends of a double's
-range, and lines of several hundred points."""
+range, phases of very small angles, and lines of several hundred points."""
 import numpy as np
 import pytest
 
@@ -77,6 +77,24 @@ def test_values_near_the_ends_of_the_range(wv, shape, power):
     for a, b in zip(k.flux_vjp(300.0, 0.0, *map(dev, A), *u), k.flux_vjp(300.0, 0.0, *map(dev, A), *map(dev, A))):
         a, b = a.cpu().numpy(), b.cpu().numpy()
         assert np.max(np.abs(a / s - b)) <= 1e-13 * np.max(np.abs(b))
+    k.close()
+
+
+@pytest.mark.parametrize("shape", [(32, 48, 17), (20, 18, 11)])
+@pytest.mark.parametrize("angle", [1e-12, 1e-7, 1.9e-3, 1.5e-2, 1.6e-2, 0.3])
+def test_sines_of_small_angles_keep_their_digits(wv, shape, angle):
+    """A wave along x with Ap = -Am has u = 2 i sin(omega t) cos(kx) times its factor: the
+    channel holds nothing but the sine, so its relative error is the sine's."""
+    c, d, A, k = _setup(wv, shape)
+    omega = d.arrays["omega"]
+    l, kk = d.l, d.k
+    mode = int(np.flatnonzero((np.abs(l) == 0.0) & (kk > 0.0))[0])
+    A = [0.0 * a for a in A]
+    A[0][mode, 1], A[1][mode, 1] = 1e-3, -1e-3
+    t = angle / float(omega[mode, 1])
+    f = k.transformWaveVortexToUVWEta(t, 0.0, *A)
+    ref = O.inverse_uvweta(d, *A, t, 0.0)
+    assert np.max(np.abs(f[0] - ref[0])) <= 1e-12 * np.max(np.abs(ref[0]))
     k.close()
 
 

@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
 // exp(i angle) rounded from fixed point: the angle in turns is the exact product of
 // its 53 bits with 1 / (2 pi) to 128 bits, the nearest of 256 table entries is
 // turned by the remainder |r| <= pi / 256 with Taylor sums (sine to r^7, cosine to
-// r^6; the next terms are below 2^-62).  About 170 integer instructions; the FP64
+// r^6; the next terms are below 2^-62).  Angles below 2^-6 rad take the Taylor sums in
+// FP64 (to a^7 and a^6), so that a small sine keeps its digits.  About 170 integer instructions; the FP64
 // sincos it replaces takes some 50 operations of a pipe that retires 1.7 per clock
 // and SM (30 clocks against 1.3 a value).
 __device__ __forceinline__ void fx_phase(double angle, const fxw* __restrict__ table, double& cs, double& sn) {
@@ -327,6 +328,12 @@ __device__ __forceinline__ void fx_phase(double angle, const fxw* __restrict__ t
     const int e = static_cast<int>((hi >> 20) & 0x7ffu);
     if (e >= 1023 + 31) {  // beyond 2^31 rad (and inf, NaN): the library's reduction
         sincos(angle, &sn, &cs);
+        return;
+    }
+    if (e < 1023 - 6) {  // below 2^-6 rad the fixed point's 2^-62 is no longer small against the sine
+        const double q = angle * angle;
+        sn = fma(angle * q, fma(q, fma(q, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), angle);
+        cs = fma(q, fma(q, fma(q, -1.0 / 720.0, 1.0 / 24.0), -0.5), 1.0);
         return;
     }
     const unsigned long long m = static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 |
