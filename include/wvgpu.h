@@ -260,7 +260,9 @@ int wv_inverse_device(wv_handle* handle, double t, double t0,
  * <a, b> = Re sum conj(a) b; a cotangent x_bar of an output x is mapped to the
  * cotangent of the inputs such that <x_bar, dx> = <in_bar, d in> for every
  * perturbation.  Device pointers, [Nj, Nkl] complex unless stated.  The first
- * adjoint call on a handle allocates its adjoint workspace.  The nonlinear
+ * adjoint call on a handle allocates its adjoint workspace, the first flux or step VJP
+ * of an FP64 handle the real rows of its x pass (without memory, or under stream capture,
+ * it runs without them).  The nonlinear
  * advection schedule only (adaptive damping's max|u_h| is not differentiable):
  * handles with adaptive damping enabled return WV_UNSUPPORTED_OPERATION. */
 

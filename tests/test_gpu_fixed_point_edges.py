@@ -1,6 +1,7 @@
 """Where the fixed-point lines of FP64 handles could lose what plain doubles keep:
 advecting velocities that are identically zero, values near both ends of a double's
-range, phases of very small angles, and lines of several hundred points."""
+range, phases of very small angles, and lines of several hundred points; and the memory
+that their VJP takes."""
 import numpy as np
 import pytest
 
@@ -120,4 +121,34 @@ def test_long_lines_against_long_double(wv, extended, shape):  # noqa: F811
           extended.inverse_uvweta(d, *wide, 123.0, 0.0))
     check(k.transformUVWEtaToWaveVortex(fields, 123.0, 0.0), O.forward(d, fields, 123.0, 0.0),
           extended.forward(d, fields.astype(np.longdouble), 123.0, 0.0))
+    k.close()
+
+
+# lane-held and run-time rows
+@pytest.mark.parametrize("shape", [(32, 32, 17), (30, 20, 9)])
+def test_rows_of_the_vjp_are_allocated_when_first_needed(wv, shape):
+    """A VJP of a state transform and a checkpointed adjoint (which keeps rows of its own)
+    do without them; a flux VJP without memory for them gives the same gradient (block
+    kernel against lines: the tolerance of the VJP against FP64's own noise, 1e-11)."""
+    import torch
+    c, d, A, k = _setup(wv, shape)
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()  # noqa: E731
+    state = list(map(dev, A))
+    k.inverse_vjp(10.0, 0.0, dev(np.ones((4, shape[2], shape[1], shape[0]))))
+    ready = k.metrics()["device_bytes"]
+    k._lib.wv_test_fail_allocation_after(0)
+    try:
+        without = k.flux_vjp(10.0, 0.0, *state, *state)
+    finally:
+        k._lib.wv_test_fail_allocation_after(-1)
+    assert k.metrics()["device_bytes"] == ready
+    k.close()
+    c, d, A, k = _setup(wv, shape)
+    k.rk4_adjoint(*state, 0.0, 0.0, 60.0, 2, 1, *state)
+    kept = k.metrics()["device_bytes"]
+    rows = k.flux_vjp(10.0, 0.0, *state, *state)
+    assert k.metrics()["device_bytes"] - kept == 15 * shape[0] * shape[1] * shape[2] * 8
+    for a, b in zip(without, rows):
+        a, b = a.cpu().numpy(), b.cpu().numpy()
+        assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
     k.close()

@@ -70,7 +70,8 @@ struct wv_handle {
     void* yadj = nullptr;   // [z][nt][y][kx]
     void* yout = nullptr;   // [z][4+2nt][y][kx]
     void* fadj = nullptr;   // [4+2nt][z][pos]
-    double* adjRows = nullptr;  // FP64: real rows of the x pass [z][3+3nt][y][Nx]
+    double* adjRows = nullptr;  // FP64: real rows of the x pass [z][3+3nt][y][Nx] (ensure_rows)
+    bool adjRowsRefused = false;
     double* st[4] = {};     // RK4 stage states (st[1..3]) for the step adjoint
     double* kb = nullptr;
     double* sb = nullptr;
@@ -1125,10 +1126,6 @@ int ensure_adjoint(wv_handle* h) {
     if (e == cudaSuccess) e = alloc(h, nIn * p.Nz * p.positions * cb, &h->fadj);
     const size_t stateBytes = 6 * p.M * sizeof(double);
     void* tmp = nullptr;
-    if (e == cudaSuccess && h->precision == WV_PRECISION_FP64 && wvgpu::fx_has_rows(p)) {
-        e = alloc(h, (3 + 3 * nt) * p.Nx * p.Ny * p.Nz * sizeof(double), &tmp);
-        h->adjRows = static_cast<double*>(tmp);
-    }
     for (int i = 1; i < 4 && e == cudaSuccess; ++i) { e = alloc(h, stateBytes, &tmp); h->st[i] = static_cast<double*>(tmp); }
     if (e == cudaSuccess) { e = alloc(h, stateBytes, &tmp); h->kb = static_cast<double*>(tmp); }
     if (e == cudaSuccess) { e = alloc(h, stateBytes, &tmp); h->sb = static_cast<double*>(tmp); }
@@ -1138,6 +1135,28 @@ int ensure_adjoint(wv_handle* h) {
     h->metrics.device_bytes = h->deviceBytes;
     h->adjointReady = true;
     return WV_SUCCESS;
+}
+
+// Rows of the x pass for VJPs of FP64 handles that have none kept (a flux VJP, a step VJP,
+// an adjoint without room for its own): allocated when first needed, since they are the
+// largest part of the workspace (1 GB at 256x256x129).  Without memory, or while the
+// stream is being captured, the VJP runs without them on the block kernel.
+void ensure_rows(wv_handle* h, cudaStream_t s) {
+    const Plan& p = h->plan;
+    if (h->adjRows || h->adjRowsRefused || h->precision != WV_PRECISION_FP64 || !wvgpu::fx_has_rows(p)) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;
+    }
+    void* rows = nullptr;
+    if (alloc(h, (3 + 3 * p.targets.count) * p.Nx * p.Ny * p.Nz * sizeof(double), &rows) != cudaSuccess) {
+        cudaGetLastError();
+        h->adjRowsRefused = true;
+        return;
+    }
+    h->adjRows = static_cast<double*>(rows);
+    h->metrics.device_bytes = h->deviceBytes;
 }
 
 // VJP of the nonlinear flux (no damping) at state A: (Fpb, Fmb, F0b) -> (Apb, Amb, A0b).
@@ -2621,6 +2640,7 @@ int wv_flux_vjp_device(wv_handle* h, double t, double t0, const double* Ap, cons
     const PairedAdjoint paired(h);
     rc = adjoint_preamble(h); if (rc) return rc;
     auto s = static_cast<cudaStream_t>(stream);
+    ensure_rows(h, s);
     const cudaError_t e = fp64_path(h)
         ? launch_flux_vjp<double>(h, t, t0, Ap, Am, A0, Fpb, Fmb, F0b, Apb, Amb, A0b, s)
         : h->precision == WV_PRECISION_MIXED ? launch_flux_vjp<float>(h, t, t0, Ap, Am, A0, Fpb, Fmb, F0b, Apb, Amb, A0b, s)
@@ -2672,6 +2692,7 @@ int wv_rk4_step_vjp_device(wv_handle* h, const double* Ap, const double* Am, con
     const PairedAdjoint paired(h);
     rc = adjoint_preamble(h); if (rc) return rc;
     auto s = static_cast<cudaStream_t>(stream);
+    ensure_rows(h, s);
     cudaError_t e = gather3(h, h->state, Ap, Am, A0, s);
     if (e == cudaSuccess) e = gather3(h, h->ybin, Apb, Amb, A0b, s);
     if (e == cudaSuccess) e = rk4_step_vjp(h, h->state, t, t0, dt, h->ybin, s);
@@ -2737,6 +2758,7 @@ int wv_rk4_adjoint_device(wv_handle* h, const double* Ap, const double* Am, cons
     if (e != cudaSuccess) return cuda_fail(h, e, "RK4 adjoint checkpoints");
     h->metrics.device_bytes = h->deviceBytes;
     const bool keepY = slots > 0;
+    if (!keepY) ensure_rows(h, s);
     std::vector<double> times(n + 1);
     times[0] = t;
     for (int i = 0; i < n; ++i) times[i + 1] = times[i] + dt;
