@@ -31,6 +31,7 @@
 #include <string>
 #include <vector>
 #include <type_traits>
+#include <utility>
 
 using wvgpu::Descriptor;
 using wvgpu::Plan;
@@ -1800,30 +1801,35 @@ static int create_handle(const wv_config* config, int precision, int members, wv
         for (dev::FFTDev* f : {&fd.fx, &fd.fy, &fd.fz})
             if (f->N) *f = fixed_point_fft(f->N);
         h->fx.x = fixed_point_fft(p.Nx);
+        // every table in one allocation and one copy
+        std::vector<int32_t> words;
+        std::vector<std::pair<size_t, const dev::fxw**>> places;
         auto table = [&](const std::vector<int32_t>& v, const dev::fxw** dst) {
-            if (e != cudaSuccess || v.empty()) return;
-            const int32_t* q = nullptr;
-            e = upload(h, v, &q);
-            *dst = reinterpret_cast<const dev::fxw*>(q);
+            if (v.empty()) return;
+            places.emplace_back(words.size(), dst);
+            words.insert(words.end(), v.begin(), v.end());
         };
+        const dev::fxw *twx = nullptr, *twy = nullptr, *twz = nullptr;
         table(wvgpu::fixed_point_twiddles(static_cast<int>(p.Nx)), &h->fx.twX);
         table(wvgpu::fx_lane_table(p.Nx), &h->fx.twXLane);
-        auto words = [&](int N, const void** dst) {
-            const dev::fxw* q = nullptr;
-            table(wvgpu::fixed_point_twiddles(N), &q);
-            *dst = q;
-        };
-        words(fd.fx.N, &fd.twx);
-        words(fd.fy.N, &fd.twy);
-        if (fd.fz.N > 0) words(fd.fz.N, &fd.twz);
+        table(wvgpu::fixed_point_twiddles(fd.fx.N), &twx);
+        table(wvgpu::fixed_point_twiddles(fd.fy.N), &twy);
+        if (fd.fz.N > 0) table(wvgpu::fixed_point_twiddles(fd.fz.N), &twz);
         table(wvgpu::fx_lane_table(p.Ny), &fd.fxTwY);
         table(wvgpu::fx_lane_table(p.fz.N), &fd.fxTwZ);
         // exp(+2 pi i k / 256): the forward table read backwards
-        const std::vector<int32_t> forward = wvgpu::fixed_point_twiddles(256);
+        const std::vector<int32_t>& forward = wvgpu::fixed_point_twiddles(256);
         std::vector<int32_t> phases(forward.size());
         for (int k = 0; k < 256; ++k)
             std::copy_n(forward.begin() + 4 * ((256 - k) % 256), 4, phases.begin() + 4 * k);
         table(phases, &fd.fxPhase);
+        const int32_t* base = nullptr;
+        if (e == cudaSuccess) e = upload(h, words, &base);
+        if (e == cudaSuccess)
+            for (const auto& q : places) *q.second = reinterpret_cast<const dev::fxw*>(base + q.first);
+        fd.twx = twx;
+        fd.twy = twy;
+        if (twz) fd.twz = twz;
         if (h->fxOn) {
             fd.tRowK = dd.rowK;
             fd.tRowL = dd.rowL;

@@ -3,6 +3,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <numeric>
 
 namespace wvgpu {
@@ -65,29 +67,40 @@ FFTFactors factor_fixed_point(int N) {
     return f;
 }
 
-std::vector<int32_t> fixed_point_twiddles(int N) {
+namespace {
+
+std::vector<int32_t> make_fixed_point_twiddles(int N) {
     // the angle is reduced to the first octant in integers; long double carries
-    // at least 64 bits on both host architectures
+    // at least 64 bits on both host architectures (software on arm64: every value of
+    // the octant is evaluated once)
     const long double pi = 3.141592653589793238462643383279502884L;
-    auto q62 = [](long double v) { return std::llroundl(v * 4611686018427387904.0L); };
+    constexpr long long unset = INT64_MIN;
+    std::vector<long long> octant[2] = {std::vector<long long>(N + 1, unset), std::vector<long long>(N + 1, unset)};
+    auto value = [&](int sine, long long num) {  // cos or sin of pi num / (2 N), 2 num <= N
+        long long& v = octant[sine][num];
+        if (v == unset) {
+            const long double x = pi * num / (2.0L * N);
+            v = std::llroundl((sine ? std::sin(x) : std::cos(x)) * 4611686018427387904.0L);
+        }
+        return v;
+    };
     auto cosQ = [&](long long k) {  // cos(2 pi k / N)
-        k %= N;
         if (2 * k > N) k = N - k;
         const bool neg = 4 * k > N;
         const long long a = neg ? N - 2 * k : 2 * k;  // angle pi a / N in [0, pi/2]
-        const long double v = 4 * a <= N ? std::cos(pi * a / N) : std::sin(pi * (N - 2 * a) / (2.0L * N));
-        return neg ? -q62(v) : q62(v);
+        const long long v = 4 * a <= N ? value(0, 2 * a) : value(1, N - 2 * a);
+        return neg ? -v : v;
     };
     auto sinQ = [&](long long k) {  // sin(2 pi k / N)
-        k %= N;
         const bool neg = 2 * k > N;
         if (neg) k = N - k;
         long long a = 2 * k;  // angle pi a / N in [0, pi]
         if (2 * a > N) a = N - a;
-        const long double v = 4 * a <= N ? std::sin(pi * a / N) : std::cos(pi * (N - 2 * a) / (2.0L * N));
-        return neg ? -q62(v) : q62(v);
+        const long long v = 4 * a <= N ? value(1, 2 * a) : value(0, N - 2 * a);
+        return neg ? -v : v;
     };
     std::vector<int32_t> out;
+    out.reserve(4 * static_cast<size_t>(N));
     auto put = [&](long long q) {
         out.push_back(static_cast<int32_t>((q + 0x80000000ll) >> 32));
         out.push_back(static_cast<int32_t>(static_cast<uint32_t>(q)));
@@ -96,8 +109,20 @@ std::vector<int32_t> fixed_point_twiddles(int N) {
     return out;
 }
 
+}  // namespace
+
+const std::vector<int32_t>& fixed_point_twiddles(int N) {
+    // one table per length for the process (lengths reach 1024: 8 MB if all are met)
+    static std::mutex mutex;
+    static std::map<int, std::vector<int32_t>> tables;
+    std::lock_guard<std::mutex> lock(mutex);
+    auto it = tables.find(N);
+    if (it == tables.end()) it = tables.emplace(N, make_fixed_point_twiddles(N)).first;
+    return it->second;
+}
+
 std::vector<int32_t> fixed_point_stage_twiddles(int N, std::initializer_list<int> radices) {
-    const std::vector<int32_t> all = fixed_point_twiddles(N);
+    const std::vector<int32_t>& all = fixed_point_twiddles(N);
     std::vector<int32_t> out;
     int Ns = 1;
     for (const int R : radices) {

@@ -33,8 +33,8 @@ FFTFactors factor_fft(int N);
 // needs the fewest twiddle products, then 4, 2 and the odd primes.
 FFTFactors factor_fixed_point(int N);
 // exp(-2 pi i k / N) in Q62, four words per entry: re_h, re_l, im_h, im_l with
-// value = h 2^32 + l and a signed low word.
-std::vector<int32_t> fixed_point_twiddles(int N);
+// value = h 2^32 + l and a signed low word.  (Kept for the process.)
+const std::vector<int32_t>& fixed_point_twiddles(int N);
 // The same entries in the order the lane-held lines read them: stages (Ns, R), for
 // r = 1 .. R-1 and k < Ns the entry r k N / (Ns R).
 std::vector<int32_t> fixed_point_stage_twiddles(int N, std::initializer_list<int> radices);
