@@ -194,12 +194,20 @@ int wv_get_vertical_kernels(const wv_handle* handle, int* inverse_kind, int* for
  * per lane, five shuffle butterfly stages; mixed and FP32X2 handles, y lines of
  * 32 R and x rows of 64 R samples for the R each precision has), the default
  * where the length allows; WV_FFT_STOCKHAM: the shared-memory Stockham kernels
- * (every length; the only form of FP64 handles).  The get call reports the
- * kernel that runs. */
+ * (every length).  The get call reports the kernel that runs where the transforms
+ * are not in fixed point (wv_get_fixed_point; FP64 handles report WV_FFT_STOCKHAM),
+ * the set call chooses one and leaves fixed point. */
 #define WV_FFT_REGISTER 0
 #define WV_FFT_STOCKHAM 1
 int wv_set_fft_variants(wv_handle* handle, int y_variant, int x_variant);
 int wv_get_fft_variants(const wv_handle* handle, int* y_variant, int* x_variant);
+/* Whether the fluxes and state transforms run on 64-bit fixed-point lines: always on
+ * FP64 handles, by default on the FP32X2 handles named at WV_PRECISION_FP32X2, never on
+ * others.  Choosing vertical kernels or FFT variants ends it on FP32X2 handles, even
+ * with the values just reported; wv_set_fixed_point(handle, 1) takes it up again where
+ * it was the default (with WV_VERTICAL_FFT in both directions), 0 leaves it. */
+int wv_set_fixed_point(wv_handle* handle, int enabled);
+int wv_get_fixed_point(const wv_handle* handle, int* enabled);
 /* Device status word of the handle (synchronous read): bit 0 is set when a
  * bounded wait inside a kernel ran out (the kernel returned without hanging). */
 int wv_get_device_status(wv_handle* handle, unsigned* status);

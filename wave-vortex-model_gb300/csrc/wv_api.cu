@@ -106,11 +106,12 @@ struct wv_handle {
     // x pass (length Nx, two rows per line) and the descriptor with their tables
     wvgpu::FxRows fx{};
     dev::DescDev fxd{};
-    // FP32X2: the fluxes, their VJP and the state transforms run on the fixed-point
-    // kernels -- more accurate than paired FP32 and, where every axis has lane-held
-    // lines, faster (2.03 against 2.34 ms a flux at 256x256x129; on the run-time
+    // FP32X2: the fluxes and the state transforms (not the adjoint: PairedAdjoint) run on
+    // the fixed-point kernels -- more accurate than paired FP32 and, where every axis has
+    // lane-held lines, faster (2.04 against 2.28 ms a flux at 256x256x129; on the run-time
     // stages 1.3 to 1.6 times slower) -- until a kernel is chosen explicitly
     bool fxOn = false;
+    bool fxTables = false;  // ... and can again (wv_set_fixed_point)
     dev::DescDev sd{};
     const void* scalarD = nullptr;
     const unsigned char* scalarFlags = nullptr;
@@ -1787,7 +1788,7 @@ static int create_handle(const wv_config* config, int precision, int members, wv
         }
     }
     // fixed-point lines: their own factors and twiddles, doubles where the working type has its copies
-    h->fxOn = precision == WV_PRECISION_FP32X2 && wvgpu::fx_beats_paired(p);
+    h->fxOn = h->fxTables = precision == WV_PRECISION_FP32X2 && wvgpu::fx_beats_paired(p);
     if (precision == WV_PRECISION_FP64 || h->fxOn) {
         dev::DescDev& fd = h->fxd;
         fd = dd;
@@ -1953,6 +1954,23 @@ int wv_get_fft_variants(const wv_handle* h, int* y_variant, int* x_variant) {
                     : h->precision == WV_PRECISION_MIXED ? warp_rx<float>(p) != 0 : warp_rx<dev::ff>(p) != 0;
     *y_variant = wy ? WV_FFT_REGISTER : WV_FFT_STOCKHAM;
     *x_variant = wx ? WV_FFT_REGISTER : WV_FFT_STOCKHAM;
+    return WV_SUCCESS;
+}
+
+int wv_set_fixed_point(wv_handle* h, int enabled) {
+    if (!h) return WV_INVALID_POINTER;
+    const bool always = h->precision == WV_PRECISION_FP64;
+    if (enabled ? !always && !h->fxTables : always)
+        return fail(h, WV_UNSUPPORTED_OPERATION, enabled ? "This handle's transforms have no fixed-point form."
+                                                         : "FP64 handles have no other form of their transforms.");
+    if (enabled && !always) h->vinvKind = h->vfwdKind = WV_VERTICAL_FFT;
+    h->fxOn = enabled != 0 && !always;
+    return WV_SUCCESS;
+}
+
+int wv_get_fixed_point(const wv_handle* h, int* enabled) {
+    if (!h || !enabled) return WV_INVALID_POINTER;
+    *enabled = fp64_path(h) ? 1 : 0;
     return WV_SUCCESS;
 }
 
