@@ -346,11 +346,19 @@ def _stage_profile(k, dev, t, t0, dt, precision, torch):
     rows = GRID["Ny"] * GRID["Nz"]
     x_flops = rows * (19 * (5 * L * math.log2(L) + 10 * L) + 4 * GRID["Nx"] * 6)
     x_ms = per_launch["x_products"]
-    compute = {"stage": "x_products", "flops_per_launch": x_flops, "achieved_tflops": x_flops / (x_ms * 1e-3) / 1e12,
-               "pipe": "fp64" if precision == "fp64" else "fp32"}
+    fixed = k.fixed_point()  # 64-bit fixed-point lines: no floating-point operations
+    form = "fixed" if fixed else precision
+    compute = {"stage": "x_products", "pipe": "integer" if fixed else "fp32"}
+    if fixed:
+        inst = traffic_from_profile("x_products_warp_instructions", form)
+        compute["warp_instructions_per_launch"] = inst
+        compute["warp_ginstructions_s"] = inst and inst / (x_ms * 1e-3) / 1e9
+        compute["warp_instructions_source"] = "smsp__inst_executed.sum of a committed ncu capture (profiles/ncu_traffic.txt)"
+    else:
+        compute.update({"flops_per_launch": x_flops, "achieved_tflops": x_flops / (x_ms * 1e-3) / 1e12})
     return {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "compute": compute,
-            "frac": achieved / peaks["hbm_gbs"], "traffic": traffic_from_profile(dominant, precision),
+            "frac": achieved / peaks["hbm_gbs"], "traffic": traffic_from_profile(dominant, form), "transforms": form,
             "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum per launch from a committed ncu capture "
                               "of this kernel on this workload (profiles/ncu_traffic.txt), not from this run",
             "peak_source": peak_kind, "algorithmic_bytes_per_launch": sbytes[dominant],
@@ -405,6 +413,7 @@ def _published_flux_comparison(wvgpu, torch, np):
             e1.synchronize()
             ms = e0.elapsed_time(e1) / 5
             row[prec + "_ms"] = ms
+            row[prec + "_fixed_point"] = k.fixed_point()
             row[prec + "_speedup_vs_published"] = ms_ref / ms
             if k is not k64:
                 k.close()
@@ -564,8 +573,6 @@ def run_ours(args):
     roofline = _stage_profile(k, dev, t, t0, dt, "fp64", torch)
     try:
         roofline["fp64_gemm_peak_tflops_measured"] = fp64_peak_tflops(torch)
-        roofline["compute"]["frac_of_fp64_gemm_peak"] = (roofline["compute"]["achieved_tflops"] /
-                                                         roofline["fp64_gemm_peak_tflops_measured"])
     except Exception:  # pragma: no cover
         roofline["fp64_gemm_peak_tflops_measured"] = None
 
@@ -596,21 +603,33 @@ def run_ours(args):
         if rank == 0:
             mixed[name]["rel_field_err_vs_fp64_after_100_steps"] = _field_error_after(k, km, state, dt, 100, torch, np)
     km.close()
-    # paired-FP32 form (FP32X2): FP64-class accuracy on the FP32 pipe
+    # FP32X2 handles: their default kernels (fixed-point lines on this grid) and the
+    # paired-FP32 ones
     kx = wvgpu.WVTransformConstantStratificationKernel(cfg, precision="fp32x2")
-    devx = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in state]
-    x_ms, tx = _time_steps(kx, devx, 0.0, t0, dt, args.steps, args.warmup, stream, barrier, flush, torch)
-    x_value = world * args.steps / max_over_ranks(x_ms / 1e3)
-    fp32x2 = {"value": x_value, "unit": UNIT, "ms_per_step": x_ms / args.steps, "speedup_vs_fp64": x_value / value,
-              "dtype": "paired f32 (float-float, ~45-48 significand bits on the FP32 pipe) for the xy transforms, "
-                       "products, phases and the vertical transforms (FFTs of the even / odd extension over z); "
-                       "f64 angles, stores and RK4",
-              "vertical_kernel": kx.vertical_kernel(),
-              "roofline": _stage_profile(kx, devx, tx, t0, dt, "fp32x2", torch)}
-    if rank == 0:
-        err = _field_error_after(k, kx, state, dt, 100, torch, np)
-        fp32x2["rel_field_err_vs_fp64_after_100_steps"] = err
-        fp32x2["meets_target_3x_and_1e-6"] = bool(fp32x2["speedup_vs_fp64"] >= 3.0 and max(err) <= 1e-6)
+    paired_dtype = ("paired f32 (float-float, ~45-48 significand bits on the FP32 pipe) for the xy transforms, "
+                    "products, phases and the vertical transforms (FFTs of the even / odd extension over z); "
+                    "f64 angles, stores and RK4")
+
+    def x2_leg():
+        devx = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in state]
+        x_ms, tx = _time_steps(kx, devx, 0.0, t0, dt, args.steps, args.warmup, stream, barrier, flush, torch)
+        x_value = world * args.steps / max_over_ranks(x_ms / 1e3)
+        leg = {"value": x_value, "unit": UNIT, "ms_per_step": x_ms / args.steps, "speedup_vs_fp64": x_value / value,
+               "fixed_point": kx.fixed_point(),
+               "dtype": "the FP64 handle's 64-bit fixed-point lines; f64 phases, projections and RK4"
+                        if kx.fixed_point() else paired_dtype,
+               "vertical_kernel": kx.vertical_kernel(),
+               "roofline": _stage_profile(kx, devx, tx, t0, dt, "fp32x2", torch)}
+        if rank == 0:
+            err = _field_error_after(k, kx, state, dt, 100, torch, np)
+            leg["rel_field_err_vs_fp64_after_100_steps"] = err
+            leg["meets_target_3x_and_1e-6"] = bool(leg["speedup_vs_fp64"] >= 3.0 and max(err) <= 1e-6)
+        return leg
+
+    fp32x2 = x2_leg()
+    if kx.fixed_point():
+        kx.set_fixed_point(False)
+        fp32x2["paired_f32"] = x2_leg()
     kx.close()
     adjoint = ({p: _adjoint_timing(wvgpu, p, stream, torch, np) for p in ("fp64", "mixed", "fp32x2")}
                if rank == 0 else None)
@@ -655,9 +674,10 @@ def run_ours(args):
                               "M5 Max: 2.20 steps/s (the reference's three-interface record; its run includes an "
                               "observer graph)",
         "dtype": "f64", "data": "synthetic",
-        "precision": "fp64 (plain drop-in); the reduced-precision forms are reported under 'mixed' (f32; its "
+        "precision": "fp64 (the drop-in: state, coefficients, phases and RK4 in double, transforms and products in "
+                     "64-bit block fixed point); the reduced-precision forms are reported under 'mixed' (f32; its "
                      "split-BF16 tensor-core vertical transforms under mixed.tensor_core_vertical) and 'fp32x2' "
-                     "(paired f32)",
+                     "(its default kernels; the paired f32 ones under fp32x2.paired_f32)",
         "vertical_kernel": k.vertical_kernel(),
         "config": {
             "workload": "fixed-step RK4, nonlinear advection, 256x256x129, 800 km x 800 km x 4 km, N0 5.2e-3, lat 33, "
@@ -725,11 +745,16 @@ def _summary(value, mixed, fp32x2, adjoint, ensemble, g512, vs_ref, roofline):
          "speedup_at_1e-6_vs_fp64": best[1]["speedup_vs_fp64"] if best else None,
          "fp32x2_speedup_vs_fp64": fp32x2["speedup_vs_fp64"],
          "fp32x2_max_field_err_100": max(fp32x2.get("rel_field_err_vs_fp64_after_100_steps", [float("nan")])),
+         "fp32x2_fixed_point": fp32x2["fixed_point"],
          "mixed_speedup_vs_fp64": mixed["speedup_vs_fp64"],
          "mixed_field_err_100": mixed.get("rel_field_err_vs_fp64_after_100_steps"),
          "mixed_all_tensor_core_vertical_speedup_vs_fp64": mixed.get("tensor_core_vertical", {}).get("speedup_vs_fp64"),
          "flux_hbm_frac_mixed": mixed["roofline"]["flux"]["frac"],
          "flux_hbm_frac_fp64": roofline["flux"]["frac"]}
+    paired = fp32x2.get("paired_f32")
+    if paired:
+        s["fp32x2_paired_speedup_vs_fp64"] = paired["speedup_vs_fp64"]
+        s["fp32x2_paired_max_field_err_100"] = max(paired.get("rel_field_err_vs_fp64_after_100_steps", [float("nan")]))
     if adjoint:
         for p, a in adjoint.items():
             s[f"adjoint_over_forward_{p}"] = a["adjoint_over_forward"]
@@ -839,7 +864,7 @@ def _leg_512(wvgpu, stream, torch, np, steps):
         finals[name] = [x.cpu().numpy() for x in dev]
         vk = kk.vertical_kernels()
         out[name] = {"value": steps / (ms * 1e-3), "ms_per_step": ms / steps,
-                     "vertical_kernel": {"inverse": vk[0], "forward": vk[1]},
+                     "vertical_kernel": {"inverse": vk[0], "forward": vk[1]}, "fixed_point": kk.fixed_point(),
                      "energy_drift": (_energy(k, finals[name], tT, 0.0, np) - E0) / E0}
         if kk is not k:
             kk.close()
