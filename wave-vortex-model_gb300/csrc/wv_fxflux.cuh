@@ -56,6 +56,7 @@ __device__ __forceinline__ void fx_load_rows(const double2* __restrict__ hA, con
     }
     // (fx_line's gap is against one entry; the first stage adds `radix` of them)
     gap = radix1 && Nx > kFxLateFrom ? max(0, fx_shared_gap(l[0].gap, l[1].gap) - fx_ceil_log2(radix)) : 0;
+    if (gap < 2) gap = 0;  // not worth the shifts
     unitA = l[0].unit;
     unitB = l[1].unit;
 #pragma unroll
@@ -73,10 +74,11 @@ __device__ __forceinline__ void fx_load_rows(const double2* __restrict__ hA, con
     }
 }
 
-// Rows of x past kFxLateFrom points have more than 64 columns (EK > 2) or keep no gap.
+// Rows of x past kFxLateFrom points have more than 64 columns (EK > 2) or keep no gap; most
+// spectra of a flow fall off and have none to speak of (fx_load_rows).
 template <int EK, bool INV>
 __device__ inline fxc* fx_row_stages(fxc* a, fxc* b, const FxFactors f, int lines, const fxw* tw, int gap) {
-    if (EK > 2 && f.N > kFxLateFrom) return fx_all_stages<INV, true, (EK > 2)>(a, b, f, lines, f.N, tw, nullptr, gap);
+    if (EK > 2 && gap > 0) return fx_all_stages<INV, true, (EK > 2)>(a, b, f, lines, f.N, tw, nullptr, gap);
     return fx_all_stages<INV, true, false>(a, b, f, lines, f.N, tw, nullptr, 0);
 }
 // Z = A + i B and its mirror into the line (every entry of it written).
