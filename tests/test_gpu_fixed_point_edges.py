@@ -47,6 +47,16 @@ def test_still_velocity_component_advects_nothing(wv, shape):
     k.close()
 
 
+@pytest.mark.parametrize("shape", [(64, 64, 33), (192, 32, 13), (256, 16, 9), (60, 50, 21), (300, 12, 9)])
+def test_own_advection_fields_give_the_flux_bit_for_bit(wv, shape):
+    """The returned velocities are the ones the flux used, to the last bit."""
+    c, d, A, k = _setup(wv, shape)
+    F, adv = k.nonlinearFluxWithAdvectionFields(50.0, 0.0, *A)
+    for a, b, f in zip(k.nonlinearFluxUsingAdvectionFields(50.0, 0.0, *A, adv), F, k.nonlinearFlux(50.0, 0.0, *A)):
+        assert np.array_equal(a, b) and np.array_equal(b, f)
+    k.close()
+
+
 @pytest.mark.parametrize("shape", [(32, 48, 17), (20, 18, 11), (516, 8, 7)])
 @pytest.mark.parametrize("power", [-900, 960])
 def test_values_near_the_ends_of_the_range(wv, shape, power):

@@ -223,12 +223,15 @@ bool fx_xadj(const Plan& p, const dev::DescDev& d, const FxRows& r, const double
     return true;
 }
 
-// Against the paired-FP32 kernels per flux: 1.05 to 1.7 times as fast where every axis
-// has lane-held lines (64x64x97 158 -> 144 us, 96x96x49 221 -> 189, RK4 step at
-// 256x256x129 9.41 -> 8.35 ms), but not with x or y lines of 192 points (RK4 step at
-// 192x192x97 4.23 -> 4.33 ms), on the run-time stages (0.6 to 0.8 times as fast), nor
-// on small grids whose y and z lines the paired form holds in warp registers
-// (32x32x17 hydrostatic 38.9 -> 44.2 us).
+// Against the paired-FP32 kernels, flux in us, paired / fixed point (nonhydrostatic):
+// every axis with lane-held lines 16x16x9 64 / 47, 48x48x25 99 / 66, 64x64x33 73 / 73,
+// 96x96x49 216 / 187, 128x128x65 328 / 297, 256x256x129 2279 / 2072; run-time stages lose
+// (0.6 to 0.8 times as fast).  On small grids whose y and z lines the paired form holds in
+// warp registers it wins below 65536 points (32x32x17 42 / 49, 64x32x17 52 / 51,
+// 32x32x33 57 / 49), hydrostatic up to twice that (64x64x17 52 / 56, 64x64x33 66 / 68:
+// within 8 %, and 1e-16 instead of 1e-12 of error).  Rows of 192 points are 12 a lane at
+// two blocks an SM and lose on wide grids (192x96x49 301 / 330, 192x192x97 1024 / 1087);
+// y lines of 192 beside other rows would win (96x192x49 409 / 326, 32x192x33 148 / 91).
 bool fx_beats_paired(const Plan& p) {
     const bool small = p.Ny % 32 == 0 && p.fz.N % 32 == 0 && p.Nx * p.Ny * p.Nz < 65536;
     return fx_x_lane(p) && fx_lane_length(p.Ny) && fx_lane_length(p.fz.N) && p.Nx != 192 && p.Ny != 192 && !small;

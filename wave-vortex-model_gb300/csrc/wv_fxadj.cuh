@@ -258,15 +258,15 @@ __global__ void __launch_bounds__(32 * kFxZWarps, 2)
     if (!live) return;
 #pragma unroll 1
     for (int i = l; i < H; i += 4) {
-    const int j = t + G * i;
-    if (j >= Nj) continue;
-    const double m = static_cast<const double*>(d.tMz)[j];
-    // u_bar = Ccos^T U + (-m) Csin^T u_z;  w_bar = Csin^T W + m Ccos^T w_z; likewise v, eta
-    const double2 e0 = X[j], o0 = X[L + j], e1 = X[2 * L + j], o1 = X[3 * L + j];
-    const double2 e2 = X[4 * L + j], o2 = X[5 * L + j], e3 = X[6 * L + j], o3 = X[7 * L + j];
-    fx_vinv_adj_store(d, j + Nj * d.modeWV[mode], elapsed, make_double2(e0.x - m * o2.x, e0.y - m * o2.y),
-                      make_double2(e1.x - m * o3.x, e1.y - m * o3.y), make_double2(o0.x + m * e2.x, o0.y + m * e2.y),
-                      make_double2(o1.x + m * e3.x, o1.y + m * e3.y), Apb, Amb, A0b);
+        const int j = t + G * i;
+        if (j >= Nj) continue;
+        const double m = static_cast<const double*>(d.tMz)[j];
+        // u_bar = Ccos^T U + (-m) Csin^T u_z;  w_bar = Csin^T W + m Ccos^T w_z; likewise v, eta
+        const double2 e0 = X[j], o0 = X[L + j], e1 = X[2 * L + j], o1 = X[3 * L + j];
+        const double2 e2 = X[4 * L + j], o2 = X[5 * L + j], e3 = X[6 * L + j], o3 = X[7 * L + j];
+        fx_vinv_adj_store(d, j + Nj * d.modeWV[mode], elapsed, make_double2(e0.x - m * o2.x, e0.y - m * o2.y),
+                          make_double2(e1.x - m * o3.x, e1.y - m * o3.y), make_double2(o0.x + m * e2.x, o0.y + m * e2.y),
+                          make_double2(o1.x + m * e3.x, o1.y + m * e3.y), Apb, Amb, A0b);
     }
 }
 
