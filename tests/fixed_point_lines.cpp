@@ -43,7 +43,7 @@ void any_line(std::vector<fxc>& line, int gap) {
     int Ns = 1;
     for (int s = 0; s < f.nstages; ++s) {
         const FxFactors factors{N, f.nstages, f.radix};
-        if (s > 0 && fx_any_radix(f.radix[s])) fx_shift_lines(line.data(), N, 1, N, fx_late_of(factors, s, Ns, nullptr, gap), 0, 1);
+        if (s > 0 && fx_any_radix(f.radix[s])) fx_shift_lines(line.data(), N, Ns, 1, N, fx_late_of(factors, s, Ns, nullptr, gap), 0, 1);
         fx_run_stage<INV, true>(line.data(), other.data(), factors, s, Ns, 1, N, tw.data(), nullptr, gap, 0, 1);
         Ns *= f.radix[s];
         std::swap(line, other);

@@ -124,3 +124,19 @@ def test_prime_lines_are_no_further_off_than_sums_of_doubles(lib, n, kind):
     for i in range(n):
         plain += rows[0][i] * tw[i * m[:n // 2 + 1] % n]
     assert _error(out[0::2].astype(np.longdouble) + 1j * out[1::2], ref) <= _error(plain, ref)
+
+
+@pytest.mark.parametrize("lanes,n", [(1, n) for n in LANES] + [(0, n) for n in (60, 200, 250, 384, 500, 512, 1000, 1024)])
+def test_line_sums_have_no_mean_error(lib, lanes, n):
+    """The first coefficient is the sum of the entries, where a mean of the roundings would
+    collect: over 400 white rows its mean error stays within five standard errors."""
+    if not np.finfo(np.longdouble).eps < 1e-18:
+        pytest.skip("no long double")
+    rng = np.random.default_rng(7 * n)
+    error = []
+    for _ in range(400):
+        rows = rng.standard_normal((2, n))
+        out = np.empty(2 * (n // 2 + 1))
+        lib.real_pair(_p(rows[0]), _p(rows[1]), n, lanes, _p(out))
+        error.append(float(out[0] - np.sum(rows[0].astype(np.longdouble))))
+    assert abs(np.mean(error)) <= 5.0 * np.std(error) / 20.0, (np.mean(error), np.std(error))

@@ -87,10 +87,9 @@ WV_HD fxc fx_cmul(fxc a, fxw w) {
 // each cuts half a unit on average, `two` gives it back), 27 instructions against 37.
 // two: the value 2 in a register the compiler cannot rebuild (fx_two); 0 on all-zero
 // lines, which stay exactly zero.  Twiddles +-1 and +-i (no low words) cut nothing.
-// SHIFT: x 2^-sh w; the operand carries two more bits, so a shift cuts at a quarter unit.
-template <bool INV, bool SHIFT>
-WV_HD fxc fx_cmul60(fxc a, fxw w, int two, int sh) {
-    const long long x4 = SHIFT ? (a.x << 2) >> sh : a.x << 2, y4 = SHIFT ? (a.y << 2) >> sh : a.y << 2;
+template <bool INV>
+WV_HD fxc fx_cmul60(fxc a, fxw w, int two) {
+    const long long x4 = a.x << 2, y4 = a.y << 2;
     const int xl = fx_lo(x4), yl = fx_lo(y4), xh = fx_hi(x4), yh = fx_hi(y4);
     const int nh = -w.sh, nl = -w.sl;
     const int sih = INV ? nh : w.sh, sil = INV ? nl : w.sl, mh = INV ? w.sh : nh, ml = INV ? w.sl : nl;
@@ -401,20 +400,25 @@ WV_HD int fx_pad(int i) { return i + (i >> 3); }
 
 // Stage of radix R behind Ns points already combined; tw[(r - 1) Ns + k].  SHIFT: the
 // inputs come down by sh bits, rounded by the half unit that the stage before added to
-// its outputs (`half` on its first input; NEXT), ties in turn over the lanes.
+// all outputs of a butterfly (on its first input; NEXT: by nextSh bits).  Ties go up and
+// down in turn over the butterflies of one k, which the following stages sum.
 template <int N, int R, int Ns, bool INV, bool SHIFT, bool NEXT>
-WV_HD void fx_wstage(fxc (&v)[FxW<N>::E], const fxw* tw, int t, int two, int sh, long long half) {
+WV_HD void fx_wstage(fxc (&v)[FxW<N>::E], const fxw* tw, int t, int two, int sh, int nextSh) {
     constexpr int G = FxW<N>::G, B = FxW<N>::E / R;
 #pragma unroll
     for (int b = 0; b < B; ++b) {
-        const int k = (t + G * b) & (Ns - 1);  // (Ns is a power of two)
+        const int j = t + G * b, k = j & (Ns - 1);  // (Ns is a power of two)
         fxc u[R];
-        u[0] = v[b];
-        if (SHIFT) u[0] = fxc{(((u[0].x << 2) >> sh) + 1 + (t & 1)) >> 2, (((u[0].y << 2) >> sh) + 1 + (t & 1)) >> 2};
-        if (NEXT) u[0] = fxc{u[0].x + half, u[0].y + half};
 #pragma unroll
-        for (int r = 1; r < R; ++r)
-            u[r] = Ns == 1 ? v[b + B * r] : fx_cmul60<INV, SHIFT>(v[b + B * r], tw[(r - 1) * Ns + k], two, sh);
+        for (int r = 0; r < R; ++r) {
+            u[r] = v[b + B * r];
+            if (SHIFT) u[r] = fxc{u[r].x >> sh, u[r].y >> sh};
+            if (r > 0 && Ns > 1) u[r] = fx_cmul60<INV>(u[r], tw[(r - 1) * Ns + k], two);
+        }
+        if (NEXT) {
+            const long long half = fx_half(nextSh, (j / Ns) & 1);
+            u[0] = fxc{u[0].x + half, u[0].y + half};
+        }
         fx_dft<R, INV>(u);
 #pragma unroll
         for (int r = 0; r < R; ++r) v[b + B * r] = u[r];
@@ -446,14 +450,13 @@ WV_DEV void fx_line_stages(fxc* x, const fxw* tw, int two, int gap, Each each) {
     constexpr bool three = W::R3 > 1, second = LATE >= 1, third = LATE >= 2 && three;
     constexpr int most2 = W::R2 == 8 ? 3 : W::R2 == 4 ? 2 : W::R2 == 2 ? 1 : 4;  // ceil log2 R2
     const int sh2 = third && gap > most2 ? most2 : gap, sh3 = gap - sh2;
-    const long long half2 = static_cast<long long>((1ull << sh2) >> 3), half3 = static_cast<long long>((1ull << sh3) >> 3);
     each([=](fxc (&v)[W::E], int t) {
-        fx_wstage<N, W::R1, 1, INV, false, second>(v, tw, t, two, 0, half2);
+        fx_wstage<N, W::R1, 1, INV, false, second>(v, tw, t, two, 0, sh2);
         fx_wscatter<N, W::R1, 1>(v, x, t);
     });
     each([=](fxc (&v)[W::E], int t) { fx_wgather<N>(v, x, t); });
     each([=](fxc (&v)[W::E], int t) {
-        fx_wstage<N, W::R2, W::R1, INV, second, third>(v, tw, t, two, sh2, half3);
+        fx_wstage<N, W::R2, W::R1, INV, second, third>(v, tw, t, two, sh2, sh3);
         if constexpr (three) fx_wscatter<N, W::R2, W::R1>(v, x, t);
     });
     if constexpr (three) {
@@ -478,10 +481,11 @@ struct FxLate {
 };
 constexpr int kFxLateFrom = 192;  // longer run-time lines start finer
 WV_HD int fx_ceil_log2(int n) { return n <= 1 ? 0 : 32 - fx_clz(static_cast<unsigned>(n - 1)); }
-// entry at place j, shifted down
-WV_HD fxc fx_late(fxc a, int sh, int j) {
+// entry of block `block` (of the Ns points that the stages so far combined), shifted down:
+// ties in turn over the blocks, which the following stages sum for one k
+WV_HD fxc fx_late(fxc a, int sh, int block) {
     if (sh == 0) return a;
-    const long long h = fx_half(sh, j & 1);
+    const long long h = fx_half(sh, block & 1);
     return fxc{(a.x + h) >> sh, (a.y + h) >> sh};
 }
 // One stage over `lines` lines (as fft_stage): radix R from src to dst.
@@ -500,10 +504,10 @@ WV_HD void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, i
             line = it / nb; j = it - line * nb; jq = j / Ns; k = j - jq * Ns;
         }
         const fxc* in = src + line * ld + j;
-        const int sh = LATE ? late(line) : 0;
+        const int sh = LATE ? late(line) : 0, blocks = LATE ? nb / Ns : 0;
         fxc v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = LATE ? fx_late(in[r * nb], sh, j) : in[r * nb];
+        for (int r = 0; r < R; ++r) v[r] = LATE ? fx_late(in[r * nb], sh, jq + r * blocks) : in[r * nb];
         if (Ns > 1) {
             const int ts = k * tstride;
 #pragma unroll
@@ -540,10 +544,10 @@ WV_HD void fx_stage_any(const fxc* __restrict__ src, fxc* __restrict__ dst, int 
 }
 
 struct FxFactors { int N, nstages; const int* radix; };
-WV_HD void fx_shift_lines(fxc* lines_, int N, int lines, int ld, FxLate late, int tid, int nt) {
+WV_HD void fx_shift_lines(fxc* lines_, int N, int Ns, int lines, int ld, FxLate late, int tid, int nt) {
     for (int it = tid; it < lines * N; it += nt) {
         const int line = it / N, i = it - line * N;
-        lines_[line * ld + i] = fx_late(lines_[line * ld + i], late(line), i);
+        lines_[line * ld + i] = fx_late(lines_[line * ld + i], late(line), i / Ns);
     }
 }
 WV_HD bool fx_any_radix(int R) { return R != 2 && R != 3 && R != 4 && R != 5 && R != 8; }
@@ -673,7 +677,7 @@ __device__ inline fxc* fx_all_stages(fxc* a, fxc* b, const FxFactors f, int line
     int Ns = 1;
     for (int s = 0; s < f.nstages; ++s) {
         if (LATE && s > 0 && fx_any_radix(f.radix[s])) {
-            fx_shift_lines(a, f.N, lines, ld, fx_late_of(f, s, Ns, gaps, gap), tid, nt);
+            fx_shift_lines(a, f.N, Ns, lines, ld, fx_late_of(f, s, Ns, gaps, gap), tid, nt);
             if (WARP) __syncwarp(); else __syncthreads();
         }
         fx_run_stage<INV, LATE>(a, b, f, s, Ns, lines, ld, tw, gaps, gap, tid, nt);
