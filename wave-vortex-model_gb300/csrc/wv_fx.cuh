@@ -481,14 +481,8 @@ struct FxLate {
 };
 constexpr int kFxLateFrom = 192;  // longer run-time lines start finer
 WV_HD int fx_ceil_log2(int n) { return n <= 1 ? 0 : 32 - fx_clz(static_cast<unsigned>(n - 1)); }
-// entry of block `block` (of the Ns points that the stages so far combined), shifted down:
-// ties in turn over the blocks, which the following stages sum for one k
-WV_HD fxc fx_late(fxc a, int sh, int block) {
-    if (sh == 0) return a;
-    const long long h = fx_half(sh, block & 1);
-    return fxc{(a.x + h) >> sh, (a.y + h) >> sh};
-}
-// One stage over `lines` lines (as fft_stage): radix R from src to dst.
+// One stage over `lines` lines (as fft_stage): radix R from src to dst.  What comes down is
+// rounded with ties in turn over the blocks of Ns points, which the stages sum for one k.
 template <int R, bool INV, bool LATE>
 WV_HD void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, int Ns, int lines, int ld,
                     const fxw* __restrict__ tw, FxLate late, int tid, int nt) {
@@ -507,7 +501,12 @@ WV_HD void fx_stage(const fxc* __restrict__ src, fxc* __restrict__ dst, int N, i
         const int sh = LATE ? late(line) : 0, blocks = LATE ? nb / Ns : 0;
         fxc v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = LATE ? fx_late(in[r * nb], sh, jq + r * blocks) : in[r * nb];
+        for (int r = 0; r < R; ++r) v[r] = in[r * nb];
+        if (LATE && sh > 0) {
+            const long long h[2] = {fx_half(sh, jq & 1), fx_half(sh, (jq + blocks) & 1)};
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = fxc{(v[r].x + h[r & 1]) >> sh, (v[r].y + h[r & 1]) >> sh};
+        }
         if (Ns > 1) {
             const int ts = k * tstride;
 #pragma unroll
@@ -547,7 +546,10 @@ struct FxFactors { int N, nstages; const int* radix; };
 WV_HD void fx_shift_lines(fxc* lines_, int N, int Ns, int lines, int ld, FxLate late, int tid, int nt) {
     for (int it = tid; it < lines * N; it += nt) {
         const int line = it / N, i = it - line * N;
-        lines_[line * ld + i] = fx_late(lines_[line * ld + i], late(line), i / Ns);
+        const int sh = late(line);
+        const long long h = fx_half(sh, (i / Ns) & 1);
+        const fxc a = lines_[line * ld + i];
+        lines_[line * ld + i] = fxc{(a.x + h) >> sh, (a.y + h) >> sh};
     }
 }
 WV_HD bool fx_any_radix(int R) { return R != 2 && R != 3 && R != 4 && R != 5 && R != 8; }
