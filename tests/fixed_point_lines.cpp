@@ -58,7 +58,9 @@ Form form_of(int N, bool lanes, bool pair, bool inverse) {
         WV_LENGTHS(X)
 #undef X
     }
-    return {0, wvgpu::factor_fixed_point(N).radix[0], N > kFxLateFrom ? 1 : 0};
+    const wvgpu::FFTFactors f = wvgpu::factor_fixed_point(N);
+    const int radix = fx_gap_radix(f.nstages, f.radix);
+    return {0, radix, N > kFxLateFrom && radix > 0 ? 1 : 0};
 }
 template <bool INV>
 void transform(std::vector<fxc>& line, const Form& form, bool pair, int gap) {

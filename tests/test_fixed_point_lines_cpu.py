@@ -140,3 +140,18 @@ def test_line_sums_have_no_mean_error(lib, lanes, n):
         lib.real_pair(_p(rows[0]), _p(rows[1]), n, lanes, _p(out))
         error.append(float(out[0] - np.sum(rows[0].astype(np.longdouble))))
     assert abs(np.mean(error)) <= 5.0 * np.std(error) / 20.0, (np.mean(error), np.std(error))
+
+
+@pytest.mark.parametrize("lanes,n", [(1, 128), (1, 192), (1, 256)] + [(0, n) for n in (200, 251, 256, 384, 500, 509, 512, 1000, 1024)])
+def test_equal_moduli_at_the_exponent_boundary(lib, lanes, n):
+    """Equal moduli near a power of two of the bounds, where the float sum may round past
+    n times the largest: every bit a line starts finer by has to come down again."""
+    rng = np.random.default_rng(n)
+    sign = rng.choice([-1.0, 1.0], (2, n))
+    ref = np.fft.rfft(sign[0])
+    out = np.empty(2 * (n // 2 + 1))
+    boundary = 2.0 ** np.arange(3) / 1.0025
+    for c in np.concatenate([b * (1.0 + np.arange(-120, 121) * 2.0 ** -23) for b in boundary]):
+        rows = np.ascontiguousarray(c * sign)
+        lib.real_pair(_p(rows[0]), _p(rows[1]), n, lanes, _p(out))
+        assert _error(out[0::2] + 1j * out[1::2], c * ref) <= 1e-15, c

@@ -162,3 +162,17 @@ def test_rows_of_the_vjp_are_allocated_when_first_needed(wv, shape):
         a, b = a.cpu().numpy(), b.cpu().numpy()
         assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
     k.close()
+
+
+@pytest.mark.parametrize("shape", [(256, 200, 9), (512, 16, 7), (16, 512, 7), (12, 10, 129), (10, 12, 201), (516, 8, 7)])
+def test_equal_samples_at_the_exponent_boundary(wv, shape):
+    """Fields of one modulus near a power of two of the lines' bounds (tests of the lines
+    alone: test_fixed_point_lines_cpu.py): the transform scales with the fields."""
+    c, d, A, k = _setup(wv, shape)
+    sign = np.random.default_rng(9).choice([-1.0, 1.0], (4, shape[2], shape[1], shape[0]))
+    ref = k.transformUVWEtaToWaveVortex(0.7 * sign, 0.0, 0.0)
+    for step in (-40, -8, -3, -1, 0, 1, 3, 8, 40):
+        f = (1.0 + step * 2.0 ** -23) / 1.0025
+        for a, b in zip(k.transformUVWEtaToWaveVortex(f * sign, 0.0, 0.0), ref):
+            assert np.max(np.abs(a - b * (f / 0.7))) <= 1e-12 * np.max(np.abs(b))
+    k.close()

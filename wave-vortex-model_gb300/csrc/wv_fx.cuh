@@ -5,12 +5,13 @@
 // integer pipes add 63 64-bit values per SM and clock and run 32 32 x 32 -> 64-bit
 // multiplies, so a butterfly costs about 10 times less there.  A line of doubles is
 // scaled by one power of two to 64-bit integers, transformed exactly in its sums and
-// to one unit in its products, and scaled back.  Flux at 256x256x129: 9.6 -> 2.05 ms.
+// to one unit in its products, and scaled back.  Flux at 256x256x129: 9.6 -> 2.06 ms.
 //
 // Range: with B = sum |x_k| over the line (every partial sum of a DFT is at most
-// B in magnitude, twiddles having modulus 1), the scale puts B into
-// (2^59, 2^61): no sum overflows 63 bits and no product its accumulator.
-// Precision: the unit is 2^-60 B at worst; quantisation contributes 0.29 units
+// B in magnitude, twiddles having modulus 1), the scale puts B into (2^60, 2^61), a bit
+// lower for two rows to a line and another for lane-held products: no sum overflows 63
+// bits and no product its accumulator.
+// Precision: the unit is 2^-58 to 2^-61 of B; quantisation contributes 0.29 units
 // per entry and each twiddle product at most about one.  B / rms and the early
 // stages' noise both grow with sqrt(N) on flat lines, so long lines start finer: an
 // output of the first s stages is a sum of P_s = R_1 ... R_s entries, at most P_s max|x|,
@@ -543,6 +544,8 @@ WV_HD void fx_stage_any(const fxc* __restrict__ src, fxc* __restrict__ dst, int 
 }
 
 struct FxFactors { int N, nstages; const int* radix; };
+// Radix of fx_gap; 0: one stage has nothing to come down before.
+WV_HD int fx_gap_radix(int nstages, const int* radix) { return nstages > 1 ? radix[0] : 0; }
 WV_HD void fx_shift_lines(fxc* lines_, int N, int Ns, int lines, int ld, FxLate late, int tid, int nt) {
     for (int it = tid; it < lines * N; it += nt) {
         const int line = it / N, i = it - line * N;
@@ -553,9 +556,10 @@ WV_HD void fx_shift_lines(fxc* lines_, int N, int Ns, int lines, int ld, FxLate 
     }
 }
 WV_HD bool fx_any_radix(int R) { return R != 2 && R != 3 && R != 4 && R != 5 && R != 8; }
-// What the lines are shifted down by before stage s > 0, which follows Ns points combined.
+// What the lines are shifted down by before stage s > 0, which follows Ns points combined:
+// all that is left before the last one (the float sums behind a gap may round it up).
 WV_HD FxLate fx_late_of(const FxFactors& f, int s, int Ns, const int* gaps, int gap) {
-    return {gaps, gap, fx_ceil_log2(Ns / f.radix[0]), fx_ceil_log2(Ns * f.radix[s] / f.radix[0])};
+    return {gaps, gap, fx_ceil_log2(Ns / f.radix[0]), Ns * f.radix[s] == f.N ? kFxAnyGap : fx_ceil_log2(Ns * f.radix[s] / f.radix[0])};
 }
 // Stage s of the lines, work items tid, tid + nt ...  LATE: lines past kFxLateFrom.
 template <bool INV, bool LATE>
@@ -574,7 +578,7 @@ WV_HD void fx_run_stage(const fxc* a, fxc* b, const FxFactors& f, int s, int Ns,
 #ifdef __CUDACC__
 // Lines of doubles (re, im) in place to fixed point: one group of warps per line
 // sums the moduli, then every entry is scaled.  unit[line] receives fx_unit, gaps[line]
-// the bits by which long lines start finer (radix: that of the first stage).
+// the bits by which the lines start finer (radix: fx_gap_radix, 0 up to kFxLateFrom).
 // Called by all threads of the block.
 __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, int radix, int* unit, int* gaps) {
     __shared__ unsigned redTop[32];
@@ -624,7 +628,7 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
         sum = total(sum);
         fxscale sc = fx_scale(sum);
         int gap = 0;
-        if (N > kFxLateFrom) gap = fx_gap(sum, largest(most), radix);
+        if (radix > 0) gap = fx_gap(sum, largest(most), radix);
         const bool odd = has && !fx_plain_sum(sum);
         if (per > 1 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) {
             unsigned top = 0;
@@ -651,7 +655,7 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
                     relMost = m > relMost ? m : relMost;
                 }
             rel = total(rel);
-            const int relGap = N > kFxLateFrom ? fx_gap(rel, largest(relMost), radix) : 0;
+            const int relGap = radix > 0 ? fx_gap(rel, largest(relMost), radix) : 0;
             if (odd) {
                 sc = fx_scale(top, rel);
                 gap = relGap;
@@ -693,7 +697,7 @@ __device__ inline fxc* fx_all_stages(fxc* a, fxc* b, const FxFactors f, int line
 template <bool INV>
 __device__ inline double2* fx_fft_lines(double2* a, double2* b, const FxFactors f, int lines, int ld, const fxw* tw) {
     __shared__ int unit[16], gaps[16];
-    fx_quantise(a, f.N, lines, ld, f.radix[0], unit, gaps);
+    fx_quantise(a, f.N, lines, ld, f.N > kFxLateFrom ? fx_gap_radix(f.nstages, f.radix) : 0, unit, gaps);
     fxc *fa = reinterpret_cast<fxc*>(a), *fb = reinterpret_cast<fxc*>(b);
     fxc* r = f.N > kFxLateFrom ? fx_all_stages<INV, false, true>(fa, fb, f, lines, ld, tw, gaps, 0)
                                : fx_all_stages<INV, false, false>(fa, fb, f, lines, ld, tw, nullptr, 0);

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
             if (mulL) v = make_double2(-rowL[i] * v.y, rowL[i] * v.x);
             row[i] = v;
         }
-        fxscale sc = fx_warp_scale(Ny, lane, LATE ? d.fy.radix[0] : 0, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
+        fxscale sc = fx_warp_scale(Ny, lane, LATE ? fx_gap_radix(d.fy.nstages, d.fy.radix) : 0, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
         if (lane == l) units = fx_unit(sc);
         if (LATE && lane == 0) gaps[warp][l] = sc.gap;
         sc.bit += sc.gap;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
     int units = 0;
     for (int l = 0; l < nl; ++l) {
         double2* row = bufA + (c0 + l) * ld;
-        fxscale sc = fx_warp_scale(Ny, lane, LATE ? d.fy.radix[0] : 0, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
+        fxscale sc = fx_warp_scale(Ny, lane, LATE ? fx_gap_radix(d.fy.nstages, d.fy.radix) : 0, [&](int i) { return row[i]; }, [](int) { return 1.0f; });
         if (lane == l) units = fx_unit(sc);
         if (LATE && lane == 0) gaps[warp][l] = sc.gap;
         sc.bit += sc.gap;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
         fxc A[EK], B[EK];
         int uA, uB, gap;
         fx_load_rows<EK>(h, cb < nch ? h + static_cast<size_t>(Ny) * KX : nullptr, ((d.c2rUseK >> ca) & 1) != 0,
-                         cb < nch && ((d.c2rUseK >> cb) & 1) != 0, KX, Nx, f.radix[0], lane, row_k<double>(d), A, B, uA, uB, gap);
+                         cb < nch && ((d.c2rUseK >> cb) & 1) != 0, KX, Nx, fx_gap_radix(f.nstages, f.radix), lane, row_k<double>(d), A, B, uA, uB, gap);
         fx_pack_rows<EK>(A, B, bufA, KX, Nx, lane);
         __syncwarp();
         const fxc* r = fx_row_stages<EK, true>(bufA, bufB, FxFactors{f.N, f.nstages, f.radix}, 1, tw, gap);
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps, 2)
         const double* s = fields + static_cast<size_t>(c) * R + (static_cast<size_t>(z) * Ny + y) * Nx;
         for (int x = lane; x < Nx; x += 32) raw[x] = make_double2(s[x], both ? s[R + x] : 0.0);
         auto one = [](int) { return 1.0f; };
-        const int radix = LATE ? f.radix[0] : 0;
+        const int radix = LATE ? fx_gap_radix(f.nstages, f.radix) : 0;
         fxscale sa = fx_warp_scale(Nx, lane, radix, [&](int x) { return make_double2(raw[x].x, 0.0); }, one);
         fxscale sb = fx_warp_scale(Nx, lane, radix, [&](int x) { return make_double2(raw[x].y, 0.0); }, one);
         sa.bit -= 1;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         const int qc = l, qs = l < 2 ? l + 2 : l - 2;
         auto atC = [&](int j) { const double2 v = fld[qc * Nj + j]; const double m = l < 2 ? 1.0 : mz[j]; return make_double2(m * v.x, m * v.y); };
         auto atD = [&](int j) { const double2 v = fld[qs * Nj + j]; const double m = l < 2 ? 1.0 : -mz[j]; return make_double2(m * v.x, m * v.y); };
-        const int radix = LATE ? d.fz.radix[0] : 0;
+        const int radix = LATE ? fx_gap_radix(d.fz.nstages, d.fz.radix) : 0;
         fxscale sC = fx_warp_scale(Nj, lane, radix, atC, count), sD = fx_warp_scale(Nj, lane, radix, atD, count);
         sC.bit -= 1; sD.bit -= 1;
         uC[l] = fx_unit(sC); uD[l] = fx_unit(sD);
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(32 * kFxAnyWarps)
         for (int z = 1 + lane; z < L; z += 32)
             rs[z] = cs >= 0 ? fspec[(static_cast<size_t>(cs) * d.zTotal + z) * P + pos] : make_double2(0.0, 0.0);
         __syncwarp();
-        const int radix = LATE ? d.fz.radix[0] : 0;
+        const int radix = LATE ? fx_gap_radix(d.fz.nstages, d.fz.radix) : 0;
         fxscale sC = fx_warp_scale(L + 1, lane, radix, [&](int z) { return rc[z]; }, count);
         fxscale sS = fx_warp_scale(L, lane, radix, [&](int z) { return z == 0 ? make_double2(0.0, 0.0) : rs[z]; }, count);
         sC.bit -= 1; sS.bit -= 1;

@@ -55,7 +55,7 @@ __device__ __forceinline__ void fx_load_rows(const double2* __restrict__ hA, con
         }
     }
     // (fx_line's gap is against one entry; the first stage adds `radix` of them)
-    gap = radix1 && Nx > kFxLateFrom ? max(0, fx_shared_gap(l[0].gap, l[1].gap) - fx_ceil_log2(radix)) : 0;
+    gap = radix1 && radix > 0 && Nx > kFxLateFrom ? max(0, fx_shared_gap(l[0].gap, l[1].gap) - fx_ceil_log2(radix)) : 0;
     if (gap < 2) gap = 0;  // not worth the shifts
     unitA = l[0].unit;
     unitB = l[1].unit;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
                     return yrow + ch * cstride;
                 };
                 const double2 *hA = spectrum(0), *hB = spectrum(1);
-                fx_load_rows<EK>(hA, hB, useK[0], useK[1], KX, Nx, f.radix[0], lane, rowK, A, B, uA, uB, gap);
+                fx_load_rows<EK>(hA, hB, useK[0], useK[1], KX, Nx, fx_gap_radix(f.nstages, f.radix), lane, rowK, A, B, uA, uB, gap);
                 if (lane == 2 * i) units = uA;
                 if (lane == 2 * i + 1) units = uB;
                 fx_pack_rows<EK>(A, B, bufA + i * Nx, KX, Nx, lane);
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(512, 1) k_xflux_fxany(DescDev d, FFTDev f, con
             int units = 0, gap = 0;
             for (int i = 0; i < nl; ++i) {
                 int sh[2] = {0, 0};
-                gap = EK > 2 && Nx > kFxLateFrom ? kFxAnyGap : 0;
+                gap = EK > 2 && Nx > kFxLateFrom && f.nstages > 1 ? kFxAnyGap : 0;
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int t = t0 + 2 * i + q;

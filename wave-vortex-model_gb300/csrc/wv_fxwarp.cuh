@@ -347,7 +347,7 @@ __device__ __forceinline__ void fx_forward_pair(const long long* __restrict__ Sa
 // time, so three blocks fit an SM.  (A warp per row with all its transforms in registers
 // gained 2 to 4 % on 12 to 40 line-sets an SM of 16 or 128 points and lost 4 to 7 % on
 // more, 10 to 30 % on fewer: flux 128x128x65 290 against 295 us, 128x256x129 1137 against
-// 1064, 128x64x33 133 against 109.)  256x256x129: 5.92 (FP64 pipe) -> 1.06 ms, 57 % of
+// 1064, 128x64x33 133 against 109.)  256x256x129: 5.92 (FP64 pipe) -> 1.07 ms, 53 % of
 // the issue slots; 192x192x97 1.00 -> 0.55 ms (run-time stages -> lanes).
 // physOut / advOut / advIn / maxSpeedBits as k_xflux.
 // EK: spectrum entries of a lane (kx < EK G; E / 2 at most, fewer under the 2/3 rule).

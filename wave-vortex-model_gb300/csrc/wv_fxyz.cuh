@@ -22,7 +22,7 @@ __device__ __forceinline__ int fx_tile(int y, int c, int cols) { return y * cols
 // Inverse FFTs along y of output channel blockIdx.z, columns blockIdx.x cols ...,
 // plane blockIdx.y: yspec[z][ch][y][kx] from zspec[src][z][pos] (times i l).  A line is
 // held by the lanes of one warp; the tile turns the result to rows for the store.
-// Bound by integer issue.  256x256x129, 12 channels: 1.71 (FP64 pipe) -> 0.457 ms;
+// Bound by integer issue.  256x256x129, 12 channels: 1.71 (FP64 pipe) -> 0.464 ms;
 // 192x192x97 0.32 -> 0.27 ms (run-time stages -> lanes).
 template <int N>
 __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
 
 // Forward FFTs along y of channel blockIdx.z, gathered to the active rows:
 // fspec[c][z][pos] from pspec[z][c][y][kx].  256x256x129, 4 channels: 0.54 (FP64 pipe)
-// -> 0.139 ms.
+// -> 0.142 ms.
 template <int N>
 __global__ void __launch_bounds__(32 * kFxYWarps, FxW<N>::E == 8 ? 3 : 2)
     k_yfwd_fx(DescDev d, const double2* __restrict__ pspec, int nch, double2* __restrict__ fspec) {
@@ -189,7 +189,7 @@ inline size_t smem_fx_field(int warps) { return (FxW<N>::twiddles + warps * FxW<
 
 // k_xc2r_fields: a warp takes two channels of a line-set of rows as one line.  KX may
 // reach N / 2 + 1 (the scalar pipeline's full half spectrum).  Inverse transform at
-// 192x192x97: 1.17 ms (FP64 pipe) -> 0.250 ms.
+// 192x192x97: 1.17 ms (FP64 pipe) -> 0.253 ms.
 template <int N>
 __global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
     k_xc2r_fx(DescDev d, const fxw* __restrict__ twg, const double2* __restrict__ yspec, int nch, double* __restrict__ fields) {
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
 
 // k_xr2c_fields: a warp takes two channels of a line-set of rows as one line.  Forward
 // transform at 256x256x65, hydrostatic: 0.305 ms with run-time lines (0.893 on the FP64
-// pipe), 0.220 with these.
+// pipe), 0.220 with these, 0.234 with the finer start of lines of samples.
 template <int N>
 __global__ void __launch_bounds__(32 * kFxFieldWarps, 4)
     k_xr2c_fx(DescDev d, const fxw* __restrict__ twg, const double* __restrict__ fields, int nch, double2* __restrict__ pspec) {
@@ -461,7 +461,7 @@ inline size_t smem_fx_z(int lines, int sets) {
 // flux, (m w | -m u), (m eta | -m v).  The two channels of a pair keep their own
 // scales (the even and the odd part separate them again), so neither rounds at the
 // other's magnitude.  Bound by integer issue and, in the field spectra, by FP64.
-// 256x256x129: 0.99 (FP64 pipe) -> 0.218 ms; 16x16x9 24 -> 14 us with a line per warp.
+// 256x256x129: 0.99 (FP64 pipe) -> 0.222 ms; 16x16x9 24 -> 14 us with a line per warp.
 template <int N, bool FLUX>
 __global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
     k_vinv_fx(DescDev d, const double* __restrict__ Ap, const double* __restrict__ Am, const double* __restrict__ A0,
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
 
 // k_vfwd_fft in fixed point: lines (u | w) and (v | eta) of a column by two warps,
 // which then share its coefficients' projection (FP64; its chain of dependent
-// operations is what small grids wait for).  256x256x129: 0.81 (FP64 pipe) -> 0.178 ms.
+// operations is what small grids wait for).  256x256x129: 0.81 (FP64 pipe) -> 0.180 ms.
 template <int N, bool FLUX>
 __global__ void __launch_bounds__(32 * kFxZWarps, FxW<N>::E == 8 ? 3 : 2)
     k_vfwd_fx(DescDev d, const double2* __restrict__ fspec, int nch, double elapsed, const double* __restrict__ Ap,
