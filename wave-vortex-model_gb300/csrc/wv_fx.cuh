@@ -480,7 +480,8 @@ struct FxLate {
         return (g < after ? g : after) - (g < before ? g : before);
     }
 };
-constexpr int kFxLateFrom = 192;  // longer run-time lines start finer
+constexpr int kFxLateFrom = 192;       // longer run-time lines of a warp start finer
+constexpr int kFxBlockLateFrom = 512;  // of a block: one complex line each, with a bit or two more
 WV_HD int fx_ceil_log2(int n) { return n <= 1 ? 0 : 32 - fx_clz(static_cast<unsigned>(n - 1)); }
 // One stage over `lines` lines (as fft_stage): radix R from src to dst.  What comes down is
 // rounded with ties in turn over the blocks of Ns points, which the stages sum for one k.
@@ -578,7 +579,7 @@ WV_HD void fx_run_stage(const fxc* a, fxc* b, const FxFactors& f, int s, int Ns,
 #ifdef __CUDACC__
 // Lines of doubles (re, im) in place to fixed point: one group of warps per line
 // sums the moduli, then every entry is scaled.  unit[line] receives fx_unit, gaps[line]
-// the bits by which the lines start finer (radix: fx_gap_radix, 0 up to kFxLateFrom).
+// the bits by which the lines start finer (radix: fx_gap_radix, 0 up to kFxBlockLateFrom).
 // Called by all threads of the block.
 __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, int radix, int* unit, int* gaps) {
     __shared__ unsigned redTop[32];
@@ -604,34 +605,18 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
             }
             return sum;
         };
-        auto largest = [&](float m) {  // over the warps of the line
-            unsigned bits = __reduce_max_sync(0xffffffffu, fx_float_bits(m));
-            if (per > 1) {
-                __syncthreads();  // (redTop may still be read)
-                if (lane == 0) redTop[warp] = bits;
-                __syncthreads();
-                if (has)
-                    for (int w = 0; w < per; ++w) bits = max(bits, redTop[g * per + w]);
-                __syncthreads();
-            }
-            return fx_float(bits);
-        };
-        float sum = 0.f, most = 0.f;
+        float sum = 0.f;
         if (has)
             for (int i = t; i < N; i += step) {
                 const double2 v = row[i];
-                const float m = fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))),
-                                           fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
-                sum += m;
-                most = m > most ? m : most;
+                sum += fx_modulus(fx_mag(static_cast<unsigned>(__double2hiint(v.x))),
+                                  fx_mag(static_cast<unsigned>(__double2hiint(v.y))));
             }
         sum = total(sum);
         fxscale sc = fx_scale(sum);
-        int gap = 0;
-        if (radix > 0) gap = fx_gap(sum, largest(most), radix);
+        unsigned top = 0;  // of an odd line
         const bool odd = has && !fx_plain_sum(sum);
         if (per > 1 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) {
-            unsigned top = 0;
             if (has)
                 for (int i = t; i < N; i += step) {
                     const double2 v = row[i];
@@ -645,21 +630,37 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
                 if (has)
                     for (int w = 0; w < per; ++w) top = max(top, redTop[g * per + w]);
             }
-            float rel = 0.f, relMost = 0.f;
+            float rel = 0.f;
             if (has)
                 for (int i = t; i < N; i += step) {
                     const double2 v = row[i];
-                    const float m = fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
-                                               fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
-                    rel += m;
-                    relMost = m > relMost ? m : relMost;
+                    rel += fx_modulus(fx_rel(static_cast<unsigned>(__double2hiint(v.x)), top),
+                                      fx_rel(static_cast<unsigned>(__double2hiint(v.y)), top));
                 }
             rel = total(rel);
-            const int relGap = radix > 0 ? fx_gap(rel, largest(relMost), radix) : 0;
             if (odd) {
                 sc = fx_scale(top, rel);
-                gap = relGap;
+                sum = rel;
             }
+        }
+        int gap = 0;
+        if (radix > 0) {  // the largest modulus of a long line
+            float most = 0.f;
+            if (has)
+                for (int i = t; i < N; i += step) {
+                    const unsigned x = static_cast<unsigned>(__double2hiint(row[i].x)), y = static_cast<unsigned>(__double2hiint(row[i].y));
+                    most = fmaxf(most, odd ? fx_modulus(fx_rel(x, top), fx_rel(y, top)) : fx_modulus(fx_mag(x), fx_mag(y)));
+                }
+            unsigned bits = __reduce_max_sync(0xffffffffu, fx_float_bits(most));
+            if (per > 1) {
+                __syncthreads();  // (redTop may still be read)
+                if (lane == 0) redTop[warp] = bits;
+                __syncthreads();
+                if (has)
+                    for (int w = 0; w < per; ++w) bits = max(bits, redTop[g * per + w]);
+                __syncthreads();
+            }
+            gap = fx_gap(sum, fx_float(bits), radix);
         }
         if (has) {
             if (t == 0) { unit[line] = fx_unit(sc); gaps[line] = gap; }
@@ -675,16 +676,23 @@ __device__ inline void fx_quantise(double2* lines_, int N, int lines, int ld, in
 }
 
 // All stages over fixed-point lines; returns the buffer holding the result.  gaps: bits by
-// which each line starts finer (null: `gap` for every line), LATE only.
+// which each line starts finer (null: `gap` for every line); LATE lines of a warp come down
+// in the stages, the block's (gaps given) after the first one, at once: its kernels hold
+// the stages a single time (twice cost k_xadj a block of an SM: flux VJP 60x50x31 285 ->
+// 339 us), and 1024 points end at 1.8e-16.
 // WARP: the lines belong to one warp (no block barrier), else to the block.
 template <bool INV, bool WARP, bool LATE>
 __device__ inline fxc* fx_all_stages(fxc* a, fxc* b, const FxFactors f, int lines, int ld, const fxw* tw, const int* gaps, int gap) {
     const int tid = WARP ? (threadIdx.x & 31) : threadIdx.x, nt = WARP ? 32 : blockDim.x;
     int Ns = 1;
     for (int s = 0; s < f.nstages; ++s) {
-        if (LATE && s > 0 && fx_any_radix(f.radix[s])) {
+        if (WARP && LATE && s > 0 && fx_any_radix(f.radix[s])) {
             fx_shift_lines(a, f.N, Ns, lines, ld, fx_late_of(f, s, Ns, gaps, gap), tid, nt);
-            if (WARP) __syncwarp(); else __syncthreads();
+            __syncwarp();
+        }
+        if (!WARP && s == 1 && gaps) {
+            fx_shift_lines(a, f.N, Ns, lines, ld, FxLate{gaps, 0, 0, kFxAnyGap}, tid, nt);
+            __syncthreads();
         }
         fx_run_stage<INV, LATE>(a, b, f, s, Ns, lines, ld, tw, gaps, gap, tid, nt);
         if (WARP) __syncwarp(); else __syncthreads();
@@ -697,10 +705,9 @@ __device__ inline fxc* fx_all_stages(fxc* a, fxc* b, const FxFactors f, int line
 template <bool INV>
 __device__ inline double2* fx_fft_lines(double2* a, double2* b, const FxFactors f, int lines, int ld, const fxw* tw) {
     __shared__ int unit[16], gaps[16];
-    fx_quantise(a, f.N, lines, ld, f.N > kFxLateFrom ? fx_gap_radix(f.nstages, f.radix) : 0, unit, gaps);
+    fx_quantise(a, f.N, lines, ld, f.N > kFxBlockLateFrom ? fx_gap_radix(f.nstages, f.radix) : 0, unit, gaps);
     fxc *fa = reinterpret_cast<fxc*>(a), *fb = reinterpret_cast<fxc*>(b);
-    fxc* r = f.N > kFxLateFrom ? fx_all_stages<INV, false, true>(fa, fb, f, lines, ld, tw, gaps, 0)
-                               : fx_all_stages<INV, false, false>(fa, fb, f, lines, ld, tw, nullptr, 0);
+    fxc* r = fx_all_stages<INV, false, false>(fa, fb, f, lines, ld, tw, f.N > kFxBlockLateFrom ? gaps : nullptr, 0);
     double2* out = reinterpret_cast<double2*>(r);
     for (int i = threadIdx.x; i < lines * f.N; i += blockDim.x) {
         const int line = i / f.N, k = i - line * f.N, u = unit[line];
